@@ -38,11 +38,14 @@ constexpr uint32_t MMA_XQ_SB = 864;               // quantized x per superblock:
 // vector's byte planes fill two or three, so the planes of a second vector ride in the next columns and both products come
 // out of the same instructions -- the weights are read, unpacked and multiplied once for the two.  Column c = vector c / NP,
 // plane c % NP.  Quantized x per superblock: [sub-block][column][32 B], then [column][8 sum bytes]; two scales per vector.
-template <int NP, int NTOK> __host__ __device__ constexpr uint32_t mma_xq_js() { return NTOK == 1 ? 96u : (uint32_t)(NTOK * NP) * 32u; }
-template <int NP, int NTOK> __host__ __device__ constexpr uint32_t mma_xq_sums() { return NTOK == 1 ? 768u : 8u * mma_xq_js<NP, NTOK>(); }
+// Four planes (products with fused neighbours): the B operand has room for them, so the fourth costs no instruction of the
+// inner loop; x is then good to fp32's own precision although its scale is shared by 256 elements.
+constexpr uint32_t MMA_XQ_SB4 = 1152;             // 8 groups x 4 planes x 32 B, then the sums (128 B)
+template <int NP, int NTOK> __host__ __device__ constexpr uint32_t mma_xq_js() { return NTOK == 1 ? (NP == 4 ? 128u : 96u) : (uint32_t)(NTOK * NP) * 32u; }
+template <int NP, int NTOK> __host__ __device__ constexpr uint32_t mma_xq_sums() { return NTOK == 1 ? 8u * mma_xq_js<NP, 1>() : 8u * mma_xq_js<NP, NTOK>(); }
 template <int NP, int NTOK> __host__ __device__ constexpr uint32_t mma_xq_sb()
 {
-    return NTOK == 1 ? MMA_XQ_SB : (mma_xq_sums<NP, NTOK>() + (uint32_t)(NTOK * NP) * 8u + 15u) / 16u * 16u;
+    return NTOK == 1 ? (NP == 4 ? MMA_XQ_SB4 : MMA_XQ_SB) : (mma_xq_sums<NP, NTOK>() + (uint32_t)(NTOK * NP) * 8u + 15u) / 16u * 16u;
 }
 
 struct MmaArgs {
@@ -53,7 +56,7 @@ struct MmaArgs {
     uint32_t in_dim, row_bytes;
     uint32_t units;            // superblocks per row
     uint32_t nwarps;           // consumer warps of one group: a group covers the kc superblocks of a stage
-    uint32_t ngroups;          // groups; stage i (counted over row tiles and their chunks) belongs to group i % ngroups
+    uint32_t ngroups;          // groups; stage i (counted over row tiles and their chunks) belongs to group i % ngroups (nstages is a multiple)
     uint32_t kc;               // superblocks per stage
     uint32_t nchunks;          // stages per row tile = ceil(units / kc)
     uint32_t dbg_tile;         // diagnostics build: first row tile whose per-warp timeline is recorded
@@ -75,6 +78,12 @@ struct MmaArgs {
     unsigned int *pub_gen, *pub_arrived;
     const uint2 *x_ll;
     const unsigned int *wait_gen;
+    // fused neighbours, as in PipeArgs: RMS-norm prologue (x is normalised while it is quantized) and residual epilogue
+    const uint16_t *norm_w;
+    const float *norm_parts;
+    float norm_eps;
+    const float *res_in;
+    float *res_parts;
     // MoE forms (template parameter MOE): the experts of a projection are one stacked tensor (expert e = rows
     // e * expert_rows .. of the tensor that map[0] describes), the chosen experts are read on the device.
     //   MOE 1, fused gate/up: segment s = expert seg_expert[s], all segments share x.
@@ -296,9 +305,16 @@ __device__ __forceinline__ Q6Lane q6_lane(uint32_t t)
 {
     auto sext = [](uint32_t b) { return b | ((8u | b) << 4) | ((8u | b) << 8) | ((8u | b) << 12); };
     Q6Lane L;
-    const uint32_t s0 = t <= 1 ? 0u : 1u, s1 = t == 0 ? 0u : 1u;   // which of the group's two scales column c0 / c1 takes
+    // which of the group's two scales column c0 / c1 takes (four planes: columns 0-3 first 16, 4-7 second 16)
+    const uint32_t s0 = t <= 1 ? 0u : 1u, s1 = NP == 4 ? s0 : (t == 0 ? 0u : 1u);
     L.sel[0][0] = sext(s0);     L.sel[0][1] = sext(s1);
     L.sel[1][0] = sext(2 + s0); L.sel[1][1] = sext(2 + s1);
+    if constexpr (NP == 4) {
+        L.cw0 = (t & 1u) ? 65536.0f : 1.0f;
+        L.cw1 = (t & 1u) ? 16777216.0f : 256.0f;
+        L.cwm = t == 0 ? 1.0f : t == 1 ? 256.0f : t == 2 ? 65536.0f : 16777216.0f;
+        return L;
+    }
     constexpr float W0 = 1.0f, W1 = 256.0f, W2 = NP == 3 ? 65536.0f : 0.0f;
     L.cw0 = t == 0 ? W0 : t == 1 ? W2 : t == 2 ? W1 : 0.0f;
     L.cw1 = t == 0 ? W1 : t == 1 ? W0 : t == 2 ? W2 : 0.0f;
@@ -344,15 +360,15 @@ __device__ __forceinline__ void q6_group(const uint32_t (&ql0)[2], const uint32_
 // the first 16 elements of a group (the word is operand b0 and b1 is zero) or the second 16 (b0 zero);
 // bsx: the digit sums of its column.  Thread t owns elements 4t..4t+3 and 16+4t..16+4t+3 of every group, so the
 // quad reads four consecutive words per row and the eight rows of a load fall into different banks.
-template <bool ALIGNED>
+template <bool ALIGNED, uint32_t JS>
 __device__ __forceinline__ void mma_superblock_q6(uint32_t s0, uint32_t s1, uint32_t t, uint32_t bx, bool first, uint32_t bsx, float xs,
                                                   const Q6Lane &L, float &y0, float &y1)
 {
     const uint32_t o = 4u * t;
     const uint32_t sel0 = (s0 & 2u) ? 0x5432u : 0x3210u, sel1 = (s1 & 2u) ? 0x5432u : 0x3210u;
     uint32_t xb[8];
-    xb[0] = lds32<0>(bx);   xb[1] = lds32<96>(bx);  xb[2] = lds32<192>(bx); xb[3] = lds32<288>(bx);
-    xb[4] = lds32<384>(bx); xb[5] = lds32<480>(bx); xb[6] = lds32<576>(bx); xb[7] = lds32<672>(bx);
+    xb[0] = lds32<0>(bx);      xb[1] = lds32<JS>(bx);     xb[2] = lds32<2 * JS>(bx); xb[3] = lds32<3 * JS>(bx);
+    xb[4] = lds32<4 * JS>(bx); xb[5] = lds32<5 * JS>(bx); xb[6] = lds32<6 * JS>(bx); xb[7] = lds32<7 * JS>(bx);
     const uint32_t bs = lds32<0>(bsx);
     uint32_t sc0[4], sc1[4];
 #pragma unroll
@@ -391,7 +407,7 @@ __device__ __forceinline__ void mma_superblock_q6(uint32_t s0, uint32_t s1, uint
 
 // Balanced base-256 digits, all elements at once: for |v| <= 0x7F7F7F (0x7F7F) the bytes of v + 0x808080 (0x8080) are
 // the digits plus 128, so a plane word is three byte permutes and one xor with 0x80808080.
-template <int NP> __device__ __forceinline__ uint32_t digit_bias() { return NP == 3 ? 0x00808080u : 0x00008080u; }
+template <int NP> __device__ __forceinline__ uint32_t digit_bias() { return NP == 4 ? 0x80808080u : NP == 3 ? 0x00808080u : 0x00008080u; }
 __device__ __forceinline__ uint32_t plane_word(uint32_t u0, uint32_t u1, uint32_t u2, uint32_t u3, int p)
 {
     const uint32_t sel = (uint32_t)p | ((uint32_t)(4 + p) << 4);
@@ -406,18 +422,28 @@ __device__ __forceinline__ uint32_t plane_word(uint32_t u0, uint32_t u1, uint32_
 // at +768 [plane p][low / high byte][16 groups].
 // With `slots` set x is a gathered vector read from its {value, tag} slots (polled for `tag`); false = a poll expired.
 // NTOK = 2: vector `b` (0 or 1) of two, into its columns of the wider layout (see mma_xq_sb).
-template <int NP, bool Q6, int NTOK = 1>
+// NORM: x is RMS-normalised on the way, (x * rsqrt(sum(norm_parts) / n + eps)) * bf16 weight; the partial sums are requested
+// before the vector and added up after it, so that the two round trips to L2 overlap.
+template <int NP, bool Q6, int NTOK = 1, bool NORM = false>
 __device__ __forceinline__ bool quantize_x_mma(const float *__restrict__ x, uint32_t units, uint8_t *xq, uint32_t warp, uint32_t lane,
-                                               uint32_t nwarps, const uint2 *slots = nullptr, unsigned int tag = 0, uint32_t b_tok = 0)
+                                               uint32_t nwarps, const uint2 *slots = nullptr, unsigned int tag = 0, uint32_t b_tok = 0,
+                                               const uint16_t *norm_w = nullptr, const float *norm_parts = nullptr, float norm_eps = 0.0f)
 {
     static_assert(NTOK == 1 || !Q6, "two vectors at once: Q4_K / Q5_K only");
     constexpr uint32_t XQSB = mma_xq_sb<NP, NTOK>(), JS = mma_xq_js<NP, NTOK>(), SUMS = mma_xq_sums<NP, NTOK>();
     const uint32_t col0 = NTOK == 1 ? 0u : b_tok * NP;
     bool ok = true;
-    constexpr int QMAXI = NP == 3 ? 127 * 65536 + 127 * 256 + 127 : 127 * 256 + 127;
+    // (four planes: the float just below 127 * (2^24 + 2^16 + 2^8 + 1), so that the clamp and the scale agree)
+    constexpr int QMAXI = NP == 4 ? 0x7F7F7F00 : NP == 3 ? 127 * 65536 + 127 * 256 + 127 : 127 * 256 + 127;
     constexpr float QMAX = (float)QMAXI;
     constexpr int XB = 4;
     float *xs = reinterpret_cast<float *>(xq + (size_t)units * XQSB), *sxs = xs + units * NTOK;
+    constexpr int NPV = PIPE_SUM_SQ_PARTS / 32;
+    float pv[NORM ? NPV : 1], rms = 0.0f;
+    if constexpr (NORM) {
+#pragma unroll
+        for (int i = 0; i < NPV; ++i) pv[i] = __ldcg(norm_parts + 32 * i + lane);
+    }
     for (uint32_t ub = warp; ub < units; ub += nwarps * XB) {
         float4 v0[XB], v1[XB];
 #pragma unroll
@@ -431,6 +457,25 @@ __device__ __forceinline__ bool quantize_x_mma(const float *__restrict__ x, uint
             } else {
                 v0[b] = u < units ? __ldcg(src) : make_float4(0.f, 0.f, 0.f, 0.f);
                 v1[b] = u < units ? __ldcg(src + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+        if constexpr (NORM) {
+            if (ub == warp) {
+                float t = 0.0f;
+#pragma unroll
+                for (int i = 0; i < NPV; ++i) t += pv[i];
+                rms = rsqrtf(warp_sum(t) / (float)(units * 256u) + norm_eps);
+            }
+#pragma unroll
+            for (int b = 0; b < XB; ++b) {
+                const uint32_t u = ub + b * nwarps;
+                if (u >= units) break;
+                const uint2 *nw = reinterpret_cast<const uint2 *>(norm_w) + (size_t)u * 64 + 2 * lane;      // 8-byte aligned bf16 weights
+                const uint2 wa = __ldg(nw), wb = __ldg(nw + 1);
+                auto lo = [](uint32_t w) { return __uint_as_float(w << 16); };
+                auto hi = [](uint32_t w) { return __uint_as_float(w & 0xffff0000u); };
+                v0[b] = make_float4(v0[b].x * rms * lo(wa.x), v0[b].y * rms * hi(wa.x), v0[b].z * rms * lo(wa.y), v0[b].w * rms * hi(wa.y));
+                v1[b] = make_float4(v1[b].x * rms * lo(wb.x), v1[b].y * rms * hi(wb.x), v1[b].z * rms * lo(wb.y), v1[b].w * rms * hi(wb.y));
             }
         }
         float amax[XB], sum[XB], smax[XB];
@@ -477,8 +522,8 @@ __device__ __forceinline__ bool quantize_x_mma(const float *__restrict__ x, uint
                     sd += __shfl_xor_sync(0xffffffffu, sd, 1);                    // 16 elements = two lanes
                     const int lo8 = (int)(signed char)(sd & 0xFF);
                     if ((lane & 1u) == 0) {
-                        sb[768 + (2 * p) * 16 + (lane >> 1)] = (uint8_t)(lo8 & 255);
-                        sb[768 + (2 * p + 1) * 16 + (lane >> 1)] = (uint8_t)(((sd - lo8) >> 8) & 255);
+                        sb[SUMS + (2 * p) * 16 + (lane >> 1)] = (uint8_t)(lo8 & 255);
+                        sb[SUMS + (2 * p + 1) * 16 + (lane >> 1)] = (uint8_t)(((sd - lo8) >> 8) & 255);
                     }
                 }
             }
@@ -581,7 +626,10 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
 
     if (producer) {
         // The weight copies do not depend on the previous kernel: no griddepcontrol.wait on this path.
-        // With two producer warps, warp p issues the stages i with i % 2 == p.
+        // With two producer warps, warp p feeds the ring slots sc with sc % 2 == p.  A slot has ONE producer because a wait by
+        // parity can only tell the last two phases of a barrier apart: a warp that fed a slot's use k - 2 but not k - 1
+        // would take "k - 2 not consumed yet" for "k - 1 consumed" and overwrite a stage that is still being read (dealing
+        // the stages out by issue number does that whenever the ring has an odd number of slots and a group lags).
         const uint32_t pw = warp - CW;
         if constexpr (MOE != 0) {      // the expert indices are the previous kernel's output
             pdl_wait();
@@ -589,15 +637,15 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
             if (lane < (uint32_t)PIPE_MAX_SEG) s_expert[lane] = lane < nsel ? a.seg_expert[blockIdx.y * a.tok_sel_stride + lane] : 0u;
             __syncwarp();
         }
-        uint32_t cur = lo, s = 0, k = 0, issued = 0, used_mask = 0, par_mask = 0;
+        uint32_t cur = lo, s = 0, k = 0, used_mask = 0, par_mask = 0;
         int seg = 0;
         bool ok = true;
         MmaTile t;
         while (ok && mma_next_tile(a, cur, hi, seg, t)) {
-            for (uint32_t c = 0; c < a.nchunks && ok; ++c, ++issued) {
+            for (uint32_t c = 0; c < a.nchunks && ok; ++c) {
                 const uint32_t sc = s, kc_ = k;
                 if (++s == a.nstages) { s = 0; ++k; }
-                if (NPROD > 1 && issued % NPROD != pw) continue;
+                if (NPROD > 1 && sc % NPROD != pw) continue;
                 if (kc_ > 0) {
                     int good = 1;
                     if (lane == 0) {
@@ -676,19 +724,24 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
     {
         const uint2 *slots = EXT ? a.x_ll : nullptr;
         const unsigned int want = EXT && a.x_ll ? *reinterpret_cast<const volatile unsigned int *>(a.wait_gen) : 0u;
-        if (!quantize_x_mma<NP, Q6, NTOK>(a.x + (MOE != 0 ? (size_t)blockIdx.y * a.tok_x_stride : 0), U, xq, warp, lane, CW, slots, want, 0u)) {
+        bool x_ok;
+        if (EXT && a.norm_w)
+            x_ok = quantize_x_mma<NP, Q6, NTOK, true>(a.x, U, xq, warp, lane, CW, nullptr, 0u, 0u, a.norm_w, a.norm_parts, a.norm_eps);
+        else
+            x_ok = quantize_x_mma<NP, Q6, NTOK>(a.x + (MOE != 0 ? (size_t)blockIdx.y * a.tok_x_stride : 0), U, xq, warp, lane, CW, slots, want, 0u);
+        if (!x_ok) {
             s_abort = 1;
             atomicExch(a.status, 3);
         }
         if constexpr (TWO) quantize_x_mma<NP, Q6, NTOK>(a.x + a.tok_x_stride, U, xq, warp, lane, CW, nullptr, 0u, 1u);
     }
     const unsigned int pub_tag = EXT && a.npeers > 0 ? *reinterpret_cast<const volatile unsigned int *>(a.pub_gen) + 1u : 0u;
-    if constexpr (Q6) {   // a block of zeros for lanes whose product column is empty
-        for (uint32_t z = tid; z < 768 / 4; z += C) reinterpret_cast<uint32_t *>(xq + (size_t)U * MMA_XQ_SB + 8 * U)[z] = 0u;
+    if constexpr (Q6 && NP < 4) {   // a block of zeros for lanes whose product column is empty
+        for (uint32_t z = tid; z < 768 / 4; z += C) reinterpret_cast<uint32_t *>(xq + (size_t)U * XQSB + 8 * U)[z] = 0u;
     }
     named_bar_sync(PIPE_BAR_CONSUMERS, (int)C);
     if constexpr (MOE == 2) {      // the routing weight of an expert goes into the scales of its input vector
-        float *xsf = reinterpret_cast<float *>(xq + (size_t)U * MMA_XQ_SB);
+        float *xsf = reinterpret_cast<float *>(xq + (size_t)U * XQSB);
         for (uint32_t u = tid; u < U; u += C) {
             const float wgt = u == tid ? moe_wgt : a.seg_weight[blockIdx.y * a.tok_sel_stride + u / a.kc];   // loaded before the quantization above
             xsf[u] *= wgt;
@@ -702,7 +755,7 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
     const uint32_t xq_s = smem_u32(xq) + plane * 32u + t4 * 8u;       // this thread's x bytes of sub-block 0, superblock 0
     const uint32_t sx_s = smem_u32(xq) + XSUMS + plane * 8u + (t4 & 1u) * 4u;
     // columns 2t, 2t+1 of the products are byte planes 2t, 2t+1
-    const float cw0 = t4 == 0 ? 1.0f : (t4 == 1 && NP == 3 ? 65536.0f : 0.0f), cw1 = t4 == 0 ? 256.0f : 0.0f;
+    const float cw0 = t4 == 0 ? 1.0f : (t4 == 1 && NP >= 3 ? 65536.0f : 0.0f), cw1 = t4 == 0 ? 256.0f : (t4 == 1 && NP == 4 ? 16777216.0f : 0.0f);
     // two vectors: column c is plane c % NP of vector c / NP; this thread's columns 2t, 2t+1 count for vector A and / or B
     auto col_w = [](uint32_t c, uint32_t vec) {
         const uint32_t pl = c % NP;
@@ -712,16 +765,19 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
     const float cwA0 = col_w(2 * t4, 0), cwA1 = col_w(2 * t4 + 1, 0), cwB0 = col_w(2 * t4, 1), cwB1 = col_w(2 * t4 + 1, 1);
 
     // Q6_K: column g = (first / second 16 elements of a group, plane g % 3); lanes of unused columns read a block of zeros
-    const uint32_t q6_plane = g % 3u;
-    const bool q6_col = Q6 && g < 6u && q6_plane < (uint32_t)NP;
-    const uint32_t q6_bx = q6_col ? smem_u32(xq) + q6_plane * 32u + (g < 3u ? 0u : 16u) + t4 * 4u : xs_s + 8u * U;
-    const uint32_t q6_bstride = q6_col ? MMA_XQ_SB : 0u;
-    const uint32_t q6_sx = smem_u32(xq) + 768u + (g < 6u ? g : 0u) * 16u + t4 * 4u;
+    // (four planes fill all eight columns: plane g % 4)
+    constexpr uint32_t Q6P = NP == 4 ? 4u : 3u;
+    const uint32_t q6_plane = g % Q6P;
+    const bool q6_first = g < Q6P, q6_col = Q6 && g < 2u * Q6P && q6_plane < (uint32_t)NP;
+    const uint32_t q6_bx = q6_col ? smem_u32(xq) + q6_plane * 32u + (q6_first ? 0u : 16u) + t4 * 4u : xs_s + 8u * U;
+    const uint32_t q6_bstride = q6_col ? XQSB : 0u;
+    const uint32_t q6_sx = smem_u32(xq) + XSUMS + (g < 2u * Q6P ? g : 0u) * 16u + t4 * 4u;
     const Q6Lane q6l = q6_lane<NP>(t4);
 
     const uint32_t CAP = a.red_rows, SLOTS = NW * NG, PLANE = CAP * SLOTS;   // every warp of every group leaves one partial sum per row
     uint32_t which = 0, buf_n = 0, buf_row0 = 0;
     int buf_seg = 0;
+    float sq = 0.0f;                          // this thread's share of the sum of squares of the outputs (residual epilogue)
     auto flush = [&]() {
         named_bar_sync(PIPE_BAR_CONSUMERS, (int)C);
         const float *src = red + (size_t)which * PLANE * (SWIGLU || TWO ? 2 : 1);
@@ -732,7 +788,13 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
                 gsum += src[r * SLOTS + w];
                 if constexpr (SWIGLU || TWO) usum += src[PLANE + r * SLOTS + w];
             }
-            const float val = SWIGLU ? silu_mul(gsum, usum) : gsum;
+            float val = SWIGLU ? silu_mul(gsum, usum) : gsum;
+            if constexpr (EXT && !SWIGLU) {
+                if (a.res_in) {               // residual add, clamped to the fp16 range as the reference's kernel does
+                    val = fminf(fmaxf(a.res_in[buf_row0 + r] + val, -65504.0f), 65504.0f);
+                    sq = fmaf(val, val, sq);
+                }
+            }
             y[r] = val;
             if constexpr (TWO) y[a.tok_y_stride + r] = usum;      // the second vector's product
             if constexpr (EXT) {
@@ -782,9 +844,9 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
                     const float xsu = __uint_as_float(lds32<0>(xs_s + 4u * ug));
                     const uint32_t sa = r0 + u * UNIT, sb = r1 + u * UNIT;
                     if (__all_sync(0xffffffffu, ((sa | sb) & 2u) == 0u))
-                        mma_superblock_q6<true>(sa, sb, t4, q6_bx + ug * q6_bstride, g < 3u, q6_sx + ug * MMA_XQ_SB, xsu, q6l, yg0, yg1);
+                        mma_superblock_q6<true, XJS>(sa, sb, t4, q6_bx + ug * q6_bstride, q6_first, q6_sx + ug * XQSB, xsu, q6l, yg0, yg1);
                     else
-                        mma_superblock_q6<false>(sa, sb, t4, q6_bx + ug * q6_bstride, g < 3u, q6_sx + ug * MMA_XQ_SB, xsu, q6l, yg0, yg1);
+                        mma_superblock_q6<false, XJS>(sa, sb, t4, q6_bx + ug * q6_bstride, q6_first, q6_sx + ug * XQSB, xsu, q6l, yg0, yg1);
                 }
             } else {
                 for (uint32_t u = wig; u < kn; u += NW) {
@@ -828,6 +890,20 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
     }
     if (tid == 0) stamp(a.trace, 6);
     if (buf_n) flush();
+    if constexpr (EXT && !SWIGLU) {
+        if (a.res_parts) {
+            __shared__ float s_sq[MMA_MAX_CONSUMER_WARPS];
+            sq = warp_sum(sq);
+            if (lane == 0) s_sq[warp] = sq;
+            named_bar_sync(PIPE_BAR_CONSUMERS, (int)C);
+            if (tid == 0) {
+                float t = 0.0f;
+                for (uint32_t w = 0; w < CW; ++w) t += s_sq[w];
+                a.res_parts[blockIdx.x] = t;
+            }
+            for (uint32_t q = gridDim.x + blockIdx.x * C + tid; q < (uint32_t)PIPE_SUM_SQ_PARTS; q += gridDim.x * C) a.res_parts[q] = 0.0f;
+        }
+    }
     if (EXT && a.npeers > 0) {
         if (tid == 0 && atomicAdd(a.pub_arrived, 1u) == gridDim.x - 1) {   // last CTA: the new generation becomes current
             *reinterpret_cast<volatile unsigned int *>(a.pub_arrived) = 0;

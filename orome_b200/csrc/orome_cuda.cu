@@ -409,6 +409,18 @@ static int arm_gather(orome_cuda_ctx *c, Args &a, uint32_t in_dim)
     return OROME_OK;
 }
 
+// Fused norm prologue / residual epilogue: the request becomes the launch's (the entry points have checked that it can take it).
+template <typename Args>
+static void arm_fuse(orome_cuda_ctx *c, Args &a)
+{
+    a.norm_w = static_cast<const uint16_t *>(c->fuse_norm_w);
+    a.norm_parts = c->fuse_norm_parts;
+    a.norm_eps = c->fuse_norm_eps;
+    a.res_in = c->fuse_res_in;
+    a.res_parts = c->fuse_res_parts;
+    c->fuse_norm_w = nullptr; c->fuse_norm_parts = nullptr; c->fuse_res_in = nullptr; c->fuse_res_parts = nullptr;
+}
+
 // Fill everything of the plan except the segments' pointers.
 static int plan_pipe(orome_cuda_ctx *c, int fmt, uint32_t in_dim, uint32_t total_rows, int mode, PipePlan &p)
 {
@@ -487,13 +499,7 @@ static int plan_pipe(orome_cuda_ctx *c, int fmt, uint32_t in_dim, uint32_t total
     a.pf_bytes = c->hint_bytes;
     c->hint_ptr = nullptr;
     c->hint_bytes = 0;
-    // fused norm prologue / residual epilogue (the entry points have checked that this launch can take them)
-    a.norm_w = static_cast<const uint16_t *>(c->fuse_norm_w);
-    a.norm_parts = c->fuse_norm_parts;
-    a.norm_eps = c->fuse_norm_eps;
-    a.res_in = c->fuse_res_in;
-    a.res_parts = c->fuse_res_parts;
-    c->fuse_norm_w = nullptr; c->fuse_norm_parts = nullptr; c->fuse_res_in = nullptr; c->fuse_res_parts = nullptr;
+    arm_fuse(c, a);
     if (a.res_parts && p.grid > PIPE_SUM_SQ_PARTS) return fail(OROME_ENOTSUP, "pipe plan: more CTAs than entries in a partials array");
     return OROME_OK;
 }
@@ -619,7 +625,6 @@ static int plan_mma(orome_cuda_ctx *c, int fmt, uint32_t in_dim, uint32_t total_
     // stages (row tiles x chunks) go round the groups: as many groups as the warp budget and the CTA's stage count allow
     const uint32_t cta_stages = (share + MMA_TILE_ROWS - 1) / MMA_TILE_ROWS * a.nchunks;
     a.ngroups = std::max(1u, std::min(std::min<uint32_t>(MMA_MAX_GROUPS, MMA_MAX_CONSUMER_WARPS / a.nwarps), cta_stages));
-    p.threads = (int)(a.nwarps * a.ngroups + (fmt == FMT_Q6_K ? 2 : 1)) * 32;
     // box width in superblocks: the smallest kb >= kc with kb = 2 (mod 4), which makes the row pitch 32 or 96 (mod 128)
     const uint32_t kb = a.kc + ((6 - a.kc % 4) % 4);
     a.pitch = kb * unit;
@@ -635,13 +640,20 @@ static int plan_mma(orome_cuda_ctx *c, int fmt, uint32_t in_dim, uint32_t total_
     a.red_rows = std::max<uint32_t>(MMA_TILE_ROWS, std::min<uint32_t>((share + MMA_TILE_ROWS - 1) / MMA_TILE_ROWS * MMA_TILE_ROWS, 128u));
     const size_t red_bytes = (size_t)2 * a.red_rows * a.nwarps * a.ngroups * (swiglu || two ? 2 : 1) * sizeof(float);
     a.xs_base = (uint32_t)((a.red_base + red_bytes + 127) / 128 * 128);
-    const size_t xq_sb = !two ? MMA_XQ_SB : (c->x_bits == 24 ? mma_xq_sb<3, 2>() : mma_xq_sb<2, 2>());
+    const bool fused = c->fuse_norm_w || c->fuse_res_in;      // fused neighbours: four byte planes (launch_mma)
+    const size_t xq_sb = !two ? (fused ? MMA_XQ_SB4 : MMA_XQ_SB) : (c->x_bits == 24 ? mma_xq_sb<3, 2>() : mma_xq_sb<2, 2>());
     const size_t xq_bytes = (size_t)a.units * xq_sb + (size_t)a.units * 8 * (two ? 2 : 1) + 768;   // planes and sums, two scales per superblock and vector, a block of zeros
     a.stage_base = (uint32_t)((a.xs_base + xq_bytes + 127) / 128 * 128);
     const size_t budget = std::min<size_t>(228 * 1024 - 1024 - 256, (size_t)c->smem_optin - 256);
     if (budget < a.stage_base + a.stage_stride) return fail(OROME_ENOTSUP, "mma plan: in_dim %u does not fit shared memory", in_dim);
     const uint32_t tiles = ((share + MMA_TILE_ROWS - 1) / MMA_TILE_ROWS + 1) * a.nchunks;
     a.nstages = (uint32_t)std::min<size_t>(std::min<size_t>(PIPE_MAX_STAGES, tiles), (budget - a.stage_base) / a.stage_stride);
+    // A whole number of ring slots per group, so that every use of a slot belongs to the same group.  A wait by parity tells
+    // only the last two phases apart: a group waiting for use k of a slot whose use k - 1 is another group's, and has not
+    // landed yet, would take phase k - 2 for phase k and read the stage too early.
+    a.ngroups = std::min(a.ngroups, a.nstages);
+    a.nstages -= a.nstages % a.ngroups;
+    p.threads = (int)(a.nwarps * a.ngroups + (fmt == FMT_Q6_K ? 2 : 1)) * 32;
     p.smem = a.stage_base + (size_t)a.stage_stride * a.nstages;
 #ifdef OROME_MMA_TILE_TRACE
     a.dbg_tile = OROME_MMA_TILE_TRACE;      // diagnostics build: first row tile whose per-warp timeline is recorded
@@ -653,6 +665,8 @@ static int plan_mma(orome_cuda_ctx *c, int fmt, uint32_t in_dim, uint32_t total_
     a.pf_bytes = c->hint_bytes;
     c->hint_ptr = nullptr;
     c->hint_bytes = 0;
+    arm_fuse(c, a);
+    if (a.res_parts && p.grid > PIPE_SUM_SQ_PARTS) return fail(OROME_ENOTSUP, "mma plan: more CTAs than entries in a partials array");
     return arm_gather(c, a, in_dim);
 }
 
@@ -744,6 +758,10 @@ static int launch_mma_moe(orome_cuda_ctx *c, int fmt, MmaPlan &p, bool gate_up, 
 template <int FMT, int NP, bool SWIGLU>
 static int launch_mma_inst(orome_cuda_ctx *c, const MmaPlan &p, cudaStream_t st)
 {
+    // Products with fused neighbours read x as four byte planes: their dp4a form (shapes and alignments this kernel does not
+    // take) scales x per 32 elements, this kernel per 256, and the spare columns of the mma hold a fourth plane for nothing
+    // (rel-L2 against fp64 on 2400 x 4352: dp4a 1.5-1.7e-7, three planes 1.7-1.9e-7, four planes 1.4-1.5e-7).
+    if (p.args.norm_w || p.args.res_in) return launch_mma_ext<FMT, 4, SWIGLU, true>(c, p, st);
     return p.args.npeers > 0 || p.args.x_ll ? launch_mma_ext<FMT, NP, SWIGLU, true>(c, p, st) : launch_mma_ext<FMT, NP, SWIGLU, false>(c, p, st);
 }
 
@@ -752,7 +770,7 @@ static int launch_mma(orome_cuda_ctx *c, int fmt, MmaPlan &p, bool swiglu, cudaS
     int rc = mma_encode_maps(c, fmt, p, swiglu);
     if (rc) return rc;
     const bool b24 = c->x_bits == 24;
-    // the fused form always reads x at 24 bits (see plan_pipe)
+    // the fused gate/up form always reads x at 24 bits (see plan_pipe)
     if (fmt == FMT_Q4_K) {
         if (swiglu) return launch_mma_inst<FMT_Q4_K, 3, true>(c, p, st);
         return b24 ? launch_mma_inst<FMT_Q4_K, 3, false>(c, p, st) : launch_mma_inst<FMT_Q4_K, 2, false>(c, p, st);
@@ -981,7 +999,7 @@ extern "C" int orome_cuda_matvec_group(orome_cuda_ctx *c, const OromeTensorRef *
     }
     bool aligned16 = true;
     for (int i = 0; i < n_refs; ++i) aligned16 = aligned16 && !(reinterpret_cast<uintptr_t>(data[i]) & 15);
-    if (!fused && (aligned16 || fmt == FMT_Q6_K) && mma_supported(c, fmt, refs[0].in_dim, false)) {   // the fused forms live in the dp4a kernel
+    if ((aligned16 || fmt == FMT_Q6_K) && mma_supported(c, fmt, refs[0].in_dim, false)) {
         MmaPlan m;
         memset(&m, 0, sizeof m);
         uint32_t rows = 0;
@@ -1317,7 +1335,7 @@ extern "C" int orome_cuda_gate_up_swiglu(orome_cuda_ctx *c, const OromeTensorRef
     }
     if (batch == 1 && !c->force_generic && orome_pipe_supported(fmt, gate->in_dim)) {
         if (reinterpret_cast<uintptr_t>(x_dev) & 15) return fail(OROME_EINVAL, "gate_up_swiglu: x must be 16-byte aligned");
-        if (!fused && !((reinterpret_cast<uintptr_t>(gd) | reinterpret_cast<uintptr_t>(ud)) & 15) && mma_supported(c, fmt, gate->in_dim, true)) {
+        if (!((reinterpret_cast<uintptr_t>(gd) | reinterpret_cast<uintptr_t>(ud)) & 15) && mma_supported(c, fmt, gate->in_dim, true)) {
             MmaPlan m;
             memset(&m, 0, sizeof m);
             m.args.seg[0] = PipeSeg{gd, ud, out_dev, gate->out_dim, 0};

@@ -152,3 +152,70 @@ def test_calls_without_a_fused_form_drop_the_request(env):
     torch.cuda.synchronize()
     want = oracle.matvec_f64(fmt, synth.host_tensor(fmt, H, H, seed=31), H, H, synth.host_x(H, 8, seed=32)[0])
     assert rel_l2(y.cpu().numpy(), want) <= REL_L2_TOL
+
+
+@pytest.mark.parametrize("fmt", [synth.Q4_K, synth.Q5_K, synth.Q6_K])
+@pytest.mark.parametrize("rows,cols", [(1, 256), (17, 512), (333, 2560), (2400, 4352), (48, 17408)])
+@pytest.mark.parametrize("x_bits", [24, 16])
+def test_fused_neighbours_on_both_kquant_kernels(env, fmt, rows, cols, x_bits):
+    """Norm prologue and residual epilogue on one product at row-tile and superblock remainders, on the mma kernel and
+    (OROME_OPT_KQUANT_MMA = 0) the dp4a kernel.  The mma kernel reads x as 32-bit fixed point at either option, so fp32 sums
+    bound its error: a few 1e-7.  The dp4a kernel at 16 bits rounds x to 2^-16 of the largest of 32 elements, 1.9e-5 per
+    element at a ratio of 2.1 between that and the deviation; a single row of 256 has a sum that may be small against
+    its terms, hence the factor of ten."""
+    torch, F, ctx = env
+    w = synth.host_tensor(fmt, rows, cols, seed=31)
+    x, resid, nw = synth.host_x(cols, seed=32), synth.host_x(rows, seed=33), bf16_weights(cols, 34)
+    _, in_parts = oracle.residual_add_sum_sq(x, np.zeros(cols, np.float32))
+    pin = np.zeros(F.SUM_SQ_PARTS, np.float32)
+    pin[:in_parts.size] = in_parts
+    t = {k: dev(torch, v) for k, v in dict(w=w, x=x, resid=resid, nw=nw, pin=pin).items()}
+    n = oracle.rms_norm_apply_partial(x, nw, in_parts, EPS)
+    prod = oracle.matvec_f64(fmt, w, rows, cols, n)
+    err = []
+    ctx.set_option(F.OPT_X_BITS, x_bits)
+    try:
+        for mma in (1, 0):
+            ctx.set_option(F.OPT_KQUANT_MMA, mma)
+            pout = torch.full((F.SUM_SQ_PARTS,), float("nan"), device="cuda")
+            y = torch.full((rows,), float("nan"), device="cuda")
+            ctx.fuse_next(F.NormPrologue(t["nw"].data_ptr(), t["pin"].data_ptr(), EPS), F.ResidualEpilogue(t["resid"].data_ptr(), pout.data_ptr()))
+            ctx.matvec(F.tensor_ref(t["w"].data_ptr(), 0, fmt, rows, cols), t["x"].data_ptr(), y.data_ptr())
+            torch.cuda.synchronize()
+            got = y.cpu().numpy().astype(np.float64)
+            err.append(rel_l2(got, np.clip(resid.astype(np.float64) + prod, -65504.0, 65504.0)))
+            assert abs(float(pout.cpu().numpy().astype(np.float64).sum()) / float((got * got).sum()) - 1.0) <= 1e-5
+    finally:
+        ctx.set_option(F.OPT_KQUANT_MMA, 1)
+        ctx.set_option(F.OPT_X_BITS, 24)
+    print(f"fmt {fmt} {rows}x{cols} x_bits {x_bits}: mma {err[0]:.2e} dp4a {err[1]:.2e}")
+    assert err[0] <= 2e-6
+    assert err[1] <= (2e-6 if x_bits == 24 else 2e-4)
+
+
+@pytest.mark.parametrize("rows,cols", [(5120, 17408), (8192, 8192), (3000, 5120)])
+def test_q6_ring_whose_slots_do_not_divide_by_its_groups(env, rows, cols):
+    """Products back to back whose shared memory holds three or five stages for two or three consumer groups (every slot must
+    keep one producer warp and one group): every repetition gives the first one's bits, and the first one is right."""
+    torch, F, ctx = env
+    fmt = synth.Q6_K
+    w = synth.host_tensor(fmt, rows, cols, seed=41)
+    x, resid = synth.host_x(cols, seed=42), synth.host_x(rows, seed=43)
+    t = {k: dev(torch, v) for k, v in dict(w=w, x=x, resid=resid).items()}
+    ref = F.tensor_ref(t["w"].data_ptr(), 0, fmt, rows, cols)
+    out = torch.full((64, rows), float("nan"), device="cuda")
+    parts = torch.zeros(F.SUM_SQ_PARTS, device="cuda")
+    for i in range(64):
+        if i % 2 == 0:
+            ctx.fuse_next(None, F.ResidualEpilogue(t["resid"].data_ptr(), parts.data_ptr()))
+        ctx.hint_next(ref)
+        ctx.matvec(ref, t["x"].data_ptr(), out[i].data_ptr())
+    torch.cuda.synchronize()
+    assert ctx.status() == 0
+    got = out.cpu().numpy()
+    assert (got[0::2] == got[0]).all() and (got[1::2] == got[1]).all()
+    pick = np.random.default_rng(44).choice(rows, 200, replace=False)
+    rb = w.size // rows
+    want = oracle.matvec_f64(fmt, np.ascontiguousarray(w.reshape(rows, rb)[pick]).reshape(-1), 200, cols, x)
+    assert rel_l2(got[1][pick], want) <= 2e-6
+    assert rel_l2(got[0][pick], np.clip(resid[pick].astype(np.float64) + want, -65504.0, 65504.0)) <= 2e-6
