@@ -61,13 +61,14 @@ struct orome_cuda_ctx {
     // scratch for the unfused gate/up fallback
     float *gu_dev = nullptr;
     size_t gu_cap = 0;
+    std::vector<void *> retired;   // scratch buffers that have been outgrown (orome_ensure)
     // scratch of the tensor-core batched form: packed fp16 X and split-K partial sums
     float *tc_xp = nullptr, *tc_part = nullptr;
     size_t tc_xp_cap = 0, tc_part_cap = 0;
     int tc_min_batch = 4;    // batches from this size on use the tensor-core kernel (smaller ones: one decode launch per vector)
     int tc_slabs = 0;        // batched form: 1 = dequantized weights staged in shared memory (the earlier form), 0 = in tensor memory
-    int tc_tiles = 0;        // batched form in tensor memory: row tiles per CTA (0: chosen by the cost model)
-    int tc_split = 0;        // batched form: K parts per row tile (0: chosen by the cost model)
+    int tc_tiles = 0;        // kept for its key: the batched form has one layout of tiles
+    int tc_split = 0;        // batched form: K parts per tile (0: equal shares of the whole product)
     int kquant_mma = 1;      // Q4_K / Q5_K batch-1 products on the mma.sync kernel (0: dp4a kernel)
     int chain_inflight = 0;  // stages a chain's producer keeps outstanding at most (0: what fits 136 KiB, two at least)
     int wait_us = 0;         // bound of every device-side wait in microseconds of SM clock (0: about one second)
@@ -89,6 +90,38 @@ int orome_check_ref(const char *who, const OromeTensorRef *r, const uint8_t **da
 uint32_t orome_pipe_group_threads(int fmt, uint32_t in_dim);
 bool orome_pipe_supported(int fmt, uint32_t in_dim);
 long long orome_wait_cycles(const orome_cuda_ctx *c);
+
+int orome_ensure(orome_cuda_ctx *c, float **p, size_t *cap, size_t floats);   // context scratch of at least that size
+typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiledFn orome_encode_tiled_fn();
+
+// Launch with programmatic stream serialization, so the kernel's launch overlaps the tail of its predecessor
+// (the kernel itself starts with griddepcontrol.wait).
+template <typename... KArgs, typename... Args>
+int orome_launch_pdl_smem(orome_cuda_ctx *c, const char *what, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = c->pdl ? 1 : 0;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+    if (e != cudaSuccess) return orome_fail(OROME_ECUDA, "%s launch: %s", what, cudaGetErrorString(e));
+    ++c->launches;
+    return OROME_OK;
+}
+template <typename... KArgs, typename... Args>
+int orome_launch_pdl(orome_cuda_ctx *c, const char *what, void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args)
+{
+    return orome_launch_pdl_smem(c, what, kern, grid, block, 0, st, args...);
+}
 
 // ---- chain recording (defined in chain.cu) --------------------------------------------------------------------
 // Called by the batch-1 entry points, after their own validation, while a recording is open.

@@ -1,0 +1,26 @@
+// gemm.h -- the batched form's launches (defined in gemm.cu).
+#pragma once
+#include "ctx.h"
+
+#include "gemv_pipe.cuh"
+
+namespace orome {
+constexpr int TC_MAX_N = 64;         // input vectors per launch of the staged form, and of a row-split product on several GPUs
+
+// Row-split form on several GPUs (the batched counterpart of the publish fields of PipeArgs): every Y value also
+// goes, as a {value, tag} slot, into this rank's and every peer's copy of the gather arena.
+struct TcPub {
+    int npeers;                               // 0: single GPU, nothing is published
+    long long peer_delta[PIPE_MAX_PEERS];
+    const uint8_t *arena_base;
+    uint8_t *ll_origin;
+    unsigned int *pub_gen, *pub_arrived;
+};
+}  // namespace orome
+
+bool orome_tc_supported(const orome_cuda_ctx *c, int fmt, uint32_t in_dim);
+// Y[b][r] for b < batch.  pub / x_ll / wait_gen: the row-split form on several GPUs (batch <= TC_MAX_N, one launch): Y is
+// published to every rank's arena by the kernel that writes it, a gathered X is read from its slots by the packing kernel.
+int orome_launch_tc(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t out_dim, uint32_t in_dim, int layout, const float *x,
+                    int batch, int ldx, float *y, int ldy, cudaStream_t st, const orome::TcPub *pub = nullptr, const uint2 *x_ll = nullptr,
+                    const unsigned int *wait_gen = nullptr);

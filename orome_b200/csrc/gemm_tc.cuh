@@ -22,7 +22,7 @@
 #include <cuda.h>
 
 #include "decode.cuh"
-#include "gemv_pipe.cuh"
+#include "gemm.h"
 
 namespace orome {
 
@@ -43,22 +43,12 @@ constexpr int TC_MAX_RING = OROME_TC_RING;   // fp16 slab buffers
 constexpr int TC_PK_MAX_STAGES = 8;
 // packed-weight stages in flight: what hides the latency of the weight stream (a Q8_0 stage is 34 KB, a Q4_K one 18 KB)
 constexpr int tc_pk_stages(int fmt) { return fmt == FMT_Q8_0 ? (OROME_TC_PK < 3 ? OROME_TC_PK : 3) : OROME_TC_PK; }
-constexpr int TC_MAX_N = 64;         // input vectors per launch (padded to a multiple of 16)
 constexpr int TC_B_STAGES = OROME_TC_BS;     // X tile stages (one chunk each)
 constexpr int TC_B_MAX_STAGES = 4;
 constexpr int TC_DEQ_WARPS = 16;     // two groups of 8 warps take alternate slabs
 constexpr int TC_SLAB_WARPS = 8;     // warps that fill one slab
 constexpr int TC_THREADS = (TC_DEQ_WARPS + 3) * 32;     // + weight producer, MMA issuer, X producer
 
-// Row-split form on several GPUs (the batched counterpart of the publish fields of PipeArgs): every Y value also
-// goes, as a {value, tag} slot, into this rank's and every peer's copy of the gather arena.
-struct TcPub {
-    int npeers;                               // 0: single GPU, nothing is published
-    long long peer_delta[PIPE_MAX_PEERS];
-    const uint8_t *arena_base;
-    uint8_t *ll_origin;
-    unsigned int *pub_gen, *pub_arrived;
-};
 __device__ __forceinline__ void tc_publish(const TcPub &g, const float *addr, float val, unsigned int tag)
 {
     uint8_t *slot = g.ll_origin + 2 * (reinterpret_cast<const uint8_t *>(addr) - g.arena_base);
@@ -90,7 +80,6 @@ struct TcArgs {
     uint32_t rows, in_dim, row_bytes, chunk_bytes;   // chunk_bytes = packed bytes of 256 weights of one row
     uint32_t batch, npad, ldy;
     uint32_t split, chunks;       // split-K parts and 256-weight chunks per row: part p takes chunks [p*chunks/split, (p+1)*chunks/split)
-    uint32_t tiles_per_cta;       // tensor-memory form: row tiles a CTA works on side by side (1, 2 or 4)
     int layout;
     int *status;
     TcPub pub;                 // split == 1 only: with split-K the reduction kernel publishes
@@ -119,33 +108,35 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint64_t da, uint64_
 // Byte offset of 16-byte piece `c` (0..7) of row `r` inside a K-major SW128 tile.
 __device__ __forceinline__ uint32_t sw128_off(uint32_t r, uint32_t c) { return (r >> 3) * 1024u + (r & 7u) * 128u + ((c ^ (r & 7u)) << 4); }
 
-// X fp32 [batch][ldx] -> fp16 tiles [k_slab][npad][64] in the same swizzled layout; rows >= batch are zero.
+// X fp32 [batch][ldx] -> fp16 tiles [n tile][k_slab][nt_rows][64] in the same swizzled layout; rows >= batch are zero.
+// One thread per 16-byte piece; blockIdx.y = vector, so that a warp reads 1 KiB of one row (bound by the L2 round trip of a
+// small batch and by HBM for a large one).
 // x_ll: X is a gathered matrix in the arena, read from its slots (every element polled, bounded, for the generation
 // *wait_gen); NULL: a plain matrix.
-__global__ void pack_x_f16_kernel(const float *__restrict__ x, int batch, int ldx, uint32_t in_dim, uint32_t npad, __half *__restrict__ xp,
-                                  const uint2 *x_ll, const unsigned int *wait_gen, long long wait_cycles, int *status)
+__global__ void __launch_bounds__(256)
+pack_x_f16_kernel(const float *__restrict__ x, int batch, int ldx, uint32_t in_dim, uint32_t nt_rows, __half *__restrict__ xp,
+                  const uint2 *x_ll, const unsigned int *wait_gen, long long wait_cycles, int *status)
 {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");      // the product's weight loads need nothing from here
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint32_t piece = blockIdx.x * 256u + threadIdx.x, n = blockIdx.y;
+    if (piece >= in_dim / 8) return;
     const unsigned int want = x_ll ? *reinterpret_cast<const volatile unsigned int *>(wait_gen) : 0u;
     bool ok = true;
-    const uint32_t slabs = in_dim / TC_SLAB_K;
-    const size_t total = (size_t)slabs * npad * 8;   // one thread per 16-byte piece
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t c = (uint32_t)(i & 7), n = (uint32_t)((i >> 3) % npad), ks = (uint32_t)(i / ((size_t)npad * 8));
-        __half2 h[4];
-        if ((int)n < batch) {
-            const size_t off = (size_t)n * ldx + (size_t)ks * TC_SLAB_K + c * 8;
-            const float4 *src = reinterpret_cast<const float4 *>(x + off);
-            const float4 a = x_ll ? ld_gathered4(x_ll + off, want, &ok, wait_cycles, status) : src[0];
-            const float4 b = x_ll ? ld_gathered4(x_ll + off + 4, want, &ok, wait_cycles, status) : src[1];
-            h[0] = __floats2half2_rn(a.x, a.y); h[1] = __floats2half2_rn(a.z, a.w);
-            h[2] = __floats2half2_rn(b.x, b.y); h[3] = __floats2half2_rn(b.z, b.w);
-        } else {
-            h[0] = h[1] = h[2] = h[3] = __floats2half2_rn(0.f, 0.f);
-        }
-        uint8_t *dst = reinterpret_cast<uint8_t *>(xp) + (size_t)ks * npad * 128 + sw128_off(n, c);
-        *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(h);
+    const uint32_t c = piece & 7u, ks = piece >> 3, tile = n / nt_rows, nn = n - tile * nt_rows;
+    __half2 h[4];
+    if ((int)n < batch) {
+        const size_t off = (size_t)n * ldx + (size_t)piece * 8;
+        const float4 *src = reinterpret_cast<const float4 *>(x + off);
+        const float4 a = x_ll ? ld_gathered4(x_ll + off, want, &ok, wait_cycles, status) : __ldcg(src);
+        const float4 b = x_ll ? ld_gathered4(x_ll + off + 4, want, &ok, wait_cycles, status) : __ldcg(src + 1);
+        h[0] = __floats2half2_rn(a.x, a.y); h[1] = __floats2half2_rn(a.z, a.w);
+        h[2] = __floats2half2_rn(b.x, b.y); h[3] = __floats2half2_rn(b.z, b.w);
+    } else {
+        h[0] = h[1] = h[2] = h[3] = __floats2half2_rn(0.f, 0.f);
     }
+    uint8_t *dst = reinterpret_cast<uint8_t *>(xp) + ((size_t)tile * (in_dim / TC_SLAB_K) + ks) * nt_rows * 128 + sw128_off(nn, c);
+    *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(h);
     if (!ok) atomicExch(status, 3);
 }
 
@@ -394,384 +385,6 @@ gemm_tc_kernel(const __grid_constant__ TcArgs a)
         tc_publish_done(a.pub, *reinterpret_cast<const volatile unsigned int *>(a.pub.pub_gen) + 1u);
 }
 
-
-// ---- the same product with the dequantized weights in TENSOR MEMORY --------------------------------------------------
-// Two findings from cycle-stamping the form above drive this one.
-// (1) A 256-weight chunk of a 128-row tile costs 64 KB of shared-memory stores (the fp16 slabs) and 64 KB of operand
-//     reads by the tensor core next to 18 KB of packed weights; its MMAs took ~100 cycles each instead of ~34.  Here
-//     the dequant warps write the fp16 weights straight into tensor memory (tcgen05.st: lane = row, two weights per
-//     32-bit column) and the MMA takes its A operand from there.
-// (2) The copy engine, not memory, set the pace after that: a tensor copy of 128 rows x 144 bytes took ~2100 cycles
-//     whether the tensor sat in HBM or in L2, and everything else queued behind it (an X tile: 4000-8000 cycles).
-//     Here the dequant threads read their packed weights with plain 16-byte loads straight into registers, one unit
-//     ahead of the one they convert; the copy engine carries only the X tiles.
-// A CTA works on `tiles_per_cta` (TT) row tiles side by side: every X tile is fetched once and multiplied with the
-// chunk of each of its row tiles, each with its own accumulator; K is split over more CTAs (args.split) instead.
-//   tensor memory (512 columns): A stages of 128 columns (one chunk of one row tile: 128 rows x 256 fp16) from column
-//   0; TT accumulators of 64 columns at the top (TT = 1, 2: three A stages; TT = 4: two).
-//   dequant warp w: rows 32 * (w % 4) + lane (the lanes of tensor memory a warp may touch), weights
-//   64 * (w / 4) .. + 63 of the chunk; every warp works on every (chunk, tile) unit.
-constexpr int TCA_B_STAGES = 4;
-constexpr int TCA_MAX_TT = 4;
-constexpr int TCA_THREADS = (TC_DEQ_WARPS + 2) * 32;     // + MMA issuer, X producer
-constexpr uint32_t tca_a_stages(uint32_t tt) { return (512u - 64u * tt) / 128u; }
-
-__device__ __forceinline__ void tc_mma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate)
-{
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n}\n"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
-}
-__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint4 (&v)[4])
-{
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-                 ::"r"(taddr), "r"(v[0].x), "r"(v[0].y), "r"(v[0].z), "r"(v[0].w), "r"(v[1].x), "r"(v[1].y), "r"(v[1].z), "r"(v[1].w),
-                   "r"(v[2].x), "r"(v[2].y), "r"(v[2].z), "r"(v[2].w), "r"(v[3].x), "r"(v[3].y), "r"(v[3].z), "r"(v[3].w) : "memory");
-}
-
-// The packed bytes one dequant thread needs for its 64 weights (sub-blocks 2kq, 2kq+1 of a K-quant superblock, blocks
-// 2kq, 2kq+1 of a Q8_0 chunk) of one row, as 16-byte pieces.
-//   Q4_K: header (d, dmin, 12 scale bytes), 32 quant bytes (low nibbles = sub-block 2kq, high = 2kq+1).
-//   Q5_K: the same plus the 32 bytes of fifth bits (all eight sub-blocks share them).
-//   Q8_0: the 80 bytes from the 16-byte boundary at or below byte 68*kq of the chunk; the thread's 68 bytes start kq words in.
-//   Q6_K (210-byte superblocks, 2-byte aligned): thread kq takes half n = kq / 2 of the superblock and the elements
-//   l = 16 (kq % 2) .. + 15 of that half's four 32-groups (weights 128 n + 32 j + l, j = 0..3): 16 bytes of ql[l],
-//   16 of ql[32 + l], 16 of qh[l], the half's eight scale bytes and d.  (Taking 64 consecutive weights instead would
-//   need all 64 ql bytes for one of their nibbles each.)
-template <int FMT> struct TcPacked { uint4 p[FMT == FMT_Q4_K ? 3 : 5]; };
-template <> struct TcPacked<FMT_Q6_K> { uint32_t qa[4], qb[4], qh[4], sc[2], d; };
-
-// N consecutive 32-bit words from a 2-byte aligned address: aligned word loads, one more and a funnel shift when the
-// address is 2 (mod 4).  Reads at most two bytes before p and never a whole word past p + 4 N.
-template <int N>
-__device__ __forceinline__ void ldg_words_a2(const uint8_t *p, uint32_t (&out)[N])
-{
-    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
-    const uint32_t *q = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
-    const bool odd = (a & 2u) != 0;
-    uint32_t w[N + 1];
-#pragma unroll
-    for (int i = 0; i < N; ++i) w[i] = __ldg(q + i);
-    w[N] = odd ? __ldg(q + N) : 0u;
-    const uint32_t sh = odd ? 16u : 0u;
-#pragma unroll
-    for (int i = 0; i < N; ++i) out[i] = __funnelshift_r(w[i], w[i + 1], sh);
-}
-
-template <int FMT>
-__device__ __forceinline__ void tc_load_packed(const uint8_t *chunk, uint32_t kq, bool live, TcPacked<FMT> &d)
-{
-    if constexpr (FMT == FMT_Q6_K) {
-        if (!live) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) d.qa[i] = d.qb[i] = d.qh[i] = 0u;
-            d.sc[0] = d.sc[1] = d.d = 0u;
-            return;
-        }
-        const uint32_t n = kq >> 1, l0 = 16u * (kq & 1u);
-        ldg_words_a2<4>(chunk + 64u * n + l0, d.qa);
-        ldg_words_a2<4>(chunk + 64u * n + 32u + l0, d.qb);
-        ldg_words_a2<4>(chunk + 128u + 32u * n + l0, d.qh);
-        ldg_words_a2<2>(chunk + 192u + 8u * n, d.sc);
-        d.d = __ldg(reinterpret_cast<const unsigned short *>(chunk + 208));
-        return;
-    } else {
-    constexpr int N = FMT == FMT_Q4_K ? 3 : 5;
-    if (!live) {
-#pragma unroll
-        for (int i = 0; i < N; ++i) d.p[i] = make_uint4(0, 0, 0, 0);
-        return;
-    }
-    if constexpr (FMT == FMT_Q8_0) {
-        const uint4 *src = reinterpret_cast<const uint4 *>(chunk + ((kq * 68u) & ~15u));
-#pragma unroll
-        for (int i = 0; i < 5; ++i) d.p[i] = __ldg(src + i);
-    } else {
-        d.p[0] = __ldg(reinterpret_cast<const uint4 *>(chunk));
-        constexpr uint32_t QOFF = FMT == FMT_Q4_K ? 16u : 48u;
-        const uint4 *q = reinterpret_cast<const uint4 *>(chunk + QOFF + 32u * kq);
-        d.p[1] = __ldg(q);
-        d.p[2] = __ldg(q + 1);
-        if constexpr (FMT == FMT_Q5_K) {
-            d.p[3] = __ldg(reinterpret_cast<const uint4 *>(chunk + 16));
-            d.p[4] = __ldg(reinterpret_cast<const uint4 *>(chunk + 32));
-        }
-    }
-    }
-}
-
-// 32 weights (half h of the thread's 64) from the packed pieces -> four 16-byte fp16 pieces, element order.
-template <int FMT, int KQ>
-__device__ __forceinline__ void tc_dequant_half(const TcPacked<FMT> &d, uint32_t h, int layout, uint4 (&out)[4])
-{
-    uint32_t w[8];
-    __half2 scale, bias, addend;
-    if constexpr (FMT == FMT_Q8_0) {
-        // words KQ .. KQ+16 of the 20 loaded: block A = fp16 scale in the low half of word KQ, quants from its upper half
-        // on; block B = scale in the upper half of word KQ+8, quants = words KQ+9 .. KQ+16
-        const uint32_t v[20] = {d.p[0].x, d.p[0].y, d.p[0].z, d.p[0].w, d.p[1].x, d.p[1].y, d.p[1].z, d.p[1].w, d.p[2].x, d.p[2].y,
-                                d.p[2].z, d.p[2].w, d.p[3].x, d.p[3].y, d.p[3].z, d.p[3].w, d.p[4].x, d.p[4].y, d.p[4].z, d.p[4].w};
-        uint32_t dbits;
-        if (h == 0) {
-            dbits = v[KQ] & 0xffffu;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) w[i] = __byte_perm(v[KQ + i], v[KQ + i + 1], 0x5432u) ^ 0x80808080u;
-        } else {
-            dbits = v[KQ + 8] >> 16;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) w[i] = v[KQ + 9 + i] ^ 0x80808080u;
-        }
-        const float dd = __half2float(__ushort_as_half((unsigned short)dbits));
-        scale = __float2half2_rn(dd); bias = __float2half2_rn(1152.0f); addend = __float2half2_rn(0.0f);   // bytes are q + 128
-    } else {
-        const uint4 hd = d.p[0];
-        uint32_t scA, scB, mnA, mnB;
-        pair_scales(hd.y, hd.z, hd.w, layout, KQ, scA, scB, mnA, mnB);
-        const uint32_t sc = h ? scB : scA, mn = h ? mnB : mnA;
-        const float dd = __half2float(__ushort_as_half((unsigned short)(hd.x & 0xffffu)));
-        const float dmin = __half2float(__ushort_as_half((unsigned short)(hd.x >> 16)));
-        w[0] = d.p[1].x; w[1] = d.p[1].y; w[2] = d.p[1].z; w[3] = d.p[1].w; w[4] = d.p[2].x; w[5] = d.p[2].y; w[6] = d.p[2].z; w[7] = d.p[2].w;
-        const uint32_t shift = h * 4u;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) w[i] = (w[i] >> shift) & 0x0F0F0F0Fu;
-        if constexpr (FMT == FMT_Q5_K) {
-            const uint32_t hb[8] = {d.p[3].x, d.p[3].y, d.p[3].z, d.p[3].w, d.p[4].x, d.p[4].y, d.p[4].z, d.p[4].w};
-            const uint32_t g32 = 2u * KQ + h;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) w[i] |= ((hb[i] >> g32) & 0x01010101u) << 4;
-        }
-        scale = __float2half2_rn(dd * (float)sc); bias = __float2half2_rn(1024.0f); addend = __float2half2_rn(-(dmin * (float)mn));
-    }
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-        out[p].x = h2_bits(two_weights(w[2 * p], 0x5140u, bias, scale, addend));
-        out[p].y = h2_bits(two_weights(w[2 * p], 0x7362u, bias, scale, addend));
-        out[p].z = h2_bits(two_weights(w[2 * p + 1], 0x5140u, bias, scale, addend));
-        out[p].w = h2_bits(two_weights(w[2 * p + 1], 0x7362u, bias, scale, addend));
-    }
-}
-
-__device__ __forceinline__ void tc_st8(uint32_t taddr, const uint32_t (&v)[8])
-{
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
-}
-
-// Q6_K, 32-group J of the thread's half: its 16 weights (q - 32) * d * scale as fp16, two per word (format.m:131-174:
-// ql nibble | two qh bits << 4, scale 8 n + 2 J + l / 16).
-template <int KQ, int J>
-__device__ __forceinline__ void tc_dequant_q6_group(const TcPacked<FMT_Q6_K> &d, uint32_t (&out)[8])
-{
-    constexpr int SI = (KQ & 1) + 2 * J;             // scale byte inside the half's eight
-    const int sc = (int)(signed char)((d.sc[SI >> 2] >> (8 * (SI & 3))) & 0xffu);
-    const float dd = __half2float(__ushort_as_half((unsigned short)d.d));
-    const __half2 scale = __float2half2_rn(dd * (float)sc), bias = __float2half2_rn(1056.0f), addend = __float2half2_rn(0.0f);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const uint32_t ql = (J & 1) ? d.qb[i] : d.qa[i];
-        const uint32_t lo = (J < 2 ? ql : ql >> 4) & 0x0F0F0F0Fu;
-        const uint32_t w = lo | (((d.qh[i] >> (2 * J)) & 0x03030303u) << 4);
-        out[2 * i] = h2_bits(two_weights(w, 0x5140u, bias, scale, addend));
-        out[2 * i + 1] = h2_bits(two_weights(w, 0x7362u, bias, scale, addend));
-    }
-}
-
-// taddr: the thread's lane and the stage's column 32 * KQ (two weights per column).
-template <int FMT, int KQ>
-__device__ __forceinline__ void tc_convert_unit(const TcPacked<FMT> &d, int layout, uint32_t taddr)
-{
-    if constexpr (FMT == FMT_Q6_K) {
-        // group J, elements 16 (KQ % 2) ..: weights 128 (KQ / 2) + 32 J + 16 (KQ % 2) .., i.e. column 64 (KQ / 2) + 16 J + 8 (KQ % 2)
-        const uint32_t col = taddr - 24u * (KQ & 1);
-        uint32_t v[8];
-        tc_dequant_q6_group<KQ, 0>(d, v); tc_st8(col, v);
-        tc_dequant_q6_group<KQ, 1>(d, v); tc_st8(col + 16u, v);
-        tc_dequant_q6_group<KQ, 2>(d, v); tc_st8(col + 32u, v);
-        tc_dequant_q6_group<KQ, 3>(d, v); tc_st8(col + 48u, v);
-    } else {
-#pragma unroll
-        for (uint32_t h = 0; h < 2; ++h) {
-            uint4 v[4];
-            tc_dequant_half<FMT, KQ>(d, h, layout, v);
-            tc_st16(taddr + h * 16u, v);
-        }
-    }
-}
-
-template <int FMT>
-__global__ void __launch_bounds__(TCA_THREADS, 1)
-gemm_tca_kernel(const __grid_constant__ TcArgs a)
-{
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    // layout: [X tiles BS x npad*512][barriers]
-    constexpr uint32_t BS = TCA_B_STAGES, MAX_AS = 3;
-    const uint32_t TT = a.tiles_per_cta, AS = tca_a_stages(TT);
-    const uint32_t b_tile_bytes = a.npad * 128u * TC_SLABS;
-    uint8_t *b_tiles = smem;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(b_tiles + BS * b_tile_bytes);
-    uint64_t *b_full = bars, *b_empty = b_full + BS;
-    uint64_t *a_full = b_empty + BS, *a_empty = a_full + MAX_AS, *acc_done = a_empty + MAX_AS;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_done + 1);
-    __shared__ volatile int s_abort;
-
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    const uint32_t tgroup = blockIdx.x / a.split, sp = blockIdx.x % a.split;
-    const uint32_t tile0 = tgroup * TT;                          // this CTA's row tiles: tile0 .. tile0 + TT - 1 (those inside the tensor)
-    const uint32_t chunk0 = sp * a.chunks / a.split, nchunks = (sp + 1) * a.chunks / a.split - chunk0;
-    const uint32_t rot = (tgroup * 5u + sp * 3u) % nchunks;      // CTAs start their walk over K at different chunks
-    const uint32_t nunits = nchunks * TT;                        // unit u = (chunk u / TT, tile u % TT)
-    const uint32_t acc_col0 = 512u - 64u * TT;
-
-    if (tid == 0) {
-        s_abort = 0;
-        for (uint32_t s = 0; s < BS; ++s) { mbar_init(smem_u32(b_full + s), 1); mbar_init(smem_u32(b_empty + s), 1); }
-        for (uint32_t s = 0; s < MAX_AS; ++s) { mbar_init(smem_u32(a_full + s), TC_DEQ_WARPS); mbar_init(smem_u32(a_empty + s), 1); }
-        mbar_init(smem_u32(acc_done), 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    if (warp == 0) {   // all 512 columns: one CTA per SM (its shared memory request sees to that)
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(tmem_slot);
-    pdl_launch_dependents();
-
-    auto wait = [&](uint64_t *bar, uint32_t parity) {
-        if (!s_abort && !mbar_wait_bounded(smem_u32(bar), parity)) { s_abort = 1; atomicExch(a.status, 4); }
-    };
-    auto chunk_of = [&](uint32_t c) { return chunk0 + (c + rot < nchunks ? c + rot : c + rot - nchunks); };
-
-    if (warp == TC_DEQ_WARPS + 1) {
-        // ---- X producer: the pre-packed fp16 tiles (the previous kernel's output), one per chunk ----
-        if (lane == 0) {
-            pdl_wait();
-            for (uint32_t c = 0; c < nchunks && !s_abort; ++c) {
-                const uint32_t sb = c % BS, kb = c / BS;
-                if (kb > 0) { wait(b_empty + sb, (kb - 1) & 1u); asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-                mbar_expect_tx(smem_u32(b_full + sb), b_tile_bytes);
-                bulk_g2s(smem_u32(b_tiles + (size_t)sb * b_tile_bytes), reinterpret_cast<const uint8_t *>(a.xp) + (size_t)chunk_of(c) * b_tile_bytes,
-                         b_tile_bytes, smem_u32(b_full + sb));
-                TC_STAMP(6, c);
-            }
-        }
-    } else if (warp == TC_DEQ_WARPS) {
-        // ---- MMA issue: one thread; 16 x (M128 x N x K16) per unit, A from tensor memory, B = the chunk's X tile ----
-        if (lane == 0) {
-            const uint32_t idesc = (1u << 4) | ((a.npad >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);   // fp32 accumulate, fp16 x fp16, K-major both
-            uint32_t sa = 0, ka = 0, u = 0;
-            for (uint32_t c = 0; c < nchunks && !s_abort; ++c) {
-                const uint32_t sb = c % BS;
-                wait(b_full + sb, (c / BS) & 1u);
-                TC_STAMP(7, c);
-                const uint32_t b_addr = smem_u32(b_tiles + (size_t)sb * b_tile_bytes);
-                for (uint32_t t = 0; t < TT; ++t, ++u) {
-                    wait(a_full + sa, ka & 1u);
-                    TC_STAMP(4, u);
-                    tc_fence_after();
-                    const uint32_t a_col = tmem_base + sa * 128u, d_col = tmem_base + acc_col0 + t * 64u;
-#pragma unroll
-                    for (uint32_t k16 = 0; k16 < 16; ++k16)
-                        tc_mma_f16_ta(d_col, a_col + k16 * 8u, tc_desc_sw128(b_addr + (k16 >> 2) * a.npad * 128u + (k16 & 3u) * 32u), idesc,
-                                      (c | k16) ? 1u : 0u);
-                    tc_commit(smem_u32(a_empty + sa));     // the A stage is free once these MMAs have read it
-                    TC_STAMP(5, u);
-                    if (++sa == AS) { sa = 0; ++ka; }
-                }
-                tc_commit(smem_u32(b_empty + sb));         // and the X tile after the chunk's last row tile
-            }
-            tc_commit(smem_u32(acc_done));
-        }
-    } else {
-        // ---- dequant warps: packed weights (global -> registers, one unit ahead) -> fp16 weights in tensor memory ----
-        const uint32_t quad = warp & 3u, kq = warp >> 2, r = quad * 32u + lane;
-        const uint32_t lane_addr = (quad * 32u) << 16;
-        uint32_t sa = 0, ka = 0, t = 0, c = 0;
-        auto unit_ptr = [&](uint32_t cc, uint32_t tt, bool &live) {
-            const uint32_t grow = (tile0 + tt) * TC_M + r;
-            live = grow < a.rows;
-            return a.w + (size_t)grow * a.row_bytes + (size_t)chunk_of(cc) * a.chunk_bytes;
-        };
-        TcPacked<FMT> cur, nxt;
-        {
-            bool live;
-            const uint8_t *p = unit_ptr(0, 0, live);
-            tc_load_packed<FMT>(p, kq, live, cur);
-        }
-        for (uint32_t u = 0; u < nunits; ++u) {
-            uint32_t tn = t + 1, cn = c;
-            if (tn == TT) { tn = 0; ++cn; }
-            if (u + 1 < nunits) {                 // the next unit's bytes are on their way while this one is converted
-                bool live;
-                const uint8_t *p = unit_ptr(cn, tn, live);
-                tc_load_packed<FMT>(p, kq, live, nxt);
-            }
-            if (tid == 0) TC_STAMP(1, u);
-            if (ka > 0) wait(a_empty + sa, (ka - 1) & 1u);
-            if (tid == 0) TC_STAMP(2, u);
-            tc_fence_after();
-            const uint32_t taddr = tmem_base + lane_addr + sa * 128u + kq * 32u;
-            switch (kq) {                         // warp-uniform; the sub-block index is a compile-time constant inside
-            case 0: tc_convert_unit<FMT, 0>(cur, a.layout, taddr); break;
-            case 1: tc_convert_unit<FMT, 1>(cur, a.layout, taddr); break;
-            case 2: tc_convert_unit<FMT, 2>(cur, a.layout, taddr); break;
-            default: tc_convert_unit<FMT, 3>(cur, a.layout, taddr); break;
-            }
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(smem_u32(a_full + sa));
-                if (tid == 0) TC_STAMP(3, u);
-            }
-            cur = nxt;
-            if (++sa == AS) { sa = 0; ++ka; }
-            t = tn; c = cn;
-        }
-        // ---- epilogue: warps 0-3, lane = row, one accumulator per row tile ----
-        if (warp < 4) {
-            wait(acc_done, 0);
-            tc_fence_after();
-            float *ybase = a.split == 1 ? a.y : a.y + (size_t)sp * a.batch * a.rows;
-            const uint32_t ld = a.split == 1 ? a.ldy : a.rows;
-            const bool publish = a.split == 1 && a.pub.npeers > 0;
-            const unsigned int pub_tag = publish ? *reinterpret_cast<const volatile unsigned int *>(a.pub.pub_gen) + 1u : 0u;
-            for (uint32_t tt = 0; tt < TT; ++tt) {
-                const uint32_t grow = (tile0 + tt) * TC_M + warp * 32 + lane;
-                for (uint32_t n0 = 0; n0 < a.npad; n0 += 16) {
-                    uint32_t v[16];
-                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-                                   "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                                 : "r"(tmem_base + ((warp * 32u) << 16) + acc_col0 + tt * 64u + n0));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (grow < a.rows && !s_abort) {
-#pragma unroll
-                        for (uint32_t i = 0; i < 16; ++i)
-                            if (n0 + i < a.batch) {
-                                float *dst = ybase + (size_t)(n0 + i) * ld + grow;
-                                *dst = __uint_as_float(v[i]);
-                                if (publish) tc_publish(a.pub, dst, __uint_as_float(v[i]), pub_tag);
-                            }
-                    }
-                }
-            }
-        }
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 0) {
-        tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
-    }
-    if (threadIdx.x == 0 && a.split == 1 && a.pub.npeers > 0)
-        tc_publish_done(a.pub, *reinterpret_cast<const volatile unsigned int *>(a.pub.pub_gen) + 1u);
-}
 
 // Y[b][r] = sum over splits of partial[s][b][r]
 __global__ void splitk_reduce_kernel(const float *__restrict__ part, uint32_t split, uint32_t batch, uint32_t rows, float *__restrict__ y, uint32_t ldy,

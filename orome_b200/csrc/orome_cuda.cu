@@ -17,7 +17,7 @@
 #include "gemv_pipe.cuh"
 #include "gemv_mma.cuh"
 #include "moe.cuh"
-#include "gemm_tc.cuh"
+#include "gemm.h"
 
 using namespace orome;
 
@@ -71,6 +71,7 @@ extern "C" void orome_cuda_ctx_destroy(orome_cuda_ctx *c)
     cudaFree(c->gu_dev);
     cudaFree(c->tc_xp);
     cudaFree(c->tc_part);
+    for (void *q : c->retired) cudaFree(q);
     cudaFree(c->trace_dev);
     cudaFree(c->g_local);
     cudaFreeHost(c->stage_x_host);
@@ -266,36 +267,6 @@ static int post_launch(orome_cuda_ctx *c, const char *what)
     return OROME_OK;
 }
 
-// Launch with programmatic stream serialization, so the kernel's launch overlaps the tail of its predecessor
-// (the kernel itself starts with griddepcontrol.wait).
-template <typename... KArgs, typename... Args>
-static int launch_pdl_smem(orome_cuda_ctx *c, const char *what, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args);
-
-template <typename... KArgs, typename... Args>
-static int launch_pdl(orome_cuda_ctx *c, const char *what, void (*kern)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args)
-{
-    return launch_pdl_smem(c, what, kern, grid, block, 0, st, args...);
-}
-
-template <typename... KArgs, typename... Args>
-static int launch_pdl_smem(orome_cuda_ctx *c, const char *what, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = c->pdl ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
-    if (e != cudaSuccess) return fail(OROME_ECUDA, "%s launch: %s", what, cudaGetErrorString(e));
-    ++c->launches;
-    return OROME_OK;
-}
-
 static int launch_generic(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t out_dim, uint32_t in_dim, int layout,
                           const float *x, int batch, int ldx, float *y, int ldy, cudaStream_t st);
 
@@ -308,14 +279,14 @@ static int launch_router(orome_cuda_ctx *c, const uint8_t *data, uint32_t ne, ui
     int rc;
     const uint32_t rows = ne + (shared_gate ? 1u : 0u);
     if (in_dim % 4 == 0 && !(reinterpret_cast<uintptr_t>(x) & 15) && (n_tokens == 1 || ldx % 4 == 0))
-        rc = launch_pdl(c, "gemv_f32", gemv_f32_kernel, dim3(rows, (unsigned)(n_tokens + 3) / 4), dim3(128), st, reinterpret_cast<const float *>(data), ne, in_dim,
+        rc = orome_launch_pdl(c, "gemv_f32", gemv_f32_kernel, dim3(rows, (unsigned)(n_tokens + 3) / 4), dim3(128), st, reinterpret_cast<const float *>(data), ne, in_dim,
                         x, n_tokens, ldx, logits, (int)rows, reinterpret_cast<const float *>(shared_gate));
     else {
         rc = launch_generic(c, FMT_F32, data, ne, in_dim, 0, x, n_tokens, ldx, logits, (int)rows, st);
         if (!rc && shared_gate) rc = launch_generic(c, FMT_F32, shared_gate, 1, in_dim, 0, x, n_tokens, ldx, logits + ne, (int)rows, st);
     }
     if (rc) return rc;
-    return launch_pdl(c, "route_topk", route_topk_kernel, dim3(n_tokens), dim3(256), st, (const float *)logits, (int)rows, ne, K, idx, w,
+    return orome_launch_pdl(c, "route_topk", route_topk_kernel, dim3(n_tokens), dim3(256), st, (const float *)logits, (int)rows, ne, K, idx, w,
                       shared_gate ? shared_logit : (float *)nullptr);
 }
 
@@ -568,11 +539,6 @@ static int launch_pipe(orome_cuda_ctx *c, int fmt, const PipePlan &p, int mode, 
 // ---------------------------------------------------------------------------
 // Q4_K / Q5_K batch-1 kernel on mma.sync: planning and launch
 // ---------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn encode_tiled_fn();
-
 struct MmaPlan {
     MmaArgs args;
     int threads, grid;
@@ -677,7 +643,7 @@ static int mma_tensor_map(orome_cuda_ctx *c, const uint8_t *w, uint32_t unit, ui
     const MapKey key{w, unit, units, rows, kb};
     auto it = c->maps.find(key);
     if (it == c->maps.end()) {
-        EncodeTiledFn enc = encode_tiled_fn();
+        EncodeTiledFn enc = orome_encode_tiled_fn();
         if (!enc) return fail(OROME_ECUDA, "mma plan: cuTensorMapEncodeTiled is not available");
         CUtensorMap m;
         const cuuint64_t dims[3] = {unit / 4, units, rows};
@@ -905,7 +871,7 @@ extern "C" int orome_cuda_gather_wait(orome_cuda_ctx *c, int flag, float *vec_de
     CU(cudaSetDevice(c->device));
     const uint2 *slots = reinterpret_cast<const uint2 *>(mine + c->g_data_bytes + 2 * (size_t)(v - mine));
     const unsigned blocks = std::max(1u, std::min((n / 4 + 255) / 256, (unsigned)c->sm_count));
-    return launch_pdl(c, "gather_unpack", gather_unpack_kernel, dim3(blocks), dim3(256), static_cast<cudaStream_t>(stream), slots, vec_dev,
+    return orome_launch_pdl(c, "gather_unpack", gather_unpack_kernel, dim3(blocks), dim3(256), static_cast<cudaStream_t>(stream), slots, vec_dev,
                       n / 4, (const unsigned int *)(c->g_local + flag), c->status_dev, orome_wait_cycles(c));
 }
 
@@ -1036,45 +1002,8 @@ extern "C" int orome_cuda_matvec_group(orome_cuda_ctx *c, const OromeTensorRef *
 // ---------------------------------------------------------------------------
 // batched form on the tensor cores
 // ---------------------------------------------------------------------------
-// Q6_K (rows only 2-byte aligned, no tensor map possible) exists in the tensor-memory form only.
-static bool tc_supported(const orome_cuda_ctx *c, int fmt, uint32_t in_dim)
-{
-    if (in_dim % TC_KC != 0) return false;
-    return fmt == FMT_Q8_0 || fmt == FMT_Q4_K || fmt == FMT_Q5_K || (fmt == FMT_Q6_K && !c->tc_slabs);
-}
-
-template <int FMT>
-static int launch_tca_fmt(orome_cuda_ctx *c, const TcArgs &a, int grid, size_t smem, cudaStream_t st)
-{
-    auto kern = gemm_tca_kernel<FMT>;
-    static bool configured[64] = {false};
-    if (!configured[c->device]) {
-        cudaFuncAttributes fa;
-        CU(cudaFuncGetAttributes(&fa, kern));
-        CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, c->smem_optin - (int)fa.sharedSizeBytes));
-        configured[c->device] = true;
-    }
-    return launch_pdl_smem(c, "gemm_tca", kern, dim3(grid), dim3(TCA_THREADS), smem, st, a);
-}
-
-template <int FMT>
-static int launch_tc_fmt(orome_cuda_ctx *c, const TcArgs &a, int grid, size_t smem, cudaStream_t st)
-{
-    auto kern = gemm_tc_kernel<FMT>;
-    static bool configured[64] = {false};
-    if (!configured[c->device]) {
-        cudaFuncAttributes fa;
-        CU(cudaFuncGetAttributes(&fa, kern));
-        CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, c->smem_optin - (int)fa.sharedSizeBytes));
-        configured[c->device] = true;
-    }
-    return launch_pdl_smem(c, "gemm_tc", kern, dim3(grid), dim3(TC_THREADS), smem, st, a);
-}
-
-static int ensure(float **p, size_t *cap, size_t floats);
-
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda)
-static EncodeTiledFn encode_tiled_fn()
+EncodeTiledFn orome_encode_tiled_fn()
 {
     static EncodeTiledFn fn = nullptr;
     if (!fn) {
@@ -1084,103 +1013,6 @@ static EncodeTiledFn encode_tiled_fn()
             fn = reinterpret_cast<EncodeTiledFn>(p);
     }
     return fn;
-}
-
-// Y[b][r] for b < batch (<= TC_MAX_N per launch; larger batches are cut into slices that each re-read the weights).
-// pub / x_ll / wait_gen: the row-split form on several GPUs (batch <= TC_MAX_N, one launch): Y is published to every
-// rank's arena by the kernel that writes it, a gathered X is read from its slots by the packing kernel.
-static int launch_tc(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t out_dim, uint32_t in_dim, int layout, const float *x,
-                     int batch, int ldx, float *y, int ldy, cudaStream_t st, const TcPub *pub = nullptr, const uint2 *x_ll = nullptr,
-                     const unsigned int *wait_gen = nullptr)
-{
-    TcPub no_pub;
-    memset(&no_pub, 0, sizeof no_pub);
-    if (!pub) pub = &no_pub;
-    const uint32_t chunk_bytes = fmt == FMT_Q8_0 ? 272u : fmt == FMT_Q4_K ? 144u : fmt == FMT_Q5_K ? 176u : 210u;
-    const uint32_t chunks = in_dim / TC_KC, tiles = (out_dim + TC_M - 1) / TC_M;
-    // Split K so that the SMs stay busy: a CTA costs about one time unit per chunk plus about five to set up (TMEM,
-    // barriers, pipeline fill -- measured: three parts in two waves were slower than one part on 96 of 148 SMs), the
-    // grid runs in waves of sm_count CTAs, a split adds a reduction pass.  Parts may be uneven.
-    // Split K so that the SMs stay busy: a CTA costs about one time unit per chunk plus about five to set up (TMEM,
-    // barriers, pipeline fill -- measured: three parts in two waves were slower than one part on 96 of 148 SMs), the
-    // grid runs in waves of sm_count CTAs, a split adds a reduction pass.  Parts may be uneven.
-    // Row tiles per CTA (tensor-memory form): one.  Two or four tiles sharing each X tile were measured slower at every
-    // split (12288 x 4096, batch 64: 29 us with one tile, 37-48 us with two): the MMA issue, not the X traffic, is what a
-    // CTA waits for.  OROME_OPT_TC_TILES keeps the choice open for experiments.
-    uint32_t split = 1;
-    const uint32_t tt = c->tc_slabs ? 1u : (c->tc_tiles ? std::min<uint32_t>((uint32_t)c->tc_tiles, tiles) : 1u);
-    double best = 1e30;
-    for (uint32_t s = c->tc_split ? (uint32_t)c->tc_split : 1u; s <= (c->tc_split ? (uint32_t)c->tc_split : 12u) && s <= chunks; ++s) {
-        const uint32_t ctas = (tiles + tt - 1) / tt * s, waves = (ctas + c->sm_count - 1) / c->sm_count;
-        const double cost = (double)waves * ((double)((chunks + s - 1) / s) * tt + 5.0) + (s > 1 ? 1.0 + 0.25 * s : 0.0);
-        if (cost < best) { best = cost; split = s; }
-    }
-    for (int b0 = 0; b0 < batch; b0 += TC_MAX_N) {
-        const int nb = std::min(batch - b0, TC_MAX_N);
-        const uint32_t npad = (uint32_t)(nb + 15) / 16 * 16;
-        int rc = ensure(&c->tc_xp, &c->tc_xp_cap, (size_t)in_dim * npad / 2 + 64);
-        if (rc) return rc;
-        if (split > 1) { rc = ensure(&c->tc_part, &c->tc_part_cap, (size_t)split * nb * out_dim); if (rc) return rc; }
-        __half *xp = reinterpret_cast<__half *>(c->tc_xp);
-        const size_t pieces = (size_t)(in_dim / TC_SLAB_K) * npad * 8;
-        rc = launch_pdl(c, "pack_x_f16", pack_x_f16_kernel, dim3((unsigned)std::min<size_t>((pieces + 255) / 256, 1184)), dim3(256), st,
-                        x + (size_t)b0 * ldx, nb, ldx, in_dim, npad, xp, x_ll, wait_gen, orome_wait_cycles(c), c->status_dev);
-        if (rc) return rc;
-        TcArgs a;
-        memset(&a, 0, sizeof a);
-        if (c->tc_slabs) {      // the staged form fetches its packed weights with tensor copies
-            EncodeTiledFn enc = encode_tiled_fn();
-            if (!enc) return fail(OROME_ECUDA, "gemm_tc: cuTensorMapEncodeTiled is not available");
-            const cuuint64_t dims[2] = {(cuuint64_t)row_bytes_of(fmt, in_dim) / 4, out_dim};
-            const cuuint64_t strides[1] = {(cuuint64_t)row_bytes_of(fmt, in_dim)};
-            const cuuint32_t box[2] = {chunk_bytes / 4, (cuuint32_t)TC_M}, estr[2] = {1, 1};
-            CUresult r = enc(&a.wmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<uint8_t *>(data), dims, strides, box, estr,
-                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            if (r != CUDA_SUCCESS) return fail(OROME_ECUDA, "gemm_tc: cuTensorMapEncodeTiled failed (%d)", (int)r);
-        }
-        a.w = data; a.xp = xp; a.y = split == 1 ? y + (size_t)b0 * ldy : c->tc_part;
-        a.rows = out_dim; a.in_dim = in_dim; a.row_bytes = (uint32_t)row_bytes_of(fmt, in_dim); a.chunk_bytes = chunk_bytes;
-        a.batch = (uint32_t)nb; a.npad = npad; a.ldy = (uint32_t)ldy; a.split = split; a.chunks = chunks; a.tiles_per_cta = tt;
-        a.layout = layout; a.status = c->status_dev;
-        a.pub = *pub;
-        // Shared memory: one chunk's worth of fp16 slab buffers, two X tile stages, two packed-weight stages (169 KB for
-        // Q4_K at batch 64).  Measured on Q4_K 12288x4096, batch 64: deeper rings (seven slab buffers, a third X stage, up
-        // to six packed-weight stages, sized at run time) made the launch slower (35-41 us against 34 us), and removing
-        // the dequant arithmetic altogether only brings it to 31 us: ring depth is not what bounds this kernel, and
-        // run-time ring sizes put integer divisions on the hand-off path of every slab.
-        const size_t pk_stage = (TC_M * chunk_bytes + 127) & ~127u, b_tile = (size_t)npad * 128 * TC_SLABS;
-        const int grid = (int)((tiles + tt - 1) / tt * split);
-        if (!c->tc_slabs) {
-            // dequantized weights in tensor memory: shared memory holds X tiles and packed stages only; at least half an
-            // SM's worth is requested so that two CTAs (each wants all 512 columns of tensor memory) never share an SM
-            size_t smem = 1024 + (size_t)TCA_B_STAGES * b_tile + 512;
-            smem = std::max<size_t>(smem, 120 * 1024);
-            if (smem > (size_t)c->smem_optin - 1024) return fail(OROME_ENOTSUP, "gemm_tca: batch %d does not fit shared memory", nb);
-            switch (fmt) {
-            case FMT_Q8_0: rc = launch_tca_fmt<FMT_Q8_0>(c, a, grid, smem, st); break;
-            case FMT_Q4_K: rc = launch_tca_fmt<FMT_Q4_K>(c, a, grid, smem, st); break;
-            case FMT_Q5_K: rc = launch_tca_fmt<FMT_Q5_K>(c, a, grid, smem, st); break;
-            default: rc = launch_tca_fmt<FMT_Q6_K>(c, a, grid, smem, st); break;
-            }
-        } else {
-            const size_t smem = 1024 + (size_t)TC_MAX_RING * 16384 + (size_t)TC_B_STAGES * b_tile + 512 + (size_t)tc_pk_stages(fmt) * pk_stage;
-            if (smem > (size_t)c->smem_optin - 1024) return fail(OROME_ENOTSUP, "gemm_tc: batch %d does not fit shared memory", nb);
-            switch (fmt) {
-            case FMT_Q8_0: rc = launch_tc_fmt<FMT_Q8_0>(c, a, grid, smem, st); break;
-            case FMT_Q4_K: rc = launch_tc_fmt<FMT_Q4_K>(c, a, grid, smem, st); break;
-            default: rc = launch_tc_fmt<FMT_Q5_K>(c, a, grid, smem, st); break;
-            }
-        }
-        if (rc) return rc;
-        if (split > 1) {
-            const size_t n = (size_t)nb * out_dim;
-            rc = launch_pdl(c, "splitk_reduce", splitk_reduce_kernel, dim3((unsigned)std::min<size_t>((n + 255) / 256, 1184)), dim3(256), st,
-                            (const float *)c->tc_part, split, (uint32_t)nb, out_dim, y + (size_t)b0 * ldy, (uint32_t)ldy, *pub);
-            if (rc) return rc;
-        }
-    }
-    return OROME_OK;
 }
 
 extern "C" int orome_cuda_matvec(orome_cuda_ctx *c, const OromeTensorRef *ref, const float *x_dev, float *y_dev, int batch,
@@ -1203,7 +1035,7 @@ extern "C" int orome_cuda_matvec(orome_cuda_ctx *c, const OromeTensorRef *ref, c
     if (rc) { c->g_wait = c->g_publish = -1; return rc; }
     CU(cudaSetDevice(c->device));
     const bool x_ok = ldx % 4 == 0 && !(reinterpret_cast<uintptr_t>(x_dev) & 15);
-    const bool tc_ok = batch >= c->tc_min_batch && !c->force_generic && tc_supported(c, (int)ref->format, ref->in_dim) && x_ok;
+    const bool tc_ok = batch >= c->tc_min_batch && !c->force_generic && orome_tc_supported(c, (int)ref->format, ref->in_dim) && x_ok;
     if (c->g_world > 1 && (c->g_wait >= 0 || c->g_publish >= 0)) {
         // Row-split batched product: only the tensor-core form has a publish / wait path, and only as one launch.  Any
         // other call drops the request and says so, rather than leave it armed for an unrelated later launch.
@@ -1235,11 +1067,11 @@ extern "C" int orome_cuda_matvec(orome_cuda_ctx *c, const OromeTensorRef *ref, c
             x_ll = reinterpret_cast<const uint2 *>(pub.ll_origin + 2 * (size_t)(xb - mine));
             wait_gen = c->g_local + wait;
         }
-        return launch_tc(c, (int)ref->format, data, ref->out_dim, ref->in_dim, (int)ref->variant, x_dev, batch, ldx, y_dev, ldy,
+        return orome_launch_tc(c, (int)ref->format, data, ref->out_dim, ref->in_dim, (int)ref->variant, x_dev, batch, ldx, y_dev, ldy,
                          static_cast<cudaStream_t>(stream), &pub, x_ll, wait_gen);
     }
     if (tc_ok)
-        return launch_tc(c, (int)ref->format, data, ref->out_dim, ref->in_dim, (int)ref->variant, x_dev, batch, ldx, y_dev, ldy,
+        return orome_launch_tc(c, (int)ref->format, data, ref->out_dim, ref->in_dim, (int)ref->variant, x_dev, batch, ldx, y_dev, ldy,
                          static_cast<cudaStream_t>(stream));
     // Small batches, and formats the tensor-core form does not take (Q6_K): one batch-1 launch per input vector.  The
     // weights are read once per vector, but the decode kernels run near the memory rate while the shape-agnostic
@@ -1289,15 +1121,20 @@ extern "C" int orome_format_dispatch_matvec(orome_cuda_ctx *c, const OromeTensor
     return orome_cuda_matvec(c, ref, x, y, 1, 0, 0, stream);
 }
 
-static int ensure(float **p, size_t *cap, size_t floats)
+int orome_ensure(orome_cuda_ctx *c, float **p, size_t *cap, size_t floats)
 {
     if (*cap >= floats) return OROME_OK;
-    if (*p) cudaFree(*p);
-    *p = nullptr;
-    *cap = 0;
-    cudaError_t e = cudaMalloc(p, floats * sizeof(float));
-    if (e != cudaSuccess) return fail(OROME_ENOMEM, "scratch of %zu floats: %s", floats, cudaGetErrorString(e));
-    *cap = floats;
+    // The old buffer may still be an operand of a captured graph: it stays until the context goes.  Doubling bounds what is
+    // kept that way by the size of the last one.
+    const size_t want = std::max(floats, 2 * *cap);
+    float *q = nullptr;
+    cudaError_t e = cudaMalloc(&q, want * sizeof(float));
+    size_t got = want;
+    if (e == cudaErrorMemoryAllocation && want > floats) { (void)cudaGetLastError(); e = cudaMalloc(&q, floats * sizeof(float)); got = floats; }
+    if (e != cudaSuccess) { (void)cudaGetLastError(); return fail(OROME_ENOMEM, "scratch of %zu floats: %s", floats, cudaGetErrorString(e)); }
+    if (*p) c->retired.push_back(*p);
+    *p = q;
+    *cap = got;
     return OROME_OK;
 }
 
@@ -1360,7 +1197,7 @@ extern "C" int orome_cuda_gate_up_swiglu(orome_cuda_ctx *c, const OromeTensorRef
     if (batch > 1 && (ldx < (int)gate->in_dim || ldo < (int)gate->out_dim))
         return fail(OROME_EINVAL, "gate_up_swiglu: ldx/ldo smaller than the row length");
     const size_t n = (size_t)gate->out_dim;
-    rc = ensure(&c->gu_dev, &c->gu_cap, 2 * n * batch);
+    rc = orome_ensure(c, &c->gu_dev, &c->gu_cap, 2 * n * batch);
     if (rc) return rc;
     float *g = c->gu_dev, *u = c->gu_dev + n * batch;
     if (batch > 1) {
@@ -1420,7 +1257,7 @@ extern "C" int orome_cuda_argmax(orome_cuda_ctx *c, const float *data_dev, uint3
     const unsigned blocks = std::max(1u, std::min((count + 1023) / 1024, (unsigned)c->sm_count));
     // reduction state: two 64-bit words of the context's status block (128 bytes in), left zero by every call
     unsigned long long *state = reinterpret_cast<unsigned long long *>(c->status_dev) + 16;
-    return launch_pdl(c, "argmax", argmax_kernel, dim3(blocks), dim3(256), static_cast<cudaStream_t>(stream), data_dev, count, result_dev, state);
+    return orome_launch_pdl(c, "argmax", argmax_kernel, dim3(blocks), dim3(256), static_cast<cudaStream_t>(stream), data_dev, count, result_dev, state);
 }
 
 // ---------------------------------------------------------------------------
@@ -1442,7 +1279,7 @@ extern "C" int orome_cuda_moe_route(orome_cuda_ctx *c, const OromeTensorRef *rou
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const uint32_t ne = router->out_dim;
     if (!logits_dev) {
-        rc = ensure(&c->logits_dev, &c->logits_cap, (size_t)ne * n_tokens);
+        rc = orome_ensure(c, &c->logits_dev, &c->logits_cap, (size_t)ne * n_tokens);
         if (rc) return rc;
         logits_dev = c->logits_dev;
     }
@@ -1475,7 +1312,7 @@ extern "C" int orome_cuda_moe_route_pair(orome_cuda_ctx *c, const OromeTensorRef
         CU(cudaMemsetAsync(shared_logit_dev, 0, (size_t)n_tokens * sizeof(float), st));      // absent gate: logit 0
     }
     if (!logits_dev) {
-        rc = ensure(&c->logits_dev, &c->logits_cap, (size_t)(ne + 1) * n_tokens);
+        rc = orome_ensure(c, &c->logits_dev, &c->logits_cap, (size_t)(ne + 1) * n_tokens);
         if (rc) return rc;
         logits_dev = c->logits_dev;
     }
@@ -1719,7 +1556,7 @@ extern "C" int orome_cuda_moe_block(orome_cuda_ctx *c, const OromeExpertLayerRef
         if (rc) return rc;
     }
     CU(cudaSetDevice(c->device));
-    return launch_pdl(c, "moe_combine", moe_combine_kernel, dim3((hidden + 255) / 256, (unsigned)n_tokens), dim3(256), static_cast<cudaStream_t>(stream),
+    return orome_launch_pdl(c, "moe_combine", moe_combine_kernel, dim3((hidden + 255) / 256, (unsigned)n_tokens), dim3(256), static_cast<cudaStream_t>(stream),
                       h_mid_dev, n_tokens == 1 ? (int)hidden : ld_mid, (const float *)moe, (int)hidden, shared ? (const float *)sout : (const float *)nullptr,
                       (int)hidden, shared_logit_dev, hidden, out_dev, n_tokens == 1 ? (int)hidden : ldo);
 }
@@ -1745,7 +1582,7 @@ extern "C" int orome_cuda_moe_ffn_shard(orome_cuda_ctx *c, const OromeExpertLaye
     }
     CU(cudaSetDevice(c->device));
     const uint32_t n = (uint32_t)n_tokens * 8;
-    int rc = launch_pdl(c, "moe_localize", moe_localize_kernel, dim3((n + 127) / 128), dim3(128), static_cast<cudaStream_t>(stream), idx_dev, n,
+    int rc = orome_launch_pdl(c, "moe_localize", moe_localize_kernel, dim3((n + 127) / 128), dim3(128), static_cast<cudaStream_t>(stream), idx_dev, n,
                         first_expert, n_local, idx_local_dev);
     if (rc) return rc;
     g_moe_may_skip = true;

@@ -635,3 +635,28 @@ def test_seeded_random_shapes_every_entry_point(env):
             assert err <= tol, (case, kind, fmt, out_dim, in_dim, variant, bits, pad, err)
         finally:
             ctx.set_option(F.OPT_X_BITS, 24)
+
+
+@pytest.mark.parametrize("fmt", [synth.Q8_0, synth.Q4_K, synth.Q5_K, synth.Q6_K])
+@pytest.mark.parametrize("shape", [(1, 256, 4), (129, 512, 16), (257, 768, 17), (1000, 1280, 64), (640, 2048, 129), (513, 768, 256), (384, 1024, 257), (2100, 2304, 300)])
+@pytest.mark.parametrize("split", [0, 1, 3])
+def test_batched_product_over_tile_edges(env, fmt, shape, split):
+    """The two-SM tensor-core form at the edges of its tiles (256 rows, 16..256 vectors, one and several tiles of vectors) and
+    of its shares of the work (tiles cut over clusters, whole tiles, a fixed number of parts).  fp16 operands, fp32 sums."""
+    torch, F, ctx = env
+    out_dim, in_dim, batch = shape
+    data = synth.host_tensor(fmt, out_dim, in_dim, seed=synth.seed_for("pair", fmt, *shape))
+    x = synth.host_x(in_dim, batch, seed=23)
+    ctx.set_option(F.OPT_TC_SPLIT, split)
+    try:
+        got = gpu_matvec(env, fmt, data, out_dim, in_dim, x)
+    finally:
+        ctx.set_option(F.OPT_TC_SPLIT, 0)
+    want = oracle.matvec_f64(fmt, data, out_dim, in_dim, x)
+    # Both operands of a term are rounded by up to 2^-11 (standard deviation of a term's error 4e-4 of the term): over many
+    # outputs that is the relative error of the result, for the four outputs of a single row it is scaled by the ratio of
+    # the terms' norm to the sums', which sums of random sign bring to several.
+    tol = TC_REL_L2_TOL if out_dim >= 64 else 5 * TC_REL_L2_TOL
+    assert got.shape == want.shape and rel_l2(got, want) <= tol
+    rows = np.linalg.norm(got.astype(np.float64) - want, axis=-1) / np.linalg.norm(want, axis=-1)
+    assert rows.max() <= (3 if out_dim >= 64 else 20) * TC_REL_L2_TOL          # no vector of the batch is off by itself
