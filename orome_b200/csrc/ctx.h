@@ -61,6 +61,8 @@ struct orome_cuda_ctx {
     // scratch for the unfused gate/up fallback
     float *gu_dev = nullptr;
     size_t gu_cap = 0;
+    float *moe_dev = nullptr;      // scratch of the grouped expert products
+    size_t moe_cap = 0;
     std::vector<void *> retired;   // scratch buffers that have been outgrown (orome_ensure)
     // scratch of the tensor-core batched form: packed fp16 X and split-K partial sums
     float *tc_xp = nullptr, *tc_part = nullptr;

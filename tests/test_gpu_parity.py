@@ -660,3 +660,57 @@ def test_batched_product_over_tile_edges(env, fmt, shape, split):
     assert got.shape == want.shape and rel_l2(got, want) <= tol
     rows = np.linalg.norm(got.astype(np.float64) - want, axis=-1) / np.linalg.norm(want, axis=-1)
     assert rows.max() <= (3 if out_dim >= 64 else 20) * TC_REL_L2_TOL          # no vector of the batch is off by itself
+
+
+@pytest.mark.parametrize("case", [
+    # T, E, K, H, M, gate format, down format, choice of experts, layout
+    (8, 6, 3, 512, 256, synth.Q4_K, synth.Q5_K, "random", 0),          # the smallest grouped batch
+    (9, 5, 2, 256, 512, synth.Q5_K, synth.Q4_K, "random", 1),
+    (40, 7, 2, 768, 256, synth.Q4_K, synth.Q4_K, "one", 0),             # an expert of 40 tokens, pair blocks of 8
+    (90, 12, 8, 512, 768, synth.Q4_K, synth.Q5_K, "one", 0),            # the same with blocks of 32 (33 and more pairs)
+    (70, 16, 8, 256, 256, synth.Q5_K, synth.Q6_K, "random", 0),         # a down format that is not grouped
+    (8, 1034, 4, 256, 256, synth.Q4_K, synth.Q5_K, "far", 1),           # experts beyond the sorted range
+    (1100, 8, 2, 256, 256, synth.Q4_K, synth.Q4_K, "random", 0),        # more tokens than one pass takes
+])
+def test_moe_ffn_grouped_by_expert(env, case):
+    """Token batches through the grouped expert products.  x and the activations are 24-bit fixed point per 256 elements and
+    the integer sums exact, so fp32 sums over K bound the error: a few 1e-7, and no larger than token by token."""
+    torch, F, ctx = env
+    T, E, K, H, M, gfmt, dfmt, choice, variant = case
+    gate = synth.host_tensor(gfmt, E * M, H, seed=81)
+    up = synth.host_tensor(gfmt, E * M, H, seed=82)
+    down = synth.host_tensor(dfmt, E * H, M, seed=83)
+    sg, sd = synth.tensor_bytes(gfmt, M, H), synth.tensor_bytes(dfmt, H, M)
+    wt = dev_bytes(torch, np.concatenate([gate, up, np.zeros((-(gate.size + up.size)) % 32, np.uint8), down]))
+    x = np.atleast_2d(synth.host_x(H, T, seed=84))
+    rng = np.random.default_rng(85)
+    idx = np.full((T, 8), 0, np.uint32)
+    w = np.zeros((T, 8), np.float32)
+    for t in range(T):
+        idx[t, :K] = rng.permutation(E)[:K]
+        if choice == "one":
+            idx[t, :K][idx[t, :K] == 3] = idx[t, 0]
+            idx[t, 0] = 3
+        if choice == "far":
+            idx[t, :K] = [1024 + t, 1033 - t, 1023, t]
+        w[t, :K] = rng.random(K)
+    w /= w.sum(1, keepdims=True)
+    layer = F.ExpertLayerRef(wt.data_ptr(), F.ExpertProjRef(0, sg, gfmt), F.ExpertProjRef(gate.size, sg, gfmt),
+                             F.ExpertProjRef((gate.size + up.size + 31) // 32 * 32, sd, dfmt))
+    xt, it, wtt = dev_bytes(torch, x), dev_bytes(torch, idx.view(np.int32)), dev_bytes(torch, w)
+    act = torch.full((T, K, M), float("nan"), device="cuda")
+    out = torch.full((T, H), float("nan"), device="cuda")
+    ctx.moe_ffn(layer, variant, xt.data_ptr(), T, H, it.data_ptr(), wtt.data_ptr(), K, H, M, act.data_ptr(), out.data_ptr(), H)
+    alone = torch.full((T, H), float("nan"), device="cuda")
+    pick = list(range(T)) if T <= 16 else sorted(rng.choice(T, 16, replace=False).tolist()) + [T - 1]
+    a1 = torch.empty((K, M), device="cuda")
+    for t in pick:
+        ctx.moe_ffn(layer, variant, xt[t].data_ptr(), 1, H, it[t].data_ptr(), wtt[t].data_ptr(), K, H, M, a1.data_ptr(), alone[t].data_ptr(), H)
+    torch.cuda.synchronize()
+    assert ctx.status() == 0
+    got, single = out.cpu().numpy(), alone.cpu().numpy()
+    assert np.isfinite(got).all()
+    want = np.stack([oracle.moe_ffn_f64(gate, up, down, (gfmt, gfmt, dfmt), (sg, sg, sd), x[t], H, M, idx[t, :K], w[t, :K], layout=variant) for t in pick])
+    err, err1 = rel_l2(got[pick], want), rel_l2(single[pick], want)
+    print(f"{case}: grouped {err:.2e} token by token {err1:.2e}")
+    assert err <= 1e-6
