@@ -6,12 +6,13 @@
 
 namespace orome {
 
-// One thread per 32-weight group: out[(r - row0) * in_dim + 32*b .. +32].
+// One thread per 32-weight group: out[(r - row0) * in_dim + 32*b .. +32].  The unquantized formats.
 // Device counterpart of format_decode_row_f32 (format.m:176-218).
 template <int FMT>
 __global__ void dequant_rows_kernel(const uint8_t *__restrict__ data, size_t row_bytes, uint32_t row0, uint32_t nrows,
                                     uint32_t in_dim, int layout, float *__restrict__ out)
 {
+    static_assert(FMT >= FMT_F16, "quantized rows: dequant_flat_kernel");
     uint32_t groups = in_dim / 32;
     size_t gid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= (size_t)nrows * groups) return;
@@ -21,6 +22,98 @@ __global__ void dequant_rows_kernel(const uint8_t *__restrict__ data, size_t row
     float4 *o = reinterpret_cast<float4 *>(out + (size_t)r * in_dim + (size_t)b * 32);
 #pragma unroll
     for (int j = 0; j < 8; ++j) o[j] = make_float4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+}
+
+// Eight bytes from a 2-byte aligned address, as two words.  Stays inside [p - 2, p + 8).
+__device__ __forceinline__ uint2 ld8_a2(const uint8_t *p)
+{
+    const bool odd = (reinterpret_cast<uintptr_t>(p) & 2u) != 0;
+    const uint32_t *q = reinterpret_cast<const uint32_t *>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)3);
+    const uint32_t a = __ldg(q), b = __ldg(q + 1), c = odd ? (uint32_t)__ldg(reinterpret_cast<const unsigned short *>(p + 6)) : 0u, sh = odd ? 16u : 0u;
+    return make_uint2(__funnelshift_r(a, b, sh), __funnelshift_r(b, c, sh));
+}
+
+// Rows of a quantized tensor lie one behind the other without gaps, so a range of rows is one run of 8-weight pieces: thread i
+// decodes pieces i, i + 32, .. of its warp's 1024 weights and stores 32 bytes a piece, so that a warp's stores are whole lines
+// and its loads fall into a few (a thread per 32-weight block, loading bytes and storing 128 bytes apart, ran at a third of the
+// memory rate: 5120 x 4096 Q6_K 47 us).  Bit-exact like decode32: the same rounded operations on the same integers.
+constexpr uint32_t DQ_PIECES = 4;            // pieces a thread has in flight
+template <int FMT>
+__global__ void __launch_bounds__(256)
+dequant_flat_kernel(const uint8_t *__restrict__ blocks, uint64_t pieces, int layout, float *__restrict__ out)
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t base = ((uint64_t)blockIdx.x * 8u + (threadIdx.x >> 5)) * (32u * DQ_PIECES) + lane;
+    uint2 q[DQ_PIECES], h[DQ_PIECES];
+    uint4 hd[DQ_PIECES];
+    uint32_t d[DQ_PIECES];
+    int sc[DQ_PIECES];
+#pragma unroll
+    for (uint32_t k = 0; k < DQ_PIECES; ++k) {
+        const uint64_t i = base + 32u * k;
+        if (i >= pieces) continue;
+        if constexpr (FMT == FMT_Q8_0) {
+            const uint8_t *blk = blocks + (i >> 2) * 34u;
+            d[k] = __ldg(reinterpret_cast<const unsigned short *>(blk));
+            q[k] = ld8_a2(blk + 2 + 8u * (i & 3u));
+        } else if constexpr (FMT == FMT_Q6_K) {
+            const uint8_t *sb = blocks + (i >> 5) * 210u;
+            const uint32_t p = (uint32_t)i & 31u, half = p >> 4, j = (p >> 2) & 3u, l = 8u * (p & 3u);
+            q[k] = ld8_a2(sb + 64u * half + 32u * (j & 1u) + l);
+            h[k] = ld8_a2(sb + 128u + 32u * half + l);
+            sc[k] = (int)(signed char)__ldg(sb + 192u + 8u * half + 2u * j + (l >> 4));
+            d[k] = __ldg(reinterpret_cast<const unsigned short *>(sb + 208));
+        } else {
+            constexpr uint32_t UNIT = FMT == FMT_Q4_K ? 144u : 176u, QOFF = FMT == FMT_Q4_K ? 16u : 48u;
+            const uint8_t *sb = blocks + (i >> 5) * UNIT;
+            const uint32_t p = (uint32_t)i & 31u;
+            hd[k] = __ldg(reinterpret_cast<const uint4 *>(sb));
+            q[k] = __ldg(reinterpret_cast<const uint2 *>(sb + QOFF + 32u * (p >> 3) + 8u * (p & 3u)));
+            if constexpr (FMT == FMT_Q5_K) h[k] = __ldg(reinterpret_cast<const uint2 *>(sb + 16u + 8u * (p & 3u)));
+        }
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");      // the packed rows are constant; what is overwritten may still be read
+#pragma unroll
+    for (uint32_t k = 0; k < DQ_PIECES; ++k) {
+        const uint64_t i = base + 32u * k;
+        if (i >= pieces) continue;
+        const uint32_t p = (uint32_t)i & 31u;
+        float w[8];
+        if constexpr (FMT == FMT_Q8_0) {
+            const float dd = half_bits_to_float(d[k]);
+#pragma unroll
+            for (int b = 0; b < 8; ++b) w[b] = __fmul_rn(dd, (float)(signed char)((b < 4 ? q[k].x : q[k].y) >> (8 * (b & 3))));
+        } else if constexpr (FMT == FMT_Q6_K) {
+            const uint32_t j = (p >> 2) & 3u;
+            const float a = __fmul_rn(half_bits_to_float(d[k]), (float)sc[k]);
+            const uint32_t lo0 = (q[k].x >> (4u * (j >> 1))) & 0x0F0F0F0Fu, lo1 = (q[k].y >> (4u * (j >> 1))) & 0x0F0F0F0Fu;
+            const uint32_t v0 = lo0 | (((h[k].x >> (2u * j)) & 0x03030303u) << 4), v1 = lo1 | (((h[k].y >> (2u * j)) & 0x03030303u) << 4);
+#pragma unroll
+            for (int b = 0; b < 8; ++b) w[b] = __fmul_rn(a, (float)((int)(((b < 4 ? v0 : v1) >> (8 * (b & 3))) & 255u) - 32));
+        } else {
+            const uint32_t sub = p >> 2, shift = 4u * (sub & 1u), w0 = hd[k].y, w1 = hd[k].z, w2 = hd[k].w;
+            auto byte = [](uint32_t v, uint32_t n) { return (v >> (8u * n)) & 255u; };
+            uint32_t s, m;                       // kq_scale_min on words: w0 = bytes 0-3, w1 = 4-7, w2 = 8-11
+            if (sub < 4) { s = byte(w0, sub) & 63u; m = byte(w1, sub) & 63u; }
+            else if (layout == LAYOUT_A) {
+                const uint32_t u = (sub - 4) >> 1, hi = sub & 1u, sp = byte(w2, u), mp = byte(w2, 2 + u);
+                s = (hi ? (sp >> 4) : (sp & 15u)) | ((byte(w0, 2 * u + hi) >> 6) << 4);
+                m = (hi ? (mp >> 4) : (mp & 15u)) | ((byte(w1, 2 * u + hi) >> 6) << 4);
+            } else {
+                s = (byte(w2, sub - 4) & 15u) | ((byte(w0, sub - 4) >> 6) << 4);
+                m = (byte(w2, sub - 4) >> 4) | ((byte(w1, sub - 4) >> 6) << 4);
+            }
+            const float a = __fmul_rn(half_bits_to_float(hd[k].x & 0xffffu), (float)s), mm = __fmul_rn(half_bits_to_float(hd[k].x >> 16), (float)m);
+            uint32_t v0 = (q[k].x >> shift) & 0x0F0F0F0Fu, v1 = (q[k].y >> shift) & 0x0F0F0F0Fu;
+            if constexpr (FMT == FMT_Q5_K) { v0 |= ((h[k].x >> sub) & 0x01010101u) << 4; v1 |= ((h[k].y >> sub) & 0x01010101u) << 4; }
+#pragma unroll
+            for (int b = 0; b < 8; ++b) w[b] = __fsub_rn(__fmul_rn(a, (float)(((b < 4 ? v0 : v1) >> (8 * (b & 3))) & 255u)), mm);
+        }
+        float4 *o = reinterpret_cast<float4 *>(out + i * 8u);
+        o[0] = make_float4(w[0], w[1], w[2], w[3]);
+        o[1] = make_float4(w[4], w[5], w[6], w[7]);
+    }
 }
 
 // Tail of an unquantized row whose length is not a multiple of 32 (F32/F16/BF16 only).

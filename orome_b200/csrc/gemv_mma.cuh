@@ -56,7 +56,7 @@ struct MmaArgs {
     uint32_t in_dim, row_bytes;
     uint32_t units;            // superblocks per row
     uint32_t nwarps;           // consumer warps of one group: a group covers the kc superblocks of a stage
-    uint32_t ngroups;          // groups; stage i (counted over row tiles and their chunks) belongs to group i % ngroups (nstages is a multiple)
+    uint32_t ngroups;          // groups; stage i (counted over row tiles and their chunks) belongs to group i % ngroups (nstages is a multiple, or odd with two groups)
     uint32_t kc;               // superblocks per stage
     uint32_t nchunks;          // stages per row tile = ceil(units / kc)
     uint32_t dbg_tile;         // diagnostics build: first row tile whose per-warp timeline is recorded
@@ -811,6 +811,7 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
 
     const uint32_t stages_s = smem_u32(stages);
     const uint32_t group = warp / NW, wig = warp - group * NW;
+    const bool odd_ring = NG == 2 && (a.nstages & 1u);
     uint32_t cur = lo, s = 0, parity = 0, i = 0, turn = 0, tile_no = 0;
     int seg = 0;
     MmaTile t;
@@ -826,6 +827,12 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
                 continue;
             }
             if (c == 0) MMA_TILE_STAMP(a, tile_no, warp, 0);
+            // Two groups on an odd ring: a slot's previous use is the other group's.  Once that has been consumed (the use
+            // before it was this group's own, so the parity is unambiguous) the slot's full barrier is in this use's phase.
+            if (odd_ring && !s_abort && !mbar_wait_bounded(smem_u32(empty + s), parity ^ 1u)) {
+                s_abort = 1;
+                atomicExch(a.status, 1);
+            }
             if (!s_abort && !mbar_wait_bounded(smem_u32(full + s), parity)) {
                 s_abort = 1;
                 atomicExch(a.status, 1);

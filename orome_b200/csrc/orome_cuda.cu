@@ -570,19 +570,6 @@ static int plan_mma(orome_cuda_ctx *c, int fmt, uint32_t in_dim, uint32_t total_
     a.units = units_row * std::max(1u, nvec);
     a.row_bytes = units_row * unit;
     a.total_rows = total_rows;
-    // a stage of about stage_kb (default 40) KiB: 16 rows (x2 in the fused form) of kc superblocks
-    const uint32_t want = (c->stage_kb ? (uint32_t)c->stage_kb : 40u) * 1024u;
-    const uint32_t kc_max = std::max(1u, std::min(units_row, want / (MMA_TILE_ROWS * unit * (swiglu ? 2u : 1u))));
-    if (nvec > 0) {
-        if (units_row > kc_max) return fail(OROME_ENOTSUP, "mma plan: combine form with rows of %u superblocks", units_row);
-        a.nchunks = nvec;
-        a.kc = units_row;
-    } else {
-        a.nchunks = (a.units + kc_max - 1) / kc_max;
-        a.kc = (a.units + a.nchunks - 1) / a.nchunks;
-    }
-    const uint32_t rounds = (a.kc + MMA_MAX_WARPS - 1) / MMA_MAX_WARPS;
-    a.nwarps = (a.kc + rounds - 1) / rounds;
     p.grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)c->sm_count, (total_rows + MMA_TILE_ROWS - 1) / MMA_TILE_ROWS));
     if (grid_cap) {
         const uint32_t tiles = (total_rows + MMA_TILE_ROWS - 1) / MMA_TILE_ROWS, cap = std::max(1u, std::min(grid_cap, tiles));
@@ -590,38 +577,65 @@ static int plan_mma(orome_cuda_ctx *c, int fmt, uint32_t in_dim, uint32_t total_
         p.grid = (int)((tiles + per - 1) / per);
     }
     const uint32_t share = (total_rows + p.grid - 1) / p.grid;
-    // stages (row tiles x chunks) go round the groups: as many groups as the warp budget and the CTA's stage count allow
-    const uint32_t cta_stages = (share + MMA_TILE_ROWS - 1) / MMA_TILE_ROWS * a.nchunks;
-    a.ngroups = std::max(1u, std::min(std::min<uint32_t>(MMA_MAX_GROUPS, MMA_MAX_CONSUMER_WARPS / a.nwarps), cta_stages));
-    // box width in superblocks: the smallest kb >= kc with kb = 2 (mod 4), which makes the row pitch 32 or 96 (mod 128)
-    const uint32_t kb = a.kc + ((6 - a.kc % 4) % 4);
-    a.pitch = kb * unit;
-    if (fmt == FMT_Q6_K) {
-        // rows arrive by their own copies, widened to 16-byte boundaries (up to 15 bytes before and after the chunk)
-        a.pitch = (a.kc * unit + 30 + 15) / 16 * 16;
-        while (a.pitch % 128 != 16) a.pitch += 16;      // the quads of the eight rows of a load then read eight different four-bank groups
-    }
-    a.box_bytes = MMA_TILE_ROWS * a.pitch;
-    a.half_stride = MMA_TILE_ROWS * a.pitch;
-    a.stage_stride = a.half_stride * (swiglu ? 2 : 1);
-    a.red_base = 2 * 8 * PIPE_MAX_STAGES;
-    a.red_rows = std::max<uint32_t>(MMA_TILE_ROWS, std::min<uint32_t>((share + MMA_TILE_ROWS - 1) / MMA_TILE_ROWS * MMA_TILE_ROWS, 128u));
-    const size_t red_bytes = (size_t)2 * a.red_rows * a.nwarps * a.ngroups * (swiglu || two ? 2 : 1) * sizeof(float);
-    a.xs_base = (uint32_t)((a.red_base + red_bytes + 127) / 128 * 128);
     const bool fused = c->fuse_norm_w || c->fuse_res_in;      // fused neighbours: four byte planes (launch_mma)
-    const size_t xq_sb = !two ? (fused ? MMA_XQ_SB4 : MMA_XQ_SB) : (c->x_bits == 24 ? mma_xq_sb<3, 2>() : mma_xq_sb<2, 2>());
-    const size_t xq_bytes = (size_t)a.units * xq_sb + (size_t)a.units * 8 * (two ? 2 : 1) + 768;   // planes and sums, two scales per superblock and vector, a block of zeros
-    a.stage_base = (uint32_t)((a.xs_base + xq_bytes + 127) / 128 * 128);
-    const size_t budget = std::min<size_t>(228 * 1024 - 1024 - 256, (size_t)c->smem_optin - 256);
-    if (budget < a.stage_base + a.stage_stride) return fail(OROME_ENOTSUP, "mma plan: in_dim %u does not fit shared memory", in_dim);
-    const uint32_t tiles = ((share + MMA_TILE_ROWS - 1) / MMA_TILE_ROWS + 1) * a.nchunks;
-    a.nstages = (uint32_t)std::min<size_t>(std::min<size_t>(PIPE_MAX_STAGES, tiles), (budget - a.stage_base) / a.stage_stride);
-    // A whole number of ring slots per group, so that every use of a slot belongs to the same group.  A wait by parity tells
-    // only the last two phases apart: a group waiting for use k of a slot whose use k - 1 is another group's, and has not
-    // landed yet, would take phase k - 2 for phase k and read the stage too early.
-    a.ngroups = std::min(a.ngroups, a.nstages);
-    a.nstages -= a.nstages % a.ngroups;
-    p.threads = (int)(a.nwarps * a.ngroups + (fmt == FMT_Q6_K ? 2 : 1)) * 32;
+    // A stage of `want` bytes: 16 rows (x2 in the fused form) of kc superblocks.  40 KiB, or less where that leaves a consumer
+    // group fewer than two ring slots: with one, a group waits out every copy into the slot it has just read.  27B shapes, one
+    // slot a group / the largest stage that leaves two: gate/up 32.6 / 23.4 us, fused down 36.5 / 28.6, lm_head 155 / 131.
+    auto lay_out = [&](uint32_t want, bool odd) -> int {
+        const uint32_t kc_max = std::max(1u, std::min(units_row, want / (MMA_TILE_ROWS * unit * (swiglu ? 2u : 1u))));
+        if (nvec > 0) {
+            if (units_row > kc_max) return fail(OROME_ENOTSUP, "mma plan: combine form with rows of %u superblocks", units_row);
+            a.nchunks = nvec;
+            a.kc = units_row;
+        } else {
+            a.nchunks = (a.units + kc_max - 1) / kc_max;
+            a.kc = (a.units + a.nchunks - 1) / a.nchunks;
+        }
+        const uint32_t rounds = (a.kc + MMA_MAX_WARPS - 1) / MMA_MAX_WARPS;
+        a.nwarps = (a.kc + rounds - 1) / rounds;
+        // stages (row tiles x chunks) go round the groups: as many groups as the warp budget and the CTA's stage count allow
+        const uint32_t cta_stages = (share + MMA_TILE_ROWS - 1) / MMA_TILE_ROWS * a.nchunks;
+        a.ngroups = std::max(1u, std::min(std::min<uint32_t>(MMA_MAX_GROUPS, MMA_MAX_CONSUMER_WARPS / a.nwarps), cta_stages));
+        // box width in superblocks: the smallest kb >= kc with kb = 2 (mod 4), which makes the row pitch 32 or 96 (mod 128)
+        const uint32_t kb = a.kc + ((6 - a.kc % 4) % 4);
+        a.pitch = kb * unit;
+        if (fmt == FMT_Q6_K) {
+            // rows arrive by their own copies, widened to 16-byte boundaries (up to 15 bytes before and after the chunk)
+            a.pitch = (a.kc * unit + 30 + 15) / 16 * 16;
+            while (a.pitch % 128 != 16) a.pitch += 16;      // the quads of the eight rows of a load then read eight different four-bank groups
+        }
+        a.box_bytes = MMA_TILE_ROWS * a.pitch;
+        a.half_stride = MMA_TILE_ROWS * a.pitch;
+        a.stage_stride = a.half_stride * (swiglu ? 2 : 1);
+        a.red_base = 2 * 8 * PIPE_MAX_STAGES;
+        a.red_rows = std::max<uint32_t>(MMA_TILE_ROWS, std::min<uint32_t>((share + MMA_TILE_ROWS - 1) / MMA_TILE_ROWS * MMA_TILE_ROWS, 128u));
+        const size_t red_bytes = (size_t)2 * a.red_rows * a.nwarps * a.ngroups * (swiglu || two ? 2 : 1) * sizeof(float);
+        a.xs_base = (uint32_t)((a.red_base + red_bytes + 127) / 128 * 128);
+        const size_t xq_sb = !two ? (fused ? MMA_XQ_SB4 : MMA_XQ_SB) : (c->x_bits == 24 ? mma_xq_sb<3, 2>() : mma_xq_sb<2, 2>());
+        const size_t xq_bytes = (size_t)a.units * xq_sb + (size_t)a.units * 8 * (two ? 2 : 1) + 768;   // planes and sums, two scales per superblock and vector, a block of zeros
+        a.stage_base = (uint32_t)((a.xs_base + xq_bytes + 127) / 128 * 128);
+        const size_t budget = std::min<size_t>(228 * 1024 - 1024 - 256, (size_t)c->smem_optin - 256);
+        if (budget < a.stage_base + a.stage_stride) return fail(OROME_ENOTSUP, "mma plan: in_dim %u does not fit shared memory", in_dim);
+        const uint32_t tiles = ((share + MMA_TILE_ROWS - 1) / MMA_TILE_ROWS + 1) * a.nchunks;
+        a.nstages = (uint32_t)std::min<size_t>(std::min<size_t>(PIPE_MAX_STAGES, tiles), (budget - a.stage_base) / a.stage_stride);
+        // A whole number of ring slots per group, so that every use of a slot belongs to the same group.  A wait by parity tells
+        // only the last two phases apart: a group waiting for use k of a slot whose use k - 1 is another group's, and has not
+        // landed yet, would take phase k - 2 for phase k and read the stage too early.
+        a.ngroups = std::min(a.ngroups, a.nstages);
+        // (odd: three or five slots for two groups, where the kernel makes a group wait for the slot's other user first.)
+        if (!(odd && a.ngroups == 2 && a.nstages >= 3)) a.nstages -= a.nstages % a.ngroups;
+        p.threads = (int)(a.nwarps * a.ngroups + (fmt == FMT_Q6_K ? 2 : 1)) * 32;
+        return a.nstages >= std::min(2 * a.ngroups, cta_stages) ? OROME_OK : 1;      // 1: a ring, but a shallow one
+    };
+    int fit = OROME_ENOTSUP;
+    if (c->stage_kb || nvec > 0) fit = lay_out((c->stage_kb ? (uint32_t)c->stage_kb : 40u) * 1024u, true);
+    else
+        for (uint32_t kb = 40; kb >= 16 && fit != OROME_OK; kb -= 4) {
+            fit = lay_out(kb * 1024u, false);
+            if (fit == OROME_OK && kb < 40 && a.nwarps * a.ngroups < 12) fit = 1;      // narrow stages that leave warps idle cost more (7-superblock rows: 3 %)
+        }
+    if (fit == 1 && !c->stage_kb && nvec == 0) fit = lay_out(40u * 1024u, true);      // shallow at every size: the largest stage
+    if (fit != OROME_OK && fit != 1) return fit;
     p.smem = a.stage_base + (size_t)a.stage_stride * a.nstages;
 #ifdef OROME_MMA_TILE_TRACE
     a.dbg_tile = OROME_MMA_TILE_TRACE;      // diagnostics build: first row tile whose per-warp timeline is recorded
@@ -1235,14 +1249,23 @@ extern "C" int orome_cuda_dequant_rows(orome_cuda_ctx *c, const OromeTensorRef *
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int fmt = (int)ref->format, layout = (int)ref->variant;
     size_t rb = row_bytes_of(fmt, ref->in_dim);
+    if (fmt <= FMT_Q8_0) {
+        const uint64_t pieces = (uint64_t)nrows * (ref->in_dim / 8);
+        const unsigned grid = (unsigned)((pieces + 256 * DQ_PIECES - 1) / (256 * DQ_PIECES));
+        const uint8_t *first = data + rb * row0;
+#define DQ(F) return orome_launch_pdl(c, "dequant_rows", dequant_flat_kernel<F>, dim3(grid), dim3(256), st, first, pieces, layout, out_dev)
+        switch (fmt) {
+        case FMT_Q4_K: DQ(FMT_Q4_K);
+        case FMT_Q5_K: DQ(FMT_Q5_K);
+        case FMT_Q6_K: DQ(FMT_Q6_K);
+        case FMT_Q8_0: DQ(FMT_Q8_0);
+        }
+#undef DQ
+    }
     size_t groups = (size_t)nrows * (ref->in_dim / 32);
     unsigned grid = (unsigned)((groups + 127) / 128);
 #define DQ(F) dequant_rows_kernel<F><<<grid, 128, 0, st>>>(data, rb, row0, nrows, ref->in_dim, layout, out_dev)
     switch (fmt) {
-    case FMT_Q4_K: DQ(FMT_Q4_K); break;
-    case FMT_Q5_K: DQ(FMT_Q5_K); break;
-    case FMT_Q6_K: DQ(FMT_Q6_K); break;
-    case FMT_Q8_0: DQ(FMT_Q8_0); break;
     case FMT_F16: DQ(FMT_F16); break;
     case FMT_BF16: DQ(FMT_BF16); break;
     case FMT_F32: DQ(FMT_F32); break;

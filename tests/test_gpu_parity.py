@@ -714,3 +714,25 @@ def test_moe_ffn_grouped_by_expert(env, case):
     err, err1 = rel_l2(got[pick], want), rel_l2(single[pick], want)
     print(f"{case}: grouped {err:.2e} token by token {err1:.2e}")
     assert err <= 1e-6
+
+
+@pytest.mark.parametrize("fmt", QUANT)
+@pytest.mark.parametrize("variant", [0, 1])
+@pytest.mark.parametrize("rows,cols,row0,n", [(1, 256, 0, 1), (9, 768, 3, 5), (7, 1280, 6, 1), (33, 1024, 0, 33), (5, 96, 1, 4), (130, 2560, 1, 129)])
+def test_dequant_rows_in_the_middle_of_a_tensor(env, fmt, variant, rows, cols, row0, n):
+    """Row ranges whose pieces do not fill a warp's share, that start and end anywhere (2-byte aligned Q6_K and Q8_0 rows, the
+    tensor's last row), at every residue of the block size: bit for bit, and nothing beside the range written."""
+    torch, F, ctx = env
+    if cols % synth.BLOCK_ELEMS[fmt]:
+        pytest.skip("not a whole number of blocks")
+    if variant == 1 and fmt in (synth.Q8_0, synth.Q6_K):
+        pytest.skip("one scale layout")
+    data = synth.host_tensor(fmt, rows, cols, seed=synth.seed_for("dq", fmt, rows, cols))
+    wt = dev_bytes(torch, data)
+    out = torch.full((n + 2, cols), float("nan"), device="cuda")
+    ctx.dequant_rows(F.tensor_ref(wt.data_ptr(), 0, fmt, rows, cols, variant), row0, n, out[1].data_ptr())
+    torch.cuda.synchronize()
+    got = out.cpu().numpy()
+    want = oracle.decode_rows(fmt, data, rows, cols, layout=variant)[row0:row0 + n]
+    assert np.array_equal(got[1:n + 1].view(np.uint32), want.view(np.uint32))
+    assert np.isnan(got[0]).all() and np.isnan(got[n + 1]).all()
