@@ -427,7 +427,8 @@ __device__ __forceinline__ uint32_t plane_word(uint32_t u0, uint32_t u1, uint32_
 template <int NP, bool Q6, int NTOK = 1, bool NORM = false>
 __device__ __forceinline__ bool quantize_x_mma(const float *__restrict__ x, uint32_t units, uint8_t *xq, uint32_t warp, uint32_t lane,
                                                uint32_t nwarps, const uint2 *slots = nullptr, unsigned int tag = 0, uint32_t b_tok = 0,
-                                               const uint16_t *norm_w = nullptr, const float *norm_parts = nullptr, float norm_eps = 0.0f)
+                                               const uint16_t *norm_w = nullptr, const float *norm_parts = nullptr, float norm_eps = 0.0f,
+                                               float *s_share = nullptr)
 {
     static_assert(NTOK == 1 || !Q6, "two vectors at once: Q4_K / Q5_K only");
     constexpr uint32_t XQSB = mma_xq_sb<NP, NTOK>(), JS = mma_xq_js<NP, NTOK>(), SUMS = mma_xq_sums<NP, NTOK>();
@@ -438,12 +439,9 @@ __device__ __forceinline__ bool quantize_x_mma(const float *__restrict__ x, uint
     constexpr float QMAX = (float)QMAXI;
     constexpr int XB = 4;
     float *xs = reinterpret_cast<float *>(xq + (size_t)units * XQSB), *sxs = xs + units * NTOK;
-    constexpr int NPV = PIPE_SUM_SQ_PARTS / 32;
-    float pv[NORM ? NPV : 1], rms = 0.0f;
-    if constexpr (NORM) {
-#pragma unroll
-        for (int i = 0; i < NPV; ++i) pv[i] = __ldcg(norm_parts + 32 * i + lane);
-    }
+    const float share = NORM ? norm_share(norm_parts, warp * 32u + lane, nwarps * 32u) : 0.0f;
+    float rms = 0.0f;
+    bool have_rms = !NORM;
     for (uint32_t ub = warp; ub < units; ub += nwarps * XB) {
         float4 v0[XB], v1[XB];
 #pragma unroll
@@ -460,12 +458,7 @@ __device__ __forceinline__ bool quantize_x_mma(const float *__restrict__ x, uint
             }
         }
         if constexpr (NORM) {
-            if (ub == warp) {
-                float t = 0.0f;
-#pragma unroll
-                for (int i = 0; i < NPV; ++i) t += pv[i];
-                rms = rsqrtf(warp_sum(t) / (float)(units * 256u) + norm_eps);
-            }
+            if (!have_rms) { rms = norm_rms(share, s_share, warp, lane, nwarps, units * 256u, norm_eps); have_rms = true; }
 #pragma unroll
             for (int b = 0; b < XB; ++b) {
                 const uint32_t u = ub + b * nwarps;
@@ -537,6 +530,7 @@ __device__ __forceinline__ bool quantize_x_mma(const float *__restrict__ x, uint
             if (lane == 0) { xs[u * NTOK + (NTOK == 1 ? 0u : b_tok)] = amax[b] / QMAX; sxs[u * NTOK + (NTOK == 1 ? 0u : b_tok)] = smax[b] / QMAX; }
         }
     }
+    if constexpr (NORM) { if (!have_rms) norm_rms(share, s_share, warp, lane, nwarps, units * 256u, norm_eps); }      // a warp without a superblock takes part in the sum
     return ok;
 }
 
@@ -725,8 +719,9 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
         const uint2 *slots = EXT ? a.x_ll : nullptr;
         const unsigned int want = EXT && a.x_ll ? *reinterpret_cast<const volatile unsigned int *>(a.wait_gen) : 0u;
         bool x_ok;
+        __shared__ float s_share[MMA_MAX_CONSUMER_WARPS];
         if (EXT && a.norm_w)
-            x_ok = quantize_x_mma<NP, Q6, NTOK, true>(a.x, U, xq, warp, lane, CW, nullptr, 0u, 0u, a.norm_w, a.norm_parts, a.norm_eps);
+            x_ok = quantize_x_mma<NP, Q6, NTOK, true>(a.x, U, xq, warp, lane, CW, nullptr, 0u, 0u, a.norm_w, a.norm_parts, a.norm_eps, s_share);
         else
             x_ok = quantize_x_mma<NP, Q6, NTOK>(a.x + (MOE != 0 ? (size_t)blockIdx.y * a.tok_x_stride : 0), U, xq, warp, lane, CW, slots, want, 0u);
         if (!x_ok) {

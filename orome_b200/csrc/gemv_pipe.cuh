@@ -389,13 +389,34 @@ __device__ __forceinline__ void quantize_piece(const float4 v, uint32_t f, bool 
     }
 }
 
-template <int NP, int G, bool SUMS>
+// This thread's share of a partials array: its loads are on their way when this returns, norm_rms() uses them.
+__device__ __forceinline__ float norm_share(const float *norm_parts, uint32_t tid, uint32_t nthreads)
+{
+    float t = 0.0f;
+    for (uint32_t i = tid; i < (uint32_t)PIPE_SUM_SQ_PARTS; i += nthreads) t += __ldcg(norm_parts + i);
+    return t;
+}
+// 1 / rms from the shares, added up over the consumer threads; every one of them calls this once.  (Each warp adding up all
+// 512 entries for itself cost 16 more loads a lane, 4.5 MB of L2 reads of the same 2 KiB per launch, ahead of the loads of x.)
+__device__ __forceinline__ float norm_rms(float share, float *s_share, uint32_t warp, uint32_t lane, uint32_t nwarps, uint32_t in_dim, float eps)
+{
+    share = warp_sum(share);
+    if (lane == 0) s_share[warp] = share;
+    named_bar_sync(PIPE_BAR_CONSUMERS, (int)(nwarps * 32u));
+    float t = 0.0f;
+    for (uint32_t w = 0; w < nwarps; ++w) t += s_share[w];
+    return rsqrtf(t / (float)in_dim + eps);
+}
+
+template <int NP, int G, bool SUMS, bool NORM = false>
 __device__ __forceinline__ bool quantize_x_to_smem(const float *__restrict__ x, uint32_t in_dim, uint32_t nvec, uint32_t x_stride,
                                                    uint8_t *xq0, uint32_t vec_bytes, uint32_t tid, uint32_t nthreads,
                                                    const uint2 *slots = nullptr, unsigned int tag = 0,
                                                    long long limit = PIPE_WAIT_CYCLES, const int *status = nullptr, uint32_t rot = 0,
-                                                   const uint16_t *norm_w = nullptr, float rms = 1.0f, uint32_t issued_bar = 0)
+                                                   uint32_t issued_bar = 0, const uint16_t *norm_w = nullptr, const float *norm_parts = nullptr,
+                                                   float norm_eps = 0.0f, float *s_share = nullptr)
 {
+    // NORM: x is RMS-normalised on the way.  The partial sums, x and the norm weights are all requested before any is used.
     // issued_bar: shared address of an mbarrier on which every warp arrives once the loads of its first batch are on
     // their way (0: none).  The weight producer holds its copies back until then, see the kernel.
     // rot (single vector only; a multiple of 32 four-float pieces): this CTA walks the vector starting rot pieces in and
@@ -409,8 +430,12 @@ __device__ __forceinline__ bool quantize_x_to_smem(const float *__restrict__ x, 
         if (lane == 0) mbar_arrive(issued_bar);
         issued_bar = 0;
     }
+    const float share = NORM ? norm_share(norm_parts, tid, nthreads) : 0.0f;
+    float rms = 0.0f;
+    bool have_rms = !NORM;
     for (uint32_t base = tid - lane; base < n4_all; base += nthreads * BATCH) {
         float4 v[BATCH];
+        uint2 nw[NORM ? BATCH : 1];
 #pragma unroll
         for (int b = 0; b < BATCH; ++b) {
             const uint32_t fa = base + b * nthreads + lane;
@@ -419,17 +444,21 @@ __device__ __forceinline__ bool quantize_x_to_smem(const float *__restrict__ x, 
             if (nvec == 1) { fl += rot; if (fl >= n4) fl -= n4; }
             if (slots) v[b] = fa < n4_all ? ld_gathered4(slots + 4 * (size_t)fl, tag, &ok, limit, status) : make_float4(0.f, 0.f, 0.f, 0.f);
             else v[b] = fa < n4_all ? __ldcg(reinterpret_cast<const float4 *>(x + (size_t)vec * x_stride) + fl) : make_float4(0.f, 0.f, 0.f, 0.f);
-            if (norm_w && fa < n4_all) {      // the RMS-norm scale and the bf16 norm weights, applied in the reference's order
-                const uint2 w = __ldg(reinterpret_cast<const uint2 *>(norm_w) + fl);
-                v[b].x = v[b].x * rms * __uint_as_float(w.x << 16);
-                v[b].y = v[b].y * rms * __uint_as_float(w.x & 0xffff0000u);
-                v[b].z = v[b].z * rms * __uint_as_float(w.y << 16);
-                v[b].w = v[b].w * rms * __uint_as_float(w.y & 0xffff0000u);
-            }
+            if constexpr (NORM) nw[b] = fa < n4_all ? __ldg(reinterpret_cast<const uint2 *>(norm_w) + fl) : make_uint2(0u, 0u);
         }
         if (issued_bar && base == tid - lane) {
             __syncwarp();
             if (lane == 0) mbar_arrive(issued_bar);
+        }
+        if constexpr (NORM) {                 // the scale and the bf16 norm weights, applied in the reference's order
+            if (!have_rms) { rms = norm_rms(share, s_share, tid >> 5, lane, nthreads / 32u, in_dim, norm_eps); have_rms = true; }
+#pragma unroll
+            for (int b = 0; b < BATCH; ++b) {
+                v[b].x = v[b].x * rms * __uint_as_float(nw[b].x << 16);
+                v[b].y = v[b].y * rms * __uint_as_float(nw[b].x & 0xffff0000u);
+                v[b].z = v[b].z * rms * __uint_as_float(nw[b].y << 16);
+                v[b].w = v[b].w * rms * __uint_as_float(nw[b].y & 0xffff0000u);
+            }
         }
 #pragma unroll
         for (int b = 0; b < BATCH; ++b) {
@@ -446,6 +475,7 @@ __device__ __forceinline__ bool quantize_x_to_smem(const float *__restrict__ x, 
         __syncwarp();
         if (lane == 0) mbar_arrive(issued_bar);
     }
+    if constexpr (NORM) { if (!have_rms) norm_rms(share, s_share, tid >> 5, lane, nthreads / 32u, in_dim, norm_eps); }   // and takes part in the sum
     return ok;
 }
 
@@ -902,17 +932,21 @@ gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
         // a gathered x: every element is polled for the generation this rank gave its own slice (visible after the wait above)
         const uint2 *slots = EXT ? a.x_ll : nullptr;
         const unsigned int want = EXT && a.x_ll ? *reinterpret_cast<const volatile unsigned int *>(a.wait_gen) : 0u;
-        const uint16_t *norm_w = EXT ? a.norm_w : nullptr;
-        float rms = 1.0f;
-        if (norm_w) {                         // every warp adds up the partial sums of squares for itself
-            float t = 0.0f;
-            for (uint32_t i = lane; i < (uint32_t)PIPE_SUM_SQ_PARTS; i += 32) t += __ldcg(a.norm_parts + i);
-            rms = rsqrtf(warp_sum(t) / (float)a.in_dim + a.norm_eps);
-        }
-        if (!quantize_x_to_smem<NP, SlotT::GROUP, SlotT::SUMS>(a.x + (EXT ? (size_t)blockIdx.y * a.tok_x_stride : 0), a.in_dim, COMBINE ? (uint32_t)a.nseg : 1u, a.x_stride, xq, a.xq_vec_bytes, tid, C,
-                                                               slots, want, a.wait_cycles, a.status,
-                                                               COMBINE ? 0u : (uint32_t)((uint64_t)blockIdx.x * (a.in_dim / 4) / gridDim.x) & ~31u,
-                                                               norm_w, rms, smem_u32(&s_x_issued))) {
+        const float *x = a.x + (EXT ? (size_t)blockIdx.y * a.tok_x_stride : 0);
+        const uint32_t rot = COMBINE ? 0u : (uint32_t)((uint64_t)blockIdx.x * (a.in_dim / 4) / gridDim.x) & ~31u;
+        bool x_ok;
+        if constexpr (EXT && !COMBINE) {
+            __shared__ float s_share[PIPE_MAX_CONSUMERS / 32];
+            if (a.norm_w)
+                x_ok = quantize_x_to_smem<NP, SlotT::GROUP, SlotT::SUMS, true>(x, a.in_dim, 1u, a.x_stride, xq, a.xq_vec_bytes, tid, C, slots, want, a.wait_cycles,
+                                                                             a.status, rot, smem_u32(&s_x_issued), a.norm_w, a.norm_parts, a.norm_eps, s_share);
+            else
+                x_ok = quantize_x_to_smem<NP, SlotT::GROUP, SlotT::SUMS>(x, a.in_dim, 1u, a.x_stride, xq, a.xq_vec_bytes, tid, C, slots, want, a.wait_cycles,
+                                                                       a.status, rot, smem_u32(&s_x_issued));
+        } else
+            x_ok = quantize_x_to_smem<NP, SlotT::GROUP, SlotT::SUMS>(x, a.in_dim, COMBINE ? (uint32_t)a.nseg : 1u, a.x_stride, xq, a.xq_vec_bytes, tid, C, slots, want,
+                                                                   a.wait_cycles, a.status, rot, smem_u32(&s_x_issued));
+        if (!x_ok) {
             s_abort = 1;
             atomicExch(a.status, 3);
         }
