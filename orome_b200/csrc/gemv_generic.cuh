@@ -217,15 +217,27 @@ gemv_f32_kernel(const float *__restrict__ W, uint32_t out_dim, uint32_t in_dim, 
     if (tid < 4 && b0 + (int)tid < batch) y[(size_t)(b0 + tid) * ldy + row] = (red[0][tid] + red[1][tid]) + (red[2][tid] + red[3][tid]);
 }
 
-// out = silu(gate) * up, elementwise (shaders.metal:1018-1030); used after two
-// generic matvecs when the fused kernel does not take the shape.
-__global__ void swiglu_kernel(const float *__restrict__ gate, const float *__restrict__ up, float *__restrict__ out,
-                              uint32_t n, int batch, int ldg, int ldo)
+// out = silu(gate) * up, elementwise (shaders.metal:1018-1030); used after two products when the fused kernel does not take the
+// shape.  Bound by memory: four elements a thread, 16-byte accesses where rows and pointers allow; blockIdx.y strides over rows.
+__global__ void __launch_bounds__(256)
+swiglu_kernel(const float *__restrict__ gate, const float *__restrict__ up, float *__restrict__ out, uint32_t n, int batch, int ldg, int ldo)
 {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)n * batch) return;
-    uint32_t b = (uint32_t)(i / n), c = (uint32_t)(i % n);
-    out[(size_t)b * ldo + c] = silu_mul(gate[(size_t)b * ldg + c], up[(size_t)b * ldg + c]);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const uint32_t c = (blockIdx.x * 256u + threadIdx.x) * 4u;
+    if (c >= n) return;
+    const bool wide = c + 4 <= n && !((reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(up) | reinterpret_cast<uintptr_t>(out)) & 15) &&
+                      !((ldg | ldo) & 3);
+    for (int b = blockIdx.y; b < batch; b += gridDim.y) {
+        const float *g = gate + (size_t)b * ldg + c, *u = up + (size_t)b * ldg + c;
+        float *o = out + (size_t)b * ldo + c;
+        if (wide) {
+            const float4 gv = __ldcg(reinterpret_cast<const float4 *>(g)), uv = __ldcg(reinterpret_cast<const float4 *>(u));
+            *reinterpret_cast<float4 *>(o) = make_float4(silu_mul(gv.x, uv.x), silu_mul(gv.y, uv.y), silu_mul(gv.z, uv.z), silu_mul(gv.w, uv.w));
+        } else {
+            for (uint32_t q = 0; q < 4 && c + q < n; ++q) o[q] = silu_mul(__ldcg(g + q), __ldcg(u + q));
+        }
+    }
 }
 
 // Index of the largest element: argmax_kernel (shaders.metal:1249-1305), dispatched after the lm_head at

@@ -1228,9 +1228,8 @@ extern "C" int orome_cuda_gate_up_swiglu(orome_cuda_ctx *c, const OromeTensorRef
         rc = launch_generic(c, fmt, ud, up->out_dim, up->in_dim, layout, x_dev, batch, ldx, u, (int)n, st);
         if (rc) return rc;
     }
-    size_t tot = n * batch;
-    swiglu_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(g, u, out_dev, (uint32_t)n, batch, (int)n, batch == 1 ? (int)n : ldo);
-    return post_launch(c, "swiglu");
+    return orome_launch_pdl(c, "swiglu", swiglu_kernel, dim3((unsigned)((n + 1023) / 1024), (unsigned)std::min(batch, 65535)), dim3(256), st, (const float *)g,
+                            (const float *)u, out_dev, (uint32_t)n, batch, (int)n, batch == 1 ? (int)n : ldo);
 }
 
 extern "C" int orome_cuda_dequant_rows(orome_cuda_ctx *c, const OromeTensorRef *ref, uint32_t row0, uint32_t nrows,
