@@ -151,13 +151,15 @@ int orome_launch_tc(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t ou
     if (c->tc_slabs) return launch_staged(c, fmt, data, out_dim, in_dim, layout, x, batch, ldx, y, ldy, st, pub, x_ll, wait_gen);
     const uint32_t chunks = in_dim / TC_KC, mtiles = (out_dim + TP_ROWS - 1) / TP_ROWS;
     // At most 4096 vectors a launch (bounds the packed X).  While a graph is being captured no scratch can grow: the slices
-    // are then as large as what is there holds, and tiles are not cut if their partial sums have no room.
+    // are then as large as what is there holds, and tiles are not cut if their partial sums have no room.  A row-split product
+    // is never sliced: a launch publishes one generation of the whole Y, and reads the gathered X from row 0 on.
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CU(cudaStreamIsCapturing(st, &cap));
     int slice = 4096;
     auto padded = [](uint32_t nb) { const uint32_t nt = (nb + TP_MAX_N - 1) / TP_MAX_N; return ((nb + nt - 1) / nt + 15) / 16 * 16 * nt; };
     auto xp_floats = [&](uint32_t nb) { return (size_t)in_dim * padded(nb) / 2 + 64; };
-    if (cap != cudaStreamCaptureStatusNone && c->tc_xp_cap < xp_floats((uint32_t)std::min(batch, slice)) && c->tc_xp_cap >= xp_floats(16)) {
+    const bool one_launch = pub->npeers > 0 || x_ll;
+    if (cap != cudaStreamCaptureStatusNone && !one_launch && c->tc_xp_cap < xp_floats((uint32_t)std::min(batch, slice)) && c->tc_xp_cap >= xp_floats(16)) {
         slice = 16;
         while (slice < 4096 && xp_floats((uint32_t)slice + 16) <= c->tc_xp_cap) slice += 16;
     }

@@ -116,3 +116,40 @@ def test_requests_the_batched_form_cannot_honour(two_ranks):
     ctx.matvec(ref, x.data_ptr(), outside.data_ptr(), 8, n, n)                 # every refusal dropped the request
     torch.cuda.synchronize()
     assert ctx.status() == 0
+
+
+def test_a_captured_row_split_product_stays_one_launch(two_ranks):
+    """Scratch warmed for 16 vectors, then a product of 64 gathered ones captured (relaxed mode: scratch may grow).  Slices as
+    large as the old scratch would each read the gathered X from its first row again."""
+    torch, F, ctxs, arenas = two_ranks
+    world, fmt, n, m, batch = 2, synth.Q4_K, 512, 512, 64
+    W1, W2 = synth.host_tensor(fmt, m, n, seed=95), synth.host_tensor(fmt, n, m, seed=96)
+    X = synth.host_x(n, batch, seed=97)
+    xt, w2 = torch.from_numpy(np.ascontiguousarray(X)).cuda(), torch.from_numpy(W2).cuda()
+    rb, half = synth.row_bytes(fmt, n), m // world
+    w1 = [torch.from_numpy(W1[r * half * rb:(r + 1) * half * rb].copy()).cuda() for r in range(world)]
+    ref2 = F.tensor_ref(w2.data_ptr(), 0, fmt, n, m)
+    y1 = [arenas[r][:batch * m].view(batch, m) for r in range(world)]
+    y2 = torch.full((batch, n), float("nan"), device="cuda")
+    # rank 1's context has seen 16 vectors at most before the capture
+    ctxs[1].matvec(ref2, xt.data_ptr(), y2.data_ptr(), 16, n, n)
+    ctxs[0].matvec(ref2, xt.data_ptr(), y2.data_ptr(), batch, n, n)
+    torch.cuda.synchronize()
+    side, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    ctxs[0].gather_next(-1, 0)
+    ctxs[0].matvec(F.tensor_ref(w1[0].data_ptr(), 0, fmt, half, n), xt.data_ptr(), y1[0].data_ptr(), batch, n, m)
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g, stream=side, capture_error_mode="relaxed"):
+        ctxs[1].gather_next(-1, 0)
+        ctxs[1].matvec(F.tensor_ref(w1[1].data_ptr(), 0, fmt, half, n), xt.data_ptr(), y1[1][:, half:].data_ptr(), batch, n, m, side.cuda_stream)
+        ctxs[1].gather_next(0, -1)
+        ctxs[1].matvec(ref2, y1[1].data_ptr(), y2.data_ptr(), batch, m, n, side.cuda_stream)
+    g.replay()
+    torch.cuda.synchronize()
+    for b in range(batch):                                  # complete rank 1's plain copy from the slots
+        ctxs[1].gather_wait(0, y1[1][b].data_ptr(), m)
+    torch.cuda.synchronize()
+    assert [c.status() for c in ctxs] == [0, 0]
+    got1 = y1[1].cpu().numpy()
+    assert rel_l2(got1, oracle.matvec_f64(fmt, W1, m, n, X)) <= TC_TOL
+    assert rel_l2(y2.cpu().numpy(), oracle.matvec_f64(fmt, W2, n, m, got1)) <= TC_TOL
