@@ -100,7 +100,8 @@ typedef struct orome_cuda_ctx orome_cuda_ctx;
 
 /* Replaces metal_setup / metal_free (orome.h:219-221, metal.m:41) for this path:
  * binds a CUDA device, allocates the context's status word.  No scratch is sized
- * from a model config; the path's kernels need none beyond their outputs. */
+ * from a model config: the batch-1 kernels need none beyond their outputs, batched
+ * products and expert layers take theirs on first use (see there). */
 int  orome_cuda_ctx_create(int device, orome_cuda_ctx **out);
 void orome_cuda_ctx_destroy(orome_cuda_ctx *ctx);
 
@@ -260,7 +261,11 @@ int  orome_cuda_moe_route_static(orome_cuda_ctx *ctx, const OromeTensorRef *rout
  * idx/w use the [t][8] layout written by orome_cuda_moe_route.  act_dev is
  * caller-provided scratch of n_tokens * K * inter floats (the reference's
  * buf_batch_expert_act, orome.h:189).  The shared-expert term and the residual
- * add of the reference's combine kernel are outside this entry point. */
+ * add of the reference's combine kernel are outside this entry point.
+ * Token batches large enough to group their tokens by expert take memory of their own besides: a direct
+ * call from a pool of the context, in stream order; a captured one memory that belongs to the graph.  Calls
+ * on several streams of a context, and replayed graphs beside them, are therefore independent as long as
+ * their act_dev and out_dev are.  Where no memory can be had the call runs without, token by token. */
 int  orome_cuda_moe_ffn(orome_cuda_ctx *ctx, const OromeExpertLayerRef *layer, uint32_t variant,
                         const float *x_dev, int n_tokens, int ldx,
                         const uint32_t *idx_dev, const float *w_dev, uint32_t K,

@@ -5,8 +5,10 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <map>
+#include <memory>
 #include <tuple>
 #include <vector>
 
@@ -16,6 +18,15 @@ struct MapKey {
     const uint8_t *w;
     uint32_t unit, units, rows, kb;
     bool operator<(const MapKey &o) const { return std::tie(w, unit, units, rows, kb) < std::tie(o.w, o.unit, o.units, o.rows, o.kb); }
+};
+
+// Device memory of calls that were captured into one graph on one stream (moe_group.cu); `gone`: that graph is no more.
+struct GraphScratch {
+    unsigned long long capture;
+    cudaStream_t stream;
+    void *mem;
+    size_t bytes;
+    std::shared_ptr<std::atomic<bool>> gone;
 };
 
 struct orome_cuda_ctx {
@@ -61,8 +72,8 @@ struct orome_cuda_ctx {
     // scratch for the unfused gate/up fallback
     float *gu_dev = nullptr;
     size_t gu_cap = 0;
-    float *moe_dev = nullptr;      // scratch of the grouped expert products
-    size_t moe_cap = 0;
+    cudaMemPool_t moe_pool = nullptr;           // scratch of the grouped expert products, one piece per call
+    std::vector<GraphScratch> graph_scratch;    // and of captured ones
     std::vector<void *> retired;   // scratch buffers that have been outgrown (orome_ensure)
     // scratch of the tensor-core batched form: packed fp16 X and split-K partial sums
     float *tc_xp = nullptr, *tc_part = nullptr;

@@ -46,19 +46,100 @@ struct MgScratch {
     }
 };
 
+// A call's scratch.  Two calls may run at the same time -- on two streams, or a replayed graph beside a direct call -- each with
+// activations and outputs of its own, so no two of them may share it:
+//   direct calls   a piece of the context's pool, allocated and freed in the order of the call's stream (2 + 1 us on the host once
+//                  the pool has grown; the pool keeps what its calls needed at once and goes with the context);
+//   captured ones  memory of the graph: calls captured on one stream of one capture follow one another in every replay and
+//                  share it, and it is used again once the graph and all that was instantiated from it are gone.
+struct MgMemory {
+    uint8_t *p = nullptr;
+    cudaStream_t st;
+    bool pooled = false;
+    explicit MgMemory(cudaStream_t s) : st(s) {}
+    ~MgMemory() { if (pooled) cudaFreeAsync(p, st); }
+    MgMemory(const MgMemory &) = delete;
+    MgMemory &operator=(const MgMemory &) = delete;
+};
+
+static void CUDART_CB graph_scratch_gone(void *flag)
+{
+    auto *f = static_cast<std::shared_ptr<std::atomic<bool>> *>(flag);
+    (*f)->store(true);
+    delete f;
+}
+
+// OROME_ENOTSUP: no memory, or a capture that cannot own any; the caller has forms that need none.
+static int take_memory(orome_cuda_ctx *c, size_t bytes, MgMemory &m)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    cudaGraph_t graph = nullptr;
+    CU(cudaStreamGetCaptureInfo(m.st, &cap, &id, &graph, nullptr, nullptr));
+    if (cap == cudaStreamCaptureStatusNone) {
+        if (!c->moe_pool) {
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = c->device;
+            CU(cudaMemPoolCreate(&c->moe_pool, &props));
+            uint64_t keep = UINT64_MAX;
+            CU(cudaMemPoolSetAttribute(c->moe_pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        }
+        void *p = nullptr;
+        if (cudaMallocFromPoolAsync(&p, bytes, c->moe_pool, m.st) != cudaSuccess) { (void)cudaGetLastError(); return OROME_ENOTSUP; }
+        m.p = static_cast<uint8_t *>(p);
+        m.pooled = true;
+        return OROME_OK;
+    }
+    if (cap != cudaStreamCaptureStatusActive) return OROME_ENOTSUP;
+    GraphScratch *g = nullptr;
+    for (GraphScratch &s : c->graph_scratch)
+        if (!s.gone->load() && s.capture == id && s.stream == m.st && s.bytes >= bytes) { m.p = static_cast<uint8_t *>(s.mem); return OROME_OK; }
+    for (GraphScratch &s : c->graph_scratch)
+        if (!g && s.gone->load() && s.bytes >= bytes) g = &s;
+    if (!g) {
+        size_t size = 1 << 20;
+        while (size < bytes) size *= 2;      // so that later captures of other sizes find it large enough
+        // cudaMalloc does not touch the capture, but has to be let through while one is going on
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        CU(cudaThreadExchangeStreamCaptureMode(&mode));
+        void *p = nullptr;
+        const cudaError_t e = cudaMalloc(&p, size);
+        CU(cudaThreadExchangeStreamCaptureMode(&mode));
+        if (e != cudaSuccess) { (void)cudaGetLastError(); return OROME_ENOTSUP; }
+        c->graph_scratch.push_back(GraphScratch{0, nullptr, p, size, std::make_shared<std::atomic<bool>>(true)});
+        g = &c->graph_scratch.back();
+    }
+    auto flag = std::make_shared<std::atomic<bool>>(false);
+    auto *held = new std::shared_ptr<std::atomic<bool>>(flag);
+    cudaUserObject_t obj = nullptr;
+    if (cudaUserObjectCreate(&obj, held, graph_scratch_gone, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+        (void)cudaGetLastError();
+        delete held;
+        return OROME_ENOTSUP;
+    }
+    if (cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+        (void)cudaGetLastError();
+        cudaUserObjectRelease(obj, 1);
+        return OROME_ENOTSUP;
+    }
+    *g = GraphScratch{id, m.st, g->mem, g->bytes, flag};
+    m.p = static_cast<uint8_t *>(g->mem);
+    return OROME_OK;
+}
+
 int orome_moe_group(orome_cuda_ctx *c, const OromeExpertLayerRef *L, int layout, bool gate_up, bool down, const float *x, int n_tokens, int ldx,
                     const uint32_t *idx, const float *w, uint32_t K, uint32_t hidden, uint32_t inter, float *act, float *out, int ldo, cudaStream_t st)
 {
     const uint8_t *base = static_cast<const uint8_t *>(L->buffer);
     const int gfmt = (int)L->gate.format, dfmt = (int)L->down.format;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    CU(cudaStreamIsCapturing(st, &cap));
     constexpr int SLICE = 1024;      // tokens a pass: bounds the pairs' results (64 MiB at a hidden size of 2048)
     const MgScratch most(std::min(n_tokens, SLICE), K, hidden, inter, down);
-    if (cap != cudaStreamCaptureStatusNone && c->moe_cap < (most.total + 3) / 4) return OROME_ENOTSUP;      // no room can be made now
-    int rc = orome_ensure(c, &c->moe_dev, &c->moe_cap, (most.total + 3) / 4);
+    MgMemory memory(st);
+    int rc = take_memory(c, most.total, memory);
     if (rc) return rc;
-    uint8_t *mem = reinterpret_cast<uint8_t *>(c->moe_dev);
+    uint8_t *mem = memory.p;
     for (int t0 = 0; t0 < n_tokens; t0 += SLICE) {
         const int T = std::min(n_tokens - t0, SLICE);
         const MgScratch sc(T, K, hidden, inter, down);

@@ -72,7 +72,8 @@ extern "C" void orome_cuda_ctx_destroy(orome_cuda_ctx *c)
     cudaFree(c->gu_dev);
     cudaFree(c->tc_xp);
     cudaFree(c->tc_part);
-    cudaFree(c->moe_dev);
+    if (c->moe_pool) cudaMemPoolDestroy(c->moe_pool);
+    for (const GraphScratch &g : c->graph_scratch) cudaFree(g.mem);
     for (void *q : c->retired) cudaFree(q);
     cudaFree(c->trace_dev);
     cudaFree(c->g_local);

@@ -1,0 +1,121 @@
+"""What calls keep to themselves: expert batches on several streams and in graphs beside direct calls."""
+import time
+
+import numpy as np
+import pytest
+
+from orome_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+class _Layer:
+    """A layer of experts on the GPU, and calls with an input, activations and an output of their own."""
+
+    def __init__(self, torch, F, E, H, M, seed):
+        self.torch, self.F, self.E, self.H, self.M = torch, F, E, H, M
+        parts = [synth.host_tensor(synth.Q4_K, E * M, H, seed=seed), synth.host_tensor(synth.Q4_K, E * M, H, seed=seed + 1),
+                 synth.host_tensor(synth.Q5_K, E * H, M, seed=seed + 2)]
+        self.mem = torch.from_numpy(np.concatenate(parts)).cuda()
+        sg, sd = synth.tensor_bytes(synth.Q4_K, M, H), synth.tensor_bytes(synth.Q5_K, H, M)
+        self.ref = F.ExpertLayerRef(self.mem.data_ptr(), F.ExpertProjRef(0, sg, synth.Q4_K), F.ExpertProjRef(E * sg, sg, synth.Q4_K),
+                                    F.ExpertProjRef(2 * E * sg, sd, synth.Q5_K))
+
+    def call(self, T, K, seed):
+        t, rng = self.torch, np.random.default_rng(seed)
+        idx, w = np.zeros((T, 8), np.int32), np.zeros((T, 8), np.float32)
+        for i in range(T):
+            idx[i, :K] = rng.permutation(self.E)[:K]
+        w[:, :K] = rng.random((T, K))
+        x = np.atleast_2d(synth.host_x(self.H, T, seed=seed))
+        return {"T": T, "K": K, "x": t.from_numpy(x).cuda(), "idx": t.from_numpy(idx).cuda(), "w": t.from_numpy(w).cuda(),
+                "act": t.empty((T, K, self.M), device="cuda"), "out": t.full((T, self.H), float("nan"), device="cuda")}
+
+    def issue(self, ctx, c, stream):
+        ctx.moe_ffn(self.ref, 0, c["x"].data_ptr(), c["T"], self.H, c["idx"].data_ptr(), c["w"].data_ptr(), c["K"], self.H, self.M,
+                    c["act"].data_ptr(), c["out"].data_ptr(), self.H, stream)
+
+
+@pytest.fixture(scope="module")
+def env():
+    import torch
+    from orome_b200 import format as F
+    ctx = F.Context(0)
+    yield torch, F, ctx
+    torch.cuda.synchronize()
+    assert ctx.status() == 0
+    ctx.close()
+
+
+def test_expert_batches_on_two_streams_of_a_context(env):
+    """Same layer, same sizes, other tokens: whatever overlaps, each call gives the bits it gives alone."""
+    torch, F, ctx = env
+    layer = _Layer(torch, F, 8, 512, 512, 11)
+    calls = [layer.call(200, 4, 21 + i) for i in range(2)]
+    want = []
+    for c in calls:
+        layer.issue(ctx, c, 0)
+        torch.cuda.synchronize()
+        want.append(c["out"].clone())
+    streams = [torch.cuda.Stream() for _ in calls]
+    for _ in range(30):
+        for c in calls:
+            c["out"].fill_(float("nan"))
+        torch.cuda.synchronize()
+        for _ in range(3):
+            for c, s in zip(calls, streams):
+                layer.issue(ctx, c, s.cuda_stream)
+        torch.cuda.synchronize()
+        for c, w in zip(calls, want):
+            assert torch.equal(c["out"], w)
+
+
+def test_captured_expert_batches_own_their_scratch(env):
+    """Graphs captured without any earlier call, replayed beside each other and beside a direct call; a graph that is gone gives
+    its memory to the next capture."""
+    torch, F, _ = env
+    layer = _Layer(torch, F, 8, 512, 512, 31)
+    ctx = F.Context(0)
+    calls = [layer.call(200, 4, 41 + i) for i in range(4)]
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    graphs = []
+    for mine in (calls[0:2], calls[2:3]):                  # two layers' worth in the first graph, one in the second
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=streams[0]):
+            for c in mine:
+                layer.issue(ctx, c, streams[0].cuda_stream)
+        graphs.append(g)
+    fresh = F.Context(0)
+    want = []
+    for c in calls:
+        layer.issue(fresh, c, 0)
+        torch.cuda.synchronize()
+        want.append(c["out"].clone())
+    for _ in range(20):
+        for c in calls:
+            c["out"].fill_(float("nan"))
+        torch.cuda.synchronize()
+        for s, g in zip(streams, graphs):
+            with torch.cuda.stream(s):
+                g.replay()
+        layer.issue(ctx, calls[3], streams[2].cuda_stream)
+        torch.cuda.synchronize()
+        for c, w in zip(calls, want):
+            assert torch.equal(c["out"], w)
+    del g, graphs
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info(0)[0]
+    for _ in range(8):                                     # memory of one graph at a time
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=streams[0]):
+            layer.issue(ctx, calls[0], streams[0].cuda_stream)
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(calls[0]["out"], want[0])
+        del g
+        torch.cuda.synchronize()
+        time.sleep(0.05)                                   # the driver tells of the graph's end from a thread of its own
+    assert free - torch.cuda.mem_get_info(0)[0] <= 16 << 20      # eight pieces of 4 MiB would be 32
+    assert ctx.status() == 0
+    ctx.close()
+    fresh.close()
