@@ -24,14 +24,11 @@
 #pragma once
 #include <cuda.h>
 #include "gemv_pipe.cuh"
+#include "mma_plan.h"
 
 namespace orome {
 
-constexpr int MMA_TILE_ROWS = 16;
-constexpr int MMA_MAX_WARPS = 8;                  // consumer warps of a group
-constexpr int MMA_MAX_GROUPS = 5;
-constexpr int MMA_MAX_CONSUMER_WARPS = 16;        // groups * warps per group
-constexpr int MMA_MAX_PRODUCERS = 2;              // producer warps (two where every row is its own copy)
+static_assert(MMA_MAX_STAGES == PIPE_MAX_STAGES, "one ring, one bound");
 constexpr int MMA_MAX_THREADS = (MMA_MAX_CONSUMER_WARPS + MMA_MAX_PRODUCERS) * 32;
 constexpr uint32_t MMA_XQ_SB = 864;               // quantized x per superblock: 8 groups x 3 planes x 32 B, then the sums (<= 96 B)
 // Two input vectors at once (NTOK = 2; Q4_K / Q5_K plain products): the mma's B operand has eight columns of which one
@@ -56,7 +53,7 @@ struct MmaArgs {
     uint32_t in_dim, row_bytes;
     uint32_t units;            // superblocks per row
     uint32_t nwarps;           // consumer warps of one group: a group covers the kc superblocks of a stage
-    uint32_t ngroups;          // groups; stage i (counted over row tiles and their chunks) belongs to group i % ngroups (nstages is a multiple, or odd with two groups)
+    uint32_t ngroups;          // groups; stage i (counted over row tiles and their chunks) belongs to group i % ngroups (nstages is a multiple, or odd with two groups and one producer)
     uint32_t kc;               // superblocks per stage
     uint32_t nchunks;          // stages per row tile = ceil(units / kc)
     uint32_t dbg_tile;         // diagnostics build: first row tile whose per-warp timeline is recorded
@@ -806,7 +803,7 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
 
     const uint32_t stages_s = smem_u32(stages);
     const uint32_t group = warp / NW, wig = warp - group * NW;
-    const bool odd_ring = NG == 2 && (a.nstages & 1u);
+    const bool odd_ring = NPROD == 1 && NG == 2 && (a.nstages & 1u);
     uint32_t cur = lo, s = 0, parity = 0, i = 0, turn = 0, tile_no = 0;
     int seg = 0;
     MmaTile t;
@@ -822,8 +819,8 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
                 continue;
             }
             if (c == 0) MMA_TILE_STAMP(a, tile_no, warp, 0);
-            // Two groups on an odd ring: a slot's previous use is the other group's.  Once that has been consumed (the use
-            // before it was this group's own, so the parity is unambiguous) the slot's full barrier is in this use's phase.
+            // Two groups on an odd ring (one producer, see mma_lay_out): a slot's previous use is the other group's.  Once that
+            // has been consumed the slot's full barrier is in this use's phase.
             if (odd_ring && !s_abort && !mbar_wait_bounded(smem_u32(empty + s), parity ^ 1u)) {
                 s_abort = 1;
                 atomicExch(a.status, 1);

@@ -568,7 +568,6 @@ static int plan_mma(orome_cuda_ctx *c, int fmt, uint32_t in_dim, uint32_t total_
     const uint32_t unit = fmt == FMT_Q4_K ? 144u : fmt == FMT_Q5_K ? 176u : 210u;
     const uint32_t units_row = in_dim / 256;
     a.in_dim = in_dim;
-    a.units = units_row * std::max(1u, nvec);
     a.row_bytes = units_row * unit;
     a.total_rows = total_rows;
     p.grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)c->sm_count, (total_rows + MMA_TILE_ROWS - 1) / MMA_TILE_ROWS));
@@ -579,64 +578,16 @@ static int plan_mma(orome_cuda_ctx *c, int fmt, uint32_t in_dim, uint32_t total_
     }
     const uint32_t share = (total_rows + p.grid - 1) / p.grid;
     const bool fused = c->fuse_norm_w || c->fuse_res_in;      // fused neighbours: four byte planes (launch_mma)
-    // A stage of `want` bytes: 16 rows (x2 in the fused form) of kc superblocks.  40 KiB, or less where that leaves a consumer
-    // group fewer than two ring slots: with one, a group waits out every copy into the slot it has just read.  27B shapes, one
-    // slot a group / the largest stage that leaves two: gate/up 32.6 / 23.4 us, fused down 36.5 / 28.6, lm_head 155 / 131.
-    auto lay_out = [&](uint32_t want, bool odd) -> int {
-        const uint32_t kc_max = std::max(1u, std::min(units_row, want / (MMA_TILE_ROWS * unit * (swiglu ? 2u : 1u))));
-        if (nvec > 0) {
-            if (units_row > kc_max) return fail(OROME_ENOTSUP, "mma plan: combine form with rows of %u superblocks", units_row);
-            a.nchunks = nvec;
-            a.kc = units_row;
-        } else {
-            a.nchunks = (a.units + kc_max - 1) / kc_max;
-            a.kc = (a.units + a.nchunks - 1) / a.nchunks;
-        }
-        const uint32_t rounds = (a.kc + MMA_MAX_WARPS - 1) / MMA_MAX_WARPS;
-        a.nwarps = (a.kc + rounds - 1) / rounds;
-        // stages (row tiles x chunks) go round the groups: as many groups as the warp budget and the CTA's stage count allow
-        const uint32_t cta_stages = (share + MMA_TILE_ROWS - 1) / MMA_TILE_ROWS * a.nchunks;
-        a.ngroups = std::max(1u, std::min(std::min<uint32_t>(MMA_MAX_GROUPS, MMA_MAX_CONSUMER_WARPS / a.nwarps), cta_stages));
-        // box width in superblocks: the smallest kb >= kc with kb = 2 (mod 4), which makes the row pitch 32 or 96 (mod 128)
-        const uint32_t kb = a.kc + ((6 - a.kc % 4) % 4);
-        a.pitch = kb * unit;
-        if (fmt == FMT_Q6_K) {
-            // rows arrive by their own copies, widened to 16-byte boundaries (up to 15 bytes before and after the chunk)
-            a.pitch = (a.kc * unit + 30 + 15) / 16 * 16;
-            while (a.pitch % 128 != 16) a.pitch += 16;      // the quads of the eight rows of a load then read eight different four-bank groups
-        }
-        a.box_bytes = MMA_TILE_ROWS * a.pitch;
-        a.half_stride = MMA_TILE_ROWS * a.pitch;
-        a.stage_stride = a.half_stride * (swiglu ? 2 : 1);
-        a.red_base = 2 * 8 * PIPE_MAX_STAGES;
-        a.red_rows = std::max<uint32_t>(MMA_TILE_ROWS, std::min<uint32_t>((share + MMA_TILE_ROWS - 1) / MMA_TILE_ROWS * MMA_TILE_ROWS, 128u));
-        const size_t red_bytes = (size_t)2 * a.red_rows * a.nwarps * a.ngroups * (swiglu || two ? 2 : 1) * sizeof(float);
-        a.xs_base = (uint32_t)((a.red_base + red_bytes + 127) / 128 * 128);
-        const size_t xq_sb = !two ? (fused ? MMA_XQ_SB4 : MMA_XQ_SB) : (c->x_bits == 24 ? mma_xq_sb<3, 2>() : mma_xq_sb<2, 2>());
-        const size_t xq_bytes = (size_t)a.units * xq_sb + (size_t)a.units * 8 * (two ? 2 : 1) + 768;   // planes and sums, two scales per superblock and vector, a block of zeros
-        a.stage_base = (uint32_t)((a.xs_base + xq_bytes + 127) / 128 * 128);
-        const size_t budget = std::min<size_t>(228 * 1024 - 1024 - 256, (size_t)c->smem_optin - 256);
-        if (budget < a.stage_base + a.stage_stride) return fail(OROME_ENOTSUP, "mma plan: in_dim %u does not fit shared memory", in_dim);
-        const uint32_t tiles = ((share + MMA_TILE_ROWS - 1) / MMA_TILE_ROWS + 1) * a.nchunks;
-        a.nstages = (uint32_t)std::min<size_t>(std::min<size_t>(PIPE_MAX_STAGES, tiles), (budget - a.stage_base) / a.stage_stride);
-        // A whole number of ring slots per group, so that every use of a slot belongs to the same group.  A wait by parity tells
-        // only the last two phases apart: a group waiting for use k of a slot whose use k - 1 is another group's, and has not
-        // landed yet, would take phase k - 2 for phase k and read the stage too early.
-        a.ngroups = std::min(a.ngroups, a.nstages);
-        // (odd: three or five slots for two groups, where the kernel makes a group wait for the slot's other user first.)
-        if (!(odd && a.ngroups == 2 && a.nstages >= 3)) a.nstages -= a.nstages % a.ngroups;
-        p.threads = (int)(a.nwarps * a.ngroups + (fmt == FMT_Q6_K ? 2 : 1)) * 32;
-        return a.nstages >= std::min(2 * a.ngroups, cta_stages) ? OROME_OK : 1;      // 1: a ring, but a shallow one
-    };
-    int fit = OROME_ENOTSUP;
-    if (c->stage_kb || nvec > 0) fit = lay_out((c->stage_kb ? (uint32_t)c->stage_kb : 40u) * 1024u, true);
-    else
-        for (uint32_t kb = 40; kb >= 16 && fit != OROME_OK; kb -= 4) {
-            fit = lay_out(kb * 1024u, false);
-            if (fit == OROME_OK && kb < 40 && a.nwarps * a.ngroups < 12) fit = 1;      // narrow stages that leave warps idle cost more (7-superblock rows: 3 %)
-        }
-    if (fit == 1 && !c->stage_kb && nvec == 0) fit = lay_out(40u * 1024u, true);      // shallow at every size: the largest stage
-    if (fit != OROME_OK && fit != 1) return fit;
+    const MmaRingShape in{fmt == FMT_Q6_K, unit, units_row, nvec, share, swiglu, two,
+                          !two ? (fused ? MMA_XQ_SB4 : MMA_XQ_SB) : (c->x_bits == 24 ? mma_xq_sb<3, 2>() : mma_xq_sb<2, 2>()),
+                          (size_t)c->smem_optin, (uint32_t)c->stage_kb};
+    MmaRing r = {};
+    if (mma_plan_ring(in, r) == MMA_RING_NO_ROOM) return fail(OROME_ENOTSUP, "mma plan: in_dim %u does not fit shared memory", in_dim);
+    a.units = r.units; a.nchunks = r.nchunks; a.kc = r.kc;
+    a.nwarps = r.nwarps; a.ngroups = r.ngroups; a.nstages = r.nstages;
+    a.pitch = r.pitch; a.half_stride = r.half_stride; a.box_bytes = r.half_stride; a.stage_stride = r.stage_stride;
+    a.red_base = r.red_base; a.red_rows = r.red_rows; a.xs_base = r.xs_base; a.stage_base = r.stage_base;
+    p.threads = (int)(a.nwarps * a.ngroups + (fmt == FMT_Q6_K ? 2 : 1)) * 32;
     p.smem = a.stage_base + (size_t)a.stage_stride * a.nstages;
 #ifdef OROME_MMA_TILE_TRACE
     a.dbg_tile = OROME_MMA_TILE_TRACE;      // diagnostics build: first row tile whose per-warp timeline is recorded

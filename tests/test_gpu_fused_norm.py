@@ -193,10 +193,11 @@ def test_fused_neighbours_on_both_kquant_kernels(env, fmt, rows, cols, x_bits):
     assert err[1] <= (2e-6 if x_bits == 24 else 2e-4)
 
 
-@pytest.mark.parametrize("rows,cols", [(5120, 17408), (8192, 8192), (3000, 5120)])
-def test_q6_ring_whose_slots_do_not_divide_by_its_groups(env, rows, cols):
-    """Products back to back whose shared memory holds three or five stages for two or three consumer groups (every slot must
-    keep one producer warp and one group): every repetition gives the first one's bits, and the first one is right."""
+@pytest.mark.parametrize("rows,cols,stage_kb", [(5120, 17408, 0), (5120, 17408, 40), (4096, 17408, 20), (8192, 8192, 0), (3000, 5120, 0)])
+def test_q6_ring_keeps_its_slots_apart(env, rows, cols, stage_kb):
+    """Products back to back on rings of several stages a group, and on those whose shared memory would hold an odd number for two
+    groups (three at 17408 columns with fused neighbours and 40-KiB stages, nine with 20-KiB ones; tests/test_mma_ring.py pins
+    the plans): every repetition gives the first one's bits, and the first one is right."""
     torch, F, ctx = env
     fmt = synth.Q6_K
     w = synth.host_tensor(fmt, rows, cols, seed=41)
@@ -205,11 +206,15 @@ def test_q6_ring_whose_slots_do_not_divide_by_its_groups(env, rows, cols):
     ref = F.tensor_ref(t["w"].data_ptr(), 0, fmt, rows, cols)
     out = torch.full((64, rows), float("nan"), device="cuda")
     parts = torch.zeros(F.SUM_SQ_PARTS, device="cuda")
-    for i in range(64):
-        if i % 2 == 0:
-            ctx.fuse_next(None, F.ResidualEpilogue(t["resid"].data_ptr(), parts.data_ptr()))
-        ctx.hint_next(ref)
-        ctx.matvec(ref, t["x"].data_ptr(), out[i].data_ptr())
+    ctx.set_option(F.OPT_STAGE_KB, stage_kb)
+    try:
+        for i in range(64):
+            if i % 2 == 0:
+                ctx.fuse_next(None, F.ResidualEpilogue(t["resid"].data_ptr(), parts.data_ptr()))
+            ctx.hint_next(ref)
+            ctx.matvec(ref, t["x"].data_ptr(), out[i].data_ptr())
+    finally:
+        ctx.set_option(F.OPT_STAGE_KB, 0)
     torch.cuda.synchronize()
     assert ctx.status() == 0
     got = out.cpu().numpy()
