@@ -201,6 +201,9 @@ moe_group_kernel(const __grid_constant__ MgArgs a)
     if (warp >= (uint32_t)MG_WARPS) {
         const uint32_t lt = tid - MG_WARPS * 32;
         uint32_t s = 0, ph = 1, fill = 0, slot = 0;
+        // `dead`: a wait ran out somewhere in this CTA.  A loader that finds out stops waiting and copying but keeps coming to the
+        // barrier below, since the others may not have found out yet and count on it; without waits the items left over are brief.
+        bool dead = false;
         uint4 bq = block_of(blockIdx.x);
         uint32_t ord = lt < bq.z ? __ldcg(a.order + bq.y + lt) : 0u;
         for (uint32_t item = blockIdx.x; item < n_items; item += gridDim.x, slot = (slot + 1) & 7u) {
@@ -208,12 +211,13 @@ moe_group_kernel(const __grid_constant__ MgArgs a)
             const uint8_t *e0 = a.w0 + bq.x * a.stride + (size_t)row0 * a.row_bytes, *e1 = SWIGLU ? a.w1 + bq.x * a.stride + (size_t)row0 * a.row_bytes : e0;
             const uint32_t live = min(ROWS, a.rows - row0), pieces = bq.z * (MG_REC / 16);
             if (lt < bq.z) s_order[slot][lt] = ord;
+            __syncwarp();
             named_bar_sync(PIPE_BAR_CONSUMERS, MG_LOADERS * 32);
             // the next item's block and pairs are on their way while this one's stages are filled
             const uint4 nq = block_of(item + gridDim.x);
-            for (uint32_t u = 0; u < U; ++u, ++fill) {
+            for (uint32_t u = 0; u < U && !dead; ++u, ++fill) {
                 if (fill >= a.nstages && !mbar_wait_bounded(smem_u32(empty + s), ph)) { if (!s_abort) { s_abort = 1; atomicExch(a.status, 2); } }
-                if (s_abort) break;
+                if (s_abort) { dead = true; break; }
                 const uint32_t st = smem_u32(smem + (size_t)s * stage_bytes);
 #pragma unroll
                 for (uint32_t j = 0; j < 16 * MG_WARPS * PPR / (MG_LOADERS * 32); ++j) {
@@ -234,7 +238,6 @@ moe_group_kernel(const __grid_constant__ MgArgs a)
                 if (++s == a.nstages) { s = 0; ph ^= 1u; }
                 if (u == 0) ord = lt < nq.z ? __ldcg(a.order + nq.y + lt) : 0u;
             }
-            if (s_abort) break;
             bq = nq;
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
@@ -252,7 +255,7 @@ moe_group_kernel(const __grid_constant__ MgArgs a)
         for (int c = 0; c < MG_MAX_CAP / 8; ++c) y[c][0] = y[c][1] = y[c][2] = y[c][3] = 0.0f;
         for (uint32_t u = 0; u < U; ++u) {
             if (!mbar_wait_bounded(smem_u32(full + s), ph)) { if (!s_abort) { s_abort = 1; atomicExch(a.status, 1); } }
-            if (s_abort) return;
+            if (__any_sync(0xffffffffu, s_abort)) return;      // the whole warp, ahead of its mma
             const uint32_t st = smem_u32(smem + (size_t)s * stage_bytes);
             const uint32_t h0 = st + (SWIGLU ? warp * 8u + g : warp * 16u + g) * PITCH, h1 = h0 + (SWIGLU ? 8 * MG_WARPS : 8) * PITCH;
             uint32_t A[8][4], sl0, sh0, sl1, sh1, ml0, mh0, ml1, mh1;
