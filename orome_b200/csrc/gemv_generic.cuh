@@ -43,6 +43,7 @@ __global__ void __launch_bounds__(256)
 dequant_flat_kernel(const uint8_t *__restrict__ blocks, uint64_t pieces, int layout, float *__restrict__ out)
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");      // the packed rows may be what the kernel before has written
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t base = ((uint64_t)blockIdx.x * 8u + (threadIdx.x >> 5)) * (32u * DQ_PIECES) + lane;
     uint2 q[DQ_PIECES], h[DQ_PIECES];
@@ -73,7 +74,6 @@ dequant_flat_kernel(const uint8_t *__restrict__ blocks, uint64_t pieces, int lay
             if constexpr (FMT == FMT_Q5_K) h[k] = __ldg(reinterpret_cast<const uint2 *>(sb + 16u + 8u * (p & 3u)));
         }
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");      // the packed rows are constant; what is overwritten may still be read
 #pragma unroll
     for (uint32_t k = 0; k < DQ_PIECES; ++k) {
         const uint64_t i = base + 32u * k;

@@ -736,3 +736,29 @@ def test_dequant_rows_in_the_middle_of_a_tensor(env, fmt, variant, rows, cols, r
     want = oracle.decode_rows(fmt, data, rows, cols, layout=variant)[row0:row0 + n]
     assert np.array_equal(got[1:n + 1].view(np.uint32), want.view(np.uint32))
     assert np.isnan(got[0]).all() and np.isnan(got[n + 1]).all()
+
+
+def test_dequant_rows_of_a_tensor_the_kernel_before_has_written(env):
+    """The packed bytes are the output of the call before, on the same stream and with nothing in between: its last rows, which it
+    writes last, decode to what they decode to after a synchronisation."""
+    torch, F, ctx = env
+    rows, cols = 8192, 4096
+    data = synth.host_tensor(synth.Q8_0, rows, cols, seed=61)
+    wt = dev_bytes(torch, data)
+    packed = torch.zeros((rows, cols), device="cuda")            # 128 MiB of fp32, read as packed blocks of every format
+    nbytes = packed.numel() * 4
+    for fmt in QUANT:
+        n = nbytes // synth.tensor_bytes(fmt, 1, cols)
+        ref = F.tensor_ref(packed.data_ptr(), 0, fmt, n, cols)
+        got = torch.zeros((64, cols), device="cuda")
+        want = torch.zeros((64, cols), device="cuda")
+        for sync, out in ((True, want), (False, got)):
+            packed.zero_()
+            torch.cuda.synchronize()
+            ctx.dequant_rows(F.tensor_ref(wt.data_ptr(), 0, synth.Q8_0, rows, cols), 0, rows, packed.data_ptr())
+            if sync:
+                torch.cuda.synchronize()
+            ctx.dequant_rows(ref, n - 64, 64, out.data_ptr())
+            torch.cuda.synchronize()
+        assert int((want.view(torch.int32) != 0).sum()) > want.numel() // 8
+        assert torch.equal(got.view(torch.int32), want.view(torch.int32)), fmt
