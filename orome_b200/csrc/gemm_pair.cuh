@@ -302,6 +302,13 @@ gemm_pair_kernel(const __grid_constant__ TpArgs a)
         if (!s_abort) { s_abort = 1; atomicExch(a.status, 4); }
         return false;
     };
+    // The same for a whole warp, with one answer for all lanes: s_abort may be set between two lanes' looks at it, and what
+    // follows (__syncwarp, tensor memory accesses) needs the warp together.
+    auto wait_warp = [&](uint64_t *bar, uint32_t parity) -> bool {
+        const bool ok = mbar_try_wait(smem_u32(bar), parity);
+        if (__all_sync(0xffffffffu, ok)) return true;
+        return __all_sync(0xffffffffu, ok || wait(bar, parity));
+    };
 
     if (warp >= (uint32_t)TP_W_LOAD) {
         // ---- loaders: packed weights of this CTA's 128 rows, independent of the previous kernel ----
@@ -409,7 +416,7 @@ gemm_pair_kernel(const __grid_constant__ TpArgs a)
         for (uint32_t i = 0; i < n_units; ++i) {
             if (FMT == FMT_Q6_K && (i == 0 || chunk == 0))
                 row_off = (uint32_t)reinterpret_cast<uintptr_t>(a.w) + ((tile / a.ntiles) * TP_ROWS + rank * TC_M + r) * a.row_bytes;
-            if (!wait(w_full + s, pw)) break;
+            if (!wait_warp(w_full + s, pw)) break;
             TcPacked<FMT> pk;
             uint32_t row_s = smem_u32(w_stages + s * STAGE) + r * PITCH;
             if constexpr (FMT == FMT_Q6_K) row_s += (row_off + chunk * 210u) & 15u;
@@ -417,7 +424,7 @@ gemm_pair_kernel(const __grid_constant__ TpArgs a)
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(w_empty + s));
             if (++s == WS) { s = 0; pw ^= 1u; }
-            if (i >= AS && !wait(a_empty + sa, pa)) break;
+            if (i >= AS && !wait_warp(a_empty + sa, pa)) break;
             __syncwarp();
             tc_fence_after();
             const uint32_t taddr = tmem_a + sa * 128u;
@@ -438,7 +445,7 @@ gemm_pair_kernel(const __grid_constant__ TpArgs a)
             const bool whole = u_lo <= t_lo && u_lo + n_units >= t_lo + a.chunks;
             const uint32_t grow = (tile / a.ntiles) * TP_ROWS + rank * TC_M + r, n_base = (tile % a.ntiles) * a.nt_rows;
             float *part = a.part + ((size_t)cl * 2 + (u_lo <= t_lo ? 1 : 0)) * a.nt_rows * TP_ROWS + rank * TC_M + r;   // 0: the share starts inside the tile
-            const bool done = wait(acc_full, seg & 1u);
+            const bool done = wait_warp(acc_full, seg & 1u);
             __syncwarp();
             tc_fence_after();
             for (uint32_t n0 = kq * 16u; n0 < a.nt_rows; n0 += 64u) {
