@@ -29,6 +29,13 @@ struct GraphScratch {
     std::shared_ptr<std::atomic<bool>> gone;
 };
 
+// Scratch that grows (orome_ensure).
+struct Scratch {
+    float *p = nullptr;
+    size_t cap = 0;            // floats
+    bool captured = false;     // a captured call has used it: its address may be in a graph
+};
+
 struct orome_cuda_ctx {
     std::map<MapKey, CUtensorMap> maps;   // tensor maps of the mma kernel's tensors
     int device = 0;
@@ -67,17 +74,14 @@ struct orome_cuda_ctx {
     size_t stage_x_cap = 0, stage_y_cap = 0;
     cudaStream_t own_stream = nullptr;
     // scratch for routing logits when the caller passes none
-    float *logits_dev = nullptr;
-    size_t logits_cap = 0;
+    Scratch logits;
     // scratch for the unfused gate/up fallback
-    float *gu_dev = nullptr;
-    size_t gu_cap = 0;
+    Scratch gu;
     cudaMemPool_t moe_pool = nullptr;           // scratch of the grouped expert products, one piece per call
     std::vector<GraphScratch> graph_scratch;    // and of captured ones
-    std::vector<void *> retired;   // scratch buffers that have been outgrown (orome_ensure)
+    std::vector<void *> retired;   // outgrown scratch that a graph may still use
     // scratch of the tensor-core batched form: packed fp16 X and split-K partial sums
-    float *tc_xp = nullptr, *tc_part = nullptr;
-    size_t tc_xp_cap = 0, tc_part_cap = 0;
+    Scratch tc_xp, tc_part;
     int tc_min_batch = 4;    // batches from this size on use the tensor-core kernel (smaller ones: one decode launch per vector)
     int tc_slabs = 0;        // batched form: 1 = dequantized weights staged in shared memory (the earlier form), 0 = in tensor memory
     int tc_tiles = 0;        // kept for its key: the batched form has one layout of tiles
@@ -104,7 +108,8 @@ uint32_t orome_pipe_group_threads(int fmt, uint32_t in_dim);
 bool orome_pipe_supported(int fmt, uint32_t in_dim);
 long long orome_wait_cycles(const orome_cuda_ctx *c);
 
-int orome_ensure(orome_cuda_ctx *c, float **p, size_t *cap, size_t floats);   // context scratch of at least that size
+// Context scratch of at least `floats` floats for a call on `st`.
+int orome_ensure(orome_cuda_ctx *c, Scratch &s, size_t floats, cudaStream_t st);
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                   const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);

@@ -57,7 +57,7 @@ static int launch_pack(orome_cuda_ctx *c, const float *x, int nb, int ldx, uint3
                        const unsigned int *wait_gen, cudaStream_t st)
 {
     return orome_launch_pdl(c, "pack_x_f16", pack_x_f16_kernel, dim3((in_dim / 8 + 255) / 256, nt_rows * ntiles), dim3(256), st, x, nb, ldx, in_dim, nt_rows,
-                            reinterpret_cast<__half *>(c->tc_xp), x_ll, wait_gen, orome_wait_cycles(c), c->status_dev);
+                            reinterpret_cast<__half *>(c->tc_xp.p), x_ll, wait_gen, orome_wait_cycles(c), c->status_dev);
 }
 
 // The form staged in shared memory (OROME_OPT_TC_SLABS): slices of TC_MAX_N vectors, each of which reads the weights again.
@@ -78,9 +78,9 @@ static int launch_staged(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32
     for (int b0 = 0; b0 < batch; b0 += TC_MAX_N) {
         const int nb = std::min(batch - b0, TC_MAX_N);
         const uint32_t npad = (uint32_t)(nb + 15) / 16 * 16;
-        int rc = orome_ensure(c, &c->tc_xp, &c->tc_xp_cap, (size_t)in_dim * npad / 2 + 64);
+        int rc = orome_ensure(c, c->tc_xp, (size_t)in_dim * npad / 2 + 64, st);
         if (rc) return rc;
-        if (split > 1) { rc = orome_ensure(c, &c->tc_part, &c->tc_part_cap, (size_t)split * nb * out_dim); if (rc) return rc; }
+        if (split > 1) { rc = orome_ensure(c, c->tc_part, (size_t)split * nb * out_dim, st); if (rc) return rc; }
         rc = launch_pack(c, x + (size_t)b0 * ldx, nb, ldx, in_dim, npad, 1, x_ll, wait_gen, st);
         if (rc) return rc;
         TcArgs a;
@@ -94,7 +94,7 @@ static int launch_staged(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) return fail(OROME_ECUDA, "gemm_tc: cuTensorMapEncodeTiled failed (%d)", (int)r);
-        a.w = data; a.xp = reinterpret_cast<__half *>(c->tc_xp); a.y = split == 1 ? y + (size_t)b0 * ldy : c->tc_part;
+        a.w = data; a.xp = reinterpret_cast<__half *>(c->tc_xp.p); a.y = split == 1 ? y + (size_t)b0 * ldy : c->tc_part.p;
         a.rows = out_dim; a.in_dim = in_dim; a.row_bytes = (uint32_t)row_bytes_of(fmt, in_dim); a.chunk_bytes = chunk_bytes;
         a.batch = (uint32_t)nb; a.npad = npad; a.ldy = (uint32_t)ldy; a.split = split; a.chunks = chunks;
         a.layout = layout; a.status = c->status_dev;
@@ -114,7 +114,7 @@ static int launch_staged(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32
         if (split > 1) {
             const size_t n = (size_t)nb * out_dim;
             rc = orome_launch_pdl(c, "splitk_reduce", splitk_reduce_kernel, dim3((unsigned)std::min<size_t>((n + 255) / 256, 1184)), dim3(256), st,
-                                  (const float *)c->tc_part, split, (uint32_t)nb, out_dim, y + (size_t)b0 * ldy, (uint32_t)ldy, *pub);
+                                  (const float *)c->tc_part.p, split, (uint32_t)nb, out_dim, y + (size_t)b0 * ldy, (uint32_t)ldy, *pub);
             if (rc) return rc;
         }
     }
@@ -150,24 +150,26 @@ int orome_launch_tc(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t ou
     if (!pub) pub = &no_pub;
     if (c->tc_slabs) return launch_staged(c, fmt, data, out_dim, in_dim, layout, x, batch, ldx, y, ldy, st, pub, x_ll, wait_gen);
     const uint32_t chunks = in_dim / TC_KC, mtiles = (out_dim + TP_ROWS - 1) / TP_ROWS;
-    // At most 4096 vectors a launch (bounds the packed X).  While a graph is being captured no scratch can grow: the slices
-    // are then as large as what is there holds, and tiles are not cut if their partial sums have no room.  A row-split product
-    // is never sliced: a launch publishes one generation of the whole Y, and reads the gathered X from row 0 on.
+    // At most 4096 vectors a launch (bounds the packed X), fewer where the packed X of that many has no room: while a graph is
+    // being captured, where no scratch can grow, as many as what is there holds; else half as many until there is room, down to
+    // 64.  Tiles are not cut if their partial sums have no room.  A row-split product is never sliced: a launch publishes one
+    // generation of the whole Y, and reads the gathered X from row 0 on.
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CU(cudaStreamIsCapturing(st, &cap));
-    int slice = 4096;
+    const bool capturing = cap != cudaStreamCaptureStatusNone, one_launch = pub->npeers > 0 || x_ll;
+    int slice = std::min(batch, 4096), rc;
     auto padded = [](uint32_t nb) { const uint32_t nt = (nb + TP_MAX_N - 1) / TP_MAX_N; return ((nb + nt - 1) / nt + 15) / 16 * 16 * nt; };
-    auto xp_floats = [&](uint32_t nb) { return (size_t)in_dim * padded(nb) / 2 + 64; };
-    const bool one_launch = pub->npeers > 0 || x_ll;
-    if (cap != cudaStreamCaptureStatusNone && !one_launch && c->tc_xp_cap < xp_floats((uint32_t)std::min(batch, slice)) && c->tc_xp_cap >= xp_floats(16)) {
+    auto xp_floats = [&](int nb) { return (size_t)in_dim * padded((uint32_t)nb) / 2 + 64; };
+    if (capturing && !one_launch && c->tc_xp.cap < xp_floats(slice) && c->tc_xp.cap >= xp_floats(16)) {
+        const int most = slice;
         slice = 16;
-        while (slice < 4096 && xp_floats((uint32_t)slice + 16) <= c->tc_xp_cap) slice += 16;
+        while (slice < most && xp_floats(slice + 16) <= c->tc_xp.cap) slice += 16;
     }
+    while ((rc = orome_ensure(c, c->tc_xp, xp_floats(slice), st)) == OROME_ENOMEM && !capturing && !one_launch && slice > 64) slice = (slice / 2 + 63) / 64 * 64;
+    if (rc) return rc;
     for (int b0 = 0; b0 < batch; b0 += slice) {
         const uint32_t nb = (uint32_t)std::min(batch - b0, slice);
         const uint32_t ntiles = (nb + TP_MAX_N - 1) / TP_MAX_N, nt_rows = ((nb + ntiles - 1) / ntiles + 15) / 16 * 16;
-        int rc = orome_ensure(c, &c->tc_xp, &c->tc_xp_cap, xp_floats(nb));
-        if (rc) return rc;
         TpArgs a;
         memset(&a, 0, sizeof a);
         auto part_floats = [&](uint32_t clusters) { return (size_t)clusters * 2 * nt_rows * TP_ROWS; };
@@ -175,13 +177,18 @@ int orome_launch_tc(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t ou
         a.units = chunks * mtiles * ntiles;
         a.clusters = tp_clusters(c, fmt, mtiles * ntiles, chunks, nt_rows, true);
         auto is_cut = [&]() { return a.units % a.clusters != 0 || (a.units / a.clusters) % chunks != 0; };
-        if (is_cut() && cap != cudaStreamCaptureStatusNone && part_floats(a.clusters) > c->tc_part_cap)
-            a.clusters = tp_clusters(c, fmt, mtiles * ntiles, chunks, nt_rows, false);
+        if (is_cut()) {
+            rc = capturing && part_floats(a.clusters) > c->tc_part.cap ? OROME_ENOMEM : orome_ensure(c, c->tc_part, part_floats(a.clusters), st);
+            if (rc == OROME_ENOMEM) {
+                a.clusters = tp_clusters(c, fmt, mtiles * ntiles, chunks, nt_rows, false);
+                rc = is_cut() ? orome_ensure(c, c->tc_part, part_floats(a.clusters), st) : OROME_OK;      // (a fixed number of parts)
+            }
+            if (rc) return rc;
+        }
         const bool cut = is_cut();
-        if (cut) { rc = orome_ensure(c, &c->tc_part, &c->tc_part_cap, part_floats(a.clusters)); if (rc) return rc; }
         rc = launch_pack(c, x + (size_t)b0 * ldx, (int)nb, ldx, in_dim, nt_rows / 2, 2 * ntiles, x_ll, wait_gen, st);      // a CTA's half of a tile lies together
         if (rc) return rc;
-        a.w = data; a.xp = reinterpret_cast<const __half *>(c->tc_xp); a.y = y + (size_t)b0 * ldy; a.part = c->tc_part;
+        a.w = data; a.xp = reinterpret_cast<const __half *>(c->tc_xp.p); a.y = y + (size_t)b0 * ldy; a.part = c->tc_part.p;
         a.rows = out_dim; a.row_bytes = (uint32_t)row_bytes_of(fmt, in_dim); a.w_bytes = (uint64_t)a.row_bytes * out_dim;
         a.batch = nb; a.nt_rows = nt_rows; a.ntiles = ntiles; a.ldy = (uint32_t)ldy;
         a.publish_done = !cut;

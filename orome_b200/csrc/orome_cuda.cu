@@ -68,10 +68,7 @@ extern "C" void orome_cuda_ctx_destroy(orome_cuda_ctx *c)
     cudaFree(c->status_dev);
     cudaFree(c->stage_x_dev);
     cudaFree(c->stage_y_dev);
-    cudaFree(c->logits_dev);
-    cudaFree(c->gu_dev);
-    cudaFree(c->tc_xp);
-    cudaFree(c->tc_part);
+    for (const Scratch *s : {&c->logits, &c->gu, &c->tc_xp, &c->tc_part}) cudaFree(s->p);
     if (c->moe_pool) cudaMemPoolDestroy(c->moe_pool);
     for (const GraphScratch &g : c->graph_scratch) cudaFree(g.mem);
     for (void *q : c->retired) cudaFree(q);
@@ -1089,20 +1086,26 @@ extern "C" int orome_format_dispatch_matvec(orome_cuda_ctx *c, const OromeTensor
     return orome_cuda_matvec(c, ref, x, y, 1, 0, 0, stream);
 }
 
-int orome_ensure(orome_cuda_ctx *c, float **p, size_t *cap, size_t floats)
+int orome_ensure(orome_cuda_ctx *c, Scratch &s, size_t floats, cudaStream_t st)
 {
-    if (*cap >= floats) return OROME_OK;
-    // The old buffer may still be an operand of a captured graph: it stays until the context goes.  Doubling bounds what is
-    // kept that way by the size of the last one.
-    const size_t want = std::max(floats, 2 * *cap);
-    float *q = nullptr;
-    cudaError_t e = cudaMalloc(&q, want * sizeof(float));
-    size_t got = want;
-    if (e == cudaErrorMemoryAllocation && want > floats) { (void)cudaGetLastError(); e = cudaMalloc(&q, floats * sizeof(float)); got = floats; }
-    if (e != cudaSuccess) { (void)cudaGetLastError(); return fail(OROME_ENOMEM, "scratch of %zu floats: %s", floats, cudaGetErrorString(e)); }
-    if (*p) c->retired.push_back(*p);
-    *p = q;
-    *cap = got;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CU(cudaStreamIsCapturing(st, &cap));
+    const bool capturing = cap != cudaStreamCaptureStatusNone;
+    if (s.cap < floats) {
+        // An outgrown buffer goes before the new one comes, so that a call needs no more than its own size.  One whose address a
+        // graph may hold stays until the context goes; doubling then bounds what is kept that way by the size of the last one.
+        const size_t want = s.captured ? std::max(floats, 2 * s.cap) : floats;
+        if (s.p && (s.captured || capturing)) c->retired.push_back(s.p);
+        else cudaFree(s.p);
+        s = Scratch();
+        for (size_t n : {want, floats}) {
+            if (cudaMalloc(&s.p, n * sizeof(float)) == cudaSuccess) { s.cap = n; break; }
+            s.p = nullptr;
+            const cudaError_t e = cudaGetLastError();
+            if (n == floats) return fail(OROME_ENOMEM, "scratch of %zu floats: %s", floats, cudaGetErrorString(e));
+        }
+    }
+    s.captured = s.captured || capturing;
     return OROME_OK;
 }
 
@@ -1165,9 +1168,9 @@ extern "C" int orome_cuda_gate_up_swiglu(orome_cuda_ctx *c, const OromeTensorRef
     if (batch > 1 && (ldx < (int)gate->in_dim || ldo < (int)gate->out_dim))
         return fail(OROME_EINVAL, "gate_up_swiglu: ldx/ldo smaller than the row length");
     const size_t n = (size_t)gate->out_dim;
-    rc = orome_ensure(c, &c->gu_dev, &c->gu_cap, 2 * n * batch);
+    rc = orome_ensure(c, c->gu, 2 * n * batch, st);
     if (rc) return rc;
-    float *g = c->gu_dev, *u = c->gu_dev + n * batch;
+    float *g = c->gu.p, *u = c->gu.p + n * batch;
     if (batch > 1) {
         // the batched product's own dispatch: tensor cores from OROME_OPT_TC_MIN_BATCH vectors on, decode launches below
         rc = orome_cuda_matvec(c, gate, x_dev, g, batch, ldx, (int)n, stream);
@@ -1255,9 +1258,9 @@ extern "C" int orome_cuda_moe_route(orome_cuda_ctx *c, const OromeTensorRef *rou
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const uint32_t ne = router->out_dim;
     if (!logits_dev) {
-        rc = orome_ensure(c, &c->logits_dev, &c->logits_cap, (size_t)ne * n_tokens);
+        rc = orome_ensure(c, c->logits, (size_t)ne * n_tokens, st);
         if (rc) return rc;
-        logits_dev = c->logits_dev;
+        logits_dev = c->logits.p;
     }
     return launch_router(c, data, ne, router->in_dim, x_dev, n_tokens, ldx, logits_dev, K, idx_dev, w_dev, st);
 }
@@ -1288,9 +1291,9 @@ extern "C" int orome_cuda_moe_route_pair(orome_cuda_ctx *c, const OromeTensorRef
         CU(cudaMemsetAsync(shared_logit_dev, 0, (size_t)n_tokens * sizeof(float), st));      // absent gate: logit 0
     }
     if (!logits_dev) {
-        rc = orome_ensure(c, &c->logits_dev, &c->logits_cap, (size_t)(ne + 1) * n_tokens);
+        rc = orome_ensure(c, c->logits, (size_t)(ne + 1) * n_tokens, st);
         if (rc) return rc;
-        logits_dev = c->logits_dev;
+        logits_dev = c->logits.p;
     }
     return launch_router(c, data, ne, router->in_dim, x_dev, n_tokens, ldx, logits_dev, K, idx_dev, w_dev, st, sg, shared_logit_dev);
 }

@@ -119,3 +119,106 @@ def test_captured_expert_batches_own_their_scratch(env):
     assert ctx.status() == 0
     ctx.close()
     fresh.close()
+
+
+class _Product:
+    """Y = X W^T with buffers of its own."""
+
+    def __init__(self, torch, F, out_dim, in_dim, batch, seed, fmt=synth.Q4_K):
+        self.out_dim, self.in_dim, self.batch = out_dim, in_dim, batch
+        self.w = torch.from_numpy(synth.host_tensor(fmt, out_dim, in_dim, seed=seed)).cuda()
+        self.ref = F.tensor_ref(self.w.data_ptr(), 0, fmt, out_dim, in_dim)
+        g = torch.Generator(device="cuda")
+        g.manual_seed(seed)
+        self.x = torch.randn(batch, in_dim, generator=g, device="cuda")
+        self.y = torch.full((batch, out_dim), float("nan"), device="cuda")
+
+    def issue(self, ctx, stream=0, batch=None):
+        ctx.matvec(self.ref, self.x.data_ptr(), self.y.data_ptr(), batch or self.batch, self.in_dim, self.out_dim, stream)
+
+    def error(self, torch, F, ctx):
+        w = torch.empty(self.out_dim, self.in_dim, device="cuda")
+        ctx.dequant_rows(self.ref, 0, self.out_dim, w.data_ptr())
+        torch.cuda.synchronize()
+        want = self.x.double() @ w.double().T
+        return float((self.y.double() - want).norm() / want.norm())
+
+
+TC_TOL = 5e-4          # fp16 operands
+
+
+def test_captured_product_on_scratch_of_a_smaller_one(env):
+    """Captured with room for a part of its packed X (slices); then a larger direct call outgrows the scratch whose address the
+    graph holds, and the graph is replayed."""
+    torch, F, _ = env
+    ctx = F.Context(0)
+    small, p, big = _Product(torch, F, 256, 512, 16, 51), _Product(torch, F, 300, 8192, 2500, 52), _Product(torch, F, 256, 16384, 3000, 53)
+    small.issue(ctx)
+    torch.cuda.synchronize()
+    side, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=side):
+        p.issue(ctx, side.cuda_stream)
+    big.issue(ctx)
+    torch.cuda.synchronize()
+    hold = [torch.full((1 << 20,), 7, dtype=torch.int32, device="cuda") for _ in range(32)]      # what a freed buffer would be given to
+    for _ in range(2):
+        p.y.fill_(float("nan"))
+        g.replay()
+        torch.cuda.synchronize()
+        assert p.error(torch, F, ctx) <= TC_TOL
+    assert big.error(torch, F, ctx) <= TC_TOL and small.error(torch, F, ctx) <= TC_TOL
+    assert all(int((h != 7).sum()) == 0 for h in hold)
+    assert ctx.status() == 0
+    ctx.close()
+
+
+def _device_bytes(torch, F, calls):
+    """Device memory that a fresh context holds after `calls` (which have run before in another one: kernels are loaded)."""
+    held = []
+    for _ in range(2):
+        ctx = F.Context(0)
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info(0)[0]
+        calls(ctx)
+        torch.cuda.synchronize()
+        held.append(free - torch.cuda.mem_get_info(0)[0])
+        ctx.close()
+        torch.cuda.synchronize()
+    return held[1]
+
+
+def test_scratch_that_grows_is_no_larger_than_its_last_size(env):
+    """Packed X of 2048, 3000 and 4096 vectors of 8192 (64 MiB at last), and at most two partial tiles per pair of SMs (37 MiB)."""
+    torch, F, _ = env
+    p = _Product(torch, F, 512, 8192, 4096, 61)
+
+    def calls(ctx):
+        for b in (2048, 3000, 4096):
+            p.issue(ctx, batch=b)
+    assert _device_bytes(torch, F, calls) <= (64 + 37 + 8) << 20
+
+
+def test_long_prompt_with_little_memory_left(env):
+    """Packed X of 4096 vectors of 16384 takes 128 MiB; with less than that left the same product runs in smaller slices."""
+    torch, F, _ = env
+    p = _Product(torch, F, 256, 16384, 4096, 71)
+    for b in (4096, 2048, 1024, 512):                      # every kernel that the slices may take is loaded
+        warm = F.Context(0)
+        p.issue(warm, batch=b)
+        torch.cuda.synchronize()
+        warm.close()
+    ctx = F.Context(0)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    p.y.fill_(float("nan"))
+    torch.cuda.synchronize()
+    hog = torch.empty(torch.cuda.mem_get_info(0)[0] - (100 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        p.issue(ctx)
+        torch.cuda.synchronize()
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    assert p.error(torch, F, ctx) <= TC_TOL
+    assert ctx.status() == 0
+    ctx.close()
