@@ -157,7 +157,8 @@ int orome_launch_tc(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t ou
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CU(cudaStreamIsCapturing(st, &cap));
     const bool capturing = cap != cudaStreamCaptureStatusNone, one_launch = pub->npeers > 0 || x_ll;
-    int slice = std::min(batch, 4096), rc;
+    // A fixed number of parts cuts every tile, at most twelve ways: 64 vectors then bound the partial sums.
+    int slice = std::min(batch, c->tc_split ? 64 : 4096), rc;
     auto padded = [](uint32_t nb) { const uint32_t nt = (nb + TP_MAX_N - 1) / TP_MAX_N; return ((nb + nt - 1) / nt + 15) / 16 * 16 * nt; };
     auto xp_floats = [&](int nb) { return (size_t)in_dim * padded((uint32_t)nb) / 2 + 64; };
     if (capturing && !one_launch && c->tc_xp.cap < xp_floats(slice) && c->tc_xp.cap >= xp_floats(16)) {
@@ -172,7 +173,8 @@ int orome_launch_tc(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t ou
         const uint32_t ntiles = (nb + TP_MAX_N - 1) / TP_MAX_N, nt_rows = ((nb + ntiles - 1) / ntiles + 15) / 16 * 16;
         TpArgs a;
         memset(&a, 0, sizeof a);
-        auto part_floats = [&](uint32_t clusters) { return (size_t)clusters * 2 * nt_rows * TP_ROWS; };
+        a.slots = c->tc_split ? 1 : 2;      // a fixed number of parts never crosses a tile's end
+        auto part_floats = [&](uint32_t clusters) { return (size_t)clusters * a.slots * nt_rows * TP_ROWS; };
         a.chunks = chunks;
         a.units = chunks * mtiles * ntiles;
         a.clusters = tp_clusters(c, fmt, mtiles * ntiles, chunks, nt_rows, true);

@@ -45,7 +45,8 @@ struct TpArgs {
     const uint8_t *w;
     const __half *xp;             // packed X: [half of an n tile][k slab of 64][nt_rows / 2][64] fp16, swizzled
     float *y;                     // [batch][ldy]
-    float *part;                  // [cluster][2][nt_rows][256]
+    float *part;                  // [cluster][slots][nt_rows][256]
+    uint32_t slots;               // partial tiles a cluster may leave: 2, or 1 where every share lies inside one tile
     uint32_t rows, row_bytes;
     uint64_t w_bytes;
     uint32_t batch, nt_rows, ntiles, ldy;      // vectors of a tile (a multiple of 16), tiles of vectors
@@ -444,7 +445,7 @@ gemm_pair_kernel(const __grid_constant__ TpArgs a)
             const uint32_t t_lo = tile * a.chunks;
             const bool whole = u_lo <= t_lo && u_lo + n_units >= t_lo + a.chunks;
             const uint32_t grow = (tile / a.ntiles) * TP_ROWS + rank * TC_M + r, n_base = (tile % a.ntiles) * a.nt_rows;
-            float *part = a.part + ((size_t)cl * 2 + (u_lo <= t_lo ? 1 : 0)) * a.nt_rows * TP_ROWS + rank * TC_M + r;   // 0: the share starts inside the tile
+            float *part = a.part + ((size_t)cl * a.slots + (u_lo <= t_lo ? a.slots - 1 : 0)) * a.nt_rows * TP_ROWS + rank * TC_M + r;   // 0: the share starts inside the tile
             const bool done = wait_warp(acc_full, seg & 1u);
             __syncwarp();
             tc_fence_after();
@@ -505,12 +506,10 @@ tile_reduce_kernel(const __grid_constant__ TpArgs a)
     const uint32_t grow = (tile / a.ntiles) * TP_ROWS + row, gn = (tile % a.ntiles) * a.nt_rows + n;
     const unsigned int tag = a.pub.npeers > 0 ? *reinterpret_cast<const volatile unsigned int *>(a.pub.pub_gen) + 1u : 0u;
     if (c_lo != c_hi && grow < a.rows && gn < a.batch) {
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        const size_t step = (size_t)2 * a.nt_rows * TP_ROWS;
+        const size_t slot = (size_t)a.nt_rows * TP_ROWS, step = a.slots * slot;
         const float *src = a.part + (size_t)c_lo * step + (size_t)n * TP_ROWS + row;
-        // only the tile's first cluster can have it as its last tile (slot 1); the others start inside it (slot 0)
-        if (tp_share_lo(a.units, a.clusters, c_lo) <= t_lo) acc = __ldcg(reinterpret_cast<const float4 *>(src + (size_t)a.nt_rows * TP_ROWS));
-        else acc = __ldcg(reinterpret_cast<const float4 *>(src));
+        // the tile's first cluster has it as its last tile (the last slot); the others start inside it (slot 0)
+        float4 acc = __ldcg(reinterpret_cast<const float4 *>(src + (a.slots - 1) * slot));
 #pragma unroll 8
         for (uint32_t c = c_lo + 1; c <= c_hi; ++c) {
             src += step;

@@ -198,6 +198,19 @@ def test_scratch_that_grows_is_no_larger_than_its_last_size(env):
     assert _device_bytes(torch, F, calls) <= (64 + 37 + 8) << 20
 
 
+def test_fixed_parts_of_a_long_prompt_bound_their_partial_sums(env):
+    """OROME_OPT_TC_SPLIT = 12 on 512 vectors: the partial sums of 64 of them at a time, 24 MiB (all at once: 384 MiB)."""
+    torch, F, _ = env
+    p = _Product(torch, F, 8192, 4096, 512, 66, synth.Q8_0)
+
+    def calls(ctx):
+        ctx.set_option(F.OPT_TC_SPLIT, 12)
+        p.issue(ctx)
+        assert p.error(torch, F, ctx) <= TC_TOL
+    p.error(torch, F, env[2])                              # torch's own workspaces
+    assert _device_bytes(torch, F, calls) <= 96 << 20
+
+
 def test_long_prompt_with_little_memory_left(env):
     """Packed X of 4096 vectors of 16384 takes 128 MiB; with less than that left the same product runs in smaller slices."""
     torch, F, _ = env
