@@ -101,7 +101,9 @@ typedef struct orome_cuda_ctx orome_cuda_ctx;
 /* Replaces metal_setup / metal_free (orome.h:219-221, metal.m:41) for this path:
  * binds a CUDA device, allocates the context's status word.  No scratch is sized
  * from a model config: the batch-1 kernels need none beyond their outputs, batched
- * products and expert layers take theirs on first use (see there). */
+ * products and expert layers take theirs on first use (see there), from a pool that the
+ * device's contexts share.  The pool keeps at most 512 MiB that none of them uses and goes
+ * with the last context that used it. */
 int  orome_cuda_ctx_create(int device, orome_cuda_ctx **out);
 void orome_cuda_ctx_destroy(orome_cuda_ctx *ctx);
 
@@ -265,7 +267,7 @@ int  orome_cuda_moe_route_static(orome_cuda_ctx *ctx, const OromeTensorRef *rout
  * buf_batch_expert_act, orome.h:189).  The shared-expert term and the residual
  * add of the reference's combine kernel are outside this entry point.
  * Token batches large enough to group their tokens by expert take memory of their own besides: a direct
- * call from a pool of the context, in stream order; a captured one memory that belongs to the graph.  Calls
+ * call from the device's pool, in stream order; a captured one memory that belongs to the graph.  Calls
  * on several streams of a context, and replayed graphs beside them, are therefore independent as long as
  * their act_dev and out_dev are.  Where no memory can be had the call runs without, token by token. */
 int  orome_cuda_moe_ffn(orome_cuda_ctx *ctx, const OromeExpertLayerRef *layer, uint32_t variant,

@@ -77,7 +77,7 @@ struct orome_cuda_ctx {
     Scratch logits;
     // scratch for the unfused gate/up fallback
     Scratch gu;
-    cudaMemPool_t moe_pool = nullptr;           // scratch of the grouped expert products, one piece per call
+    cudaMemPool_t pool = nullptr;               // the device's scratch pool, once this context has used it (orome_pool)
     std::vector<GraphScratch> graph_scratch;    // and of captured ones
     std::vector<void *> retired;   // outgrown scratch that a graph may still use
     // scratch of the tensor-core batched form: packed fp16 X and split-K partial sums
@@ -108,8 +108,10 @@ uint32_t orome_pipe_group_threads(int fmt, uint32_t in_dim);
 bool orome_pipe_supported(int fmt, uint32_t in_dim);
 long long orome_wait_cycles(const orome_cuda_ctx *c);
 
-// Context scratch of at least `floats` floats for a call on `st`.
-int orome_ensure(orome_cuda_ctx *c, Scratch &s, size_t floats, cudaStream_t st);
+// Context scratch of at least `floats` floats for a call on `st`; `usual` floats where nothing is there yet and that many fit.
+int orome_ensure(orome_cuda_ctx *c, Scratch &s, size_t floats, cudaStream_t st, size_t usual = 0);
+// The pool scratch comes from: one per device, shared by its contexts and gone with the last one that used it.
+int orome_pool(orome_cuda_ctx *c);
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                   const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);

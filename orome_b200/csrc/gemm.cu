@@ -166,7 +166,9 @@ int orome_launch_tc(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t ou
         slice = 16;
         while (slice < most && xp_floats(slice + 16) <= c->tc_xp.cap) slice += 16;
     }
-    while ((rc = orome_ensure(c, c->tc_xp, xp_floats(slice), st)) == OROME_ENOMEM && !capturing && !one_launch && slice > 64) slice = (slice / 2 + 63) / 64 * 64;
+    // (first sizes: 32 MiB of packed X, 960 vectors of 17408, and all that shares can leave, two tiles of 256 vectors per pair of SMs,
+    // so that the products of a layer do not each outgrow the one before)
+    while ((rc = orome_ensure(c, c->tc_xp, xp_floats(slice), st, (size_t)8 << 20)) == OROME_ENOMEM && !capturing && !one_launch && slice > 64) slice = (slice / 2 + 63) / 64 * 64;
     if (rc) return rc;
     for (int b0 = 0; b0 < batch; b0 += slice) {
         const uint32_t nb = (uint32_t)std::min(batch - b0, slice);
@@ -180,7 +182,7 @@ int orome_launch_tc(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t ou
         a.clusters = tp_clusters(c, fmt, mtiles * ntiles, chunks, nt_rows, true);
         auto is_cut = [&]() { return a.units % a.clusters != 0 || (a.units / a.clusters) % chunks != 0; };
         if (is_cut()) {
-            rc = capturing && part_floats(a.clusters) > c->tc_part.cap ? OROME_ENOMEM : orome_ensure(c, c->tc_part, part_floats(a.clusters), st);
+            rc = capturing && part_floats(a.clusters) > c->tc_part.cap ? OROME_ENOMEM : orome_ensure(c, c->tc_part, part_floats(a.clusters), st, (size_t)std::max(1, c->sm_count / 2) * 2 * TP_MAX_N * TP_ROWS);
             if (rc == OROME_ENOMEM) {
                 a.clusters = tp_clusters(c, fmt, mtiles * ntiles, chunks, nt_rows, false);
                 rc = is_cut() ? orome_ensure(c, c->tc_part, part_floats(a.clusters), st) : OROME_OK;      // (a fixed number of parts)

@@ -48,8 +48,8 @@ struct MgScratch {
 
 // A call's scratch.  Two calls may run at the same time -- on two streams, or a replayed graph beside a direct call -- each with
 // activations and outputs of its own, so no two of them may share it:
-//   direct calls   a piece of the context's pool, allocated and freed in the order of the call's stream (2 + 1 us on the host once
-//                  the pool has grown; the pool keeps what its calls needed at once and goes with the context);
+//   direct calls   a piece of the device's pool, allocated and freed in the order of the call's stream (2 + 1 us on the host once
+//                  the pool has grown);
 //   captured ones  memory of the graph: calls captured on one stream of one capture follow one another in every replay and
 //                  share it, and it is used again once the graph and all that was instantiated from it are gone.
 struct MgMemory {
@@ -77,17 +77,9 @@ static int take_memory(orome_cuda_ctx *c, size_t bytes, MgMemory &m)
     cudaGraph_t graph = nullptr;
     CU(cudaStreamGetCaptureInfo(m.st, &cap, &id, &graph, nullptr, nullptr));
     if (cap == cudaStreamCaptureStatusNone) {
-        if (!c->moe_pool) {
-            cudaMemPoolProps props = {};
-            props.allocType = cudaMemAllocationTypePinned;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = c->device;
-            CU(cudaMemPoolCreate(&c->moe_pool, &props));
-            uint64_t keep = UINT64_MAX;
-            CU(cudaMemPoolSetAttribute(c->moe_pool, cudaMemPoolAttrReleaseThreshold, &keep));
-        }
+        if (orome_pool(c) != OROME_OK) return OROME_ENOTSUP;
         void *p = nullptr;
-        if (cudaMallocFromPoolAsync(&p, bytes, c->moe_pool, m.st) != cudaSuccess) { (void)cudaGetLastError(); return OROME_ENOTSUP; }
+        if (cudaMallocFromPoolAsync(&p, bytes, c->pool, m.st) != cudaSuccess) { (void)cudaGetLastError(); return OROME_ENOTSUP; }
         m.p = static_cast<uint8_t *>(p);
         m.pooled = true;
         return OROME_OK;

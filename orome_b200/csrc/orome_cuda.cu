@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <string>
 #include <tuple>
 
@@ -60,6 +61,40 @@ extern "C" int orome_cuda_ctx_create(int device, orome_cuda_ctx **out)
     return OROME_OK;
 }
 
+// A cudaMalloc costs a millisecond and more whatever its size (measured 0.4-4 ms on a shared host), memory that the pool already
+// has 2 us.  It keeps at most POOL_KEEP bytes that nobody uses.
+constexpr uint64_t POOL_KEEP = 512ull << 20;
+static std::mutex g_pool_mutex;
+static struct { cudaMemPool_t pool; int users; } g_pools[64];      // per device ordinal
+
+int orome_pool(orome_cuda_ctx *c)
+{
+    if (c->pool) return OROME_OK;
+    if (c->device >= 64) return fail(OROME_ENOTSUP, "device ordinal %d out of range", c->device);
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    auto &g = g_pools[c->device];
+    if (!g.users) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = c->device;
+        CU(cudaMemPoolCreate(&g.pool, &props));
+        uint64_t keep = POOL_KEEP;
+        CU(cudaMemPoolSetAttribute(g.pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    }
+    ++g.users;
+    c->pool = g.pool;
+    return OROME_OK;
+}
+
+static void release_pool(orome_cuda_ctx *c)
+{
+    if (!c->pool) return;
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    auto &g = g_pools[c->device];
+    if (--g.users == 0) cudaMemPoolDestroy(g.pool);
+}
+
 extern "C" void orome_cuda_ctx_destroy(orome_cuda_ctx *c)
 {
     if (!c) return;
@@ -68,8 +103,8 @@ extern "C" void orome_cuda_ctx_destroy(orome_cuda_ctx *c)
     cudaFree(c->status_dev);
     cudaFree(c->stage_x_dev);
     cudaFree(c->stage_y_dev);
+    cudaDeviceSynchronize();                 // memory of the pool is freed without one
     for (const Scratch *s : {&c->logits, &c->gu, &c->tc_xp, &c->tc_part}) cudaFree(s->p);
-    if (c->moe_pool) cudaMemPoolDestroy(c->moe_pool);
     for (const GraphScratch &g : c->graph_scratch) cudaFree(g.mem);
     for (void *q : c->retired) cudaFree(q);
     cudaFree(c->trace_dev);
@@ -77,6 +112,7 @@ extern "C" void orome_cuda_ctx_destroy(orome_cuda_ctx *c)
     cudaFreeHost(c->stage_x_host);
     cudaFreeHost(c->stage_y_host);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
+    release_pool(c);
     delete c;
 }
 
@@ -1086,7 +1122,7 @@ extern "C" int orome_format_dispatch_matvec(orome_cuda_ctx *c, const OromeTensor
     return orome_cuda_matvec(c, ref, x, y, 1, 0, 0, stream);
 }
 
-int orome_ensure(orome_cuda_ctx *c, Scratch &s, size_t floats, cudaStream_t st)
+int orome_ensure(orome_cuda_ctx *c, Scratch &s, size_t floats, cudaStream_t st, size_t usual)
 {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CU(cudaStreamIsCapturing(st, &cap));
@@ -1094,14 +1130,24 @@ int orome_ensure(orome_cuda_ctx *c, Scratch &s, size_t floats, cudaStream_t st)
     if (s.cap < floats) {
         // An outgrown buffer goes before the new one comes, so that a call needs no more than its own size.  One whose address a
         // graph may hold stays until the context goes; doubling then bounds what is kept that way by the size of the last one.
-        const size_t want = s.captured ? std::max(floats, 2 * s.cap) : floats;
+        const size_t want = std::max({floats, s.captured ? 2 * s.cap : 0, s.cap ? 0 : usual});
         if (s.p && (s.captured || capturing)) c->retired.push_back(s.p);
-        else cudaFree(s.p);
+        else if (s.p) {
+            CU(cudaDeviceSynchronize());
+            cudaFree(s.p);
+        }
         s = Scratch();
         for (size_t n : {want, floats}) {
-            if (cudaMalloc(&s.p, n * sizeof(float)) == cudaSuccess) { s.cap = n; break; }
-            s.p = nullptr;
-            const cudaError_t e = cudaGetLastError();
+            // From the pool, on the context's own stream and waited for (nothing else is queued there), so that any stream may use
+            // it; plainly during a capture, whose mode decides whether that may be.
+            void *p = nullptr;
+            cudaError_t e = cudaErrorMemoryAllocation;
+            if (!capturing && orome_pool(c) == OROME_OK) {
+                e = cudaMallocFromPoolAsync(&p, n * sizeof(float), c->pool, c->own_stream);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(c->own_stream);
+            } else e = cudaMalloc(&p, n * sizeof(float));
+            if (e == cudaSuccess) { s.p = static_cast<float *>(p); s.cap = n; break; }
+            (void)cudaGetLastError();
             if (n == floats) return fail(OROME_ENOMEM, "scratch of %zu floats: %s", floats, cudaGetErrorString(e));
         }
     }

@@ -36,7 +36,7 @@ class _Layer:
                     c["act"].data_ptr(), c["out"].data_ptr(), self.H, stream)
 
 
-@pytest.fixture(scope="module")
+@pytest.fixture()
 def env():
     import torch
     from orome_b200 import format as F
@@ -73,9 +73,8 @@ def test_expert_batches_on_two_streams_of_a_context(env):
 def test_captured_expert_batches_own_their_scratch(env):
     """Graphs captured without any earlier call, replayed beside each other and beside a direct call; a graph that is gone gives
     its memory to the next capture."""
-    torch, F, _ = env
+    torch, F, ctx = env
     layer = _Layer(torch, F, 8, 512, 512, 31)
-    ctx = F.Context(0)
     calls = [layer.call(200, 4, 41 + i) for i in range(4)]
     streams = [torch.cuda.Stream() for _ in range(3)]
     graphs = []
@@ -116,8 +115,6 @@ def test_captured_expert_batches_own_their_scratch(env):
         torch.cuda.synchronize()
         time.sleep(0.05)                                   # the driver tells of the graph's end from a thread of its own
     assert free - torch.cuda.mem_get_info(0)[0] <= 16 << 20      # eight pieces of 4 MiB would be 32
-    assert ctx.status() == 0
-    ctx.close()
     fresh.close()
 
 
@@ -150,8 +147,7 @@ TC_TOL = 5e-4          # fp16 operands
 def test_captured_product_on_scratch_of_a_smaller_one(env):
     """Captured with room for a part of its packed X (slices); then a larger direct call outgrows the scratch whose address the
     graph holds, and the graph is replayed."""
-    torch, F, _ = env
-    ctx = F.Context(0)
+    torch, F, ctx = env
     small, p, big = _Product(torch, F, 256, 512, 16, 51), _Product(torch, F, 300, 8192, 2500, 52), _Product(torch, F, 256, 16384, 3000, 53)
     small.issue(ctx)
     torch.cuda.synchronize()
@@ -168,12 +164,11 @@ def test_captured_product_on_scratch_of_a_smaller_one(env):
         assert p.error(torch, F, ctx) <= TC_TOL
     assert big.error(torch, F, ctx) <= TC_TOL and small.error(torch, F, ctx) <= TC_TOL
     assert all(int((h != 7).sum()) == 0 for h in hold)
-    assert ctx.status() == 0
-    ctx.close()
 
 
 def _device_bytes(torch, F, calls):
-    """Device memory that a fresh context holds after `calls` (which have run before in another one: kernels are loaded)."""
+    """Device memory that the only context with scratch holds after `calls` (which have run before in another one: kernels are
+    loaded, and torch has what it needs)."""
     held = []
     for _ in range(2):
         ctx = F.Context(0)
@@ -207,7 +202,6 @@ def test_fixed_parts_of_a_long_prompt_bound_their_partial_sums(env):
         ctx.set_option(F.OPT_TC_SPLIT, 12)
         p.issue(ctx)
         assert p.error(torch, F, ctx) <= TC_TOL
-    p.error(torch, F, env[2])                              # torch's own workspaces
     assert _device_bytes(torch, F, calls) <= 96 << 20
 
 
@@ -220,7 +214,7 @@ def test_long_prompt_with_little_memory_left(env):
         p.issue(warm, batch=b)
         torch.cuda.synchronize()
         warm.close()
-    ctx = F.Context(0)
+    ctx = env[2]
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
     p.y.fill_(float("nan"))
@@ -233,5 +227,25 @@ def test_long_prompt_with_little_memory_left(env):
         del hog
         torch.cuda.empty_cache()
     assert p.error(torch, F, ctx) <= TC_TOL
-    assert ctx.status() == 0
-    ctx.close()
+
+
+def test_contexts_share_the_pool(env):
+    """Scratch of a context that is gone serves the next one, and the last one gives everything back."""
+    torch, F, ctx = env
+    p, layer = _Product(torch, F, 512, 1024, 100, 81), _Layer(torch, F, 8, 512, 512, 82)
+    c = layer.call(200, 4, 83)
+    held = []
+    for _ in range(3):
+        a, b = F.Context(0), F.Context(0)
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info(0)[0]
+        for x in (a, b):
+            p.issue(x)
+            layer.issue(x, c, 0)
+        a.close()
+        p.issue(b)
+        torch.cuda.synchronize()
+        b.close()
+        held.append(free - torch.cuda.mem_get_info(0)[0])
+    assert max(held[1:]) <= 4 << 20
+    assert p.error(torch, F, ctx) <= TC_TOL
