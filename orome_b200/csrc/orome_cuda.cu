@@ -1390,6 +1390,20 @@ static thread_local bool g_moe_may_skip = false;
 // tiles never leave an expert's rows, so the extent only has to cover every expert).
 constexpr uint32_t MOE_STACK_ROWS = 1u << 24;
 
+// The number of experts of a layer, from above: a stack of whole experts ends before the next one of the three begins.  256, what
+// the routing kernels take at most, where the offsets say nothing (experts whose projections lie between each other's).
+static uint64_t moe_experts_at_most(const OromeExpertLayerRef *L)
+{
+    const OromeExpertProjRef *const p[3] = {&L->gate, &L->up, &L->down};
+    uint64_t most = 0;
+    for (const OromeExpertProjRef *a : p)
+        for (const OromeExpertProjRef *b : p) {
+            const uint64_t room = b->offset > a->offset && a->expert_stride ? (b->offset - a->offset) / a->expert_stride : 0;
+            if (room && (!most || room < most)) most = room;
+        }
+    return most ? most : 256;
+}
+
 extern "C" int orome_cuda_moe_ffn(orome_cuda_ctx *c, const OromeExpertLayerRef *L, uint32_t variant, const float *x_dev,
                                   int n_tokens, int ldx, const uint32_t *idx_dev, const float *w_dev, uint32_t K, uint32_t hidden,
                                   uint32_t inter, float *act_dev, float *out_dev, int ldo, void *stream)
@@ -1422,12 +1436,16 @@ extern "C" int orome_cuda_moe_ffn(orome_cuda_ctx *c, const OromeExpertLayerRef *
     const size_t out_ld_m = n_tokens == 1 ? hidden : (size_t)ldo;
     const bool sizes_ok = (size_t)n_tokens * K * inter <= 0xFFFFFFFFull && out_ld_m * (size_t)n_tokens <= 0xFFFFFFFFull;
     // Token batches: grouped by expert, so that an expert's weights are unpacked once for all of its tokens instead of once for
-    // each (moe_group.cuh).  From eight tokens on: it takes three more launches, so below that the forms that walk the tokens
-    // are faster (a layer of 128 experts, top-8, 2048 x 768, token by token / grouped: 4 tokens 43 / 58 us, 8 tokens 68 / 68,
-    // 16 tokens 115 / 102, 32 tokens 201 / 124, 300 tokens 2383 / 278).
-    const int group_min = 8;
+    // each (moe_group.cuh).  That takes three more launches, and pays by how many (token, slot) pairs an expert gets: 4/3 of the
+    // number of experts means about 1.8 for each one hit.  Walk / grouped, us a layer, down Q5_K: 2048 x 768, 128 experts, 16
+    // tokens of 2 pairs 43 / 57, 8 of 8 68 / 77, 16 of 8 114 / 100, 24 of 8 154 / 118; 64 experts, 12 of 4 52 / 58, 24 of 4 85 / 65;
+    // 32 experts, 16 of 2 42 / 44, 8 of 8 67 / 59; 3072 x 1536, 128 experts, 16 of 8 229 / 239, 24 of 8 326 / 281.  With a down
+    // format that is walked (2048 x 768, Q6_K) both ends of it meet at the same place: 128 experts, 16 of 2 77 / 89, 16 of 8
+    // 244 / 242, 32 of 8 449 / 413; 32 experts, 8 of 8 139 / 138.
+    const uint64_t pairs = (uint64_t)n_tokens * K;
+    const bool shared = pairs >= 64 && 3 * pairs >= 4 * moe_experts_at_most(L);
     auto group_ok = [&](int fmt, uint32_t in_dim, const OromeExpertProjRef &p) {
-        return n_tokens >= group_min && c->kquant_mma && !c->force_generic && !g_moe_may_skip && x_ok16 && orome_moe_group_supported(fmt, in_dim) && p.expert_stride % 16 == 0;
+        return shared && c->kquant_mma && !c->force_generic && !g_moe_may_skip && x_ok16 && orome_moe_group_supported(fmt, in_dim) && p.expert_stride % 16 == 0;
     };
     bool gate_up_done = false;
     const bool group_gu = group_ok(gfmt, hidden, L->gate) && L->up.expert_stride == L->gate.expert_stride, group_dn = group_gu && group_ok(dfmt, inter, L->down);

@@ -664,12 +664,12 @@ def test_batched_product_over_tile_edges(env, fmt, shape, split):
 
 @pytest.mark.parametrize("case", [
     # T, E, K, H, M, gate format, down format, choice of experts, layout
-    (8, 6, 3, 512, 256, synth.Q4_K, synth.Q5_K, "random", 0),          # the smallest grouped batch
-    (9, 5, 2, 256, 512, synth.Q5_K, synth.Q4_K, "random", 1),
+    (8, 9, 8, 512, 256, synth.Q4_K, synth.Q5_K, "random", 0),          # the smallest grouped batch
+    (33, 5, 2, 256, 512, synth.Q5_K, synth.Q4_K, "random", 1),
     (40, 7, 2, 768, 256, synth.Q4_K, synth.Q4_K, "one", 0),             # an expert of 40 tokens, pair blocks of 8
     (90, 12, 8, 512, 768, synth.Q4_K, synth.Q5_K, "one", 0),            # the same with blocks of 32 (33 and more pairs)
     (70, 16, 8, 256, 256, synth.Q5_K, synth.Q6_K, "random", 0),         # a down format that is not grouped
-    (8, 1034, 4, 256, 256, synth.Q4_K, synth.Q5_K, "far", 1),           # experts beyond the sorted range
+    (345, 1034, 4, 256, 256, synth.Q4_K, synth.Q5_K, "far", 1),         # experts beyond the sorted range
     (1100, 8, 2, 256, 256, synth.Q4_K, synth.Q4_K, "random", 0),        # more tokens than one pass takes
 ])
 def test_moe_ffn_grouped_by_expert(env, case):
@@ -692,7 +692,7 @@ def test_moe_ffn_grouped_by_expert(env, case):
             idx[t, :K][idx[t, :K] == 3] = idx[t, 0]
             idx[t, 0] = 3
         if choice == "far":
-            idx[t, :K] = [1024 + t, 1033 - t, 1023, t]
+            idx[t, :K] = [1024 + t % 10, 1033 - t % 10, 1023, t]
         w[t, :K] = rng.random(K)
     w /= w.sum(1, keepdims=True)
     layer = F.ExpertLayerRef(wt.data_ptr(), F.ExpertProjRef(0, sg, gfmt), F.ExpertProjRef(gate.size, sg, gfmt),
@@ -700,7 +700,9 @@ def test_moe_ffn_grouped_by_expert(env, case):
     xt, it, wtt = dev_bytes(torch, x), dev_bytes(torch, idx.view(np.int32)), dev_bytes(torch, w)
     act = torch.full((T, K, M), float("nan"), device="cuda")
     out = torch.full((T, H), float("nan"), device="cuda")
+    before = ctx.launch_count
     ctx.moe_ffn(layer, variant, xt.data_ptr(), T, H, it.data_ptr(), wtt.data_ptr(), K, H, M, act.data_ptr(), out.data_ptr(), H)
+    assert ctx.launch_count - before >= 3                   # two launches walk the tokens
     alone = torch.full((T, H), float("nan"), device="cuda")
     pick = list(range(T)) if T <= 16 else sorted(rng.choice(T, 16, replace=False).tolist()) + [T - 1]
     a1 = torch.empty((K, M), device="cuda")
@@ -714,6 +716,40 @@ def test_moe_ffn_grouped_by_expert(env, case):
     err, err1 = rel_l2(got[pick], want), rel_l2(single[pick], want)
     print(f"{case}: grouped {err:.2e} token by token {err1:.2e}")
     assert err <= 1e-6
+
+
+@pytest.mark.parametrize("T,E,K,lay,grouped", [
+    (8, 128, 2, "stacks", False), (16, 128, 2, "stacks", False), (8, 128, 8, "stacks", False), (22, 128, 8, "stacks", True),
+    (21, 128, 8, "stacks", False), (16, 64, 4, "stacks", False), (22, 64, 4, "stacks", True), (15, 32, 4, "stacks", False),
+    (16, 32, 4, "stacks", True), (7, 9, 8, "stacks", False), (42, 32, 8, "between", False), (43, 32, 8, "between", True)])
+def test_moe_ffn_groups_tokens_where_they_share_experts(env, T, E, K, lay, grouped):
+    """Which way a token batch goes, by the number of launches (grouped: sort, gate/up, quantize, down, sum): by pairs of token and
+    slot for each expert, whose number follows from where the three stacks lie, or is taken to be 256."""
+    torch, F, ctx = env
+    H = M = 256
+    size = synth.tensor_bytes(synth.Q4_K, M, H)
+    gate, up, down = (synth.host_tensor(synth.Q4_K, E * M, H, seed=s) for s in (91, 92, 93))
+    if lay == "stacks":
+        mem, at, stride = np.concatenate([gate, up, down]), [0, E * size, 2 * E * size], size
+    else:                                                    # expert 0's gate, up, down, then expert 1's
+        mem = np.concatenate([v.reshape(E, size) for v in (gate, up, down)], axis=1).reshape(-1)
+        at, stride = [0, size, 2 * size], 3 * size
+    wt = dev_bytes(torch, np.ascontiguousarray(mem))
+    layer = F.ExpertLayerRef(wt.data_ptr(), *(F.ExpertProjRef(o, stride, synth.Q4_K) for o in at))
+    x = np.atleast_2d(synth.host_x(H, T, seed=94))
+    rng = np.random.default_rng(95)
+    idx, w = np.zeros((T, 8), np.uint32), np.zeros((T, 8), np.float32)
+    for t in range(T):
+        idx[t, :K] = rng.permutation(E)[:K]
+    w[:, :K] = rng.random((T, K))
+    xt, it, wtt = dev_bytes(torch, x), dev_bytes(torch, idx.view(np.int32)), dev_bytes(torch, w)
+    act, out = torch.empty((T, K, M), device="cuda"), torch.full((T, H), float("nan"), device="cuda")
+    before = ctx.launch_count
+    ctx.moe_ffn(layer, 0, xt.data_ptr(), T, H, it.data_ptr(), wtt.data_ptr(), K, H, M, act.data_ptr(), out.data_ptr(), H)
+    assert ctx.launch_count - before == (5 if grouped else 2)
+    torch.cuda.synchronize()
+    want = np.stack([oracle.moe_ffn_f64(gate, up, down, (synth.Q4_K,) * 3, (size,) * 3, x[t], H, M, idx[t, :K], w[t, :K], layout=0) for t in (0, T - 1)])
+    assert rel_l2(out.cpu().numpy()[[0, T - 1]], want) <= 1e-6
 
 
 @pytest.mark.parametrize("fmt", QUANT)
