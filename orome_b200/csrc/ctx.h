@@ -110,8 +110,9 @@ long long orome_wait_cycles(const orome_cuda_ctx *c);
 
 // Context scratch of at least `floats` floats for a call on `st`; `usual` floats where nothing is there yet and that many fit.
 int orome_ensure(orome_cuda_ctx *c, Scratch &s, size_t floats, cudaStream_t st, size_t usual = 0);
-// The pool scratch comes from: one per device, shared by its contexts and gone with the last one that used it.
-int orome_pool(orome_cuda_ctx *c);
+// `bytes` in the order of `st` from the pool scratch comes from: one per device, shared by its contexts and gone with the last one
+// that used it.  nullptr: there is no room.
+void *orome_pool_alloc(orome_cuda_ctx *c, size_t bytes, cudaStream_t st);
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                   const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);

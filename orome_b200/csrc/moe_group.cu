@@ -77,10 +77,8 @@ static int take_memory(orome_cuda_ctx *c, size_t bytes, MgMemory &m)
     cudaGraph_t graph = nullptr;
     CU(cudaStreamGetCaptureInfo(m.st, &cap, &id, &graph, nullptr, nullptr));
     if (cap == cudaStreamCaptureStatusNone) {
-        if (orome_pool(c) != OROME_OK) return OROME_ENOTSUP;
-        void *p = nullptr;
-        if (cudaMallocFromPoolAsync(&p, bytes, c->pool, m.st) != cudaSuccess) { (void)cudaGetLastError(); return OROME_ENOTSUP; }
-        m.p = static_cast<uint8_t *>(p);
+        m.p = static_cast<uint8_t *>(orome_pool_alloc(c, bytes, m.st));
+        if (!m.p) return OROME_ENOTSUP;
         m.pooled = true;
         return OROME_OK;
     }

@@ -67,7 +67,7 @@ constexpr uint64_t POOL_KEEP = 512ull << 20;
 static std::mutex g_pool_mutex;
 static struct { cudaMemPool_t pool; int users; } g_pools[64];      // per device ordinal
 
-int orome_pool(orome_cuda_ctx *c)
+static int use_pool(orome_cuda_ctx *c)
 {
     if (c->pool) return OROME_OK;
     if (c->device >= 64) return fail(OROME_ENOTSUP, "device ordinal %d out of range", c->device);
@@ -85,6 +85,18 @@ int orome_pool(orome_cuda_ctx *c)
     ++g.users;
     c->pool = g.pool;
     return OROME_OK;
+}
+
+void *orome_pool_alloc(orome_cuda_ctx *c, size_t bytes, cudaStream_t st)
+{
+    void *p = nullptr;
+    if (use_pool(c) != OROME_OK) return nullptr;
+    if (cudaMallocFromPoolAsync(&p, bytes, c->pool, st) == cudaSuccess) return p;
+    (void)cudaGetLastError();
+    cudaMemPoolTrimTo(c->pool, 0);           // what it keeps in pieces may make room in one
+    if (cudaMallocFromPoolAsync(&p, bytes, c->pool, st) == cudaSuccess) return p;
+    (void)cudaGetLastError();
+    return nullptr;
 }
 
 static void release_pool(orome_cuda_ctx *c)
@@ -1135,20 +1147,22 @@ int orome_ensure(orome_cuda_ctx *c, Scratch &s, size_t floats, cudaStream_t st, 
         else if (s.p) {
             CU(cudaDeviceSynchronize());
             cudaFree(s.p);
+            if (c->pool) cudaMemPoolTrimTo(c->pool, 0);      // the pool would keep it beside the larger one
         }
         s = Scratch();
         for (size_t n : {want, floats}) {
             // From the pool, on the context's own stream and waited for (nothing else is queued there), so that any stream may use
             // it; plainly during a capture, whose mode decides whether that may be.
             void *p = nullptr;
-            cudaError_t e = cudaErrorMemoryAllocation;
-            if (!capturing && orome_pool(c) == OROME_OK) {
-                e = cudaMallocFromPoolAsync(&p, n * sizeof(float), c->pool, c->own_stream);
-                if (e == cudaSuccess) e = cudaStreamSynchronize(c->own_stream);
-            } else e = cudaMalloc(&p, n * sizeof(float));
-            if (e == cudaSuccess) { s.p = static_cast<float *>(p); s.cap = n; break; }
-            (void)cudaGetLastError();
-            if (n == floats) return fail(OROME_ENOMEM, "scratch of %zu floats: %s", floats, cudaGetErrorString(e));
+            if (!capturing) {
+                p = orome_pool_alloc(c, n * sizeof(float), c->own_stream);
+                if (p) CU(cudaStreamSynchronize(c->own_stream));
+            } else if (cudaMalloc(&p, n * sizeof(float)) != cudaSuccess) {
+                (void)cudaGetLastError();
+                p = nullptr;
+            }
+            if (p) { s.p = static_cast<float *>(p); s.cap = n; break; }
+            if (n == floats) return fail(OROME_ENOMEM, "scratch of %zu floats: no device memory%s", floats, capturing ? " (a stream is being captured)" : "");
         }
     }
     s.captured = s.captured || capturing;
