@@ -198,9 +198,9 @@ int orome_launch_tc(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t ou
         a.publish_done = !cut;
         a.layout = layout; a.status = c->status_dev;
         a.pub = *pub;
-        // Rings: four X stages (128 KiB at 256 vectors, where a stage is half a chunk; 128 KiB down to 8 KiB below), the rest for
-        // packed weights (two 34-KiB stages of Q8_0 at 256 vectors, five of Q4_K; six of anything where there is room).  At
-        // least half an SM's shared memory, so that two CTAs (each takes all of tensor memory) never share an SM.
+        // Rings: four X stages of 128 k (256 up to 128 vectors), 128 KiB from 128 vectors on, more of them below, at least 32 KiB;
+        // the rest for packed weights (two 34-KiB stages of Q8_0 at 256 vectors, five of Q4_K; six of anything where there is
+        // room).  At least half an SM's shared memory, so that two CTAs (each takes all of tensor memory) never share an SM.
         const size_t x_stage = (size_t)nt_rows * 64 * (nt_rows > 128 ? 2 : 4), stage = tp_stage_bytes(fmt), room = (size_t)c->smem_optin - 1024 - 1024 - 512;
         a.bs = (uint32_t)std::max<size_t>(4, std::min<size_t>(8, 65536 / x_stage));
         a.ws = (uint32_t)std::min<size_t>(TP_MAX_WS, (room - a.bs * x_stage) / stage);

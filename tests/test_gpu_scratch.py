@@ -145,15 +145,17 @@ TC_TOL = 5e-4          # fp16 operands
 
 
 def test_captured_product_on_scratch_of_a_smaller_one(env):
-    """Captured with room for a part of its packed X (slices); then a larger direct call outgrows the scratch whose address the
-    graph holds, and the graph is replayed."""
+    """Captured with room for a part of its packed X (two slices) and none for partial sums (whole tiles: no third launch a slice);
+    then a larger direct call outgrows the scratch whose address the graph holds, and the graph is replayed."""
     torch, F, ctx = env
     small, p, big = _Product(torch, F, 256, 512, 16, 51), _Product(torch, F, 300, 8192, 2500, 52), _Product(torch, F, 256, 16384, 3000, 53)
     small.issue(ctx)
     torch.cuda.synchronize()
     side, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    before = ctx.launch_count
     with torch.cuda.graph(g, stream=side):
         p.issue(ctx, side.cuda_stream)
+    assert ctx.launch_count - before == 4
     big.issue(ctx)
     torch.cuda.synchronize()
     hold = [torch.full((1 << 20,), 7, dtype=torch.int32, device="cuda") for _ in range(32)]      # what a freed buffer would be given to
