@@ -1450,14 +1450,15 @@ extern "C" int orome_cuda_moe_ffn(orome_cuda_ctx *c, const OromeExpertLayerRef *
     const size_t out_ld_m = n_tokens == 1 ? hidden : (size_t)ldo;
     const bool sizes_ok = (size_t)n_tokens * K * inter <= 0xFFFFFFFFull && out_ld_m * (size_t)n_tokens <= 0xFFFFFFFFull;
     // Token batches: grouped by expert, so that an expert's weights are unpacked once for all of its tokens instead of once for
-    // each (moe_group.cuh).  That takes three more launches, and pays by how many (token, slot) pairs an expert gets: 4/3 of the
-    // number of experts means about 1.8 for each one hit.  Walk / grouped, us a layer, down Q5_K: 2048 x 768, 128 experts, 16
-    // tokens of 2 pairs 43 / 57, 8 of 8 68 / 77, 16 of 8 114 / 100, 24 of 8 154 / 118; 64 experts, 12 of 4 52 / 58, 24 of 4 85 / 65;
+    // each (moe_group.cuh).  That takes three more launches, and pays by how many (token, slot) pairs an expert gets: 3/2 of the
+    // number of experts means about 1.9 for each one hit.  Walk / grouped, us a layer, down Q5_K: 2048 x 768, 128 experts, 16
+    // tokens of 2 pairs 43 / 57, 8 of 8 68 / 77, 16 of 8 114 / 100, 24 of 8 154 / 118; 64 experts, 12 of 4 52 / 58, 24 of 4 85 / 65
+    // (1024 x 512, Q4_K: 22 of 4 39 / 41, 32 of 4 51 / 41); 256 experts, 43 of 8 289 / 186;
     // 32 experts, 16 of 2 42 / 44, 8 of 8 67 / 59; 3072 x 1536, 128 experts, 16 of 8 229 / 239, 24 of 8 326 / 281.  With a down
     // format that is walked (2048 x 768, Q6_K) both ends of it meet at the same place: 128 experts, 16 of 2 77 / 89, 16 of 8
     // 244 / 242, 32 of 8 449 / 413; 32 experts, 8 of 8 139 / 138.
     const uint64_t pairs = (uint64_t)n_tokens * K;
-    const bool shared = pairs >= 64 && 3 * pairs >= 4 * moe_experts_at_most(L);
+    const bool shared = pairs >= 64 && 2 * pairs >= 3 * moe_experts_at_most(L);
     auto group_ok = [&](int fmt, uint32_t in_dim, const OromeExpertProjRef &p) {
         return shared && c->kquant_mma && !c->force_generic && !g_moe_may_skip && x_ok16 && orome_moe_group_supported(fmt, in_dim) && p.expert_stride % 16 == 0;
     };

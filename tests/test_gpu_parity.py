@@ -669,7 +669,7 @@ def test_batched_product_over_tile_edges(env, fmt, shape, split):
     (40, 7, 2, 768, 256, synth.Q4_K, synth.Q4_K, "one", 0),             # an expert of 40 tokens, pair blocks of 8
     (90, 12, 8, 512, 768, synth.Q4_K, synth.Q5_K, "one", 0),            # the same with blocks of 32 (33 and more pairs)
     (70, 16, 8, 256, 256, synth.Q5_K, synth.Q6_K, "random", 0),         # a down format that is not grouped
-    (345, 1034, 4, 256, 256, synth.Q4_K, synth.Q5_K, "far", 1),         # experts beyond the sorted range
+    (388, 1034, 4, 256, 256, synth.Q4_K, synth.Q5_K, "far", 1),         # experts beyond the sorted range
     (1100, 8, 2, 256, 256, synth.Q4_K, synth.Q4_K, "random", 0),        # more tokens than one pass takes
 ])
 def test_moe_ffn_grouped_by_expert(env, case):
@@ -719,9 +719,9 @@ def test_moe_ffn_grouped_by_expert(env, case):
 
 
 @pytest.mark.parametrize("T,E,K,lay,grouped", [
-    (8, 128, 2, "stacks", False), (16, 128, 2, "stacks", False), (8, 128, 8, "stacks", False), (22, 128, 8, "stacks", True),
-    (21, 128, 8, "stacks", False), (16, 64, 4, "stacks", False), (22, 64, 4, "stacks", True), (15, 32, 4, "stacks", False),
-    (16, 32, 4, "stacks", True), (7, 9, 8, "stacks", False), (42, 32, 8, "between", False), (43, 32, 8, "between", True)])
+    (8, 128, 2, "stacks", False), (16, 128, 2, "stacks", False), (8, 128, 8, "stacks", False), (23, 128, 8, "stacks", False),
+    (24, 128, 8, "stacks", True), (23, 64, 4, "stacks", False), (24, 64, 4, "stacks", True), (15, 32, 4, "stacks", False),
+    (16, 32, 4, "stacks", True), (7, 9, 8, "stacks", False), (47, 32, 8, "between", False), (48, 32, 8, "between", True)])
 def test_moe_ffn_groups_tokens_where_they_share_experts(env, T, E, K, lay, grouped):
     """Which way a token batch goes, by the number of launches (grouped: sort, gate/up, quantize, down, sum): by pairs of token and
     slot for each expert, whose number follows from where the three stacks lie, or is taken to be 256."""
