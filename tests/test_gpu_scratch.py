@@ -185,14 +185,15 @@ def _device_bytes(torch, F, calls):
 
 
 def test_scratch_that_grows_is_no_larger_than_its_last_size(env):
-    """Packed X of 2048, 3000 and 4096 vectors of 8192 (64 MiB at last), and at most two partial tiles per pair of SMs (37 MiB)."""
+    """Packed X of 2400, 3600 and 4096 vectors of 16384 (128 MiB at last; each kept and doubled: 225), and two partial tiles per
+    pair of SMs (37 MiB); the pool takes memory 32 MiB at a time."""
     torch, F, _ = env
-    p = _Product(torch, F, 512, 8192, 4096, 61)
+    p = _Product(torch, F, 512, 16384, 4096, 61)
 
     def calls(ctx):
-        for b in (2048, 3000, 4096):
+        for b in (2400, 3600, 4096):
             p.issue(ctx, batch=b)
-    assert _device_bytes(torch, F, calls) <= (64 + 37 + 8) << 20
+    assert _device_bytes(torch, F, calls) <= (128 + 37 + 2 * 32) << 20
 
 
 def test_fixed_parts_of_a_long_prompt_bound_their_partial_sums(env):
