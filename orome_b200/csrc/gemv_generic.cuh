@@ -29,7 +29,7 @@ __device__ __forceinline__ uint2 ld8_a2(const uint8_t *p)
 {
     const bool odd = (reinterpret_cast<uintptr_t>(p) & 2u) != 0;
     const uint32_t *q = reinterpret_cast<const uint32_t *>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)3);
-    const uint32_t a = __ldg(q), b = __ldg(q + 1), c = odd ? (uint32_t)__ldg(reinterpret_cast<const unsigned short *>(p + 6)) : 0u, sh = odd ? 16u : 0u;
+    const uint32_t a = __ldcg(q), b = __ldcg(q + 1), c = odd ? (uint32_t)__ldcg(reinterpret_cast<const unsigned short *>(p + 6)) : 0u, sh = odd ? 16u : 0u;
     return make_uint2(__funnelshift_r(a, b, sh), __funnelshift_r(b, c, sh));
 }
 
@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(256)
 dequant_flat_kernel(const uint8_t *__restrict__ blocks, uint64_t pieces, int layout, float *__restrict__ out)
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");      // the packed rows may be what the kernel before has written
+    asm volatile("griddepcontrol.wait;" ::: "memory");      // the packed rows may be what the kernel before has written (hence no non-coherent loads)
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t base = ((uint64_t)blockIdx.x * 8u + (threadIdx.x >> 5)) * (32u * DQ_PIECES) + lane;
     uint2 q[DQ_PIECES], h[DQ_PIECES];
@@ -56,22 +56,22 @@ dequant_flat_kernel(const uint8_t *__restrict__ blocks, uint64_t pieces, int lay
         if (i >= pieces) continue;
         if constexpr (FMT == FMT_Q8_0) {
             const uint8_t *blk = blocks + (i >> 2) * 34u;
-            d[k] = __ldg(reinterpret_cast<const unsigned short *>(blk));
+            d[k] = __ldcg(reinterpret_cast<const unsigned short *>(blk));
             q[k] = ld8_a2(blk + 2 + 8u * (i & 3u));
         } else if constexpr (FMT == FMT_Q6_K) {
             const uint8_t *sb = blocks + (i >> 5) * 210u;
             const uint32_t p = (uint32_t)i & 31u, half = p >> 4, j = (p >> 2) & 3u, l = 8u * (p & 3u);
             q[k] = ld8_a2(sb + 64u * half + 32u * (j & 1u) + l);
             h[k] = ld8_a2(sb + 128u + 32u * half + l);
-            sc[k] = (int)(signed char)__ldg(sb + 192u + 8u * half + 2u * j + (l >> 4));
-            d[k] = __ldg(reinterpret_cast<const unsigned short *>(sb + 208));
+            sc[k] = (int)(signed char)__ldcg(sb + 192u + 8u * half + 2u * j + (l >> 4));
+            d[k] = __ldcg(reinterpret_cast<const unsigned short *>(sb + 208));
         } else {
             constexpr uint32_t UNIT = FMT == FMT_Q4_K ? 144u : 176u, QOFF = FMT == FMT_Q4_K ? 16u : 48u;
             const uint8_t *sb = blocks + (i >> 5) * UNIT;
             const uint32_t p = (uint32_t)i & 31u;
-            hd[k] = __ldg(reinterpret_cast<const uint4 *>(sb));
-            q[k] = __ldg(reinterpret_cast<const uint2 *>(sb + QOFF + 32u * (p >> 3) + 8u * (p & 3u)));
-            if constexpr (FMT == FMT_Q5_K) h[k] = __ldg(reinterpret_cast<const uint2 *>(sb + 16u + 8u * (p & 3u)));
+            hd[k] = __ldcg(reinterpret_cast<const uint4 *>(sb));
+            q[k] = __ldcg(reinterpret_cast<const uint2 *>(sb + QOFF + 32u * (p >> 3) + 8u * (p & 3u)));
+            if constexpr (FMT == FMT_Q5_K) h[k] = __ldcg(reinterpret_cast<const uint2 *>(sb + 16u + 8u * (p & 3u)));
         }
     }
 #pragma unroll
