@@ -407,13 +407,12 @@ gemm_pair_kernel(const __grid_constant__ TpArgs a)
         const uint32_t tmem_a = tmem_base + lane_addr + kq * 32u;
         uint32_t s = 0, pw = 0, sa = 0, pa = 1, seg = 0, tile = tile0, chunk = chunk0;
         uint32_t row_off = 0;        // Q6_K: the row's first byte inside its 16-byte piece, before the chunk's offset
-        // A lane whose wait has run out goes through the motions to the end: s_abort may be set between two lanes' looks at it, and
-        // what follows a wait (__syncwarp, tensor memory accesses) needs the warp together.
-        bool alive = true;
+        // s_abort may be set between two lanes' looks at it, but what follows a wait (__syncwarp, tensor memory accesses) needs the
+        // warp together: the lanes vote, where they have to meet anyway, and give up as a whole.
         for (uint32_t i = 0; i < n_units; ++i) {
             if (FMT == FMT_Q6_K && (i == 0 || chunk == 0))
                 row_off = (uint32_t)reinterpret_cast<uintptr_t>(a.w) + ((tile / a.ntiles) * TP_ROWS + rank * TC_M + r) * a.row_bytes;
-            if (alive) alive = wait(w_full + s, pw);
+            bool ok = wait(w_full + s, pw);
             TcPacked<FMT> pk;
             uint32_t row_s = smem_u32(w_stages + s * STAGE) + r * PITCH;
             if constexpr (FMT == FMT_Q6_K) row_s += (row_off + chunk * 210u) & 15u;
@@ -421,8 +420,8 @@ gemm_pair_kernel(const __grid_constant__ TpArgs a)
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(w_empty + s));
             if (++s == WS) { s = 0; pw ^= 1u; }
-            if (alive && i >= AS) alive = wait(a_empty + sa, pa);
-            __syncwarp();
+            if (ok && i >= AS) ok = wait(a_empty + sa, pa);
+            if (!__all_sync(0xffffffffu, ok)) break;
             tc_fence_after();
             const uint32_t taddr = tmem_a + sa * 128u;
             switch (kq) {                         // warp-uniform; the sub-block index is a compile-time constant inside
@@ -442,8 +441,7 @@ gemm_pair_kernel(const __grid_constant__ TpArgs a)
             const bool whole = u_lo <= t_lo && u_lo + n_units >= t_lo + a.chunks;
             const uint32_t grow = (tile / a.ntiles) * TP_ROWS + rank * TC_M + r, n_base = (tile % a.ntiles) * a.nt_rows;
             float *part = a.part + ((size_t)cl * a.slots + (u_lo <= t_lo ? a.slots - 1 : 0)) * a.nt_rows * TP_ROWS + rank * TC_M + r;   // 0: the share starts inside the tile
-            if (alive) alive = wait(acc_full, seg & 1u);
-            __syncwarp();
+            const bool done = __all_sync(0xffffffffu, wait(acc_full, seg & 1u));
             tc_fence_after();
             for (uint32_t n0 = kq * 16u; n0 < a.nt_rows; n0 += 64u) {
                 uint32_t v[16];
@@ -453,7 +451,7 @@ gemm_pair_kernel(const __grid_constant__ TpArgs a)
                                "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
                              : "r"(tmem_base + lane_addr + ACC_COL + n0));
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (!alive) continue;
+                if (!done) continue;
                 if (!whole) {
 #pragma unroll
                     for (uint32_t q = 0; q < 16; ++q) part[(size_t)(n0 + q) * TP_ROWS] = __uint_as_float(v[q]);
@@ -470,6 +468,7 @@ gemm_pair_kernel(const __grid_constant__ TpArgs a)
             }
             tc_fence_before();
             __syncwarp();
+            if (!done) break;
             if (lane == 0) mbar_arrive_cluster(acc_empty0);
             ++seg;
             if (chunk == a.chunks) { chunk = 0; ++tile; }
