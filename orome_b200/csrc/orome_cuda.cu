@@ -5,6 +5,7 @@
 #include "ctx.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -1450,15 +1451,17 @@ extern "C" int orome_cuda_moe_ffn(orome_cuda_ctx *c, const OromeExpertLayerRef *
     const size_t out_ld_m = n_tokens == 1 ? hidden : (size_t)ldo;
     const bool sizes_ok = (size_t)n_tokens * K * inter <= 0xFFFFFFFFull && out_ld_m * (size_t)n_tokens <= 0xFFFFFFFFull;
     // Token batches: grouped by expert, so that an expert's weights are unpacked once for all of its tokens instead of once for
-    // each (moe_group.cuh).  That takes three more launches, and pays by how many (token, slot) pairs an expert gets: 3/2 of the
-    // number of experts means about 1.9 for each one hit.  Walk / grouped, us a layer, down Q5_K: 2048 x 768, 128 experts, 16
-    // tokens of 2 pairs 43 / 57, 8 of 8 68 / 77, 16 of 8 114 / 100, 24 of 8 154 / 118; 64 experts, 12 of 4 52 / 58, 24 of 4 85 / 65
-    // (1024 x 512, Q4_K: 22 of 4 39 / 41, 32 of 4 51 / 41); 256 experts, 43 of 8 289 / 186;
-    // 32 experts, 16 of 2 42 / 44, 8 of 8 67 / 59; 3072 x 1536, 128 experts, 16 of 8 229 / 239, 24 of 8 326 / 281.  With a down
-    // format that is walked (2048 x 768, Q6_K) both ends of it meet at the same place: 128 experts, 16 of 2 77 / 89, 16 of 8
-    // 244 / 242, 32 of 8 449 / 413; 32 experts, 8 of 8 139 / 138.
-    const uint64_t pairs = (uint64_t)n_tokens * K;
-    const bool shared = pairs >= 64 && 2 * pairs >= 3 * moe_experts_at_most(L);
+    // each (moe_group.cuh).  Whether that pays depends on how many (token, slot) pairs an expert gets.  A model in us a layer, fitted
+    // to 190 measured shapes (it picks the faster form or one within 6 %): three more launches and their passes cost 7 + 0.7 m,
+    // m = 2^20 weights of a projection; an expert hit costs 0.46 m grouped, a pair about 0.1 + 0.3 to 0.4 m walked; three quarters
+    // of the last two where the down format is walked either way.  Walk / grouped, Q4_K gate/up, Q5_K down: 2048 x 768, 128 experts,
+    // 16 tokens of 2 43 / 57, 8 of 8 68 / 77, 16 of 8 114 / 100, 32 of 8 201 / 125; 64 experts, 12 of 4 52 / 58, 24 of 4 85 / 65;
+    // 32 experts, 16 of 2 42 / 44, 8 of 8 67 / 59; 3072 x 1536, 128 experts, 16 of 8 229 / 239, 24 of 8 326 / 281; 1024 x 512, 128
+    // experts, 8 of 8 36 / 43, 24 of 8 73 / 55; Q6_K down, 2048 x 768, 128 experts, 8 of 8 140 / 150, 16 of 8 244 / 242, 32 of 8
+    // 449 / 413.  Fewer than 48 pairs were not faster anywhere.
+    const double pairs = (double)n_tokens * K, experts = (double)moe_experts_at_most(L), m = (double)hidden * inter / 1048576.0;
+    const double hit = experts * (1.0 - std::pow(1.0 - 1.0 / experts, pairs)), part = orome_moe_group_supported(dfmt, inter) ? 1.0 : 0.75;
+    const bool shared = pairs >= 48.0 && 7.0 + 0.7 * m + part * 0.46 * m * hit <= part * pairs * std::min(0.075 + 0.38 * m, 0.14 + 0.29 * m);
     auto group_ok = [&](int fmt, uint32_t in_dim, const OromeExpertProjRef &p) {
         return shared && c->kquant_mma && !c->force_generic && !g_moe_may_skip && x_ok16 && orome_moe_group_supported(fmt, in_dim) && p.expert_stride % 16 == 0;
     };

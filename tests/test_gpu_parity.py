@@ -664,8 +664,8 @@ def test_batched_product_over_tile_edges(env, fmt, shape, split):
 
 @pytest.mark.parametrize("case", [
     # T, E, K, H, M, gate format, down format, choice of experts, layout
-    (8, 9, 8, 512, 256, synth.Q4_K, synth.Q5_K, "random", 0),          # the smallest grouped batch
-    (33, 5, 2, 256, 512, synth.Q5_K, synth.Q4_K, "random", 1),
+    (24, 9, 8, 512, 256, synth.Q4_K, synth.Q5_K, "random", 0),
+    (90, 5, 2, 256, 512, synth.Q5_K, synth.Q4_K, "random", 1),
     (40, 7, 2, 768, 256, synth.Q4_K, synth.Q4_K, "one", 0),             # an expert of 40 tokens, pair blocks of 8
     (90, 12, 8, 512, 768, synth.Q4_K, synth.Q5_K, "one", 0),            # the same with blocks of 32 (33 and more pairs)
     (70, 16, 8, 256, 256, synth.Q5_K, synth.Q6_K, "random", 0),         # a down format that is not grouped
@@ -719,12 +719,12 @@ def test_moe_ffn_grouped_by_expert(env, case):
 
 
 @pytest.mark.parametrize("T,E,K,lay,grouped", [
-    (8, 128, 2, "stacks", False), (16, 128, 2, "stacks", False), (8, 128, 8, "stacks", False), (23, 128, 8, "stacks", False),
-    (24, 128, 8, "stacks", True), (23, 64, 4, "stacks", False), (24, 64, 4, "stacks", True), (15, 32, 4, "stacks", False),
-    (16, 32, 4, "stacks", True), (7, 9, 8, "stacks", False), (47, 32, 8, "between", False), (48, 32, 8, "between", True)])
+    (8, 128, 2, "stacks", False), (16, 128, 2, "stacks", False), (8, 128, 8, "stacks", False), (10, 128, 8, "stacks", False),
+    (13, 128, 8, "stacks", True), (16, 64, 4, "stacks", False), (24, 64, 4, "stacks", True), (5, 9, 8, "stacks", False),
+    (9, 32, 8, "stacks", False), (11, 32, 8, "stacks", True), (11, 32, 8, "between", False), (14, 32, 8, "between", True)])
 def test_moe_ffn_groups_tokens_where_they_share_experts(env, T, E, K, lay, grouped):
-    """Which way a token batch goes, by the number of launches (grouped: sort, gate/up, quantize, down, sum): by pairs of token and
-    slot for each expert, whose number follows from where the three stacks lie, or is taken to be 256."""
+    """Which way a token batch goes, by the number of launches (grouped: sort, gate/up, quantize, down, sum): by how many pairs of
+    token and slot an expert gets, the number of experts following from where the three stacks lie, or taken to be 256."""
     torch, F, ctx = env
     H = M = 256
     size = synth.tensor_bytes(synth.Q4_K, M, H)
