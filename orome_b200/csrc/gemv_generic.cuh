@@ -43,9 +43,15 @@ __global__ void __launch_bounds__(256)
 dequant_flat_kernel(const uint8_t *__restrict__ blocks, uint64_t pieces, int layout, float *__restrict__ out)
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");      // the packed rows may be what the kernel before has written (hence no non-coherent loads)
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t base = ((uint64_t)blockIdx.x * 8u + (threadIdx.x >> 5)) * (32u * DQ_PIECES) + lane;
+    // The packed rows may be what the kernel before has written: nothing of them is loaded before the wait (nor without coherence
+    // after it), but their lines may come to the L2, where that kernel's writes go too (5120 x 4096 Q6_K, back to back: 29.8 us
+    // without, 25.7 with).
+    constexpr uint32_t GROUP = FMT == FMT_Q8_0 ? 4u : 32u, BLOCK = FMT == FMT_Q8_0 ? 34u : FMT == FMT_Q4_K ? 144u : FMT == FMT_Q5_K ? 176u : 210u;
+    const uint64_t first = (base - lane) / GROUP * BLOCK + 128u * lane;
+    if (128u * lane < 32u * DQ_PIECES / GROUP * BLOCK && first < pieces / GROUP * BLOCK) asm volatile("prefetch.global.L2 [%0];" ::"l"(blocks + first));
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     uint2 q[DQ_PIECES], h[DQ_PIECES];
     uint4 hd[DQ_PIECES];
     uint32_t d[DQ_PIECES];
