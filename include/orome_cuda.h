@@ -238,7 +238,7 @@ int  orome_cuda_moe_route_pair(orome_cuda_ctx *ctx, const OromeTensorRef *router
  * Same result as orome_cuda_moe_route called without a logits buffer, but the router
  * logits go to a fixed array that is part of the library image (device memory of
  * OROME_ROUTE_STATIC_MAX_LOGITS floats, 64 KiB, held by every GPU that loads the library
- * until the process exits) instead of context scratch obtained with cudaMalloc.  It is
+ * until the process exits) instead of context scratch allocated on demand.  It is
  * meant for the per-token loop of an engine that, like the reference, reserves all device
  * memory up front and then forbids allocation - cudaMalloc synchronises the whole device
  * and can fail once the model has filled HBM - and for hosts whose device memory belongs
