@@ -395,7 +395,7 @@ __global__ void splitk_reduce_kernel(const float *__restrict__ part, uint32_t sp
     const size_t n = (size_t)batch * rows;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         float acc = 0.0f;
-        for (uint32_t s = 0; s < split; ++s) acc += part[(size_t)s * n + i];
+        for (uint32_t s = 0; s < split; ++s) acc += __ldcg(part + (size_t)s * n + i);
         float *dst = y + (i / rows) * ldy + (i % rows);
         *dst = acc;
         if (pub.npeers > 0) tc_publish(pub, dst, acc, pub_tag);

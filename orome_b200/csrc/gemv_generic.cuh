@@ -206,7 +206,7 @@ gemv_f32_kernel(const float *__restrict__ W, uint32_t out_dim, uint32_t in_dim, 
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     if (c0 + 128 * u < n4) {
-                        const float4 xv = x4[c0 + 128 * u];
+                        const float4 xv = __ldcg(x4 + c0 + 128 * u);
                         acc[i] = fmaf(w[u].x, xv.x, fmaf(w[u].y, xv.y, fmaf(w[u].z, xv.z, fmaf(w[u].w, xv.w, acc[i]))));
                     }
                 }

@@ -212,6 +212,9 @@ __device__ __forceinline__ float4 ld_gathered4(const uint2 *slots, unsigned int 
     }
     return make_float4(__uint_as_float(a.x), __uint_as_float(a.z), __uint_as_float(b.x), __uint_as_float(b.z));
 }
+// What a predecessor wrote is read after this with coherent loads (__ldcg): ld.global.nc, which the compiler also makes of loads
+// through const __restrict__ pointers, promises that nothing writes the data while the kernel runs, and a kernel launched ahead
+// runs while its predecessor writes (such a load was seen served before the wait).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -24,7 +24,7 @@ route_topk_kernel(const float *__restrict__ logits, int ld_logits, uint32_t n_ex
     asm volatile("griddepcontrol.wait;" ::: "memory");   // the logits are the previous kernel's output
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const float *lg = logits + (size_t)blockIdx.x * ld_logits;
-    float my = tid < n_experts ? lg[tid] : -INFINITY;
+    float my = tid < n_experts ? __ldcg(lg + tid) : -INFINITY;
     const uint32_t limit = K < 8 ? K : 8;
     for (uint32_t round = 0; round < limit; ++round) {
         const uint32_t buf = round & 1u;
@@ -62,7 +62,7 @@ route_topk_kernel(const float *__restrict__ logits, int ld_logits, uint32_t n_ex
             wo[k] = k < limit ? w[k] * inv : 0.0f;
         }
         // the raw logit of the shared-expert gate, which sits after the router logits (out_params[8], shaders.metal:1232)
-        if (shared_logit_out) shared_logit_out[blockIdx.x] = lg[n_experts];
+        if (shared_logit_out) shared_logit_out[blockIdx.x] = __ldcg(lg + n_experts);
     }
 }
 
@@ -76,11 +76,11 @@ moe_combine_kernel(const float *__restrict__ h_mid, int ld_mid, const float *__r
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t t = blockIdx.y, h = blockIdx.x * blockDim.x + threadIdx.x;
     if (h >= hidden) return;
-    float v = moe[(size_t)t * ld_moe + h];
-    if (h_mid) v = h_mid[(size_t)t * ld_mid + h] + v;
+    float v = __ldcg(moe + (size_t)t * ld_moe + h);
+    if (h_mid) v = __ldcg(h_mid + (size_t)t * ld_mid + h) + v;
     if (shared_out) {
-        const float gate = 1.0f / (1.0f + expf(-shared_logit[t]));
-        v += gate * shared_out[(size_t)t * ld_shared + h];
+        const float gate = 1.0f / (1.0f + expf(-__ldcg(shared_logit + t)));
+        v += gate * __ldcg(shared_out + (size_t)t * ld_shared + h);
     }
     out[(size_t)t * ldo + h] = v;
 }
@@ -92,7 +92,7 @@ __global__ void moe_localize_kernel(const uint32_t *__restrict__ idx, uint32_t n
     asm volatile("griddepcontrol.wait;" ::: "memory");   // the indices are the routing kernel's output
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
-        const uint32_t e = idx[i] - first;
+        const uint32_t e = __ldcg(idx + i) - first;
         out[i] = e < count ? e : 0xFFFFFFFFu;
     }
 }

@@ -119,7 +119,7 @@ moe_prepare_kernel(const uint32_t *__restrict__ idx, uint32_t n_tokens, uint32_t
     __syncthreads();
     const uint32_t n = n_tokens * K;
     for (uint32_t i = tid; i < n; i += 1024u) {
-        const uint32_t e = idx[(i / K) * 8u + i % K];
+        const uint32_t e = __ldcg(idx + (i / K) * 8u + i % K);
         if (e < (uint32_t)MG_BINS) atomicAdd(&s_count[e], 1u);
     }
     __syncthreads();
@@ -158,7 +158,7 @@ moe_prepare_kernel(const uint32_t *__restrict__ idx, uint32_t n_tokens, uint32_t
     s_count[tid] = start;                          // from here on: where the expert's next pair goes
     __syncthreads();
     for (uint32_t i = tid; i < n; i += 1024u) {
-        const uint32_t t = i / K, k = i - t * K, e = idx[t * 8u + k];
+        const uint32_t t = i / K, k = i - t * K, e = __ldcg(idx + t * 8u + k);
         uint32_t pos;
         if (e < (uint32_t)MG_BINS) pos = atomicAdd(&s_count[e], 1u);
         else {
