@@ -78,6 +78,12 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t mapped)      // an 
 {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(mapped) : "memory");
 }
+__device__ __forceinline__ bool elect_one()      // one lane of the (whole) warp, always the same
+{
+    uint32_t p;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ void tp_commit(uint32_t bar)      // both CTAs' barrier at this offset
 {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
@@ -346,7 +352,7 @@ gemm_pair_kernel(const __grid_constant__ TpArgs a)
             for (uint32_t i = 0; i < n_units && ok; ++i) {
                 const uint8_t *src = reinterpret_cast<const uint8_t *>(a.xp) + ((size_t)(2 * nt + rank) * a.chunks + chunk) * (TC_SLABS * slab_bytes);
                 for (uint32_t j = 0; j < XPU; ++j, ++n) {
-                    if (n >= BS) { ok = wait(b_empty + s, ph); if (!ok) break; asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+                    if (n >= BS) { ok = wait(b_empty + s, ph); if (!ok) break; }      // only MMAs and bulk copies touch X: no proxy to order
                     mbar_expect_tx(smem_u32(b_full + s), x_bytes);
                     bulk_g2s(smem_u32(x_stages + s * x_bytes), src + j * x_bytes, x_bytes, smem_u32(b_full + s));
                     if (++s == BS) { s = 0; ph ^= 1u; }
@@ -368,36 +374,45 @@ gemm_pair_kernel(const __grid_constant__ TpArgs a)
                 mbar_arrive_cluster(peer + 8u * s);
                 if (++s == BS) { s = 0; ph ^= 1u; }
             }
-        } else if (lane == 0) {
+        } else if (rank == 0) {
             // ---- MMA issue ----
+            // The whole warp walks the loop and one elected lane issues: descriptors and columns then stay in uniform registers.  As
+            // the body of `if (lane == 0)` every operand of every MMA had to be moved there, and with the dequant warps competing for
+            // issue slots the 16 MMAs of a unit took ~600-900 clocks longer (12288 x 4096 Q8_0 at 2048 vectors 3180 -> 2580 clocks a
+            // unit, 17408 x 5120 Q4_K at 333 2680 -> 1830, 12288 x 4096 Q4_K at 64 2200 -> 1420).
             const uint32_t idesc = (1u << 4) | ((a.nt_rows >> 3) << 17) | ((uint32_t)(TP_ROWS >> 4) << 24);   // fp32 accumulate, fp16 x fp16, K-major both
             const uint32_t slab_step = slab_bytes >> 4, acc = tmem_base + ACC_COL;
             uint32_t sa = 0, pa = 0, sb = 0, pb = 0, seg = 0, chunk = chunk0;
             bool ok = true;
             for (uint32_t i = 0; i < n_units && ok; ++i) {
                 const bool first = i == 0 || chunk == 0;
-                if (first && seg > 0) { if (!wait(acc_empty, (seg - 1) & 1u)) break; }      // the previous tile's sums have been read
-                if (!wait(a_full + sa, pa)) break;
-                uint32_t a_col = tmem_base + sa * 128u, accumulate = !first;
+                if (first && seg > 0 && !__all_sync(0xffffffffu, wait(acc_empty, (seg - 1) & 1u))) break;      // the previous tile's sums have been read
+                if (!__all_sync(0xffffffffu, wait(a_full + sa, pa))) break;
+                const uint32_t a_col = tmem_base + sa * 128u;
 #pragma unroll
                 for (uint32_t j = 0; j < XPU; ++j) {
-                    if (!wait(b_full + sb, pb)) { ok = false; break; }
+                    if (!__all_sync(0xffffffffu, wait(b_full + sb, pb))) { ok = false; break; }
                     tc_fence_after();
-                    const uint64_t db0 = tc_desc_sw128(smem_u32(x_stages + sb * x_bytes));
+                    if (elect_one()) {
+                        const uint64_t db0 = tc_desc_sw128(smem_u32(x_stages + sb * x_bytes));
 #pragma unroll
-                    for (uint32_t k16 = 0; k16 < 4 * SL; ++k16) {
-                        tp_mma(acc, a_col, db0 + (k16 >> 2) * slab_step + (k16 & 3u) * 2u, idesc, accumulate);      // a step of 32 bytes is 2 in the descriptor
-                        accumulate = 1;
-                        a_col += 8u;
+                        for (uint32_t k16 = 0; k16 < 4 * SL; ++k16)      // a step of 32 bytes is 2 in the descriptor
+                            tp_mma(acc, a_col + (j * 4 * SL + k16) * 8u, db0 + (k16 >> 2) * slab_step + (k16 & 3u) * 2u, idesc, j == 0 && k16 == 0 ? !first : 1u);
+                        tp_commit(smem_u32(b_empty + sb));
                     }
-                    tp_commit(smem_u32(b_empty + sb));
+                    __syncwarp();
                     if (++sb == BS) { sb = 0; pb ^= 1u; }
                 }
                 if (!ok) break;
-                tp_commit(smem_u32(a_empty + sa));
+                if (elect_one()) tp_commit(smem_u32(a_empty + sa));
+                __syncwarp();
                 if (++sa == AS) { sa = 0; pa ^= 1u; }
                 if (++chunk == a.chunks) chunk = 0;
-                if (chunk == 0 || i + 1 == n_units) { tp_commit(smem_u32(acc_full)); ++seg; }
+                if (chunk == 0 || i + 1 == n_units) {
+                    if (elect_one()) tp_commit(smem_u32(acc_full));
+                    __syncwarp();
+                    ++seg;
+                }
             }
         }
     } else {
