@@ -411,104 +411,125 @@ __device__ __forceinline__ uint32_t plane_word(uint32_t u0, uint32_t u1, uint32_
     return __byte_perm(__byte_perm(u0, u1, sel), __byte_perm(u2, u3, sel), 0x5410) ^ 0x80808080u;
 }
 
+// The four (three, two) byte planes of four elements.
+template <int NP>
+__device__ __forceinline__ void plane_words(uint32_t u0, uint32_t u1, uint32_t u2, uint32_t u3, uint32_t (&pl)[NP])
+{
+    const uint32_t a = __byte_perm(u0, u1, 0x5140), b = __byte_perm(u2, u3, 0x5140);      // bytes 0, 0, 1, 1 of a pair
+    pl[0] = __byte_perm(a, b, 0x5410) ^ 0x80808080u;
+    pl[1] = __byte_perm(a, b, 0x7632) ^ 0x80808080u;
+    if constexpr (NP > 2) {
+        const uint32_t c = __byte_perm(u0, u1, 0x7362), d = __byte_perm(u2, u3, 0x7362);
+        pl[2] = __byte_perm(c, d, 0x5410) ^ 0x80808080u;
+        if constexpr (NP > 3) pl[3] = __byte_perm(c, d, 0x7632) ^ 0x80808080u;
+    }
+}
+// Eight floats, not from L1.  In one access where x is 32-byte aligned: lanes 32 bytes apart in 16-byte accesses touch every line
+// twice (12288-wide, all CTAs at once: 2180 clocks against 1540).
+__device__ __forceinline__ void ldcg8(const float *p, bool whole, float4 &a, float4 &b)
+{
+    if (whole) asm volatile("ld.global.cg.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                            : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "l"(p));
+    else { a = __ldcg(reinterpret_cast<const float4 *>(p)); b = __ldcg(reinterpret_cast<const float4 *>(p) + 1); }
+}
+// max |v| over the warp; NaN where all lanes hold one, as fmaxf gives it
+__device__ __forceinline__ float warp_abs_max(float v)
+{
+    float r;
+    asm volatile("redux.sync.max.abs.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
 // x -> shared memory, one warp per superblock: lane l owns elements 8l..8l+7 (sub-block l / 4, bytes 8 (l % 4)..).
 // Layout per superblock u at xq + u * MMA_XQ_SB: [sub-block j][plane p][32 bytes], then at +768 [plane p][8 sum bytes];
-// xs[u], sxs[u] after all superblocks.  A warp takes up to four superblocks at a time: their loads are issued together
-// and their shuffle reductions interleave.
+// xs[u], sxs[u] after all superblocks.  A warp takes up to five superblocks at a time: their loads are issued together
+// and their reductions interleave.
 // Q6 form: instead of the float sums, the sums of the signed digits over every 16 elements, as two balanced bytes:
 // at +768 [plane p][low / high byte][16 groups].
 // With `slots` set x is a gathered vector read from its {value, tag} slots (polled for `tag`); false = a poll expired.
 // NTOK = 2: vector `b` (0 or 1) of two, into its columns of the wider layout (see mma_xq_sb).
-// NORM: x is RMS-normalised on the way, (x * rsqrt(sum(norm_parts) / n + eps)) * bf16 weight; the partial sums are requested
-// before the vector and added up after it, so that the two round trips to L2 overlap.
+// NORM: x is multiplied by the bf16 norm weights on the way; the common factor 1 / rms is the caller's, who applies it to the sums,
+// since nothing before them needs it.
+// What bounds it: every CTA does this between its predecessor's end and its own first mma, so it is latency, and then issue slots:
+// a maximum is one redux instead of five shuffles, and the up to ten factors of a round are worked out by ten lanes at once.
 template <int NP, bool Q6, int NTOK = 1, bool NORM = false>
 __device__ __forceinline__ bool quantize_x_mma(const float *__restrict__ x, uint32_t units, uint8_t *xq, uint32_t warp, uint32_t lane,
                                                uint32_t nwarps, const uint2 *slots = nullptr, unsigned int tag = 0, uint32_t b_tok = 0,
-                                               const uint16_t *norm_w = nullptr, const float *norm_parts = nullptr, float norm_eps = 0.0f,
-                                               float *s_share = nullptr)
+                                               const uint16_t *norm_w = nullptr)
 {
     static_assert(NTOK == 1 || !Q6, "two vectors at once: Q4_K / Q5_K only");
     constexpr uint32_t XQSB = mma_xq_sb<NP, NTOK>(), JS = mma_xq_js<NP, NTOK>(), SUMS = mma_xq_sums<NP, NTOK>();
     const uint32_t col0 = NTOK == 1 ? 0u : b_tok * NP;
     bool ok = true;
-    // (four planes: the float just below 127 * (2^24 + 2^16 + 2^8 + 1), so that the clamp and the scale agree)
-    constexpr int QMAXI = NP == 4 ? 0x7F7F7F00 : NP == 3 ? 127 * 65536 + 127 * 256 + 127 : 127 * 256 + 127;
+    // The largest digits are 127 each; a little below that, so that v * factor rounds to no more.
+    constexpr int QMAXI = NP == 4 ? 0x7F7F7C00 : NP == 3 ? 127 * 65536 + 127 * 256 + 123 : 127 * 256 + 126;
     constexpr float QMAX = (float)QMAXI;
-    constexpr int XB = 4;
+    constexpr int XB = 5;
+    const bool whole = (reinterpret_cast<uintptr_t>(x) & 31) == 0;
     float *xs = reinterpret_cast<float *>(xq + (size_t)units * XQSB), *sxs = xs + units * NTOK;
-    const float share = NORM ? norm_share(norm_parts, warp * 32u + lane, nwarps * 32u) : 0.0f;
-    float rms = 0.0f;
-    bool have_rms = !NORM;
     for (uint32_t ub = warp; ub < units; ub += nwarps * XB) {
         float4 v0[XB], v1[XB];
+        uint4 nw[NORM ? XB : 1];
 #pragma unroll
         for (int b = 0; b < XB; ++b) {
             const uint32_t u = ub + b * nwarps;
-            const float4 *src = reinterpret_cast<const float4 *>(x + (size_t)u * 256) + 2 * lane;
             if (slots) {
                 const uint2 *sl = slots + (size_t)u * 256 + 8 * lane;
                 v0[b] = u < units ? ld_gathered4(sl, tag, &ok) : make_float4(0.f, 0.f, 0.f, 0.f);
                 v1[b] = u < units ? ld_gathered4(sl + 4, tag, &ok) : make_float4(0.f, 0.f, 0.f, 0.f);
             } else {
-                v0[b] = u < units ? __ldcg(src) : make_float4(0.f, 0.f, 0.f, 0.f);
-                v1[b] = u < units ? __ldcg(src + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v0[b] = v1[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (u < units) ldcg8(x + (size_t)u * 256 + 8 * lane, whole, v0[b], v1[b]);
             }
         }
         if constexpr (NORM) {
-            if (!have_rms) { rms = norm_rms(share, s_share, warp, lane, nwarps, units * 256u, norm_eps); have_rms = true; }
+#pragma unroll
+            for (int b = 0; b < XB; ++b) {      // 8-byte aligned bf16 weights
+                const uint2 *w = reinterpret_cast<const uint2 *>(norm_w) + (size_t)(ub + b * nwarps) * 64 + 2 * lane;
+                const uint2 wa = ub + b * nwarps < units ? __ldg(w) : make_uint2(0u, 0u), wb = ub + b * nwarps < units ? __ldg(w + 1) : make_uint2(0u, 0u);
+                nw[b] = make_uint4(wa.x, wa.y, wb.x, wb.y);
+            }
 #pragma unroll
             for (int b = 0; b < XB; ++b) {
-                const uint32_t u = ub + b * nwarps;
-                if (u >= units) break;
-                const uint2 *nw = reinterpret_cast<const uint2 *>(norm_w) + (size_t)u * 64 + 2 * lane;      // 8-byte aligned bf16 weights
-                const uint2 wa = __ldg(nw), wb = __ldg(nw + 1);
                 auto lo = [](uint32_t w) { return __uint_as_float(w << 16); };
                 auto hi = [](uint32_t w) { return __uint_as_float(w & 0xffff0000u); };
-                v0[b] = make_float4(v0[b].x * rms * lo(wa.x), v0[b].y * rms * hi(wa.x), v0[b].z * rms * lo(wa.y), v0[b].w * rms * hi(wa.y));
-                v1[b] = make_float4(v1[b].x * rms * lo(wb.x), v1[b].y * rms * hi(wb.x), v1[b].z * rms * lo(wb.y), v1[b].w * rms * hi(wb.y));
+                v0[b] = make_float4(v0[b].x * lo(nw[b].x), v0[b].y * hi(nw[b].x), v0[b].z * lo(nw[b].y), v0[b].w * hi(nw[b].y));
+                v1[b] = make_float4(v1[b].x * lo(nw[b].z), v1[b].y * hi(nw[b].z), v1[b].z * lo(nw[b].w), v1[b].w * hi(nw[b].w));
             }
         }
-        float amax[XB], sum[XB], smax[XB];
+        float sum[XB], mine = 0.0f;             // lane b: the maximum of superblock b, lane XB + b: of its sums
 #pragma unroll
         for (int b = 0; b < XB; ++b) {
-            amax[b] = fmaxf(fmaxf(fmaxf(fabsf(v0[b].x), fabsf(v0[b].y)), fmaxf(fabsf(v0[b].z), fabsf(v0[b].w))),
-                            fmaxf(fmaxf(fabsf(v1[b].x), fabsf(v1[b].y)), fmaxf(fabsf(v1[b].z), fabsf(v1[b].w))));
-            sum[b] = ((v0[b].x + v0[b].y) + (v0[b].z + v0[b].w)) + ((v1[b].x + v1[b].y) + (v1[b].z + v1[b].w));
-        }
-#pragma unroll
-        for (int o = 1; o < 4; o <<= 1) {
-#pragma unroll
-            for (int b = 0; b < XB; ++b) {
-                amax[b] = fmaxf(amax[b], __shfl_xor_sync(0xffffffffu, amax[b], o));
-                sum[b] += __shfl_xor_sync(0xffffffffu, sum[b], o);      // ends as the sum of x over the lane's sub-block
+            if (ub + b * nwarps >= units) break;
+            const float amax = warp_abs_max(fmaxf(fmaxf(fmaxf(fabsf(v0[b].x), fabsf(v0[b].y)), fmaxf(fabsf(v0[b].z), fabsf(v0[b].w))),
+                                                  fmaxf(fmaxf(fabsf(v1[b].x), fabsf(v1[b].y)), fmaxf(fabsf(v1[b].z), fabsf(v1[b].w)))));
+            if (lane == (uint32_t)b) mine = amax;
+            if constexpr (!Q6) {
+                sum[b] = ((v0[b].x + v0[b].y) + (v0[b].z + v0[b].w)) + ((v1[b].x + v1[b].y) + (v1[b].z + v1[b].w));
+                sum[b] += __shfl_xor_sync(0xffffffffu, sum[b], 1);
+                sum[b] += __shfl_xor_sync(0xffffffffu, sum[b], 2);      // ends as the sum of x over the lane's sub-block
+                const float smax = warp_abs_max(sum[b]);
+                if (lane == (uint32_t)(XB + b)) mine = smax;
             }
         }
-#pragma unroll
-        for (int b = 0; b < XB; ++b) smax[b] = fabsf(sum[b]);
-#pragma unroll
-        for (int o = 4; o < 32; o <<= 1) {
-#pragma unroll
-            for (int b = 0; b < XB; ++b) {
-                amax[b] = fmaxf(amax[b], __shfl_xor_sync(0xffffffffu, amax[b], o));
-                smax[b] = fmaxf(smax[b], __shfl_xor_sync(0xffffffffu, smax[b], o));
-            }
-        }
+        const float inv_mine = fixed_factor(mine, QMAX);
 #pragma unroll
         for (int b = 0; b < XB; ++b) {
             const uint32_t u = ub + b * nwarps;
             if (u >= units) break;
-            const float inv = amax[b] > 0.0f ? QMAX / amax[b] : 0.0f, sinv = smax[b] > 0.0f ? QMAX / smax[b] : 0.0f;
+            const float inv = __shfl_sync(0xffffffffu, inv_mine, b);
             const float v[8] = {v0[b].x, v0[b].y, v0[b].z, v0[b].w, v1[b].x, v1[b].y, v1[b].z, v1[b].w};
-            uint32_t uq[8];
+            uint32_t uq[8], pa[NP], pb[NP];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) uq[i] = (uint32_t)max(-QMAXI, min(QMAXI, __float2int_rn(v[i] * inv))) + digit_bias<NP>();
+            for (int i = 0; i < 8; ++i) uq[i] = (uint32_t)__float2int_rn(v[i] * inv) + digit_bias<NP>();
+            plane_words<NP>(uq[0], uq[1], uq[2], uq[3], pa);
+            plane_words<NP>(uq[4], uq[5], uq[6], uq[7], pb);
             uint8_t *sb = xq + (size_t)u * XQSB;
 #pragma unroll
             for (int p = 0; p < NP; ++p) {
-                const uint2 pw = make_uint2(plane_word(uq[0], uq[1], uq[2], uq[3], p), plane_word(uq[4], uq[5], uq[6], uq[7], p));
-                *reinterpret_cast<uint2 *>(sb + (lane >> 2) * JS + (col0 + p) * 32 + (lane & 3u) * 8) = pw;
+                *reinterpret_cast<uint2 *>(sb + (lane >> 2) * JS + (col0 + p) * 32 + (lane & 3u) * 8) = make_uint2(pa[p], pb[p]);
                 if constexpr (Q6) {
-                    int sd = __dp4a((int)pw.x, 0x01010101, __dp4a((int)pw.y, 0x01010101, 0));
+                    int sd = __dp4a((int)pa[p], 0x01010101, __dp4a((int)pb[p], 0x01010101, 0));
                     sd += __shfl_xor_sync(0xffffffffu, sd, 1);                    // 16 elements = two lanes
                     const int lo8 = (int)(signed char)(sd & 0xFF);
                     if ((lane & 1u) == 0) {
@@ -518,16 +539,18 @@ __device__ __forceinline__ bool quantize_x_mma(const float *__restrict__ x, uint
                 }
             }
             if constexpr (!Q6) {
-                const uint32_t us = (uint32_t)max(-QMAXI, min(QMAXI, __float2int_rn(sum[b] * sinv))) + digit_bias<NP>();
+                const uint32_t us = (uint32_t)__float2int_rn(sum[b] * __shfl_sync(0xffffffffu, inv_mine, XB + b)) + digit_bias<NP>();
                 if ((lane & 3u) == 0) {
 #pragma unroll
                     for (int p = 0; p < NP; ++p) sb[SUMS + (col0 + p) * 8 + (lane >> 2)] = (uint8_t)(((us >> (8 * p)) & 255u) ^ 0x80u);
                 }
             }
-            if (lane == 0) { xs[u * NTOK + (NTOK == 1 ? 0u : b_tok)] = amax[b] / QMAX; sxs[u * NTOK + (NTOK == 1 ? 0u : b_tok)] = smax[b] / QMAX; }
+        }
+        {
+            const uint32_t b = lane < (uint32_t)XB ? lane : lane - XB, u = ub + b * nwarps;
+            if (lane < (uint32_t)(Q6 ? XB : 2 * XB) && u < units) (lane < (uint32_t)XB ? xs : sxs)[u * NTOK + (NTOK == 1 ? 0u : b_tok)] = fixed_unit(inv_mine);
         }
     }
-    if constexpr (NORM) { if (!have_rms) norm_rms(share, s_share, warp, lane, nwarps, units * 256u, norm_eps); }      // a warp without a superblock takes part in the sum
     return ok;
 }
 
@@ -707,20 +730,29 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
 
     // ---- consumers ------------------------------------------------------------------------
     const uint32_t g = lane >> 2, t4 = lane & 3u;
+    if (EXT && a.norm_w) {        // from memory, so on their way to L2 before the wait; read after it, next to x
+        for (uint32_t u = warp * 32u + lane; u < U * 4u; u += C) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t *>(a.norm_w) + u * 128u));
+    }
     pdl_wait();   // x is the previous kernel's output
     if (tid == 0) stamp(a.trace, 2);
     uint8_t *xq = smem + a.xs_base;
+    // of the fused neighbours, what the flush will need: this thread's share of the partial sums of squares, its residual
+    __shared__ float s_share[MMA_MAX_CONSUMER_WARPS];
+    float share = 0.0f, res0 = 0.0f;
     float moe_wgt = 1.0f;      // MoE form 2: the routing weight of the expert whose input this thread's superblock belongs to
     if constexpr (MOE == 2) { if (tid < U) moe_wgt = a.seg_weight[blockIdx.y * a.tok_sel_stride + tid / a.kc]; }
     {
         const uint2 *slots = EXT ? a.x_ll : nullptr;
         const unsigned int want = EXT && a.x_ll ? *reinterpret_cast<const volatile unsigned int *>(a.wait_gen) : 0u;
         bool x_ok;
-        __shared__ float s_share[MMA_MAX_CONSUMER_WARPS];
-        if (EXT && a.norm_w)
-            x_ok = quantize_x_mma<NP, Q6, NTOK, true>(a.x, U, xq, warp, lane, CW, nullptr, 0u, 0u, a.norm_w, a.norm_parts, a.norm_eps, s_share);
-        else
+        if (EXT && a.norm_w) {
+            share = norm_share(a.norm_parts, tid, C);
+            x_ok = quantize_x_mma<NP, Q6, NTOK, true>(a.x, U, xq, warp, lane, CW, nullptr, 0u, 0u, a.norm_w);
+            share = warp_sum(share);
+            if (lane == 0) s_share[warp] = share;
+        } else
             x_ok = quantize_x_mma<NP, Q6, NTOK>(a.x + (MOE != 0 ? (size_t)blockIdx.y * a.tok_x_stride : 0), U, xq, warp, lane, CW, slots, want, 0u);
+        if (EXT && !SWIGLU && a.res_in && tid < hi - lo) res0 = __ldcg(a.res_in + lo + tid);
         if (!x_ok) {
             s_abort = 1;
             atomicExch(a.status, 3);
@@ -770,7 +802,10 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
     uint32_t which = 0, buf_n = 0, buf_row0 = 0;
     int buf_seg = 0;
     float sq = 0.0f;                          // this thread's share of the sum of squares of the outputs (residual epilogue)
+    float rms = 1.0f;                         // 1 / rms of a normalised x
+    bool have_rms = !(EXT && a.norm_w);
     auto flush = [&]() {
+        if (EXT && !have_rms) { rms = norm_rms(s_share, CW, a.in_dim, a.norm_eps); have_rms = true; }
         named_bar_sync(PIPE_BAR_CONSUMERS, (int)C);
         const float *src = red + (size_t)which * PLANE * (SWIGLU || TWO ? 2 : 1);
         float *y = a.seg[buf_seg].y + buf_row0 + (MOE != 0 ? (size_t)blockIdx.y * a.tok_y_stride : 0);
@@ -780,10 +815,12 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
                 gsum += src[r * SLOTS + w];
                 if constexpr (SWIGLU || TWO) usum += src[PLANE + r * SLOTS + w];
             }
+            if constexpr (EXT) { gsum *= rms; usum *= rms; }
             float val = SWIGLU ? silu_mul(gsum, usum) : gsum;
             if constexpr (EXT && !SWIGLU) {
                 if (a.res_in) {               // residual add, clamped to the fp16 range as the reference's kernel does
-                    val = fminf(fmaxf(a.res_in[buf_row0 + r] + val, -65504.0f), 65504.0f);
+                    const float res = buf_row0 + r == lo + tid ? res0 : __ldcg(a.res_in + buf_row0 + r);      // (one tensor: its rows are the CTA's)
+                    val = fminf(fmaxf(res + val, -65504.0f), 65504.0f);
                     sq = fmaf(val, val, sq);
                 }
             }

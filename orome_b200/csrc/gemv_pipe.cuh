@@ -343,6 +343,18 @@ __device__ __forceinline__ void dot_s(uint32_t q, const XGroup<NP, N> &g, int k,
     for (int p = 0; p < NP; ++p) I[p] = (p == NP - 1) ? dp4a_ss(q, g.pc[p][k], I[p]) : dp4a_su(q, g.pc[p][k], I[p]);
 }
 
+// Fixed point of a group whose largest magnitude is `m`: X = rn(v * inv), v ~= X * unit.  Any factor near qmax / m will do as long as
+// unit is its exact reciprocal: an approximate one and one rounded reciprocal instead of two divisions, whose ~340 clocks every
+// launch waited for between its input and its first product.  qmax leaves room for the factor's error (2^-22).  m = 0 or infinite:
+// all X are zero (F2I of NaN), unit 0 or infinite.
+__device__ __forceinline__ float fixed_factor(float m, float qmax)
+{
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(m));
+    return qmax * r;
+}
+__device__ __forceinline__ float fixed_unit(float inv) { return __frcp_rn(inv); }
+
 // ---- x in shared memory, quantized once per CTA --------------------------------------------
 // Layout at xq: NP byte planes of in_dim bytes (plane p holds byte p of every X_i), then one fp32
 // scale per group of G elements, then (Q4_K/Q5_K only) one fp32 sum of x per 32 elements.
@@ -358,7 +370,7 @@ __device__ __forceinline__ void dot_s(uint32_t q, const XGroup<NP, N> &g, int k,
 template <int NP, int G, bool SUMS>
 __device__ __forceinline__ void quantize_piece(const float4 v, uint32_t f, bool valid, uint32_t lane, uint8_t *xq, uint32_t in_dim)
 {
-    constexpr float QMAX = NP == 3 ? 8388607.0f : 32767.0f;
+    constexpr float QMAX = NP == 3 ? 8388603.0f : 32766.0f;
     const uint32_t n4 = in_dim / 4;
     uint32_t *planes = reinterpret_cast<uint32_t *>(xq);
     float *scales = reinterpret_cast<float *>(xq + (size_t)NP * in_dim);
@@ -366,12 +378,10 @@ __device__ __forceinline__ void quantize_piece(const float4 v, uint32_t f, bool 
     float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
 #pragma unroll
     for (int o = 1; o < G / 4; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const float inv = amax > 0.0f ? QMAX / amax : 0.0f;
+    const float inv = fixed_factor(amax, QMAX);
     int X[4];
     X[0] = __float2int_rn(v.x * inv); X[1] = __float2int_rn(v.y * inv);
     X[2] = __float2int_rn(v.z * inv); X[3] = __float2int_rn(v.w * inv);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) X[j] = max(-(int)QMAX, min((int)QMAX, X[j]));
     float sum = 0.0f;
     if constexpr (SUMS) {
         sum = (v.x + v.y) + (v.z + v.w);
@@ -386,7 +396,7 @@ __device__ __forceinline__ void quantize_piece(const float4 v, uint32_t f, bool 
             const uint32_t hi = __byte_perm((uint32_t)X[2], (uint32_t)X[3], sel);
             planes[(size_t)p * n4 + 4 * plane_swz(f >> 2) + (f & 3u)] = __byte_perm(lo, hi, 0x5410);
         }
-        if ((lane & (G / 4 - 1)) == 0) scales[f / (G / 4)] = amax / QMAX;
+        if ((lane & (G / 4 - 1)) == 0) scales[f / (G / 4)] = fixed_unit(inv);
         if constexpr (SUMS)
             if ((lane & 7u) == 0) sums[f / 8] = sum;
     }
@@ -399,13 +409,11 @@ __device__ __forceinline__ float norm_share(const float *norm_parts, uint32_t ti
     for (uint32_t i = tid; i < (uint32_t)PIPE_SUM_SQ_PARTS; i += nthreads) t += __ldcg(norm_parts + i);
     return t;
 }
-// 1 / rms from the shares, added up over the consumer threads; every one of them calls this once.  (Each warp adding up all
-// 512 entries for itself cost 16 more loads a lane, 4.5 MB of L2 reads of the same 2 KiB per launch, ahead of the loads of x.)
-__device__ __forceinline__ float norm_rms(float share, float *s_share, uint32_t warp, uint32_t lane, uint32_t nwarps, uint32_t in_dim, float eps)
+// 1 / rms from the warps' sums of their shares (written before the barrier behind the quantization).  It is a common factor of every
+// output, so it is applied to the sums: ahead of the quantization it cost a barrier and a round trip there (with the mma kernel's
+// late loads of the norm weights 5120-wide 4.5 us from x to the barrier, 1.8 without a norm).
+__device__ __forceinline__ float norm_rms(const float *s_share, uint32_t nwarps, uint32_t in_dim, float eps)
 {
-    share = warp_sum(share);
-    if (lane == 0) s_share[warp] = share;
-    named_bar_sync(PIPE_BAR_CONSUMERS, (int)(nwarps * 32u));
     float t = 0.0f;
     for (uint32_t w = 0; w < nwarps; ++w) t += s_share[w];
     return rsqrtf(t / (float)in_dim + eps);
@@ -416,10 +424,9 @@ __device__ __forceinline__ bool quantize_x_to_smem(const float *__restrict__ x, 
                                                    uint8_t *xq0, uint32_t vec_bytes, uint32_t tid, uint32_t nthreads,
                                                    const uint2 *slots = nullptr, unsigned int tag = 0,
                                                    long long limit = PIPE_WAIT_CYCLES, const int *status = nullptr, uint32_t rot = 0,
-                                                   uint32_t issued_bar = 0, const uint16_t *norm_w = nullptr, const float *norm_parts = nullptr,
-                                                   float norm_eps = 0.0f, float *s_share = nullptr)
+                                                   uint32_t issued_bar = 0, const uint16_t *norm_w = nullptr)
 {
-    // NORM: x is RMS-normalised on the way.  The partial sums, x and the norm weights are all requested before any is used.
+    // NORM: x is multiplied by the bf16 norm weights on the way (1 / rms: see norm_rms); both are requested before any is used.
     // issued_bar: shared address of an mbarrier on which every warp arrives once the loads of its first batch are on
     // their way (0: none).  The weight producer holds its copies back until then, see the kernel.
     // rot (single vector only; a multiple of 32 four-float pieces): this CTA walks the vector starting rot pieces in and
@@ -433,9 +440,6 @@ __device__ __forceinline__ bool quantize_x_to_smem(const float *__restrict__ x, 
         if (lane == 0) mbar_arrive(issued_bar);
         issued_bar = 0;
     }
-    const float share = NORM ? norm_share(norm_parts, tid, nthreads) : 0.0f;
-    float rms = 0.0f;
-    bool have_rms = !NORM;
     for (uint32_t base = tid - lane; base < n4_all; base += nthreads * BATCH) {
         float4 v[BATCH];
         uint2 nw[NORM ? BATCH : 1];
@@ -453,14 +457,13 @@ __device__ __forceinline__ bool quantize_x_to_smem(const float *__restrict__ x, 
             __syncwarp();
             if (lane == 0) mbar_arrive(issued_bar);
         }
-        if constexpr (NORM) {                 // the scale and the bf16 norm weights, applied in the reference's order
-            if (!have_rms) { rms = norm_rms(share, s_share, tid >> 5, lane, nthreads / 32u, in_dim, norm_eps); have_rms = true; }
+        if constexpr (NORM) {
 #pragma unroll
             for (int b = 0; b < BATCH; ++b) {
-                v[b].x = v[b].x * rms * __uint_as_float(nw[b].x << 16);
-                v[b].y = v[b].y * rms * __uint_as_float(nw[b].x & 0xffff0000u);
-                v[b].z = v[b].z * rms * __uint_as_float(nw[b].y << 16);
-                v[b].w = v[b].w * rms * __uint_as_float(nw[b].y & 0xffff0000u);
+                v[b].x *= __uint_as_float(nw[b].x << 16);
+                v[b].y *= __uint_as_float(nw[b].x & 0xffff0000u);
+                v[b].z *= __uint_as_float(nw[b].y << 16);
+                v[b].w *= __uint_as_float(nw[b].y & 0xffff0000u);
             }
         }
 #pragma unroll
@@ -478,7 +481,6 @@ __device__ __forceinline__ bool quantize_x_to_smem(const float *__restrict__ x, 
         __syncwarp();
         if (lane == 0) mbar_arrive(issued_bar);
     }
-    if constexpr (NORM) { if (!have_rms) norm_rms(share, s_share, tid >> 5, lane, nthreads / 32u, in_dim, norm_eps); }   // and takes part in the sum
     return ok;
 }
 
@@ -926,9 +928,18 @@ gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
     const int part = (int)(j / U);
     const uint32_t unit = j % U;
 
+    if constexpr (EXT && !COMBINE) {
+        if (a.norm_w) {           // from memory, so on their way to L2 before the wait; read after it, next to x
+            for (uint32_t p = tid * 128u; p < a.in_dim * 2u; p += C * 128u) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t *>(a.norm_w) + p));
+        }
+    }
     pdl_wait();   // x is the previous kernel's output
     if (tid == 0) stamp(a.trace, 2);
 
+    // of the fused neighbours, what the flush will need: this thread's share of the partial sums of squares, its residual
+    __shared__ float s_share[PIPE_MAX_CONSUMERS / 32];
+    float share = 0.0f, res0 = 0.0f;
+    const uint32_t cta_row0 = (uint32_t)((uint64_t)blockIdx.x * a.total_rows / gridDim.x);
     SlotT slot;
     {
         uint8_t *xq = smem + a.xs_base;
@@ -939,16 +950,21 @@ gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
         const uint32_t rot = COMBINE ? 0u : (uint32_t)((uint64_t)blockIdx.x * (a.in_dim / 4) / gridDim.x) & ~31u;
         bool x_ok;
         if constexpr (EXT && !COMBINE) {
-            __shared__ float s_share[PIPE_MAX_CONSUMERS / 32];
-            if (a.norm_w)
+            if (a.norm_w) {
+                share = norm_share(a.norm_parts, tid, C);
                 x_ok = quantize_x_to_smem<NP, SlotT::GROUP, SlotT::SUMS, true>(x, a.in_dim, 1u, a.x_stride, xq, a.xq_vec_bytes, tid, C, slots, want, a.wait_cycles,
-                                                                             a.status, rot, smem_u32(&s_x_issued), a.norm_w, a.norm_parts, a.norm_eps, s_share);
-            else
+                                                                             a.status, rot, smem_u32(&s_x_issued), a.norm_w);
+                share = warp_sum(share);
+                if (lane == 0) s_share[tid >> 5] = share;
+            } else
                 x_ok = quantize_x_to_smem<NP, SlotT::GROUP, SlotT::SUMS>(x, a.in_dim, 1u, a.x_stride, xq, a.xq_vec_bytes, tid, C, slots, want, a.wait_cycles,
                                                                        a.status, rot, smem_u32(&s_x_issued));
         } else
             x_ok = quantize_x_to_smem<NP, SlotT::GROUP, SlotT::SUMS>(x, a.in_dim, COMBINE ? (uint32_t)a.nseg : 1u, a.x_stride, xq, a.xq_vec_bytes, tid, C, slots, want,
                                                                    a.wait_cycles, a.status, rot, smem_u32(&s_x_issued));
+        if constexpr (EXT && MODE == 0) {
+            if (a.res_in && cta_row0 + tid < (uint32_t)((uint64_t)(blockIdx.x + 1) * a.total_rows / gridDim.x)) res0 = __ldcg(a.res_in + cta_row0 + tid);
+        }
         if (!x_ok) {
             s_abort = 1;
             atomicExch(a.status, 3);
@@ -988,7 +1004,10 @@ gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
     uint32_t which = 0, buf_n = 0, buf_row0 = 0;
     int buf_seg = 0;
     float sq = 0.0f;                          // this thread's share of the sum of squares of the outputs (residual epilogue)
+    float rms = 1.0f;                         // 1 / rms of a normalised x
+    bool have_rms = COMBINE || !(EXT && a.norm_w);
     auto flush = [&]() {
+        if (EXT && !COMBINE && !have_rms) { rms = norm_rms(s_share, C >> 5, a.in_dim, a.norm_eps); have_rms = true; }
         named_bar_sync(PIPE_BAR_CONSUMERS, (int)C);
         const float *src = pbuf + (size_t)which * PLANE * (SWIGLU ? 2 : 1);
         float *y = a.seg[buf_seg].y + buf_row0 + (EXT ? (size_t)blockIdx.y * a.tok_y_stride : 0);
@@ -1001,10 +1020,12 @@ gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
             }
             if constexpr (COMBINE) accbuf[buf_row0 - wk.lo + r] += (comb_acc ? 1.0f : a.seg_weight[blockIdx.y * a.tok_sel_stride + buf_seg]) * g;   // one owner per row and flush
             else {
+                if constexpr (EXT) { g *= rms; u *= rms; }
                 float val = SWIGLU ? silu_mul(g, u) : g;
                 if constexpr (EXT && MODE == 0) {
                     if (a.res_in) {           // residual add, clamped to the fp16 range as the reference's kernel does
-                        val = fminf(fmaxf(a.res_in[buf_row0 + r] + val, -65504.0f), 65504.0f);
+                        const float res = buf_row0 + r == cta_row0 + tid ? res0 : __ldcg(a.res_in + buf_row0 + r);      // (one tensor: its rows are the CTA's)
+                        val = fminf(fmaxf(res + val, -65504.0f), 65504.0f);
                         sq = fmaf(val, val, sq);
                     }
                 }
