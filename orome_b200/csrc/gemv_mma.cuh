@@ -430,7 +430,7 @@ __device__ __forceinline__ void ldcg8(const float *p, bool whole, float4 &a, flo
 {
     if (whole) asm volatile("ld.global.cg.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                             : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "l"(p));
-    else { a = __ldcg(reinterpret_cast<const float4 *>(p)); b = __ldcg(reinterpret_cast<const float4 *>(p) + 1); }
+    else { a = ldcg4_here(reinterpret_cast<const float4 *>(p)); b = ldcg4_here(reinterpret_cast<const float4 *>(p) + 1); }
 }
 // max |v| over the warp; NaN where all lanes hold one, as fmaxf gives it
 __device__ __forceinline__ float warp_abs_max(float v)
@@ -442,17 +442,18 @@ __device__ __forceinline__ float warp_abs_max(float v)
 
 // x -> shared memory, one warp per superblock: lane l owns elements 8l..8l+7 (sub-block l / 4, bytes 8 (l % 4)..).
 // Layout per superblock u at xq + u * MMA_XQ_SB: [sub-block j][plane p][32 bytes], then at +768 [plane p][8 sum bytes];
-// xs[u], sxs[u] after all superblocks.  A warp takes up to five superblocks at a time: their loads are issued together
-// and their reductions interleave.
+// xs[u], sxs[u] after all superblocks.  A warp takes XB superblocks a round, the next round's loads ahead of this one's arithmetic.
 // Q6 form: instead of the float sums, the sums of the signed digits over every 16 elements, as two balanced bytes:
 // at +768 [plane p][low / high byte][16 groups].
-// With `slots` set x is a gathered vector read from its {value, tag} slots (polled for `tag`); false = a poll expired.
+// GATHERED: x is read from its {value, tag} slots (polled for `tag`); false = a poll expired.  (An instance of its own: with the
+// choice made load by load, a round's loads waited for one another.)
 // NTOK = 2: vector `b` (0 or 1) of two, into its columns of the wider layout (see mma_xq_sb).
-// NORM: x is multiplied by the bf16 norm weights on the way; the common factor 1 / rms is the caller's, who applies it to the sums,
+// NORM: x is multiplied by the bf16 norm weights (none: by one) on the way; the common factor 1 / rms is the caller's, who applies it to the sums,
 // since nothing before them needs it.
-// What bounds it: every CTA does this between its predecessor's end and its own first mma, so it is latency, and then issue slots:
-// a maximum is one redux instead of five shuffles, and the up to ten factors of a round are worked out by ten lanes at once.
-template <int NP, bool Q6, int NTOK = 1, bool NORM = false>
+// What bounds it: every CTA does this between its predecessor's end and its own first mma, so it is latency, and then issue slots and
+// instructions fetched: a maximum is one redux instead of five shuffles, the factors of a round are worked out by as many lanes at once,
+// and the rounds are a rolled loop (run once a launch from cold instruction caches).
+template <int NP, bool Q6, int NTOK = 1, bool NORM = false, bool GATHERED = false>
 __device__ __forceinline__ bool quantize_x_mma(const float *__restrict__ x, uint32_t units, uint8_t *xq, uint32_t warp, uint32_t lane,
                                                uint32_t nwarps, const uint2 *slots = nullptr, unsigned int tag = 0, uint32_t b_tok = 0,
                                                const uint16_t *norm_w = nullptr)
@@ -464,37 +465,45 @@ __device__ __forceinline__ bool quantize_x_mma(const float *__restrict__ x, uint
     // The largest digits are 127 each; a little below that, so that v * factor rounds to no more.
     constexpr int QMAXI = NP == 4 ? 0x7F7F7C00 : NP == 3 ? 127 * 65536 + 127 * 256 + 123 : 127 * 256 + 126;
     constexpr float QMAX = (float)QMAXI;
-    constexpr int XB = 5;
+    constexpr int XB = 2;
     const bool whole = (reinterpret_cast<uintptr_t>(x) & 31) == 0;
     float *xs = reinterpret_cast<float *>(xq + (size_t)units * XQSB), *sxs = xs + units * NTOK;
-    for (uint32_t ub = warp; ub < units; ub += nwarps * XB) {
-        float4 v0[XB], v1[XB];
-        uint4 nw[NORM ? XB : 1];
+    struct Round { float4 v0[XB], v1[XB]; uint4 nw[NORM ? XB : 1]; };
+    auto load = [&](uint32_t ub, Round &r) {
 #pragma unroll
         for (int b = 0; b < XB; ++b) {
             const uint32_t u = ub + b * nwarps;
-            if (slots) {
+            r.v0[b] = r.v1[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if constexpr (NORM) r.nw[b] = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
+            if (u >= units) continue;
+            if constexpr (GATHERED) {
                 const uint2 *sl = slots + (size_t)u * 256 + 8 * lane;
-                v0[b] = u < units ? ld_gathered4(sl, tag, &ok) : make_float4(0.f, 0.f, 0.f, 0.f);
-                v1[b] = u < units ? ld_gathered4(sl + 4, tag, &ok) : make_float4(0.f, 0.f, 0.f, 0.f);
-            } else {
-                v0[b] = v1[b] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (u < units) ldcg8(x + (size_t)u * 256 + 8 * lane, whole, v0[b], v1[b]);
+                r.v0[b] = ld_gathered4(sl, tag, &ok);
+                r.v1[b] = ld_gathered4(sl + 4, tag, &ok);
+            } else ldcg8(x + (size_t)u * 256 + 8 * lane, whole, r.v0[b], r.v1[b]);
+            if constexpr (NORM) {
+                if (norm_w) {      // 8-byte aligned
+                    const uint2 *w = reinterpret_cast<const uint2 *>(norm_w) + (size_t)u * 64 + 2 * lane;
+                    const uint2 wa = ldnc2_here(w), wb = ldnc2_here(w + 1);
+                    r.nw[b] = make_uint4(wa.x, wa.y, wb.x, wb.y);
+                }
             }
         }
+    };
+    Round r, next;
+    if (warp < units) load(warp, r);
+#pragma unroll 1
+    for (uint32_t ub = warp; ub < units; ub += nwarps * XB) {
+        if (ub + nwarps * XB < units) load(ub + nwarps * XB, next);
+        float4 (&v0)[XB] = r.v0, (&v1)[XB] = r.v1;
         if constexpr (NORM) {
 #pragma unroll
-            for (int b = 0; b < XB; ++b) {      // 8-byte aligned bf16 weights
-                const uint2 *w = reinterpret_cast<const uint2 *>(norm_w) + (size_t)(ub + b * nwarps) * 64 + 2 * lane;
-                const uint2 wa = ub + b * nwarps < units ? __ldg(w) : make_uint2(0u, 0u), wb = ub + b * nwarps < units ? __ldg(w + 1) : make_uint2(0u, 0u);
-                nw[b] = make_uint4(wa.x, wa.y, wb.x, wb.y);
-            }
-#pragma unroll
             for (int b = 0; b < XB; ++b) {
+                const uint4 nw = r.nw[b];
                 auto lo = [](uint32_t w) { return __uint_as_float(w << 16); };
                 auto hi = [](uint32_t w) { return __uint_as_float(w & 0xffff0000u); };
-                v0[b] = make_float4(v0[b].x * lo(nw[b].x), v0[b].y * hi(nw[b].x), v0[b].z * lo(nw[b].y), v0[b].w * hi(nw[b].y));
-                v1[b] = make_float4(v1[b].x * lo(nw[b].z), v1[b].y * hi(nw[b].z), v1[b].z * lo(nw[b].w), v1[b].w * hi(nw[b].w));
+                v0[b] = make_float4(v0[b].x * lo(nw.x), v0[b].y * hi(nw.x), v0[b].z * lo(nw.y), v0[b].w * hi(nw.y));
+                v1[b] = make_float4(v1[b].x * lo(nw.z), v1[b].y * hi(nw.z), v1[b].z * lo(nw.w), v1[b].w * hi(nw.w));
             }
         }
         float sum[XB], mine = 0.0f;             // lane b: the maximum of superblock b, lane XB + b: of its sums
@@ -550,6 +559,7 @@ __device__ __forceinline__ bool quantize_x_mma(const float *__restrict__ x, uint
             const uint32_t b = lane < (uint32_t)XB ? lane : lane - XB, u = ub + b * nwarps;
             if (lane < (uint32_t)(Q6 ? XB : 2 * XB) && u < units) (lane < (uint32_t)XB ? xs : sxs)[u * NTOK + (NTOK == 1 ? 0u : b_tok)] = fixed_unit(inv_mine);
         }
+        r = next;
     }
     return ok;
 }
@@ -591,13 +601,14 @@ __device__ __forceinline__ bool mma_next_tile(const MmaArgs &a, uint32_t &cur, u
     return true;
 }
 
-template <int FMT, int NP, bool SWIGLU, bool EXT, int MOE = 0, int NTOK = 1>
+// EXT: as in gemv_pipe_kernel (1: multi-GPU publish / wait, 2: fused norm / residual neighbours).
+template <int FMT, int NP, bool SWIGLU, int EXT, int MOE = 0, int NTOK = 1>
 __global__ void __launch_bounds__(MMA_MAX_THREADS, 1)
 gemv_mma_kernel(const __grid_constant__ MmaArgs a)
 {
     static_assert(MOE == 0 || (FMT != FMT_Q6_K && !EXT), "the MoE forms are built for Q4_K / Q5_K on one GPU");
     static_assert(NTOK == 1 || (NTOK == 2 && FMT != FMT_Q6_K && !SWIGLU && !EXT && MOE == 0), "two vectors at once: plain Q4_K / Q5_K products on one GPU");
-    constexpr bool TWO = NTOK == 2;
+    constexpr bool TWO = NTOK == 2, PEER = EXT == 1, FUSE = EXT == 2;
     constexpr uint32_t XQSB = mma_xq_sb<NP, NTOK>(), XJS = mma_xq_js<NP, NTOK>(), XSUMS = mma_xq_sums<NP, NTOK>();
     static_assert(MOE != 1 || SWIGLU, "MOE 1 is the fused gate/up form");
     static_assert(MOE != 2 || !SWIGLU, "MOE 2 is the down + combine form");
@@ -730,7 +741,7 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
 
     // ---- consumers ------------------------------------------------------------------------
     const uint32_t g = lane >> 2, t4 = lane & 3u;
-    if (EXT && a.norm_w) {        // from memory, so on their way to L2 before the wait; read after it, next to x
+    if (FUSE && a.norm_w) {       // from memory, so on their way to L2 before the wait; read after it, next to x
         for (uint32_t u = warp * 32u + lane; u < U * 4u; u += C) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t *>(a.norm_w) + u * 128u));
     }
     pdl_wait();   // x is the previous kernel's output
@@ -742,24 +753,24 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
     float moe_wgt = 1.0f;      // MoE form 2: the routing weight of the expert whose input this thread's superblock belongs to
     if constexpr (MOE == 2) { if (tid < U) moe_wgt = a.seg_weight[blockIdx.y * a.tok_sel_stride + tid / a.kc]; }
     {
-        const uint2 *slots = EXT ? a.x_ll : nullptr;
-        const unsigned int want = EXT && a.x_ll ? *reinterpret_cast<const volatile unsigned int *>(a.wait_gen) : 0u;
         bool x_ok;
-        if (EXT && a.norm_w) {
-            share = norm_share(a.norm_parts, tid, C);
+        if constexpr (FUSE) {
+            if (a.norm_w) share = norm_share(a.norm_parts, tid, C);
             x_ok = quantize_x_mma<NP, Q6, NTOK, true>(a.x, U, xq, warp, lane, CW, nullptr, 0u, 0u, a.norm_w);
             share = warp_sum(share);
             if (lane == 0) s_share[warp] = share;
-        } else
-            x_ok = quantize_x_mma<NP, Q6, NTOK>(a.x + (MOE != 0 ? (size_t)blockIdx.y * a.tok_x_stride : 0), U, xq, warp, lane, CW, slots, want, 0u);
-        if (EXT && !SWIGLU && a.res_in && tid < hi - lo) res0 = __ldcg(a.res_in + lo + tid);
+        } else if (PEER && a.x_ll)
+            x_ok = quantize_x_mma<NP, Q6, NTOK, false, true>(a.x, U, xq, warp, lane, CW, a.x_ll, *reinterpret_cast<const volatile unsigned int *>(a.wait_gen), 0u);
+        else
+            x_ok = quantize_x_mma<NP, Q6, NTOK, false, false>(a.x + (MOE != 0 ? (size_t)blockIdx.y * a.tok_x_stride : 0), U, xq, warp, lane, CW, nullptr, 0u, 0u);
+        if (FUSE && !SWIGLU && a.res_in && tid < hi - lo) res0 = __ldcg(a.res_in + lo + tid);
         if (!x_ok) {
             s_abort = 1;
             atomicExch(a.status, 3);
         }
         if constexpr (TWO) quantize_x_mma<NP, Q6, NTOK>(a.x + a.tok_x_stride, U, xq, warp, lane, CW, nullptr, 0u, 1u);
     }
-    const unsigned int pub_tag = EXT && a.npeers > 0 ? *reinterpret_cast<const volatile unsigned int *>(a.pub_gen) + 1u : 0u;
+    const unsigned int pub_tag = PEER && a.npeers > 0 ? *reinterpret_cast<const volatile unsigned int *>(a.pub_gen) + 1u : 0u;
     if constexpr (Q6 && NP < 4) {   // a block of zeros for lanes whose product column is empty
         for (uint32_t z = tid; z < 768 / 4; z += C) reinterpret_cast<uint32_t *>(xq + (size_t)U * XQSB + 8 * U)[z] = 0u;
     }
@@ -803,9 +814,9 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
     int buf_seg = 0;
     float sq = 0.0f;                          // this thread's share of the sum of squares of the outputs (residual epilogue)
     float rms = 1.0f;                         // 1 / rms of a normalised x
-    bool have_rms = !(EXT && a.norm_w);
+    bool have_rms = !(FUSE && a.norm_w);
     auto flush = [&]() {
-        if (EXT && !have_rms) { rms = norm_rms(s_share, CW, a.in_dim, a.norm_eps); have_rms = true; }
+        if (FUSE && !have_rms) { rms = norm_rms(s_share, CW, a.in_dim, a.norm_eps); have_rms = true; }
         named_bar_sync(PIPE_BAR_CONSUMERS, (int)C);
         const float *src = red + (size_t)which * PLANE * (SWIGLU || TWO ? 2 : 1);
         float *y = a.seg[buf_seg].y + buf_row0 + (MOE != 0 ? (size_t)blockIdx.y * a.tok_y_stride : 0);
@@ -815,9 +826,9 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
                 gsum += src[r * SLOTS + w];
                 if constexpr (SWIGLU || TWO) usum += src[PLANE + r * SLOTS + w];
             }
-            if constexpr (EXT) { gsum *= rms; usum *= rms; }
+            if constexpr (FUSE) { gsum *= rms; usum *= rms; }
             float val = SWIGLU ? silu_mul(gsum, usum) : gsum;
-            if constexpr (EXT && !SWIGLU) {
+            if constexpr (FUSE && !SWIGLU) {
                 if (a.res_in) {               // residual add, clamped to the fp16 range as the reference's kernel does
                     const float res = buf_row0 + r == lo + tid ? res0 : __ldcg(a.res_in + buf_row0 + r);      // (one tensor: its rows are the CTA's)
                     val = fminf(fmaxf(res + val, -65504.0f), 65504.0f);
@@ -826,7 +837,7 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
             }
             y[r] = val;
             if constexpr (TWO) y[a.tok_y_stride + r] = usum;      // the second vector's product
-            if constexpr (EXT) {
+            if constexpr (PEER) {
                 if (a.npeers > 0) {
                     uint8_t *slot = a.ll_origin + 2 * (reinterpret_cast<const uint8_t *>(y + r) - a.arena_base);
                     st_slot(reinterpret_cast<uint2 *>(slot), val, pub_tag);
@@ -926,7 +937,7 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
     }
     if (tid == 0) stamp(a.trace, 6);
     if (buf_n) flush();
-    if constexpr (EXT && !SWIGLU) {
+    if constexpr (FUSE && !SWIGLU) {
         if (a.res_parts) {
             __shared__ float s_sq[MMA_MAX_CONSUMER_WARPS];
             sq = warp_sum(sq);
@@ -940,7 +951,7 @@ gemv_mma_kernel(const __grid_constant__ MmaArgs a)
             for (uint32_t q = gridDim.x + blockIdx.x * C + tid; q < (uint32_t)PIPE_SUM_SQ_PARTS; q += gridDim.x * C) a.res_parts[q] = 0.0f;
         }
     }
-    if (EXT && a.npeers > 0) {
+    if (PEER && a.npeers > 0) {
         if (tid == 0 && atomicAdd(a.pub_arrived, 1u) == gridDim.x - 1) {   // last CTA: the new generation becomes current
             *reinterpret_cast<volatile unsigned int *>(a.pub_arrived) = 0;
             *reinterpret_cast<volatile unsigned int *>(a.pub_gen) = pub_tag;

@@ -29,6 +29,8 @@
 //   * Every wait on a copy barrier is bounded by a timer; on expiry the kernel
 //     records a code in the status word, stops waiting and runs to completion.
 #pragma once
+#include <type_traits>
+
 #include "decode.cuh"
 
 namespace orome {
@@ -363,8 +365,8 @@ __device__ __forceinline__ float fixed_unit(float inv) { return __frcp_rn(inv); 
 // consecutive floats, a group of G elements is G/4 adjacent lanes.
 // `nvec` vectors of in_dim floats, x_stride floats apart, are quantized in one pass (all loads of a batch are in
 // flight together); vector v goes to xq + v * vec_bytes.  in_dim is a multiple of 32, so groups never straddle vectors.
-// With `slots` set, x is a gathered vector: its elements come from {value, tag} slots and are polled for `tag`;
-// the return value is false when a poll expired.
+// GATHERED: the elements of x come from {value, tag} slots and are polled for `tag`; the return value is false when a poll
+// expired.  (An instance of its own: with the choice made load by load, the loads of a batch waited for one another.)
 // One four-float piece (piece number f of its vector) into the quantized copy at xq: the lanes of a group agree on the
 // group's scale by shuffles, so whole warps must call this together (`valid` false for lanes past the end).
 template <int NP, int G, bool SUMS>
@@ -419,65 +421,93 @@ __device__ __forceinline__ float norm_rms(const float *s_share, uint32_t nwarps,
     return rsqrtf(t / (float)in_dim + eps);
 }
 
-template <int NP, int G, bool SUMS, bool NORM = false>
+// Loads that stay where they are written: left to itself the compiler moved the loads of a batch down to their uses in some
+// instances, one round trip to L2 after the other (4096-wide x with fused neighbours: 3.0 us from the wait to the last piece, 1.6
+// where it did not).
+__device__ __forceinline__ float4 ldcg4_here(const float4 *p)
+{
+    float4 v;
+    asm volatile("ld.global.cg.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint2 ldnc2_here(const uint2 *p)
+{
+    uint2 v;
+    asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+
+template <int NP, int G, bool SUMS, bool NORM = false, bool GATHERED = false>
 __device__ __forceinline__ bool quantize_x_to_smem(const float *__restrict__ x, uint32_t in_dim, uint32_t nvec, uint32_t x_stride,
                                                    uint8_t *xq0, uint32_t vec_bytes, uint32_t tid, uint32_t nthreads,
                                                    const uint2 *slots = nullptr, unsigned int tag = 0,
                                                    long long limit = PIPE_WAIT_CYCLES, const int *status = nullptr, uint32_t rot = 0,
                                                    uint32_t issued_bar = 0, const uint16_t *norm_w = nullptr)
 {
-    // NORM: x is multiplied by the bf16 norm weights on the way (1 / rms: see norm_rms); both are requested before any is used.
+    // NORM: x is multiplied by the bf16 norm weights (none: by one) on the way (1 / rms: see norm_rms).
     // issued_bar: shared address of an mbarrier on which every warp arrives once the loads of its first batch are on
     // their way (0: none).  The weight producer holds its copies back until then, see the kernel.
     // rot (single vector only; a multiple of 32 four-float pieces): this CTA walks the vector starting rot pieces in and
     // wraps around.  When every CTA of a grid reads the same vector at the same moment, different rot values keep them
     // on different cache lines (L2 slices) at any one time instead of all queueing on the same line.
+    // (Rolled, four pieces a round and the next round's loads ahead of this one's arithmetic, it is a third of the instructions; 1 % slower.)
     bool ok = true;
     constexpr int BATCH = 8;
     const uint32_t n4 = in_dim / 4, n4_all = n4 * nvec, lane = tid & 31u;
-    if (issued_bar && slots) {      // a gathered x is polled until the peers have written it: nothing to order the copies behind
+    if (GATHERED && issued_bar) {   // a gathered x is polled until the peers have written it: nothing to order the copies behind
         __syncwarp();
         if (lane == 0) mbar_arrive(issued_bar);
         issued_bar = 0;
     }
-    for (uint32_t base = tid - lane; base < n4_all; base += nthreads * BATCH) {
-        float4 v[BATCH];
-        uint2 nw[NORM ? BATCH : 1];
+    struct Round { float4 v[BATCH]; uint2 nw[NORM ? BATCH : 1]; };
+    auto place = [&](uint32_t fa, uint32_t &vec) {      // piece fa of all: its vector, and its place there
+        vec = nvec == 1 ? 0u : fa / n4;                 // no division on the single-vector path
+        uint32_t f = fa - vec * n4;
+        if (nvec == 1) { f += rot; if (f >= n4) f -= n4; }
+        return f;
+    };
+    auto load = [&](uint32_t base, Round &r) {
 #pragma unroll
         for (int b = 0; b < BATCH; ++b) {
             const uint32_t fa = base + b * nthreads + lane;
-            const uint32_t vec = nvec == 1 ? 0u : fa / n4;      // no division on the single-vector path
-            uint32_t fl = fa - vec * n4;
-            if (nvec == 1) { fl += rot; if (fl >= n4) fl -= n4; }
-            if (slots) v[b] = fa < n4_all ? ld_gathered4(slots + 4 * (size_t)fl, tag, &ok, limit, status) : make_float4(0.f, 0.f, 0.f, 0.f);
-            else v[b] = fa < n4_all ? __ldcg(reinterpret_cast<const float4 *>(x + (size_t)vec * x_stride) + fl) : make_float4(0.f, 0.f, 0.f, 0.f);
-            if constexpr (NORM) nw[b] = fa < n4_all ? __ldg(reinterpret_cast<const uint2 *>(norm_w) + fl) : make_uint2(0u, 0u);
+            uint32_t vec;
+            const uint32_t fl = place(fa, vec);
+            if constexpr (GATHERED) r.v[b] = fa < n4_all ? ld_gathered4(slots + 4 * (size_t)fl, tag, &ok, limit, status) : make_float4(0.f, 0.f, 0.f, 0.f);
+            else {
+                r.v[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (fa < n4_all) r.v[b] = ldcg4_here(reinterpret_cast<const float4 *>(x + (size_t)vec * x_stride) + fl);
+            }
+            if constexpr (NORM) {
+                r.nw[b] = make_uint2(0x3F803F80u, 0x3F803F80u);
+                if (norm_w && fa < n4_all) r.nw[b] = ldnc2_here(reinterpret_cast<const uint2 *>(norm_w) + fl);
+            }
         }
-        if (issued_bar && base == tid - lane) {
+    };
+#pragma unroll 1
+    for (uint32_t base = tid - lane; base < n4_all; base += nthreads * BATCH) {
+        Round r;
+        load(base, r);
+        if (issued_bar) {
             __syncwarp();
             if (lane == 0) mbar_arrive(issued_bar);
-        }
-        if constexpr (NORM) {
-#pragma unroll
-            for (int b = 0; b < BATCH; ++b) {
-                v[b].x *= __uint_as_float(nw[b].x << 16);
-                v[b].y *= __uint_as_float(nw[b].x & 0xffff0000u);
-                v[b].z *= __uint_as_float(nw[b].y << 16);
-                v[b].w *= __uint_as_float(nw[b].y & 0xffff0000u);
-            }
+            issued_bar = 0;
         }
 #pragma unroll
         for (int b = 0; b < BATCH; ++b) {
             const uint32_t fb = base + b * nthreads;       // warp-uniform
             if (fb >= n4_all) break;
-            const uint32_t fa = fb + lane;
-            const uint32_t vec = nvec == 1 ? 0u : fa / n4;
-            uint32_t f = fa - vec * n4;
-            if (nvec == 1) { f += rot; if (f >= n4) f -= n4; }
-            quantize_piece<NP, G, SUMS>(v[b], f, fa < n4_all, lane, xq0 + (size_t)vec * vec_bytes, in_dim);
+            uint32_t vec;
+            const uint32_t f = place(fb + lane, vec);
+            if constexpr (NORM) {
+                r.v[b].x *= __uint_as_float(r.nw[b].x << 16);
+                r.v[b].y *= __uint_as_float(r.nw[b].x & 0xffff0000u);
+                r.v[b].z *= __uint_as_float(r.nw[b].y << 16);
+                r.v[b].w *= __uint_as_float(r.nw[b].y & 0xffff0000u);
+            }
+            quantize_piece<NP, G, SUMS>(r.v[b], f, fb + lane < n4_all, lane, xq0 + (size_t)vec * vec_bytes, in_dim);
         }
     }
-    if (issued_bar && tid - lane >= n4_all) {      // a warp without a piece of x arrives all the same
+    if (issued_bar) {      // a warp without a piece of x arrives all the same
         __syncwarp();
         if (lane == 0) mbar_arrive(issued_bar);
     }
@@ -839,13 +869,15 @@ __device__ __forceinline__ void issue_tile(const PipeArgs &a, const PipeTile &t,
 }
 
 // MODE 0: y = W x.  MODE 1: fused gate/up, y = silu(Wg x) * (Wu x).  MODE 2: combine, y = sum_s weight_s * (W_s x_s).
-// EXT compiles in the expert indirection and the multi-GPU publish / wait paths; dense single-GPU launches use the
-// EXT = false instance, which carries none of that code.
-template <int FMT, int NP, int MODE, int MINB, bool EXT>
+// EXT 1 compiles in the expert indirection and the multi-GPU publish / wait paths, EXT 2 the fused norm / residual neighbours; plain
+// launches use EXT 0, which carries none of that code.  (1 and 2 never meet in a launch.  As one instance they were 100 KB of
+// instructions, 50-65 now, and a launch starts with cold instruction caches: 9B token 1726 -> 1549 us.)
+template <int FMT, int NP, int MODE, int MINB, int EXT>
 __global__ void __launch_bounds__(MINB == 2 ? PIPE_THREADS_2CTA : PIPE_MAX_THREADS, MINB)
 gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
 {
-    constexpr bool SWIGLU = MODE == 1, COMBINE = MODE == 2;
+    constexpr bool SWIGLU = MODE == 1, COMBINE = MODE == 2, PEER = EXT == 1, FUSE = EXT == 2;
+    static_assert(!(COMBINE && FUSE), "the combine form has no fused neighbours");
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem);
     uint64_t *empty = full + PIPE_MAX_STAGES;
@@ -883,12 +915,12 @@ gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
     if (producer) {
         // The weight copies do not depend on the previous kernel: no griddepcontrol.wait on this path.
         if (lane == 0) {
-            if constexpr (EXT) { if (a.seg_expert) pdl_wait(); }   // the expert indices are the previous kernel's output
+            if constexpr (PEER) { if (a.seg_expert) pdl_wait(); }   // the expert indices are the previous kernel's output
             PipeWalk w;
             walk_init<COMBINE>(a, w);
             uint32_t i = 0, s = 0, k = 0;       // tile index, its stage and how many times the ring has wrapped
             PipeTile t;
-            while (next_tile<COMBINE, EXT>(a, w, t)) {
+            while (next_tile<COMBINE, PEER>(a, w, t)) {
                 if (k > 0) {
                     if (s_abort || !mbar_wait_bounded(smem_u32(empty + s), (k - 1) & 1u)) {
                         if (!s_abort) { s_abort = 1; atomicExch(a.status, 2); }
@@ -896,7 +928,7 @@ gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 }
-                issue_tile<SWIGLU, EXT>(a, t, stages + (size_t)s * a.stage_stride, smem_u32(full + s));
+                issue_tile<SWIGLU, PEER>(a, t, stages + (size_t)s * a.stage_stride, smem_u32(full + s));
                 ++i;
                 if (++s == a.nstages) { s = 0; ++k; }
                 if (i == 1) mbar_wait_bounded(smem_u32(&s_x_issued), 0);      // x first (see above); an expired wait only loses the ordering
@@ -928,7 +960,7 @@ gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
     const int part = (int)(j / U);
     const uint32_t unit = j % U;
 
-    if constexpr (EXT && !COMBINE) {
+    if constexpr (FUSE) {
         if (a.norm_w) {           // from memory, so on their way to L2 before the wait; read after it, next to x
             for (uint32_t p = tid * 128u; p < a.in_dim * 2u; p += C * 128u) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t *>(a.norm_w) + p));
         }
@@ -944,25 +976,28 @@ gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
     {
         uint8_t *xq = smem + a.xs_base;
         // a gathered x: every element is polled for the generation this rank gave its own slice (visible after the wait above)
-        const uint2 *slots = EXT ? a.x_ll : nullptr;
-        const unsigned int want = EXT && a.x_ll ? *reinterpret_cast<const volatile unsigned int *>(a.wait_gen) : 0u;
-        const float *x = a.x + (EXT ? (size_t)blockIdx.y * a.tok_x_stride : 0);
+        const float *x = a.x + (PEER ? (size_t)blockIdx.y * a.tok_x_stride : 0);
         const uint32_t rot = COMBINE ? 0u : (uint32_t)((uint64_t)blockIdx.x * (a.in_dim / 4) / gridDim.x) & ~31u;
-        bool x_ok;
-        if constexpr (EXT && !COMBINE) {
-            if (a.norm_w) {
-                share = norm_share(a.norm_parts, tid, C);
-                x_ok = quantize_x_to_smem<NP, SlotT::GROUP, SlotT::SUMS, true>(x, a.in_dim, 1u, a.x_stride, xq, a.xq_vec_bytes, tid, C, slots, want, a.wait_cycles,
-                                                                             a.status, rot, smem_u32(&s_x_issued), a.norm_w);
-                share = warp_sum(share);
-                if (lane == 0) s_share[tid >> 5] = share;
-            } else
-                x_ok = quantize_x_to_smem<NP, SlotT::GROUP, SlotT::SUMS>(x, a.in_dim, 1u, a.x_stride, xq, a.xq_vec_bytes, tid, C, slots, want, a.wait_cycles,
-                                                                       a.status, rot, smem_u32(&s_x_issued));
-        } else
-            x_ok = quantize_x_to_smem<NP, SlotT::GROUP, SlotT::SUMS>(x, a.in_dim, COMBINE ? (uint32_t)a.nseg : 1u, a.x_stride, xq, a.xq_vec_bytes, tid, C, slots, want,
-                                                                   a.wait_cycles, a.status, rot, smem_u32(&s_x_issued));
-        if constexpr (EXT && MODE == 0) {
+        bool x_ok = true;
+        auto pass = [&](auto norm, auto gathered) {
+            constexpr bool N = decltype(norm)::value, GA = decltype(gathered)::value;
+            return quantize_x_to_smem<NP, SlotT::GROUP, SlotT::SUMS, N, GA>(x, a.in_dim, COMBINE ? (uint32_t)a.nseg : 1u, a.x_stride, xq, a.xq_vec_bytes, tid, C, GA ? a.x_ll : nullptr,
+                                                                         GA ? *reinterpret_cast<const volatile unsigned int *>(a.wait_gen) : 0u, a.wait_cycles, a.status,
+                                                                         rot, smem_u32(&s_x_issued), N ? a.norm_w : nullptr);
+        };
+        constexpr std::true_type yes{};
+        constexpr std::false_type no{};
+        if constexpr (FUSE) {
+            if (a.norm_w) share = norm_share(a.norm_parts, tid, C);
+            x_ok = pass(yes, no);
+            share = warp_sum(share);
+            if (lane == 0) s_share[tid >> 5] = share;
+        } else if (PEER && a.x_ll) {
+            if constexpr (PEER) x_ok = pass(no, yes);
+        } else {
+            x_ok = pass(no, no);
+        }
+        if constexpr (FUSE && MODE == 0) {
             if (a.res_in && cta_row0 + tid < (uint32_t)((uint64_t)(blockIdx.x + 1) * a.total_rows / gridDim.x)) res0 = __ldcg(a.res_in + cta_row0 + tid);
         }
         if (!x_ok) {
@@ -980,7 +1015,7 @@ gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
     // Per-row partial sums (one per warp of the row's group) collect in shared memory and are added up, a whole
     // batch of rows at a time, by all consumer threads: one consumer-wide barrier per batch, coalesced stores of y.
     // Two buffers alternate, so the barrier that opens a flush also protects the buffer written two flushes ago.
-    const unsigned int pub_tag = EXT && a.npeers > 0 ? *reinterpret_cast<const volatile unsigned int *>(a.pub_gen) + 1u : 0u;
+    const unsigned int pub_tag = PEER && a.npeers > 0 ? *reinterpret_cast<const volatile unsigned int *>(a.pub_gen) + 1u : 0u;
     const uint32_t CAP = a.red_rows, PLANE = CAP * GW;                 // floats per buffer (per tensor)
     PipeWalk wk;
     walk_init<COMBINE>(a, wk);
@@ -1005,12 +1040,12 @@ gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
     int buf_seg = 0;
     float sq = 0.0f;                          // this thread's share of the sum of squares of the outputs (residual epilogue)
     float rms = 1.0f;                         // 1 / rms of a normalised x
-    bool have_rms = COMBINE || !(EXT && a.norm_w);
+    bool have_rms = !(FUSE && a.norm_w);
     auto flush = [&]() {
-        if (EXT && !COMBINE && !have_rms) { rms = norm_rms(s_share, C >> 5, a.in_dim, a.norm_eps); have_rms = true; }
+        if (FUSE && !have_rms) { rms = norm_rms(s_share, C >> 5, a.in_dim, a.norm_eps); have_rms = true; }
         named_bar_sync(PIPE_BAR_CONSUMERS, (int)C);
         const float *src = pbuf + (size_t)which * PLANE * (SWIGLU ? 2 : 1);
-        float *y = a.seg[buf_seg].y + buf_row0 + (EXT ? (size_t)blockIdx.y * a.tok_y_stride : 0);
+        float *y = a.seg[buf_seg].y + buf_row0 + (PEER ? (size_t)blockIdx.y * a.tok_y_stride : 0);
         for (uint32_t r = tid; r < buf_n; r += C) {
             float g = 0.0f, u = 0.0f;
             const uint32_t nsl = comb_acc ? SL : GW;
@@ -1020,9 +1055,9 @@ gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
             }
             if constexpr (COMBINE) accbuf[buf_row0 - wk.lo + r] += (comb_acc ? 1.0f : a.seg_weight[blockIdx.y * a.tok_sel_stride + buf_seg]) * g;   // one owner per row and flush
             else {
-                if constexpr (EXT) { g *= rms; u *= rms; }
+                if constexpr (FUSE) { g *= rms; u *= rms; }
                 float val = SWIGLU ? silu_mul(g, u) : g;
-                if constexpr (EXT && MODE == 0) {
+                if constexpr (FUSE && MODE == 0) {
                     if (a.res_in) {           // residual add, clamped to the fp16 range as the reference's kernel does
                         const float res = buf_row0 + r == cta_row0 + tid ? res0 : __ldcg(a.res_in + buf_row0 + r);      // (one tensor: its rows are the CTA's)
                         val = fminf(fmaxf(res + val, -65504.0f), 65504.0f);
@@ -1030,7 +1065,7 @@ gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
                     }
                 }
                 y[r] = val;
-                if constexpr (EXT) {
+                if constexpr (PEER) {
                     if (a.npeers > 0) {
                         uint8_t *slot = a.ll_origin + 2 * (reinterpret_cast<const uint8_t *>(y + r) - a.arena_base);
                         st_slot(reinterpret_cast<uint2 *>(slot), val, pub_tag);
@@ -1050,7 +1085,7 @@ gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
     uint32_t delta = 0, delta2 = 0;
     const bool rows16 = (a.row_bytes & 15u) == 0;     // then every row starts at the same offset inside its 16-byte piece
     PipeTile t;
-    while (next_tile<COMBINE, EXT>(a, wk, t)) {
+    while (next_tile<COMBINE, PEER>(a, wk, t)) {
         if (!comb_acc && buf_n && (t.seg != buf_seg || buf_n + t.n > CAP)) flush();
         if (!comb_acc && buf_n == 0) { buf_seg = t.seg; buf_row0 = t.row0; }
         const bool mine = !comb_acc || (uint32_t)t.seg % a.rows_par == group;    // segment-parallel combine: one group per segment
@@ -1080,8 +1115,8 @@ gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
         if (i == 0 && tid == 0) stamp(a.trace, 5);
         if (!rows16 || t.seg != delta_seg) {   // offset of the tile's first byte inside its 16-byte piece
             delta_seg = t.seg;
-            delta = ((uint32_t)reinterpret_cast<uintptr_t>(seg_w<EXT>(a, t.seg)) + t.row0 * a.row_bytes) & 15u;
-            if constexpr (SWIGLU) delta2 = ((uint32_t)reinterpret_cast<uintptr_t>(seg_w2<EXT>(a, t.seg)) + t.row0 * a.row_bytes) & 15u;
+            delta = ((uint32_t)reinterpret_cast<uintptr_t>(seg_w<PEER>(a, t.seg)) + t.row0 * a.row_bytes) & 15u;
+            if constexpr (SWIGLU) delta2 = ((uint32_t)reinterpret_cast<uintptr_t>(seg_w2<PEER>(a, t.seg)) + t.row0 * a.row_bytes) & 15u;
         }
         const uint32_t base = stages_s + s * a.stage_stride + delta + unit_off;
         uint32_t base2 = 0;
@@ -1132,9 +1167,9 @@ gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
     if constexpr (COMBINE) {
         named_bar_sync(PIPE_BAR_CONSUMERS, (int)C);
         for (uint32_t r = tid; r < wk.hi - wk.lo; r += C) {
-            float *dst = a.seg[0].y + wk.lo + r + (EXT ? (size_t)blockIdx.y * a.tok_y_stride : 0);
+            float *dst = a.seg[0].y + wk.lo + r + (PEER ? (size_t)blockIdx.y * a.tok_y_stride : 0);
             *dst = accbuf[r];
-            if constexpr (EXT) {
+            if constexpr (PEER) {
                 if (a.npeers > 0) {
                     uint8_t *slot = a.ll_origin + 2 * (reinterpret_cast<const uint8_t *>(dst) - a.arena_base);
                     st_slot(reinterpret_cast<uint2 *>(slot), accbuf[r], pub_tag);
@@ -1143,7 +1178,7 @@ gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
             }
         }
     }
-    if constexpr (EXT && MODE == 0) {
+    if constexpr (FUSE && MODE == 0) {
         if (a.res_parts) {
             __shared__ float s_sq[PIPE_MAX_CONSUMERS / 32];
             sq = warp_sum(sq);
@@ -1157,7 +1192,7 @@ gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
             for (uint32_t i = gridDim.x + blockIdx.x * C + tid; i < (uint32_t)PIPE_SUM_SQ_PARTS; i += gridDim.x * C) a.res_parts[i] = 0.0f;
         }
     }
-    if (EXT && a.npeers > 0) {
+    if (PEER && a.npeers > 0) {
         // the last CTA to get here makes the new generation this rank's current one; a launch that consumes the
         // vector reads it after its griddepcontrol.wait, i.e. after this grid has completed
         if (tid == 0 && atomicAdd(a.pub_arrived, 1u) == gridDim.x - 1) {

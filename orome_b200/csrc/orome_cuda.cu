@@ -524,7 +524,7 @@ static int plan_pipe(orome_cuda_ctx *c, int fmt, uint32_t in_dim, uint32_t total
     return OROME_OK;
 }
 
-template <int FMT, int NP, int MODE, int MINB, bool EXT>
+template <int FMT, int NP, int MODE, int MINB, int EXT>
 static int launch_pipe_ext(orome_cuda_ctx *c, const PipePlan &p, cudaStream_t st)
 {
     auto kern = gemv_pipe_kernel<FMT, NP, MODE, MINB, EXT>;
@@ -555,9 +555,10 @@ static int launch_pipe_ext(orome_cuda_ctx *c, const PipePlan &p, cudaStream_t st
 template <int FMT, int NP, int MODE, int MINB>
 static int launch_pipe_inst(orome_cuda_ctx *c, const PipePlan &p, cudaStream_t st)
 {
-    const bool ext = p.args.seg_expert || p.args.npeers > 0 || p.args.x_ll || p.args.norm_w || p.args.res_in || p.tokens > 1;
-    if constexpr (MODE == 2) return launch_pipe_ext<FMT, NP, MODE, MINB, true>(c, p, st);
-    else return ext ? launch_pipe_ext<FMT, NP, MODE, MINB, true>(c, p, st) : launch_pipe_ext<FMT, NP, MODE, MINB, false>(c, p, st);
+    const bool ext = p.args.seg_expert || p.args.npeers > 0 || p.args.x_ll || p.tokens > 1;
+    if constexpr (MODE == 2) return launch_pipe_ext<FMT, NP, MODE, MINB, 1>(c, p, st);
+    else if (p.args.norm_w || p.args.res_in) return launch_pipe_ext<FMT, NP, MODE, MINB, 2>(c, p, st);
+    else return ext ? launch_pipe_ext<FMT, NP, MODE, MINB, 1>(c, p, st) : launch_pipe_ext<FMT, NP, MODE, MINB, 0>(c, p, st);
 }
 
 template <int FMT, int NP>
@@ -687,7 +688,7 @@ static int mma_encode_maps(orome_cuda_ctx *c, int fmt, MmaPlan &p, bool swiglu)
     return OROME_OK;
 }
 
-template <int FMT, int NP, bool SWIGLU, bool EXT, int MOE = 0, int NTOK = 1>
+template <int FMT, int NP, bool SWIGLU, int EXT, int MOE = 0, int NTOK = 1>
 static int launch_mma_ext(orome_cuda_ctx *c, const MmaPlan &p, cudaStream_t st)
 {
     auto kern = gemv_mma_kernel<FMT, NP, SWIGLU, EXT, MOE, NTOK>;
@@ -721,8 +722,8 @@ static int launch_mma_two(orome_cuda_ctx *c, int fmt, MmaPlan &p, cudaStream_t s
     int rc = mma_encode_maps(c, fmt, p, false);
     if (rc) return rc;
     const bool b24 = c->x_bits == 24;
-    if (fmt == FMT_Q4_K) return b24 ? launch_mma_ext<FMT_Q4_K, 3, false, false, 0, 2>(c, p, st) : launch_mma_ext<FMT_Q4_K, 2, false, false, 0, 2>(c, p, st);
-    return b24 ? launch_mma_ext<FMT_Q5_K, 3, false, false, 0, 2>(c, p, st) : launch_mma_ext<FMT_Q5_K, 2, false, false, 0, 2>(c, p, st);
+    if (fmt == FMT_Q4_K) return b24 ? launch_mma_ext<FMT_Q4_K, 3, false, 0, 0, 2>(c, p, st) : launch_mma_ext<FMT_Q4_K, 2, false, 0, 0, 2>(c, p, st);
+    return b24 ? launch_mma_ext<FMT_Q5_K, 3, false, 0, 0, 2>(c, p, st) : launch_mma_ext<FMT_Q5_K, 2, false, 0, 0, 2>(c, p, st);
 }
 
 // The MoE forms of the mma kernel (Q4_K / Q5_K): fused gate/up over device-chosen experts, down + weighted combine.
@@ -730,9 +731,9 @@ static int launch_mma_moe(orome_cuda_ctx *c, int fmt, MmaPlan &p, bool gate_up, 
 {
     const bool b24 = c->x_bits == 24;
     if (gate_up)      // the fused form always reads x at 24 bits
-        return fmt == FMT_Q4_K ? launch_mma_ext<FMT_Q4_K, 3, true, false, 1>(c, p, st) : launch_mma_ext<FMT_Q5_K, 3, true, false, 1>(c, p, st);
-    if (fmt == FMT_Q4_K) return b24 ? launch_mma_ext<FMT_Q4_K, 3, false, false, 2>(c, p, st) : launch_mma_ext<FMT_Q4_K, 2, false, false, 2>(c, p, st);
-    return b24 ? launch_mma_ext<FMT_Q5_K, 3, false, false, 2>(c, p, st) : launch_mma_ext<FMT_Q5_K, 2, false, false, 2>(c, p, st);
+        return fmt == FMT_Q4_K ? launch_mma_ext<FMT_Q4_K, 3, true, 0, 1>(c, p, st) : launch_mma_ext<FMT_Q5_K, 3, true, 0, 1>(c, p, st);
+    if (fmt == FMT_Q4_K) return b24 ? launch_mma_ext<FMT_Q4_K, 3, false, 0, 2>(c, p, st) : launch_mma_ext<FMT_Q4_K, 2, false, 0, 2>(c, p, st);
+    return b24 ? launch_mma_ext<FMT_Q5_K, 3, false, 0, 2>(c, p, st) : launch_mma_ext<FMT_Q5_K, 2, false, 0, 2>(c, p, st);
 }
 
 template <int FMT, int NP, bool SWIGLU>
@@ -741,8 +742,8 @@ static int launch_mma_inst(orome_cuda_ctx *c, const MmaPlan &p, cudaStream_t st)
     // Products with fused neighbours read x as four byte planes: their dp4a form (shapes and alignments this kernel does not
     // take) scales x per 32 elements, this kernel per 256, and the spare columns of the mma hold a fourth plane for nothing
     // (rel-L2 against fp64 on 2400 x 4352: dp4a 1.5-1.7e-7, three planes 1.7-1.9e-7, four planes 1.4-1.5e-7).
-    if (p.args.norm_w || p.args.res_in) return launch_mma_ext<FMT, 4, SWIGLU, true>(c, p, st);
-    return p.args.npeers > 0 || p.args.x_ll ? launch_mma_ext<FMT, NP, SWIGLU, true>(c, p, st) : launch_mma_ext<FMT, NP, SWIGLU, false>(c, p, st);
+    if (p.args.norm_w || p.args.res_in) return launch_mma_ext<FMT, 4, SWIGLU, 2>(c, p, st);
+    return p.args.npeers > 0 || p.args.x_ll ? launch_mma_ext<FMT, NP, SWIGLU, 1>(c, p, st) : launch_mma_ext<FMT, NP, SWIGLU, 0>(c, p, st);
 }
 
 static int launch_mma(orome_cuda_ctx *c, int fmt, MmaPlan &p, bool swiglu, cudaStream_t st)
