@@ -147,7 +147,12 @@ int orome_launch_tc(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t ou
 {
     TcPub no_pub;
     memset(&no_pub, 0, sizeof no_pub);
+    const bool single = !pub && !x_ll;
     if (!pub) pub = &no_pub;
+    if (single && orome_few_supported(c, fmt, out_dim, in_dim, batch, false)) {
+        const int rc = orome_launch_few(c, fmt, data, nullptr, out_dim, in_dim, layout, x, batch, ldx, y, ldy, st);
+        if (rc != OROME_ENOTSUP) return rc;
+    }
     if (c->tc_slabs) return launch_staged(c, fmt, data, out_dim, in_dim, layout, x, batch, ldx, y, ldy, st, pub, x_ll, wait_gen);
     const uint32_t chunks = in_dim / TC_KC, mtiles = (out_dim + TP_ROWS - 1) / TP_ROWS;
     // At most 4096 vectors a launch (bounds the packed X), fewer where the packed X of that many has no room: while a graph is

@@ -24,3 +24,9 @@ bool orome_tc_supported(const orome_cuda_ctx *c, int fmt, uint32_t in_dim);
 int orome_launch_tc(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t out_dim, uint32_t in_dim, int layout, const float *x,
                     int batch, int ldx, float *y, int ldy, cudaStream_t st, const orome::TcPub *pub = nullptr, const uint2 *x_ll = nullptr,
                     const unsigned int *wait_gen = nullptr);
+
+// Few vectors (gemm_few.cuh): Y, or with w1 (at most eight vectors) silu(W0 x) * (W1 x), in one launch behind the packing of X.  packed: X
+// is the one the previous launch on the stream has packed.  OROME_ENOTSUP: no scratch for X.
+bool orome_few_supported(const orome_cuda_ctx *c, int fmt, uint32_t out_dim, uint32_t in_dim, int batch, bool fused);      // ... and the faster form there
+int orome_launch_few(orome_cuda_ctx *c, int fmt, const uint8_t *w0, const uint8_t *w1, uint32_t out_dim, uint32_t in_dim, int layout, const float *x,
+                     int batch, int ldx, float *y, int ldy, cudaStream_t st, bool packed = false);

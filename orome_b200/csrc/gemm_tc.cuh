@@ -113,7 +113,7 @@ __device__ __forceinline__ uint32_t sw128_off(uint32_t r, uint32_t c) { return (
 // small batch and by HBM for a large one).
 // x_ll: X is a gathered matrix in the arena, read from its slots (every element polled, bounded, for the generation
 // *wait_gen); NULL: a plain matrix.
-__global__ void __launch_bounds__(256)
+static __global__ void __launch_bounds__(256)
 pack_x_f16_kernel(const float *__restrict__ x, int batch, int ldx, uint32_t in_dim, uint32_t nt_rows, __half *__restrict__ xp,
                   const uint2 *x_ll, const unsigned int *wait_gen, long long wait_cycles, int *status)
 {
@@ -387,7 +387,7 @@ gemm_tc_kernel(const __grid_constant__ TcArgs a)
 
 
 // Y[b][r] = sum over splits of partial[s][b][r]
-__global__ void splitk_reduce_kernel(const float *__restrict__ part, uint32_t split, uint32_t batch, uint32_t rows, float *__restrict__ y, uint32_t ldy,
+static __global__ void splitk_reduce_kernel(const float *__restrict__ part, uint32_t split, uint32_t batch, uint32_t rows, float *__restrict__ y, uint32_t ldy,
                                      const TcPub pub)
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -1229,11 +1229,23 @@ extern "C" int orome_cuda_gate_up_swiglu(orome_cuda_ctx *c, const OromeTensorRef
     // two matvecs into context scratch, then the elementwise epilogue (the reference's unfused branch, engine.m:388-404)
     if (batch > 1 && (ldx < (int)gate->in_dim || ldo < (int)gate->out_dim))
         return fail(OROME_EINVAL, "gate_up_swiglu: ldx/ldo smaller than the row length");
+    // few vectors: gate, up and the epilogue in one launch; more than eight: two products of one packed X
+    const bool few = batch > 1 && batch >= c->tc_min_batch && !c->force_generic && ldx % 4 == 0 && !(reinterpret_cast<uintptr_t>(x_dev) & 15);
+    if (few && orome_few_supported(c, fmt, gate->out_dim, gate->in_dim, batch, true)) {
+        rc = orome_launch_few(c, fmt, gd, ud, gate->out_dim, gate->in_dim, layout, x_dev, batch, ldx, out_dev, ldo, st);
+        if (rc != OROME_ENOTSUP) return rc;
+    }
     const size_t n = (size_t)gate->out_dim;
     rc = orome_ensure(c, c->gu, 2 * n * batch, st);
     if (rc) return rc;
     float *g = c->gu.p, *u = c->gu.p + n * batch;
-    if (batch > 1) {
+    rc = few && orome_few_supported(c, fmt, gate->out_dim, gate->in_dim, batch, false) ?
+             orome_launch_few(c, fmt, gd, nullptr, gate->out_dim, gate->in_dim, layout, x_dev, batch, ldx, g, (int)n, st) : OROME_ENOTSUP;
+    if (rc == OROME_OK) {
+        rc = orome_launch_few(c, fmt, ud, nullptr, gate->out_dim, gate->in_dim, layout, x_dev, batch, ldx, u, (int)n, st, true);
+        if (rc) return rc;
+    } else if (rc != OROME_ENOTSUP) return rc;
+    else if (batch > 1) {
         // the batched product's own dispatch: tensor cores from OROME_OPT_TC_MIN_BATCH vectors on, decode launches below
         rc = orome_cuda_matvec(c, gate, x_dev, g, batch, ldx, (int)n, stream);
         if (rc) return rc;

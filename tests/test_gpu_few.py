@@ -1,0 +1,76 @@
+"""The batched form for few vectors (up to 32): plain and fused gate/up, against the fp64 oracle.
+
+Bound: weights and x are rounded to fp16 once (2^-11 each, about 3e-4 of a product of many terms); 1e-3 asked of a product, twice
+that and the gate's slope of a fused one.  A handful of outputs spreads more: their bound is four times as wide."""
+import numpy as np
+import pytest
+
+import oracle
+from orome_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+FORMATS = [(synth.Q8_0, 0), (synth.Q4_K, 0), (synth.Q4_K, 1), (synth.Q5_K, 0), (synth.Q5_K, 1), (synth.Q6_K, 0)]
+# one row; a row tile and its neighbours; one tile a CTA and more; two passes of eight tiles; chunks that warps share unevenly
+SHAPES = [(1, 512), (15, 256), (17, 768), (333, 2560), (2500, 512), (300, 9728), (19200, 256)]
+
+
+@pytest.fixture(scope="module")
+def env():
+    import torch
+    from orome_b200 import format as F
+    ctx = F.Context(0)
+    yield torch, F, ctx
+    assert ctx.status() == 0
+    ctx.close()
+
+
+def _rel(got, want):
+    return float(np.linalg.norm(got - want) / np.linalg.norm(want))
+
+
+@pytest.mark.parametrize("fmt,variant", FORMATS)
+@pytest.mark.parametrize("rows,cols", SHAPES)
+@pytest.mark.parametrize("batch", [4, 8, 9, 24, 32])
+def test_few_vectors(env, fmt, variant, rows, cols, batch):
+    torch, F, ctx = env
+    ldx, ldy = cols + 4, rows + 3
+    w = [synth.host_tensor(fmt, rows, cols, seed=s) for s in (rows, cols)]
+    x = synth.host_x(cols, batch, seed=batch)
+    wt = [torch.from_numpy(t).cuda() for t in w]
+    xt = torch.full((batch, ldx), float("nan"), device="cuda")
+    xt[:, :cols] = torch.from_numpy(x).cuda()
+    y, act = (torch.full((batch, ldy), float("nan"), device="cuda") for _ in range(2))
+    refs = [F.tensor_ref(t.data_ptr(), 0, fmt, rows, cols, variant) for t in wt]
+    ctx.matvec(refs[0], xt.data_ptr(), y.data_ptr(), batch, ldx, ldy)
+    ctx.gate_up_swiglu(refs[0], refs[1], xt.data_ptr(), act.data_ptr(), batch, ldx, ldy)
+    torch.cuda.synchronize()
+    gate, up = (oracle.matvec_f64(fmt, t, rows, cols, x, layout=variant).reshape(batch, rows) for t in w)
+    few = 4 if rows * batch < 1000 else 1
+    assert torch.isnan(y[:, rows:]).all() and torch.isnan(act[:, rows:]).all()
+    assert _rel(y[:, :rows].cpu().numpy(), gate) <= 1e-3 * few
+    assert _rel(act[:, :rows].cpu().numpy(), oracle.swiglu_f64(gate, up).reshape(batch, rows)) <= 3e-3 * few
+
+
+def test_a_captured_product_repeats_its_bits(env):
+    torch, F, _ = env
+    rows, cols = 256, 1024
+    ctx = F.Context(0)
+    w, x = synth.host_tensor(synth.Q4_K, rows, cols, seed=1), synth.host_x(cols, 32, seed=2)
+    wt, xt, y = torch.from_numpy(w).cuda(), torch.from_numpy(x).cuda(), torch.zeros(32, rows, device="cuda")
+    ref = F.tensor_ref(wt.data_ptr(), 0, synth.Q4_K, rows, cols)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        ctx.matvec(ref, xt.data_ptr(), y.data_ptr(), 32, cols, rows, side.cuda_stream)
+    torch.cuda.synchronize()
+    want = y.clone()
+    y.zero_()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        ctx.matvec(ref, xt.data_ptr(), y.data_ptr(), 32, cols, rows, torch.cuda.current_stream().cuda_stream)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
+    assert ctx.status() == 0
+    del graph
+    ctx.close()
