@@ -143,13 +143,13 @@ static uint32_t tp_clusters(const orome_cuda_ctx *c, int fmt, uint32_t tiles, ui
 }
 
 int orome_launch_tc(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t out_dim, uint32_t in_dim, int layout, const float *x,
-                    int batch, int ldx, float *y, int ldy, cudaStream_t st, const TcPub *pub, const uint2 *x_ll, const unsigned int *wait_gen)
+                    int batch, int ldx, float *y, int ldy, cudaStream_t st, const TcPub *pub, const uint2 *x_ll, const unsigned int *wait_gen, bool *x_packed)
 {
     TcPub no_pub;
     memset(&no_pub, 0, sizeof no_pub);
     const bool single = !pub && !x_ll;
     if (!pub) pub = &no_pub;
-    if (single && orome_few_supported(c, fmt, out_dim, in_dim, batch, false)) {
+    if (single && !x_packed && orome_few_supported(c, fmt, out_dim, in_dim, batch, false)) {
         const int rc = orome_launch_few(c, fmt, data, nullptr, out_dim, in_dim, layout, x, batch, ldx, y, ldy, st);
         if (rc != OROME_ENOTSUP) return rc;
     }
@@ -175,6 +175,8 @@ int orome_launch_tc(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t ou
     // so that the products of a layer do not each outgrow the one before)
     while ((rc = orome_ensure(c, c->tc_xp, xp_floats(slice), st, (size_t)8 << 20)) == OROME_ENOMEM && !capturing && !one_launch && slice > 64) slice = (slice / 2 + 63) / 64 * 64;
     if (rc) return rc;
+    const bool packed = x_packed && *x_packed && slice >= batch;
+    if (x_packed) *x_packed = slice >= batch;
     for (int b0 = 0; b0 < batch; b0 += slice) {
         const uint32_t nb = (uint32_t)std::min(batch - b0, slice);
         const uint32_t ntiles = (nb + TP_MAX_N - 1) / TP_MAX_N, nt_rows = ((nb + ntiles - 1) / ntiles + 15) / 16 * 16;
@@ -195,8 +197,10 @@ int orome_launch_tc(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t ou
             if (rc) return rc;
         }
         const bool cut = is_cut();
-        rc = launch_pack(c, x + (size_t)b0 * ldx, (int)nb, ldx, in_dim, nt_rows / 2, 2 * ntiles, x_ll, wait_gen, st);      // a CTA's half of a tile lies together
-        if (rc) return rc;
+        if (!packed) {
+            rc = launch_pack(c, x + (size_t)b0 * ldx, (int)nb, ldx, in_dim, nt_rows / 2, 2 * ntiles, x_ll, wait_gen, st);      // a CTA's half of a tile lies together
+            if (rc) return rc;
+        }
         a.w = data; a.xp = reinterpret_cast<const __half *>(c->tc_xp.p); a.y = y + (size_t)b0 * ldy; a.part = c->tc_part.p;
         a.rows = out_dim; a.row_bytes = (uint32_t)row_bytes_of(fmt, in_dim); a.w_bytes = (uint64_t)a.row_bytes * out_dim;
         a.batch = nb; a.nt_rows = nt_rows; a.ntiles = ntiles; a.ldy = (uint32_t)ldy;

@@ -21,9 +21,11 @@ struct TcPub {
 bool orome_tc_supported(const orome_cuda_ctx *c, int fmt, uint32_t in_dim);
 // Y[b][r] for b < batch.  pub / x_ll / wait_gen: the row-split form on several GPUs (batch <= TC_MAX_N, one launch): Y is
 // published to every rank's arena by the kernel that writes it, a gathered X is read from its slots by the packing kernel.
+// x_packed (never with pub; the tensor-memory form is then the one taken): in, X is the one the previous call on the stream packed; out,
+// all of it lies packed in scratch.
 int orome_launch_tc(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t out_dim, uint32_t in_dim, int layout, const float *x,
                     int batch, int ldx, float *y, int ldy, cudaStream_t st, const orome::TcPub *pub = nullptr, const uint2 *x_ll = nullptr,
-                    const unsigned int *wait_gen = nullptr);
+                    const unsigned int *wait_gen = nullptr, bool *x_packed = nullptr);
 
 // Few vectors (gemm_few.cuh): Y, or with w1 (at most eight vectors) silu(W0 x) * (W1 x), in one launch behind the packing of X.  packed: X
 // is the one the previous launch on the stream has packed.  OROME_ENOTSUP: no scratch for X.
