@@ -33,6 +33,13 @@ __device__ __forceinline__ uint2 ld8_a2(const uint8_t *p)
     return make_uint2(__funnelshift_r(a, b, sh), __funnelshift_r(b, c, sh));
 }
 
+// Byte `b` of a word less `bias` (an integer), exactly, as a float: on top of the bits of 2^23 the byte is a float that much too large.  I2F
+// runs at an eighth of the rate of the permute and the subtraction.
+__device__ __forceinline__ float byte_float(uint32_t v, int b, float bias)
+{
+    return __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7440u + (uint32_t)b)) - (8388608.0f + bias);
+}
+
 // Rows of a quantized tensor lie one behind the other without gaps, so a range of rows is one run of 8-weight pieces: thread i
 // decodes pieces i, i + 32, .. of its warp's 1024 weights and stores 32 bytes a piece, so that a warp's stores are whole lines
 // and its loads fall into a few (a thread per 32-weight block, loading bytes and storing 128 bytes apart, ran at a third of the
@@ -52,6 +59,7 @@ dequant_flat_kernel(const uint8_t *__restrict__ blocks, uint64_t pieces, int lay
     const uint64_t first = (base - lane) / GROUP * BLOCK + 128u * lane;
     if (128u * lane < 32u * DQ_PIECES / GROUP * BLOCK && first < pieces / GROUP * BLOCK) asm volatile("prefetch.global.L2 [%0];" ::"l"(blocks + first));
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    const bool whole = (reinterpret_cast<uintptr_t>(out) & 31) == 0;      // a piece in one store: whole lines a warp
     uint2 q[DQ_PIECES], h[DQ_PIECES];
     uint4 hd[DQ_PIECES];
     uint32_t d[DQ_PIECES];
@@ -89,14 +97,14 @@ dequant_flat_kernel(const uint8_t *__restrict__ blocks, uint64_t pieces, int lay
         if constexpr (FMT == FMT_Q8_0) {
             const float dd = half_bits_to_float(d[k]);
 #pragma unroll
-            for (int b = 0; b < 8; ++b) w[b] = __fmul_rn(dd, (float)(signed char)((b < 4 ? q[k].x : q[k].y) >> (8 * (b & 3))));
+            for (int b = 0; b < 8; ++b) w[b] = __fmul_rn(dd, byte_float((b < 4 ? q[k].x : q[k].y) ^ 0x80808080u, b & 3, 128.0f));
         } else if constexpr (FMT == FMT_Q6_K) {
             const uint32_t j = (p >> 2) & 3u;
             const float a = __fmul_rn(half_bits_to_float(d[k]), (float)sc[k]);
             const uint32_t lo0 = (q[k].x >> (4u * (j >> 1))) & 0x0F0F0F0Fu, lo1 = (q[k].y >> (4u * (j >> 1))) & 0x0F0F0F0Fu;
             const uint32_t v0 = lo0 | (((h[k].x >> (2u * j)) & 0x03030303u) << 4), v1 = lo1 | (((h[k].y >> (2u * j)) & 0x03030303u) << 4);
 #pragma unroll
-            for (int b = 0; b < 8; ++b) w[b] = __fmul_rn(a, (float)((int)(((b < 4 ? v0 : v1) >> (8 * (b & 3))) & 255u) - 32));
+            for (int b = 0; b < 8; ++b) w[b] = __fmul_rn(a, byte_float(b < 4 ? v0 : v1, b & 3, 32.0f));
         } else {
             const uint32_t sub = p >> 2, shift = 4u * (sub & 1u), w0 = hd[k].y, w1 = hd[k].z, w2 = hd[k].w;
             auto byte = [](uint32_t v, uint32_t n) { return (v >> (8u * n)) & 255u; };
@@ -114,11 +122,15 @@ dequant_flat_kernel(const uint8_t *__restrict__ blocks, uint64_t pieces, int lay
             uint32_t v0 = (q[k].x >> shift) & 0x0F0F0F0Fu, v1 = (q[k].y >> shift) & 0x0F0F0F0Fu;
             if constexpr (FMT == FMT_Q5_K) { v0 |= ((h[k].x >> sub) & 0x01010101u) << 4; v1 |= ((h[k].y >> sub) & 0x01010101u) << 4; }
 #pragma unroll
-            for (int b = 0; b < 8; ++b) w[b] = __fsub_rn(__fmul_rn(a, (float)(((b < 4 ? v0 : v1) >> (8 * (b & 3))) & 255u)), mm);
+            for (int b = 0; b < 8; ++b) w[b] = __fsub_rn(__fmul_rn(a, byte_float(b < 4 ? v0 : v1, b & 3, 0.0f)), mm);
         }
         float4 *o = reinterpret_cast<float4 *>(out + i * 8u);
-        o[0] = make_float4(w[0], w[1], w[2], w[3]);
-        o[1] = make_float4(w[4], w[5], w[6], w[7]);
+        if (whole) asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                                ::"l"(o), "f"(w[0]), "f"(w[1]), "f"(w[2]), "f"(w[3]), "f"(w[4]), "f"(w[5]), "f"(w[6]), "f"(w[7]) : "memory");
+        else {
+            o[0] = make_float4(w[0], w[1], w[2], w[3]);
+            o[1] = make_float4(w[4], w[5], w[6], w[7]);
+        }
     }
 }
 
