@@ -28,18 +28,20 @@ static int allow_smem(orome_cuda_ctx *c, K kern, bool (&configured)[64])
     return OROME_OK;
 }
 
-template <int FMT, bool BIG>
+template <int FMT, bool BIG, bool PUB>
 static int launch_pair_inst(orome_cuda_ctx *c, const TpArgs &a, size_t smem, cudaStream_t st)
 {
     static bool configured[64] = {false};
-    int rc = allow_smem(c, gemm_pair_kernel<FMT, BIG>, configured);
+    int rc = allow_smem(c, gemm_pair_kernel<FMT, BIG, PUB>, configured);
     if (rc) return rc;
-    return orome_launch_pdl_smem(c, "gemm_pair", gemm_pair_kernel<FMT, BIG>, dim3(2 * a.clusters), dim3(TP_THREADS), smem, st, a);
+    return orome_launch_pdl_smem(c, "gemm_pair", gemm_pair_kernel<FMT, BIG, PUB>, dim3(2 * a.clusters), dim3(TP_THREADS), smem, st, a);
 }
 template <int FMT>
 static int launch_pair_fmt(orome_cuda_ctx *c, const TpArgs &a, size_t smem, cudaStream_t st)
 {
-    return a.nt_rows > 128 ? launch_pair_inst<FMT, true>(c, a, smem, st) : launch_pair_inst<FMT, false>(c, a, smem, st);
+    static_assert(TC_MAX_N <= 128, "a published product fits the smaller tiles");
+    if (a.pub.npeers > 0) return launch_pair_inst<FMT, false, true>(c, a, smem, st);
+    return a.nt_rows > 128 ? launch_pair_inst<FMT, true, false>(c, a, smem, st) : launch_pair_inst<FMT, false, false>(c, a, smem, st);
 }
 
 template <int FMT>

@@ -42,6 +42,35 @@ struct GfArgs {
     int *status;
 };
 
+// One superblock of 32 Q6_K rows, by a warp: half a warp per row, its 14 pieces from the 16-byte boundary at or below the row (rows
+// are only 2-byte aligned).  INTERLEAVED: eight rows of `src`, eight of `src2`, and so on.  CHECK: near the tensor's end, past
+// which nothing is read.  (Pieces dealt out 32 in a row, as in the other formats, cost a row's address and the end's comparison for
+// every piece: 2400 clocks for 128 rows, twice what the product behind them needs.)
+template <bool CHECK, bool INTERLEAVED>
+__device__ __forceinline__ void load_q6_rows(uint32_t dst, uint32_t pitch, const uint8_t *src, const uint8_t *src2, uint32_t row_bytes, uint32_t rows_left,
+                                             uint32_t stage_rows_left, const uint8_t *end, const uint8_t *end2, uint32_t lane)
+{
+    const uint32_t hw = lane >> 4, p = lane & 15u;
+    src += hw * row_bytes;
+    if constexpr (INTERLEAVED) src2 += hw * row_bytes;
+    dst += hw * pitch + p * 16u;
+#pragma unroll
+    for (uint32_t i = 0; i < 16; ++i) {
+        const bool second = INTERLEAVED && ((i >> 2) & 1u);
+        const uint32_t out = INTERLEAVED ? (i >> 3) * 8u + ((2u * i) & 7u) : 2u * i;       // + hw
+        if (p < 14u && out + hw < rows_left && 2u * i + hw < stage_rows_left) {
+            const uint8_t *a = reinterpret_cast<const uint8_t *>(reinterpret_cast<uintptr_t>((second ? src2 : src) + out * row_bytes) & ~(uintptr_t)15) + p * 16u;
+            uint32_t bytes = 16u;
+            if constexpr (CHECK) {
+                const uint8_t *e = second ? end2 : end;
+                if (a + 16 > e) bytes = a < e ? (uint32_t)(e - a) : 0u;
+                if (!bytes) a = reinterpret_cast<const uint8_t *>(reinterpret_cast<uintptr_t>(second ? src2 : src) & ~(uintptr_t)15);
+            }
+            cp_async16(dst + 2u * i * pitch, a, bytes);
+        }
+    }
+}
+
 // X fp32 [batch][ldx] -> the layout above; vectors >= batch are zero.  One thread per eight elements.
 __global__ void __launch_bounds__(256)
 pack_x_few_kernel(const float *__restrict__ x, uint32_t batch, uint32_t ldx, uint32_t in_dim, uint32_t nt, uint4 *__restrict__ xp)

@@ -106,35 +106,6 @@ __device__ __forceinline__ void tc_st16(uint32_t taddr, const uint4 (&v)[4])
                    "r"(v[2].x), "r"(v[2].y), "r"(v[2].z), "r"(v[2].w), "r"(v[3].x), "r"(v[3].y), "r"(v[3].z), "r"(v[3].w) : "memory");
 }
 
-// One superblock of 32 Q6_K rows, by a warp: half a warp per row, its 14 pieces from the 16-byte boundary at or below the row (rows
-// are only 2-byte aligned).  INTERLEAVED: eight rows of `src`, eight of `src2`, and so on.  CHECK: near the tensor's end, past
-// which nothing is read.  (Pieces dealt out 32 in a row, as in the other formats, cost a row's address and the end's comparison for
-// every piece: 2400 clocks for 128 rows, twice what the product behind them needs.)
-template <bool CHECK, bool INTERLEAVED>
-__device__ __forceinline__ void load_q6_rows(uint32_t dst, uint32_t pitch, const uint8_t *src, const uint8_t *src2, uint32_t row_bytes, uint32_t rows_left,
-                                             uint32_t stage_rows_left, const uint8_t *end, const uint8_t *end2, uint32_t lane)
-{
-    const uint32_t hw = lane >> 4, p = lane & 15u;
-    src += hw * row_bytes;
-    if constexpr (INTERLEAVED) src2 += hw * row_bytes;
-    dst += hw * pitch + p * 16u;
-#pragma unroll
-    for (uint32_t i = 0; i < 16; ++i) {
-        const bool second = INTERLEAVED && ((i >> 2) & 1u);
-        const uint32_t out = INTERLEAVED ? (i >> 3) * 8u + ((2u * i) & 7u) : 2u * i;       // + hw
-        if (p < 14u && out + hw < rows_left && 2u * i + hw < stage_rows_left) {
-            const uint8_t *a = reinterpret_cast<const uint8_t *>(reinterpret_cast<uintptr_t>((second ? src2 : src) + out * row_bytes) & ~(uintptr_t)15) + p * 16u;
-            uint32_t bytes = 16u;
-            if constexpr (CHECK) {
-                const uint8_t *e = second ? end2 : end;
-                if (a + 16 > e) bytes = a < e ? (uint32_t)(e - a) : 0u;
-                if (!bytes) a = reinterpret_cast<const uint8_t *>(reinterpret_cast<uintptr_t>(second ? src2 : src) & ~(uintptr_t)15);
-            }
-            cp_async16(dst + 2u * i * pitch, a, bytes);
-        }
-    }
-}
-
 // The packed bytes one dequant thread needs for its 64 weights (sub-blocks 2kq, 2kq+1 of a K-quant superblock, blocks
 // 2kq, 2kq+1 of a Q8_0 chunk) of one row, as 16-byte pieces.
 //   Q4_K: header (d, dmin, 12 scale bytes), 32 quant bytes (low nibbles = sub-block 2kq, high = 2kq+1).
@@ -286,7 +257,9 @@ template <bool BIG> struct TpShape {
     static constexpr uint32_t AS = BIG ? 2 : 3, ACC_COL = BIG ? 256 : 384, SL = BIG ? 2 : 4;      // A stages, accumulator column, slabs of an X stage
 };
 
-template <int FMT, bool BIG>
+// PUB: Y is published to the peers (a row-split product, at most 64 vectors).  Its code, inlined behind every store, is not in the other
+// instances: a launch starts with cold instruction caches.
+template <int FMT, bool BIG, bool PUB>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ TpArgs a)
 {
@@ -355,15 +328,17 @@ gemm_pair_kernel(const __grid_constant__ TpArgs a)
             if (i >= WS && !wait(w_empty + s, ph)) break;
             const uint8_t *src0 = rows0 + chunk * CB;
             const uint32_t dst0 = smem_u32(w_stages + s * STAGE) + lw * 32u * PITCH;
-            if constexpr (FMT == FMT_Q6_K) {
-                if (src0 + (size_t)32 * a.row_bytes + 16 <= w_end) load_q6_rows<false, false>(dst0, PITCH, src0, nullptr, a.row_bytes, live, 32u, nullptr, nullptr, lane);
-                else load_q6_rows<true, false>(dst0, PITCH, src0, nullptr, a.row_bytes, live, 32u, w_end, nullptr, lane);
-            } else {
 #pragma unroll
-                for (uint32_t j = 0; j < PPR; ++j) {
-                    const uint32_t q = lane + 32u * j, r = q / PPR, p = q - r * PPR;
-                    cp_async16(dst0 + r * PITCH + p * 16u, r < live ? src0 + r * a.row_bytes + p * 16u : a.w, r < live ? 16u : 0u);
+            for (uint32_t j = 0; j < PPR; ++j) {
+                const uint32_t q = lane + 32u * j, r = q / PPR, p = q - r * PPR;
+                const uint8_t *src = src0 + r * a.row_bytes;
+                if constexpr (FMT == FMT_Q6_K) src = reinterpret_cast<const uint8_t *>(reinterpret_cast<uintptr_t>(src) & ~(uintptr_t)15);
+                src += p * 16u;
+                uint32_t bytes = r < live ? 16u : 0u;
+                if constexpr (FMT == FMT_Q6_K) {      // the tensor may end inside or before a row's last piece
+                    if (bytes && src + 16 > w_end) bytes = src < w_end ? (uint32_t)(w_end - src) : 0u;
                 }
+                cp_async16(dst0 + r * PITCH + p * 16u, bytes ? src : a.w, bytes);
             }
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(w_full + s)) : "memory");
             if (++s == WS) { s = 0; ph ^= 1u; }
@@ -503,7 +478,7 @@ gemm_pair_kernel(const __grid_constant__ TpArgs a)
                     for (uint32_t q = 0; q < 16; ++q) {
                         if (n_base + n0 + q < a.batch) {
                             dst[(size_t)q * a.ldy] = __uint_as_float(v[q]);
-                            if (a.pub.npeers > 0) tc_publish(a.pub, dst + (size_t)q * a.ldy, __uint_as_float(v[q]), *reinterpret_cast<const volatile unsigned int *>(a.pub.pub_gen) + 1u);
+                            if (PUB && a.pub.npeers > 0) tc_publish(a.pub, dst + (size_t)q * a.ldy, __uint_as_float(v[q]), *reinterpret_cast<const volatile unsigned int *>(a.pub.pub_gen) + 1u);
                         }
                     }
                 }
@@ -524,7 +499,7 @@ gemm_pair_kernel(const __grid_constant__ TpArgs a)
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
     }
-    if (tid == 0 && a.publish_done && a.pub.npeers > 0)
+    if (PUB && tid == 0 && a.publish_done && a.pub.npeers > 0)
         tc_publish_done(a.pub, *reinterpret_cast<const volatile unsigned int *>(a.pub.pub_gen) + 1u);
 }
 
