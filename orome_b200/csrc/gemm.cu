@@ -144,6 +144,13 @@ static uint32_t tp_clusters(const orome_cuda_ctx *c, int fmt, uint32_t tiles, ui
     return pick;
 }
 
+size_t orome_tc_part_floats(const orome_cuda_ctx *c, int fmt, uint32_t out_dim, uint32_t in_dim, int batch)
+{
+    const uint32_t chunks = in_dim / TC_KC, tiles = (out_dim + TP_ROWS - 1) / TP_ROWS, nt_rows = ((uint32_t)batch + 15) / 16 * 16;
+    const uint32_t units = tiles * chunks, clusters = tp_clusters(c, fmt, tiles, chunks, nt_rows, true);
+    return units % clusters != 0 || (units / clusters) % chunks != 0 ? (size_t)clusters * 2 * nt_rows * TP_ROWS : 0;
+}
+
 int orome_launch_tc(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t out_dim, uint32_t in_dim, int layout, const float *x,
                     int batch, int ldx, float *y, int ldy, cudaStream_t st, const TcPub *pub, const uint2 *x_ll, const unsigned int *wait_gen, bool *x_packed)
 {
@@ -173,8 +180,8 @@ int orome_launch_tc(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t ou
         slice = 16;
         while (slice < most && xp_floats(slice + 16) <= c->tc_xp.cap) slice += 16;
     }
-    // (first sizes: 32 MiB of packed X, 960 vectors of 17408, and all that shares can leave, two tiles of 256 vectors per pair of SMs,
-    // so that the products of a layer do not each outgrow the one before)
+    // (first sizes: 32 MiB of packed X, 960 vectors of 17408, and all the partial sums that shares can leave, so that the products of
+    // a layer do not each outgrow the one before)
     while ((rc = orome_ensure(c, c->tc_xp, xp_floats(slice), st, (size_t)8 << 20)) == OROME_ENOMEM && !capturing && !one_launch && slice > 64) slice = (slice / 2 + 63) / 64 * 64;
     if (rc) return rc;
     const bool packed = x_packed && *x_packed && slice >= batch;
@@ -191,7 +198,7 @@ int orome_launch_tc(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32_t ou
         a.clusters = tp_clusters(c, fmt, mtiles * ntiles, chunks, nt_rows, true);
         auto is_cut = [&]() { return a.units % a.clusters != 0 || (a.units / a.clusters) % chunks != 0; };
         if (is_cut()) {
-            rc = capturing && part_floats(a.clusters) > c->tc_part.cap ? OROME_ENOMEM : orome_ensure(c, c->tc_part, part_floats(a.clusters), st, (size_t)std::max(1, c->sm_count / 2) * 2 * TP_MAX_N * TP_ROWS);
+            rc = capturing && part_floats(a.clusters) > c->tc_part.cap ? OROME_ENOMEM : orome_ensure(c, c->tc_part, part_floats(a.clusters), st, tp_part_usual(c));
             if (rc == OROME_ENOMEM) {
                 a.clusters = tp_clusters(c, fmt, mtiles * ntiles, chunks, nt_rows, false);
                 rc = is_cut() ? orome_ensure(c, c->tc_part, part_floats(a.clusters), st) : OROME_OK;      // (a fixed number of parts)

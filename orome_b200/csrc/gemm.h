@@ -18,6 +18,11 @@ struct TcPub {
 };
 }  // namespace orome
 
+// Partial sums that the tensor-memory form's shares of a product leave (at most 256 vectors; 0: no tile is cut), and the most that any
+// leave: two tiles of 256 x 256 per pair of SMs.
+size_t orome_tc_part_floats(const orome_cuda_ctx *c, int fmt, uint32_t out_dim, uint32_t in_dim, int batch);
+inline size_t tp_part_usual(const orome_cuda_ctx *c) { return (size_t)(c->sm_count < 2 ? 1 : c->sm_count / 2) * 2 * 256 * 256; }
+
 bool orome_tc_supported(const orome_cuda_ctx *c, int fmt, uint32_t in_dim);
 // Y[b][r] for b < batch.  pub / x_ll / wait_gen: the row-split form on several GPUs (batch <= TC_MAX_N, one launch): Y is
 // published to every rank's arena by the kernel that writes it, a gathered X is read from its slots by the packing kernel.

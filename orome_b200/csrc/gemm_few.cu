@@ -78,6 +78,10 @@ int orome_launch_few(orome_cuda_ctx *c, int fmt, const uint8_t *w0, const uint8_
     if (cap != cudaStreamCaptureStatusNone && c->tc_xp.cap < xp_floats) return OROME_ENOTSUP;
     int rc = orome_ensure(c, c->tc_xp, xp_floats, st, (size_t)8 << 20);
     if (rc) return rc == OROME_ENOMEM ? OROME_ENOTSUP : rc;
+    if (cap == cudaStreamCaptureStatusNone && !c->tc_part.cap) {
+        rc = orome_reserve(c, c->tc_part, orome_tc_part_floats(c, fmt, out_dim, in_dim, batch), st, tp_part_usual(c));
+        if (rc) return rc;
+    }
     GfArgs a;
     memset(&a, 0, sizeof a);
     // the warps that a pass's row tiles leave split the chunks of a row

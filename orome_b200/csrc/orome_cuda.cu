@@ -1171,6 +1171,16 @@ int orome_ensure(orome_cuda_ctx *c, Scratch &s, size_t floats, cudaStream_t st, 
     return OROME_OK;
 }
 
+int orome_reserve(orome_cuda_ctx *c, Scratch &s, size_t floats, cudaStream_t st, size_t usual)
+{
+    if (s.cap >= floats) return OROME_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CU(cudaStreamIsCapturing(st, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return OROME_OK;
+    const int rc = orome_ensure(c, s, floats, st, usual);
+    return rc == OROME_ENOMEM ? OROME_OK : rc;
+}
+
 extern "C" int orome_cuda_gate_up_swiglu(orome_cuda_ctx *c, const OromeTensorRef *gate, const OromeTensorRef *up,
                                          const float *x_dev, float *out_dev, int batch, int ldx, int ldo, void *stream)
 {
@@ -1231,11 +1241,13 @@ extern "C" int orome_cuda_gate_up_swiglu(orome_cuda_ctx *c, const OromeTensorRef
         return fail(OROME_EINVAL, "gate_up_swiglu: ldx/ldo smaller than the row length");
     // few vectors: gate, up and the epilogue in one launch; more than eight: two products of one packed X
     const bool few = batch > 1 && batch >= c->tc_min_batch && !c->force_generic && ldx % 4 == 0 && !(reinterpret_cast<uintptr_t>(x_dev) & 15);
+    const size_t n = (size_t)gate->out_dim;
     if (few && orome_few_supported(c, fmt, gate->out_dim, gate->in_dim, batch, true)) {
+        rc = orome_reserve(c, c->gu, 2 * n * batch, st);
+        if (rc) return rc;
         rc = orome_launch_few(c, fmt, gd, ud, gate->out_dim, gate->in_dim, layout, x_dev, batch, ldx, out_dev, ldo, st);
         if (rc != OROME_ENOTSUP) return rc;
     }
-    const size_t n = (size_t)gate->out_dim;
     rc = orome_ensure(c, c->gu, 2 * n * batch, st);
     if (rc) return rc;
     float *g = c->gu.p, *u = c->gu.p + n * batch;

@@ -252,3 +252,47 @@ def test_contexts_share_the_pool(env):
         held.append(free - torch.cuda.mem_get_info(0)[0])
     assert max(held[1:]) <= 4 << 20
     assert p.error(torch, F, ctx) <= TC_TOL
+
+
+@pytest.mark.parametrize("fmt", [synth.Q8_0, synth.Q4_K])
+def test_smaller_and_larger_batches_captured_after_a_warm_up_of_eight(env, fmt):
+    """A token loop warms up once and captures its other batch sizes: what eight vectors leave behind (whichever form they took) serves a
+    gate/up of two and of three, and 64 vectors of a product in as many launches as a direct call of them (tiles cut, sums added up)."""
+    torch, F, ctx = env
+    gate, up = (_Product(torch, F, 512, 1024, 8, s, fmt) for s in (91, 92))
+    p = _Product(torch, F, 1024, 4096, 64, 93, fmt)
+    act = torch.full((8, 512), float("nan"), device="cuda")
+
+    def gate_up(c, batch, stream=0):
+        c.gate_up_swiglu(gate.ref, up.ref, gate.x.data_ptr(), act.data_ptr(), batch, 1024, 512, stream)
+    fresh = F.Context(0)
+    want = []
+    for b in (2, 3):
+        gate_up(fresh, b)
+        torch.cuda.synchronize()
+        want.append(act[:b].clone())
+    before = fresh.launch_count
+    p.issue(fresh)
+    direct = fresh.launch_count - before
+    assert direct == 3                                     # pack, product, sums of cut tiles
+    gate_up(ctx, 8)
+    p.issue(ctx, batch=8)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    for b, w in zip((2, 3), want):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=side):
+            gate_up(ctx, b, side.cuda_stream)
+        act.fill_(float("nan"))
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(act[:b], w)
+    before, g = ctx.launch_count, torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=side):
+        p.issue(ctx, side.cuda_stream)
+    assert ctx.launch_count - before == direct
+    p.y.fill_(float("nan"))
+    g.replay()
+    torch.cuda.synchronize()
+    assert p.error(torch, F, ctx) <= TC_TOL
+    fresh.close()
