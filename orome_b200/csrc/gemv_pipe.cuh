@@ -404,7 +404,7 @@ __device__ __forceinline__ void quantize_piece(const float4 v, uint32_t f, bool 
     }
 }
 
-// This thread's share of a partials array: its loads are on their way when this returns, norm_rms() uses them.
+// This thread's share of a partials array; the warps' sums of the shares are what norm_rms() adds up.
 __device__ __forceinline__ float norm_share(const float *norm_parts, uint32_t tid, uint32_t nthreads)
 {
     float t = 0.0f;
@@ -414,11 +414,22 @@ __device__ __forceinline__ float norm_share(const float *norm_parts, uint32_t ti
 // 1 / rms from the warps' sums of their shares (written before the barrier behind the quantization).  It is a common factor of every
 // output, so it is applied to the sums: ahead of the quantization it cost a barrier and a round trip there (with the mma kernel's
 // late loads of the norm weights 5120-wide 4.5 us from x to the barrier, 1.8 without a norm).
+// The quantization's fixed point ends at about 1e-29 where 1 / rms would have raised x by up to eps^-1/2, so the norm weights raise it by
+// 2^32 instead and this takes that back.  (x is below 2^64, or its sum of squares is infinite.)
+constexpr uint32_t NORM_RAISE_BF16X2 = 0x4F804F80u, NORM_ONE_BF16X2 = 0x3F803F80u;
 __device__ __forceinline__ float norm_rms(const float *s_share, uint32_t nwarps, uint32_t in_dim, float eps)
 {
     float t = 0.0f;
     for (uint32_t w = 0; w < nwarps; ++w) t += s_share[w];
-    return rsqrtf(t / (float)in_dim + eps);
+    return rsqrtf(t / (float)in_dim + eps) * 0x1p-32f;
+}
+// An output of a normalised x: zero, whatever the sums are, where the sum of squares is infinite.
+__device__ __forceinline__ float norm_scaled(float sum, float rms) { return rms == 0.0f ? 0.0f : sum * rms; }
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b)
+{
+    uint32_t r;
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
 }
 
 // Loads that stay where they are written: left to itself the compiler moved the loads of a batch down to their uses in some
@@ -444,7 +455,7 @@ __device__ __forceinline__ bool quantize_x_to_smem(const float *__restrict__ x, 
                                                    long long limit = PIPE_WAIT_CYCLES, const int *status = nullptr, uint32_t rot = 0,
                                                    uint32_t issued_bar = 0, const uint16_t *norm_w = nullptr)
 {
-    // NORM: x is multiplied by the bf16 norm weights (none: by one) on the way (1 / rms: see norm_rms).
+    // NORM: x is multiplied by the bf16 norm weights, raised (none: by one) on the way (1 / rms: see norm_rms).
     // issued_bar: shared address of an mbarrier on which every warp arrives once the loads of its first batch are on
     // their way (0: none).  The weight producer holds its copies back until then, see the kernel.
     // rot (single vector only; a multiple of 32 four-float pieces): this CTA walks the vector starting rot pieces in and
@@ -460,6 +471,7 @@ __device__ __forceinline__ bool quantize_x_to_smem(const float *__restrict__ x, 
         issued_bar = 0;
     }
     struct Round { float4 v[BATCH]; uint2 nw[NORM ? BATCH : 1]; };
+    const uint32_t raise = norm_w ? NORM_RAISE_BF16X2 : NORM_ONE_BF16X2;
     auto place = [&](uint32_t fa, uint32_t &vec) {      // piece fa of all: its vector, and its place there
         vec = nvec == 1 ? 0u : fa / n4;                 // no division on the single-vector path
         uint32_t f = fa - vec * n4;
@@ -478,7 +490,7 @@ __device__ __forceinline__ bool quantize_x_to_smem(const float *__restrict__ x, 
                 if (fa < n4_all) r.v[b] = ldcg4_here(reinterpret_cast<const float4 *>(x + (size_t)vec * x_stride) + fl);
             }
             if constexpr (NORM) {
-                r.nw[b] = make_uint2(0x3F803F80u, 0x3F803F80u);
+                r.nw[b] = make_uint2(NORM_ONE_BF16X2, NORM_ONE_BF16X2);
                 if (norm_w && fa < n4_all) r.nw[b] = ldnc2_here(reinterpret_cast<const uint2 *>(norm_w) + fl);
             }
         }
@@ -499,10 +511,11 @@ __device__ __forceinline__ bool quantize_x_to_smem(const float *__restrict__ x, 
             uint32_t vec;
             const uint32_t f = place(fb + lane, vec);
             if constexpr (NORM) {
-                r.v[b].x *= __uint_as_float(r.nw[b].x << 16);
-                r.v[b].y *= __uint_as_float(r.nw[b].x & 0xffff0000u);
-                r.v[b].z *= __uint_as_float(r.nw[b].y << 16);
-                r.v[b].w *= __uint_as_float(r.nw[b].y & 0xffff0000u);
+                const uint32_t w0 = mul_bf16x2(r.nw[b].x, raise), w1 = mul_bf16x2(r.nw[b].y, raise);
+                r.v[b].x *= __uint_as_float(w0 << 16);
+                r.v[b].y *= __uint_as_float(w0 & 0xffff0000u);
+                r.v[b].z *= __uint_as_float(w1 << 16);
+                r.v[b].w *= __uint_as_float(w1 & 0xffff0000u);
             }
             quantize_piece<NP, G, SUMS>(r.v[b], f, fb + lane < n4_all, lane, xq0 + (size_t)vec * vec_bytes, in_dim);
         }
@@ -1055,7 +1068,7 @@ gemv_pipe_kernel(const __grid_constant__ PipeArgs a)
             }
             if constexpr (COMBINE) accbuf[buf_row0 - wk.lo + r] += (comb_acc ? 1.0f : a.seg_weight[blockIdx.y * a.tok_sel_stride + buf_seg]) * g;   // one owner per row and flush
             else {
-                if constexpr (FUSE) { g *= rms; u *= rms; }
+                if constexpr (FUSE) { g = norm_scaled(g, rms); u = norm_scaled(u, rms); }
                 float val = SWIGLU ? silu_mul(g, u) : g;
                 if constexpr (FUSE && MODE == 0) {
                     if (a.res_in) {           // residual add, clamped to the fp16 range as the reference's kernel does

@@ -74,3 +74,31 @@ def test_norm_and_residual_around_a_product(env, fmt, rows):
     got = y.cpu().numpy()
     assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 2e-6
     assert abs(float(out.double().sum()) / float((got.astype(np.float64) ** 2).sum()) - 1) <= 1e-5
+
+
+# the same bound where x without 1 / rms would be out of the fixed point's range; zeros where its sum of squares is infinite
+@pytest.mark.parametrize("fmt", [synth.Q8_0, synth.Q4_K, synth.Q6_K])
+@pytest.mark.parametrize("bits,scale", [(24, 1e-31), (24, 1e-25), (24, 1e17), (24, 1e36), (16, 1e36)])
+def test_magnitudes_of_a_normalised_x(env, fmt, bits, scale):
+    torch, F, ctx = env
+    rows, cols = 48, 2048
+    w, nw = synth.host_tensor(fmt, rows, cols, seed=5), (synth.host_x(cols, seed=8).view(np.uint32) >> 16).astype(np.uint16)
+    x = (synth.host_x(cols, seed=6) * np.float32(scale)).astype(np.float32)
+    total = (x.astype(np.float64) ** 2).sum()
+    wt, xt, nwt = (torch.from_numpy(a).cuda() for a in (w, x, nw.view(np.int16)))
+    parts, y = torch.zeros(F.SUM_SQ_PARTS, device="cuda"), torch.full((rows,), float("nan"), device="cuda")
+    parts[0] = total if total < 3e38 else float("inf")
+    ctx.set_option(F.OPT_X_BITS, bits)
+    try:
+        ctx.fuse_next(F.NormPrologue(nwt.data_ptr(), parts.data_ptr(), 1e-6), None)
+        ctx.matvec(F.tensor_ref(wt.data_ptr(), 0, fmt, rows, cols), xt.data_ptr(), y.data_ptr())
+        torch.cuda.synchronize()
+    finally:
+        ctx.set_option(F.OPT_X_BITS, 24)
+    got = y.cpu().numpy().astype(np.float64)
+    if total > 3e38:
+        assert (got == 0).all()
+        return
+    xn = x.astype(np.float64) / np.sqrt(total / cols + 1e-6) * (nw.astype(np.uint32) << 16).view(np.float32)
+    want = oracle.decode_rows(fmt, w, rows, cols).reshape(rows, cols).astype(np.float64) @ xn
+    assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 2e-6
