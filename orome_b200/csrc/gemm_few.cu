@@ -20,7 +20,7 @@ static int launch_inst(orome_cuda_ctx *c, const GfArgs &a, int grid, size_t smem
         CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, c->smem_optin - (int)fa.sharedSizeBytes));
         configured[c->device] = true;
     }
-    return orome_launch_pdl_smem(c, "gemm_few", kern, dim3(grid), dim3((a.rt * a.kp + GF_LOADERS + 1) * 32), smem, st, a);
+    return orome_launch_pdl_smem(c, "gemm_few", kern, dim3(grid), dim3((a.rt * a.kp + gf_loaders(NT) + 1) * 32), smem, st, a);
 }
 template <int FMT, bool SWIGLU>
 static int launch_nt(orome_cuda_ctx *c, const GfArgs &a, uint32_t nt, int grid, size_t smem, cudaStream_t st)

@@ -9,7 +9,7 @@
 //
 //   warps 0 .. rt * kp - 1   warp = row tile (16 rows; fused: 8 of gate and the same 8 of up) x share of the 256-weight chunks;
 //                            a chunk of a tile: fragments from shared memory, fp16 in registers, 16 mma (m16n8k16) per 8 vectors
-//   4 loader warps           packed weights as 16-byte cp.async, rows 32 or 96 bytes apart (mod 128): rows g .. g + 3 of a fragment
+//   8 (7) loader warps       packed weights as 16-byte cp.async, rows 32 or 96 bytes apart (mod 128): rows g .. g + 3 of a fragment
 //                            load hit different banks
 //   1 X warp                 the chunks' packed X, one bulk copy a stage
 //
@@ -25,7 +25,10 @@
 
 namespace orome {
 
-constexpr int GF_MAX_VECTORS = 32, GF_MAX_WARPS = 16, GF_LOADERS = 8, GF_MAX_STAGES = 8;
+constexpr int GF_MAX_VECTORS = 32, GF_MAX_WARPS = 16, GF_MAX_STAGES = 8;
+// Four groups: one fewer, for 80 registers a thread instead of 72 (17408 x 5120 Q4_K 31.4 -> 30.1 us, Q5_K 37.2 -> 34.4); with fewer groups the
+// loads are what a stage waits for (three: 28.2 -> 28.5, 5120 x 5120 12.5 -> 14.2).
+constexpr int gf_loaders(int nt) { return nt == 4 ? 7 : 8; }
 constexpr uint32_t GF_X_CHUNK = 4096;        // packed X of one chunk and eight vectors
 __host__ __device__ constexpr uint32_t gf_pitch(int fmt) { return fmt == FMT_Q8_0 ? 288u : fmt == FMT_Q4_K ? 160u : 224u; }
 
@@ -209,13 +212,14 @@ __device__ __forceinline__ void gf_pair(GfRow &r0, GfRow &r1, uint32_t t, uint32
 }
 
 template <int FMT, int NT, bool SWIGLU>
-__global__ void __launch_bounds__((GF_MAX_WARPS + GF_LOADERS + 1) * 32, 1)
+__global__ void __launch_bounds__((GF_MAX_WARPS + gf_loaders(NT) + 1) * 32, 1)
 gemm_few_kernel(const __grid_constant__ GfArgs a)
 {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr uint32_t PITCH = gf_pitch(FMT), PPR = tp_pieces(FMT);
     constexpr uint32_t CB = FMT == FMT_Q8_0 ? 272u : FMT == FMT_Q4_K ? 144u : FMT == FMT_Q5_K ? 176u : 210u;
     constexpr uint32_t TROWS = SWIGLU ? 8u : 16u;        // output rows of a tile
+    constexpr uint32_t LOADERS = gf_loaders(NT);
     __shared__ uint64_t full[GF_MAX_STAGES], empty[GF_MAX_STAGES];
     __shared__ volatile int s_abort;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -224,7 +228,7 @@ gemm_few_kernel(const __grid_constant__ GfArgs a)
     const uint32_t steps = (a.chunks + KP - 1) / KP, x_off = SR * KP * PITCH;
     if (tid == 0) {
         s_abort = 0;
-        for (uint32_t s = 0; s < a.nstages; ++s) { mbar_init(smem_u32(full + s), GF_LOADERS * 32 + 1); mbar_init(smem_u32(empty + s), CW); }
+        for (uint32_t s = 0; s < a.nstages; ++s) { mbar_init(smem_u32(full + s), LOADERS * 32 + 1); mbar_init(smem_u32(empty + s), CW); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -238,7 +242,7 @@ gemm_few_kernel(const __grid_constant__ GfArgs a)
         return false;
     };
 
-    if (warp >= CW + GF_LOADERS) {
+    if (warp >= CW + LOADERS) {
         // ---- X: one bulk copy a stage ----
         if (lane == 0) {
             pdl_wait();          // the packed X is the previous kernel's output
@@ -273,7 +277,7 @@ gemm_few_kernel(const __grid_constant__ GfArgs a)
                 if (fill >= a.nstages && !(ok = wait(empty + s, ph))) break;
                 const uint32_t st = smem_u32(smem + a.stage_base + s * a.stage_bytes), n = min(KP, a.chunks - k * KP);
                 uint32_t j = 0, b = lw;
-                for (;; b += GF_LOADERS) {
+                for (;; b += LOADERS) {
                     while (b >= blocks) { b -= blocks; ++j; }
                     if (j >= n) break;
                     const uint32_t first = row + b * 2u * TROWS, rows_left = first < hi ? hi - first : 0u, dst0 = st + (j * SR + b * 32u) * PITCH;
@@ -308,10 +312,23 @@ gemm_few_kernel(const __grid_constant__ GfArgs a)
     uint32_t s = 0, ph = 0;
     for (uint32_t row = lo; row < hi; row += RT * TROWS) {
         const uint32_t row0 = row + tile * TROWS;            // this warp's output rows
+        // The mma truncates where it adds: from two groups on a chunk's 16 have sums of their own, added up as fp32 (one chain over a warp's
+        // chunks: 1024 x 4096 at 32 vectors 1.3e-6 off the exact product of the same operands, 3.5e-7 like this and in the tensor-memory
+        // form; a single group has two chains, and more warps for its chunks: 2e-7, and 1 % slower like this).
         constexpr int NA = NT == 1 ? 2 : NT;
-        float acc[NA][4];
+        float acc[NA][4], sum[NT][4];
+#pragma unroll
+        for (int n = 0; n < NT; ++n) sum[n][0] = sum[n][1] = sum[n][2] = sum[n][3] = 0.0f;
 #pragma unroll
         for (int n = 0; n < NA; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
+        auto add_up = [&]() {
+#pragma unroll
+            for (int n = 0; n < NA; ++n) {
+                const int m = n < NT ? n : n - NT;
+                sum[m][0] += acc[n][0]; sum[m][1] += acc[n][1]; sum[m][2] += acc[n][2]; sum[m][3] += acc[n][3];
+                acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
+            }
+        };
         for (uint32_t k = 0; k < steps; ++k) {
             const bool ok = wait(full + s, ph);
             const uint32_t c = k * KP + kph;
@@ -330,18 +347,19 @@ gemm_few_kernel(const __grid_constant__ GfArgs a)
                 gf_pair<FMT, NT, NA, 1>(r0, r1, t, xl, acc);
                 gf_pair<FMT, NT, NA, 2>(r0, r1, t, xl, acc);
                 gf_pair<FMT, NT, NA, 3>(r0, r1, t, xl, acc);
+                if constexpr (NT > 1) add_up();
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(empty + s));
             if (++s == a.nstages) { s = 0; ph ^= 1u; }
         }
-        if constexpr (NA > NT) { acc[0][0] += acc[1][0]; acc[0][1] += acc[1][1]; acc[0][2] += acc[1][2]; acc[0][3] += acc[1][3]; }
+        if constexpr (NT == 1) add_up();
         // the shares of a tile meet: all but the first leave theirs, the first adds them up in order
         if (KP > 1) {
             if (row != lo) named_bar_sync(PIPE_BAR_CONSUMERS, (int)(CW * 32u));      // the last pass's have been read
             if (kph > 0) {
 #pragma unroll
-                for (int n = 0; n < NT; ++n) *reinterpret_cast<float4 *>(red + ((size_t)(warp * NT + n) * 32u + lane) * 4u) = make_float4(acc[n][0], acc[n][1], acc[n][2], acc[n][3]);
+                for (int n = 0; n < NT; ++n) *reinterpret_cast<float4 *>(red + ((size_t)(warp * NT + n) * 32u + lane) * 4u) = make_float4(sum[n][0], sum[n][1], sum[n][2], sum[n][3]);
             }
             named_bar_sync(PIPE_BAR_CONSUMERS, (int)(CW * 32u));
             if (kph > 0) continue;
@@ -349,7 +367,7 @@ gemm_few_kernel(const __grid_constant__ GfArgs a)
 #pragma unroll
                 for (int n = 0; n < NT; ++n) {
                     const float4 v = *reinterpret_cast<const float4 *>(red + ((size_t)((o * RT + tile) * NT + n) * 32u + lane) * 4u);
-                    acc[n][0] += v.x; acc[n][1] += v.y; acc[n][2] += v.z; acc[n][3] += v.w;
+                    sum[n][0] += v.x; sum[n][1] += v.y; sum[n][2] += v.z; sum[n][3] += v.w;
                 }
             }
         }
@@ -363,10 +381,10 @@ gemm_few_kernel(const __grid_constant__ GfArgs a)
                 if (v >= a.batch) continue;
                 float *dst = a.y + (size_t)v * a.ldy + row0 + g;
                 if constexpr (SWIGLU) {
-                    if (row0 + g < hi) *dst = silu_mul(acc[n][q], acc[n][2 + q]);
+                    if (row0 + g < hi) *dst = silu_mul(sum[n][q], sum[n][2 + q]);
                 } else {
-                    if (row0 + g < hi) dst[0] = acc[n][q];
-                    if (row0 + g + 8u < hi) dst[8] = acc[n][2 + q];
+                    if (row0 + g < hi) dst[0] = sum[n][q];
+                    if (row0 + g + 8u < hi) dst[8] = sum[n][2 + q];
                 }
             }
         }

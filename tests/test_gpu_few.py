@@ -52,6 +52,25 @@ def test_few_vectors(env, fmt, variant, rows, cols, batch):
     assert _rel(act[:, :rows].cpu().numpy(), oracle.swiglu_f64(gate, up).reshape(batch, rows)) <= 3e-3 * few
 
 
+@pytest.mark.parametrize("fmt", [synth.Q8_0, synth.Q4_K, synth.Q5_K, synth.Q6_K])
+@pytest.mark.parametrize("batch", [8, 16, 24, 32])
+def test_sums_are_as_exact_as_the_tensor_memory_form(env, fmt, batch):
+    """Against the exact product of the same fp16 operands (the weights as they come out for one-hot vectors).  16 mma in a row, each
+    truncating at 2^-24 of a sum that grows to its end: 16 / 3 * 2^-24 = 3.2e-7 on average, twice that asked."""
+    torch, F, ctx = env
+    rows, cols = 200, 4096
+    wt = torch.from_numpy(synth.host_tensor(fmt, rows, cols, seed=9)).cuda()
+    ref = F.tensor_ref(wt.data_ptr(), 0, fmt, rows, cols)
+    eye, w = torch.eye(cols, device="cuda"), torch.empty(cols, rows, device="cuda")
+    for b in range(0, cols, 256):
+        ctx.matvec(ref, eye[b:].data_ptr(), w[b:].data_ptr(), 256, cols, rows)
+    x, y = torch.from_numpy(synth.host_x(cols, batch, seed=batch)).cuda(), torch.full((batch, rows), float("nan"), device="cuda")
+    ctx.matvec(ref, x.data_ptr(), y.data_ptr(), batch, cols, rows)
+    torch.cuda.synchronize()
+    want = x.half().double() @ w.double()
+    assert float((y.double() - want).norm() / want.norm()) <= 6.4e-7
+
+
 def test_a_captured_product_repeats_its_bits(env):
     torch, F, _ = env
     rows, cols = 256, 1024
