@@ -20,17 +20,15 @@
 // delivers the 2304 bytes in 102), and from 24 vectors on the mma (one per two clocks) and the reads of X (32 wavefronts per 8
 // vectors and piece).
 #pragma once
+#include "few_plan.h"
 #include "gemm_pair.cuh"
 #include "gemv_mma.cuh"
 
 namespace orome {
 
-constexpr int GF_MAX_VECTORS = 32, GF_MAX_WARPS = 16, GF_MAX_STAGES = 8;
 // Four groups: one fewer, for 80 registers a thread instead of 72 (17408 x 5120 Q4_K 31.4 -> 30.1 us, Q5_K 37.2 -> 34.4); with fewer groups the
 // loads are what a stage waits for (three: 28.2 -> 28.5, 5120 x 5120 12.5 -> 14.2).
 constexpr int gf_loaders(int nt) { return nt == 4 ? 7 : 8; }
-constexpr uint32_t GF_X_CHUNK = 4096;        // packed X of one chunk and eight vectors
-__host__ __device__ constexpr uint32_t gf_pitch(int fmt) { return fmt == FMT_Q8_0 ? 288u : fmt == FMT_Q4_K ? 160u : 224u; }
 
 struct GfArgs {
     const uint8_t *w0, *w1;        // the tensor; fused: gate and up
