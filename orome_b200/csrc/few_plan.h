@@ -26,7 +26,7 @@ struct FewPlan {
     uint32_t grid, tiles;          // CTAs take equal row ranges; row tiles (16 rows; fused: 8 of gate and 8 of up) of the busiest one
     uint32_t passes, rt;           // a pass covers rt row tiles, at most eight
     uint32_t kp, steps;            // the warps that a pass's row tiles leave split the chunks of a row: kp of them a stage, steps stages a pass
-    uint32_t nstages, stage_base, stage_bytes;
+    uint32_t nstages, stage_base, stage_bytes, bytes;      // shared memory: the sums of a row's shares, then the stages; all of it
 };
 
 inline uint32_t few_tile_rows(bool fused) { return fused ? 8u : 16u; }
@@ -51,9 +51,10 @@ inline bool few_plan(const FewShape &in, FewPlan &p)
         p.steps = (chunks + kp - 1) / kp;
         p.kp = (chunks + p.steps - 1) / p.steps;
         p.stage_bytes = p.rt * 16 * p.kp * gf_pitch(in.fmt) + p.kp * nt * GF_X_CHUNK;
-        p.stage_base = (p.kp > 1 ? p.rt * p.kp * nt * 512u : 0u);
+        p.stage_base = p.kp > 1 ? p.rt * p.kp * nt * 512 : 0;
         p.nstages = p.stage_base + (size_t)p.stage_bytes <= room ? (uint32_t)std::min<size_t>(GF_MAX_STAGES, (room - p.stage_base) / p.stage_bytes) : 0u;
         p.nstages = std::min(p.nstages, p.steps * p.passes);
+        p.bytes = p.stage_base + p.nstages * p.stage_bytes;
         if (p.nstages >= std::min(2u, p.steps * p.passes) || kp == 1) break;      // two stages at least, so that loads and products overlap
     }
     return p.nstages > 0;

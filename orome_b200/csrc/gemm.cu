@@ -125,8 +125,9 @@ static int launch_staged(orome_cuda_ctx *c, int fmt, const uint8_t *data, uint32
 
 // How many clusters share the (tile, chunk) units.  In clocks: a unit costs the longest of its MMAs (8 a vector), its dequant
 // (~1100) and its packed bytes at an SM's share of memory (~22 a clock); a share costs ~5000 to set up, fill and drain; cut
-// tiles are written and read back at ~2000 bytes a clock and cost one more launch (~4000).  As many clusters as there are SM
-// pairs wins nearly everywhere; small products with many vectors take fewer, since their partial sums would outweigh the gain.
+// tiles are written and read back at ~2000 bytes a clock and cost one more launch (~4000).  (896 products with their number of clusters
+// swept: the choice is 5 % slower than the best count on average.  Equal parts of a tile are cheaper than this says, 4096 x 4096 at 128
+// vectors 20.1 us as whole tiles, 15.3 in halves; models that know it made others slower, 12288 x 4096 at 2048 164 -> 180.)
 static uint32_t tp_clusters(const orome_cuda_ctx *c, int fmt, uint32_t tiles, uint32_t chunks, uint32_t nt_rows, bool may_cut)
 {
     const uint32_t pairs = std::max(1u, (uint32_t)c->sm_count / 2), units = tiles * chunks;

@@ -21,7 +21,7 @@
 // vectors and piece).
 #pragma once
 #include "few_plan.h"
-#include "gemm_pair.cuh"
+#include "gemm_common.cuh"
 #include "gemv_mma.cuh"
 
 namespace orome {
@@ -38,6 +38,8 @@ struct GfArgs {
     uint64_t w_bytes;
     uint32_t batch, ldy, chunks;
     uint32_t rt, kp, nstages;      // row tiles of a pass, chunks of a stage; warps = rt * kp
+    // Shared memory: the shares' sums, then the stages.  The sums begin at its start, but as an address that is known when the kernel is
+    // compiled it made two 9B layers at eight vectors slower (Q8_0, 138.8 -> 139.7 us): other registers, another order.
     uint32_t red_base, stage_base, stage_bytes;
     int layout;
     int *status;
@@ -98,8 +100,8 @@ __device__ __forceinline__ void mma_f16_k16(float (&d)[4], uint32_t a0, uint32_t
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// The eight quants of 32-group `J` that this thread holds of one row (bytes 8t .. 8t + 7 of the group), as fp16 pairs.
-//   h: the row's chunk;  sc / mn: scale and min of the group as fp16 in both halves, products rounded once as in the other forms
+// What a thread holds of a row's chunk at shared address `h` besides its quants (bytes 8t .. 8t + 7 of every 32-group): d and -dmin in both
+// halves, the K-quants' eight scales and minimums as bytes, Q5_K's fifth bits (Q6_K: the half's upper bits), Q6_K's scales.
 struct GfRow { uint32_t h; __half2 d, dmin; uint32_t scl, sch, mnl, mnh; uint2 qh; uint32_t sc[4]; };
 
 __device__ __forceinline__ __half2 gf_byte_pair(uint32_t w, int j, float bias)       // bytes j, j + 1 of a word as fp16, less bias
@@ -316,17 +318,11 @@ gemm_few_kernel(const __grid_constant__ GfArgs a)
         constexpr int NA = NT == 1 ? 2 : NT;
         float acc[NA][4], sum[NT][4];
 #pragma unroll
-        for (int n = 0; n < NT; ++n) sum[n][0] = sum[n][1] = sum[n][2] = sum[n][3] = 0.0f;
-#pragma unroll
         for (int n = 0; n < NA; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
-        auto add_up = [&]() {
+        if constexpr (NT > 1) {
 #pragma unroll
-            for (int n = 0; n < NA; ++n) {
-                const int m = n < NT ? n : n - NT;
-                sum[m][0] += acc[n][0]; sum[m][1] += acc[n][1]; sum[m][2] += acc[n][2]; sum[m][3] += acc[n][3];
-                acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
-            }
-        };
+            for (int n = 0; n < NT; ++n) sum[n][0] = sum[n][1] = sum[n][2] = sum[n][3] = 0.0f;
+        }
         for (uint32_t k = 0; k < steps; ++k) {
             const bool ok = wait(full + s, ph);
             const uint32_t c = k * KP + kph;
@@ -345,13 +341,22 @@ gemm_few_kernel(const __grid_constant__ GfArgs a)
                 gf_pair<FMT, NT, NA, 1>(r0, r1, t, xl, acc);
                 gf_pair<FMT, NT, NA, 2>(r0, r1, t, xl, acc);
                 gf_pair<FMT, NT, NA, 3>(r0, r1, t, xl, acc);
-                if constexpr (NT > 1) add_up();
+                if constexpr (NT > 1) {
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) {
+                        sum[n][0] += acc[n][0]; sum[n][1] += acc[n][1]; sum[n][2] += acc[n][2]; sum[n][3] += acc[n][3];
+                        acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
+                    }
+                }
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(empty + s));
             if (++s == a.nstages) { s = 0; ph ^= 1u; }
         }
-        if constexpr (NT == 1) add_up();
+        if constexpr (NT == 1) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) sum[0][i] = acc[0][i] + acc[1][i];
+        }
         // the shares of a tile meet: all but the first leave theirs, the first adds them up in order
         if (KP > 1) {
             if (row != lo) named_bar_sync(PIPE_BAR_CONSUMERS, (int)(CW * 32u));      // the last pass's have been read

@@ -35,9 +35,7 @@ constexpr int TP_MAX_N = 256;            // input vectors of a tile
 constexpr int TP_MAX_WS = 6, TP_MAX_BS = 8, TP_MAX_AS = 3;
 constexpr int TP_ROWS = 2 * TC_M;        // rows of a tile (a cluster)
 
-// 16-byte pieces a row of a stage is fetched as, and the pieces between rows (odd).  Q6_K rows are only 2-byte aligned: the
-// 210 bytes of a superblock lie in 14 pieces from the boundary below.
-__host__ __device__ constexpr uint32_t tp_pieces(int fmt) { return fmt == FMT_Q8_0 ? 17 : fmt == FMT_Q4_K ? 9 : fmt == FMT_Q5_K ? 11 : 14; }
+// Pieces between rows: odd.
 __host__ __device__ constexpr uint32_t tp_pitch(int fmt) { return 16u * (tp_pieces(fmt) | 1u); }
 __host__ __device__ constexpr uint32_t tp_stage_bytes(int fmt) { return TC_M * tp_pitch(fmt); }
 
@@ -95,10 +93,6 @@ __device__ __forceinline__ void tp_mma(uint32_t tmem_d, uint32_t tmem_a, uint64_
                  " tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
                  ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32_t bytes)      // bytes < 16: the rest is zero-filled
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ void tc_st16(uint32_t taddr, const uint4 (&v)[4])
 {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
@@ -117,18 +111,6 @@ __device__ __forceinline__ void tc_st16(uint32_t taddr, const uint4 (&v)[4])
 //   need all 64 ql bytes for one of their nibbles each.)
 template <int FMT> struct TcPacked { uint4 p[FMT == FMT_Q4_K ? 3 : 5]; };
 template <> struct TcPacked<FMT_Q6_K> { uint32_t qa[4], qb[4], qh[4], sc[2], d; };
-
-// N consecutive 32-bit words of shared memory from a 2-byte aligned address.
-template <int N>
-__device__ __forceinline__ void lds_words_a2(uint32_t a, uint32_t (&out)[N])
-{
-    const uint32_t q = a & ~3u, sh = (a & 2u) * 8u;
-    uint32_t w[N + 1];
-#pragma unroll
-    for (int i = 0; i <= N; ++i) w[i] = lds32<0>(q + 4u * i);
-#pragma unroll
-    for (int i = 0; i < N; ++i) out[i] = __funnelshift_r(w[i], w[i + 1], sh);
-}
 
 // row: shared address of the row's chunk (Q6_K: of its first byte, 2-byte aligned).
 template <int FMT>
@@ -506,7 +488,7 @@ gemm_pair_kernel(const __grid_constant__ TpArgs a)
 // Tiles that were cut over several clusters: Y = the sum of their partial sums, in cluster order.  blockIdx.x = tile,
 // blockIdx.y = four of its vectors; a thread adds up four rows of one vector, so that a tile cut six ways is one round of
 // independent 16-byte loads (with 16 vectors a thread in turn this pass took longer than the product it follows).
-static __global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256)
 tile_reduce_kernel(const __grid_constant__ TpArgs a)
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

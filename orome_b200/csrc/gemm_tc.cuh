@@ -22,7 +22,7 @@
 #include <cuda.h>
 
 #include "decode.cuh"
-#include "gemm.h"
+#include "gemm_common.cuh"
 
 namespace orome {
 
@@ -113,7 +113,7 @@ __device__ __forceinline__ uint32_t sw128_off(uint32_t r, uint32_t c) { return (
 // small batch and by HBM for a large one).
 // x_ll: X is a gathered matrix in the arena, read from its slots (every element polled, bounded, for the generation
 // *wait_gen); NULL: a plain matrix.
-static __global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256)
 pack_x_f16_kernel(const float *__restrict__ x, int batch, int ldx, uint32_t in_dim, uint32_t nt_rows, __half *__restrict__ xp,
                   const uint2 *x_ll, const unsigned int *wait_gen, long long wait_cycles, int *status)
 {
@@ -138,17 +138,6 @@ pack_x_f16_kernel(const float *__restrict__ x, int batch, int ldx, uint32_t in_d
     uint8_t *dst = reinterpret_cast<uint8_t *>(xp) + ((size_t)tile * (in_dim / TC_SLAB_K) + ks) * nt_rows * 128 + sw128_off(nn, c);
     *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(h);
     if (!ok) atomicExch(status, 3);
-}
-
-// 8 consecutive weights of one row as fp16 -> one 16-byte piece.
-__device__ __forceinline__ uint32_t h2_bits(__half2 v) { return *reinterpret_cast<uint32_t *>(&v); }
-
-// Two byte lanes of `w` (selected by `sel`) -> fp16 pair (byte - bias) * scale + addend.  0x6400 | byte is the
-// fp16 number 1024 + byte exactly, so the bias comes off exactly before the one rounded multiply-add.
-__device__ __forceinline__ __half2 two_weights(uint32_t w, uint32_t sel, __half2 bias, __half2 scale, __half2 addend)
-{
-    const uint32_t bits = __byte_perm(w, 0x64646464u, sel);
-    return __hfma2(__hsub2(*reinterpret_cast<const __half2 *>(&bits), bias), scale, addend);
 }
 
 // 32 consecutive weights of one row (a Q8_0 block / a K-quant sub-block) -> four 16-byte fp16 pieces.
@@ -387,7 +376,7 @@ gemm_tc_kernel(const __grid_constant__ TcArgs a)
 
 
 // Y[b][r] = sum over splits of partial[s][b][r]
-static __global__ void splitk_reduce_kernel(const float *__restrict__ part, uint32_t split, uint32_t batch, uint32_t rows, float *__restrict__ y, uint32_t ldy,
+__global__ void splitk_reduce_kernel(const float *__restrict__ part, uint32_t split, uint32_t batch, uint32_t rows, float *__restrict__ y, uint32_t ldy,
                                      const TcPub pub)
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -13,6 +13,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SMEM_OPTIN, SMS = 232448, 148      # of a B200
 NAMES = {synth.Q4_K: "q4_k", synth.Q5_K: "q5_k", synth.Q6_K: "q6_k", synth.Q8_0: "q8_0"}
 FMT = {v: k for k, v in NAMES.items()}
+PITCH = {synth.Q4_K: 160, synth.Q5_K: 224, synth.Q6_K: 224, synth.Q8_0: 288}      # bytes between the rows of a stage's chunk
 
 PROGRAM = r"""
 #include "few_plan.h"
@@ -26,7 +27,7 @@ int main()
         FewShape in{fmt, rows, cols, batch, fused != 0, SMS, SMEM};
         FewPlan p = {};
         const bool fits = few_plan(in, p);
-        printf("%d %d %u %u %u %u %u %u %u %u %u\n", (int)few_faster(in), (int)fits, p.grid, p.tiles, p.passes, p.rt, p.kp, p.steps, p.nstages, p.stage_base, p.stage_bytes);
+        printf("%d %d %u %u %u %u %u %u %u %u %u %u\n", (int)few_faster(in), (int)fits, p.grid, p.tiles, p.passes, p.rt, p.kp, p.steps, p.nstages, p.stage_base, p.stage_bytes, p.bytes);
     }
 }
 """
@@ -35,7 +36,7 @@ int main()
 class Plan:
     def __init__(self, shape, values):
         self.fmt, self.rows, self.cols, self.batch, self.fused = shape
-        (self.faster, self.fits, self.grid, self.tiles, self.passes, self.rt, self.kp, self.steps, self.nstages, self.base, self.stage) = values
+        (self.faster, self.fits, self.grid, self.tiles, self.passes, self.rt, self.kp, self.steps, self.nstages, self.base, self.stage, self.bytes) = values
         self.chunks, self.fills = self.cols // 256, self.passes * self.steps
 
 
@@ -60,7 +61,10 @@ def test_every_plan_covers_its_rows_and_chunks_and_fits(plans):
         assert p.fits and 1 <= p.grid <= SMS and p.rt <= 8 and 1 <= p.rt * p.kp <= 16
         assert p.rt * p.passes * t >= -(-p.rows // p.grid) and (p.passes - 1) * p.rt < p.tiles
         assert p.kp * p.steps >= p.chunks > p.kp * (p.steps - 1)
-        assert 1 <= p.nstages <= min(8, p.fills) and p.base + p.nstages * p.stage <= SMEM_OPTIN - 1024 and p.base % 128 == 0 and p.stage % 16 == 0
+        assert 1 <= p.nstages <= min(8, p.fills) and p.base % 128 == 0 and p.stage % 16 == 0
+        groups = (p.batch + 7) // 8
+        assert p.stage == p.rt * 16 * p.kp * PITCH[p.fmt] + p.kp * groups * 4096
+        assert p.base == (p.rt * p.kp * groups * 512 if p.kp > 1 else 0) and p.bytes == p.base + p.nstages * p.stage <= SMEM_OPTIN - 1024
 
 
 def test_the_gpu_tests_reach_what_they_are_for(plans):
