@@ -296,3 +296,37 @@ def test_smaller_and_larger_batches_captured_after_a_warm_up_of_eight(env, fmt):
     torch.cuda.synchronize()
     assert p.error(torch, F, ctx) <= TC_TOL
     fresh.close()
+
+
+def test_captured_gate_up_on_scratch_of_a_smaller_one(env):
+    """2500 vectors of 8192 take 40 MiB of packed X, a first call leaves 32: captured, gate and up pack it in slices, each for itself.
+    The bound: the same operands, but tiles that are not cut, 512 mma in a row that truncate at 2^-24 of a sum growing to its end, 512 / 3 *
+    2^-24 = 1e-5 of a product on average; the activation is a product of two, and as much again for spread."""
+    torch, F, ctx = env
+    rows, batch, cols = 300, 2500, 8192
+    first = [_Product(torch, F, rows, 256, batch, s) for s in (101, 102)]
+    gate, up = (_Product(torch, F, rows, cols, batch, s) for s in (103, 104))
+    act = torch.full((batch, rows), float("nan"), device="cuda")
+
+    def gate_up(c, a, b, stream=0):
+        c.gate_up_swiglu(a.ref, b.ref, a.x.data_ptr(), act.data_ptr(), batch, a.in_dim, rows, stream)
+    gate_up(ctx, *first)                                   # room for both products' values
+    torch.cuda.synchronize()
+    side, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    before = ctx.launch_count
+    with torch.cuda.graph(g, stream=side):
+        gate_up(ctx, gate, up, side.cuda_stream)
+    assert ctx.launch_count - before >= 9                  # two slices of each: packing and product; the elementwise pass
+    up.x = gate.x
+    fresh = F.Context(0)
+    for p in (gate, up):
+        p.issue(fresh)
+    torch.cuda.synchronize()
+    want = torch.nn.functional.silu(gate.y.double()) * up.y.double()
+    for _ in range(2):
+        act.fill_(float("nan"))
+        g.replay()
+        torch.cuda.synchronize()
+        assert float((act.double() - want).norm() / want.norm()) <= 4e-5
+    assert gate.error(torch, F, fresh) <= TC_TOL and up.error(torch, F, fresh) <= TC_TOL
+    fresh.close()
