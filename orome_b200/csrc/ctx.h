@@ -34,6 +34,7 @@ struct Scratch {
     float *p = nullptr;
     size_t cap = 0;            // floats
     bool captured = false;     // a captured call has used it: its address may be in a graph
+    bool refused = false;      // orome_reserve found no room
 };
 
 struct orome_cuda_ctx {
@@ -111,7 +112,8 @@ long long orome_wait_cycles(const orome_cuda_ctx *c);
 // Context scratch of at least `floats` floats for a call on `st`; `usual` floats where nothing is there yet and that many fit.
 int orome_ensure(orome_cuda_ctx *c, Scratch &s, size_t floats, cudaStream_t st, size_t usual = 0);
 // The same for scratch that this call does without and another form of it would use: a direct call of either form leaves what calls
-// captured after it run on (nothing can grow there, and tiles are cut only if their partial sums have room).  While capturing it does nothing; no room is no error.
+// captured after it run on (nothing can grow there, and tiles are cut only if their partial sums have room).  While capturing it does nothing; no room is no
+// error, and is not looked for again.
 int orome_reserve(orome_cuda_ctx *c, Scratch &s, size_t floats, cudaStream_t st, size_t usual = 0);
 // `bytes` in the order of `st` from the pool scratch comes from: one per device, shared by its contexts and gone with the last one
 // that used it.  nullptr: there is no room.

@@ -1173,12 +1173,14 @@ int orome_ensure(orome_cuda_ctx *c, Scratch &s, size_t floats, cudaStream_t st, 
 
 int orome_reserve(orome_cuda_ctx *c, Scratch &s, size_t floats, cudaStream_t st, size_t usual)
 {
-    if (s.cap >= floats) return OROME_OK;
+    if (s.cap >= floats || s.refused) return OROME_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CU(cudaStreamIsCapturing(st, &cap));
     if (cap != cudaStreamCaptureStatusNone) return OROME_OK;
     const int rc = orome_ensure(c, s, floats, st, usual);
-    return rc == OROME_ENOMEM ? OROME_OK : rc;
+    if (rc != OROME_ENOMEM) return rc;
+    s.refused = true;
+    return OROME_OK;
 }
 
 extern "C" int orome_cuda_gate_up_swiglu(orome_cuda_ctx *c, const OromeTensorRef *gate, const OromeTensorRef *up,

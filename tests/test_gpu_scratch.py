@@ -232,6 +232,34 @@ def test_long_prompt_with_little_memory_left(env):
     assert p.error(torch, F, ctx) <= TC_TOL
 
 
+def test_few_vectors_with_little_memory_left(env):
+    """Room for the packed X, none for what only another form of the calls would use."""
+    torch, F, ctx = env
+    p, gate, up = _Product(torch, F, 1024, 4096, 8, 76), _Product(torch, F, 512, 1024, 8, 77), _Product(torch, F, 512, 1024, 8, 78)
+    act = torch.full((8, 512), float("nan"), device="cuda")
+
+    def calls(c):
+        p.issue(c)
+        c.gate_up_swiglu(gate.ref, up.ref, gate.x.data_ptr(), act.data_ptr(), 8, 1024, 512)
+        torch.cuda.synchronize()
+    warm = F.Context(0)
+    calls(warm)                                            # every kernel is loaded
+    want = p.y.clone(), act.clone()
+    warm.close()
+    p.y.fill_(float("nan"))
+    act.fill_(float("nan"))
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    hog = torch.empty(torch.cuda.mem_get_info(0)[0] - (48 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        calls(ctx)
+        calls(ctx)
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    assert torch.equal(p.y, want[0]) and torch.equal(act, want[1])
+
+
 def test_contexts_share_the_pool(env):
     """Scratch of a context that is gone serves the next one, and the last one gives everything back."""
     torch, F, ctx = env
