@@ -448,8 +448,8 @@ __device__ __forceinline__ float warp_abs_max(float v)
 // GATHERED: x is read from its {value, tag} slots (polled for `tag`); false = a poll expired.  (An instance of its own: with the
 // choice made load by load, a round's loads waited for one another.)
 // NTOK = 2: vector `b` (0 or 1) of two, into its columns of the wider layout (see mma_xq_sb).
-// NORM: x is multiplied by the bf16 norm weights, raised (none: by one) on the way; the common factor 1 / rms is the caller's, who applies it to
-// the sums (norm_rms), since nothing before them needs it.
+// NORM: x is multiplied by the bf16 norm weights (none: by one) on the way; the common factor 1 / rms is the caller's, who applies it to the
+// sums, since nothing before them needs it (the lift: see norm_rms).
 // What bounds it: every CTA does this between its predecessor's end and its own first mma, so it is latency, and then issue slots and
 // instructions fetched: a maximum is one redux instead of five shuffles, the factors of a round are worked out by as many lanes at once,
 // and the rounds are a rolled loop (run once a launch from cold instruction caches).
@@ -469,13 +469,13 @@ __device__ __forceinline__ bool quantize_x_mma(const float *__restrict__ x, uint
     const bool whole = (reinterpret_cast<uintptr_t>(x) & 31) == 0;
     float *xs = reinterpret_cast<float *>(xq + (size_t)units * XQSB), *sxs = xs + units * NTOK;
     struct Round { float4 v0[XB], v1[XB]; uint4 nw[NORM ? XB : 1]; };
-    const uint32_t raise = norm_w ? NORM_RAISE_BF16X2 : NORM_ONE_BF16X2;
+    const float lift = NORM && norm_w ? NORM_LIFT : 1.0f;
     auto load = [&](uint32_t ub, Round &r) {
 #pragma unroll
         for (int b = 0; b < XB; ++b) {
             const uint32_t u = ub + b * nwarps;
             r.v0[b] = r.v1[b] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if constexpr (NORM) r.nw[b] = make_uint4(NORM_ONE_BF16X2, NORM_ONE_BF16X2, NORM_ONE_BF16X2, NORM_ONE_BF16X2);
+            if constexpr (NORM) r.nw[b] = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
             if (u >= units) continue;
             if constexpr (GATHERED) {
                 const uint2 *sl = slots + (size_t)u * 256 + 8 * lane;
@@ -500,7 +500,7 @@ __device__ __forceinline__ bool quantize_x_mma(const float *__restrict__ x, uint
         if constexpr (NORM) {
 #pragma unroll
             for (int b = 0; b < XB; ++b) {
-                const uint4 nw = make_uint4(mul_bf16x2(r.nw[b].x, raise), mul_bf16x2(r.nw[b].y, raise), mul_bf16x2(r.nw[b].z, raise), mul_bf16x2(r.nw[b].w, raise));
+                const uint4 nw = r.nw[b];
                 auto lo = [](uint32_t w) { return __uint_as_float(w << 16); };
                 auto hi = [](uint32_t w) { return __uint_as_float(w & 0xffff0000u); };
                 v0[b] = make_float4(v0[b].x * lo(nw.x), v0[b].y * hi(nw.x), v0[b].z * lo(nw.y), v0[b].w * hi(nw.y));
@@ -522,7 +522,7 @@ __device__ __forceinline__ bool quantize_x_mma(const float *__restrict__ x, uint
                 if (lane == (uint32_t)(XB + b)) mine = smax;
             }
         }
-        const float inv_mine = fixed_factor(mine, QMAX);
+        const float inv_mine = fixed_group<NORM>(mine, QMAX);
 #pragma unroll
         for (int b = 0; b < XB; ++b) {
             const uint32_t u = ub + b * nwarps;
@@ -558,7 +558,7 @@ __device__ __forceinline__ bool quantize_x_mma(const float *__restrict__ x, uint
         }
         {
             const uint32_t b = lane < (uint32_t)XB ? lane : lane - XB, u = ub + b * nwarps;
-            if (lane < (uint32_t)(Q6 ? XB : 2 * XB) && u < units) (lane < (uint32_t)XB ? xs : sxs)[u * NTOK + (NTOK == 1 ? 0u : b_tok)] = fixed_unit(inv_mine);
+            if (lane < (uint32_t)(Q6 ? XB : 2 * XB) && u < units) (lane < (uint32_t)XB ? xs : sxs)[u * NTOK + (NTOK == 1 ? 0u : b_tok)] = fixed_unit<NORM>(inv_mine, lift);
         }
         r = next;
     }

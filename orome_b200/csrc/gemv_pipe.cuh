@@ -355,7 +355,11 @@ __device__ __forceinline__ float fixed_factor(float m, float qmax)
     asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(m));
     return qmax * r;
 }
-__device__ __forceinline__ float fixed_unit(float inv) { return __frcp_rn(inv); }
+// NORM: of a normalised x (see norm_rms): the factor stays finite, the unit is lifted.
+template <bool NORM = false>
+__device__ __forceinline__ float fixed_group(float m, float qmax) { return NORM ? fminf(fixed_factor(m, qmax), 0x1p125f) : fixed_factor(m, qmax); }
+template <bool NORM = false>
+__device__ __forceinline__ float fixed_unit(float inv, float lift = 1.0f) { return NORM ? __frcp_rn(inv) * lift : __frcp_rn(inv); }
 
 // ---- x in shared memory, quantized once per CTA --------------------------------------------
 // Layout at xq: NP byte planes of in_dim bytes (plane p holds byte p of every X_i), then one fp32
@@ -369,8 +373,8 @@ __device__ __forceinline__ float fixed_unit(float inv) { return __frcp_rn(inv); 
 // expired.  (An instance of its own: with the choice made load by load, the loads of a batch waited for one another.)
 // One four-float piece (piece number f of its vector) into the quantized copy at xq: the lanes of a group agree on the
 // group's scale by shuffles, so whole warps must call this together (`valid` false for lanes past the end).
-template <int NP, int G, bool SUMS>
-__device__ __forceinline__ void quantize_piece(const float4 v, uint32_t f, bool valid, uint32_t lane, uint8_t *xq, uint32_t in_dim)
+template <int NP, int G, bool SUMS, bool NORM = false>
+__device__ __forceinline__ void quantize_piece(const float4 v, uint32_t f, bool valid, uint32_t lane, uint8_t *xq, uint32_t in_dim, float lift = 1.0f)
 {
     constexpr float QMAX = NP == 3 ? 8388603.0f : 32766.0f;
     const uint32_t n4 = in_dim / 4;
@@ -380,7 +384,7 @@ __device__ __forceinline__ void quantize_piece(const float4 v, uint32_t f, bool 
     float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
 #pragma unroll
     for (int o = 1; o < G / 4; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const float inv = fixed_factor(amax, QMAX);
+    const float inv = fixed_group<NORM>(amax, QMAX);
     int X[4];
     X[0] = __float2int_rn(v.x * inv); X[1] = __float2int_rn(v.y * inv);
     X[2] = __float2int_rn(v.z * inv); X[3] = __float2int_rn(v.w * inv);
@@ -398,9 +402,9 @@ __device__ __forceinline__ void quantize_piece(const float4 v, uint32_t f, bool 
             const uint32_t hi = __byte_perm((uint32_t)X[2], (uint32_t)X[3], sel);
             planes[(size_t)p * n4 + 4 * plane_swz(f >> 2) + (f & 3u)] = __byte_perm(lo, hi, 0x5410);
         }
-        if ((lane & (G / 4 - 1)) == 0) scales[f / (G / 4)] = fixed_unit(inv);
+        if ((lane & (G / 4 - 1)) == 0) scales[f / (G / 4)] = fixed_unit<NORM>(inv, lift);
         if constexpr (SUMS)
-            if ((lane & 7u) == 0) sums[f / 8] = sum;
+            if ((lane & 7u) == 0) sums[f / 8] = NORM ? sum * lift : sum;
     }
 }
 
@@ -414,23 +418,18 @@ __device__ __forceinline__ float norm_share(const float *norm_parts, uint32_t ti
 // 1 / rms from the warps' sums of their shares (written before the barrier behind the quantization).  It is a common factor of every
 // output, so it is applied to the sums: ahead of the quantization it cost a barrier and a round trip there (with the mma kernel's
 // late loads of the norm weights 5120-wide 4.5 us from x to the barrier, 1.8 without a norm).
-// The quantization's fixed point ends at about 1e-29 where 1 / rms would have raised x by up to eps^-1/2, so the norm weights raise it by
-// 2^32 instead and this takes that back.  (x is below 2^64, or its sum of squares is infinite.)
-constexpr uint32_t NORM_RAISE_BF16X2 = 0x4F804F80u, NORM_ONE_BF16X2 = 0x3F803F80u;
+// Small elements are then not raised by up to eps^-1/2 ahead of the fixed point: a group's factor is kept finite (below about 1e-32 with the
+// digits that are left), and its unit, times a block's scale, out of fp32's small end by a lift of 2^32 that this takes back.  (x is
+// below 2^64, or its sum of squares is infinite.)
+constexpr float NORM_LIFT = 0x1p32f;
 __device__ __forceinline__ float norm_rms(const float *s_share, uint32_t nwarps, uint32_t in_dim, float eps)
 {
     float t = 0.0f;
     for (uint32_t w = 0; w < nwarps; ++w) t += s_share[w];
-    return rsqrtf(t / (float)in_dim + eps) * 0x1p-32f;
+    return rsqrtf(t / (float)in_dim + eps) * (1.0f / NORM_LIFT);
 }
 // An output of a normalised x: zero, whatever the sums are, where the sum of squares is infinite.
 __device__ __forceinline__ float norm_scaled(float sum, float rms) { return rms == 0.0f ? 0.0f : sum * rms; }
-__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b)
-{
-    uint32_t r;
-    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
 
 // Loads that stay where they are written: left to itself the compiler moved the loads of a batch down to their uses in some
 // instances, one round trip to L2 after the other (4096-wide x with fused neighbours: 3.0 us from the wait to the last piece, 1.6
@@ -455,7 +454,7 @@ __device__ __forceinline__ bool quantize_x_to_smem(const float *__restrict__ x, 
                                                    long long limit = PIPE_WAIT_CYCLES, const int *status = nullptr, uint32_t rot = 0,
                                                    uint32_t issued_bar = 0, const uint16_t *norm_w = nullptr)
 {
-    // NORM: x is multiplied by the bf16 norm weights, raised (none: by one) on the way (1 / rms: see norm_rms).
+    // NORM: x is multiplied by the bf16 norm weights (none: by one) on the way (1 / rms, the lift: see norm_rms).
     // issued_bar: shared address of an mbarrier on which every warp arrives once the loads of its first batch are on
     // their way (0: none).  The weight producer holds its copies back until then, see the kernel.
     // rot (single vector only; a multiple of 32 four-float pieces): this CTA walks the vector starting rot pieces in and
@@ -471,7 +470,7 @@ __device__ __forceinline__ bool quantize_x_to_smem(const float *__restrict__ x, 
         issued_bar = 0;
     }
     struct Round { float4 v[BATCH]; uint2 nw[NORM ? BATCH : 1]; };
-    const uint32_t raise = norm_w ? NORM_RAISE_BF16X2 : NORM_ONE_BF16X2;
+    const float lift = NORM && norm_w ? NORM_LIFT : 1.0f;
     auto place = [&](uint32_t fa, uint32_t &vec) {      // piece fa of all: its vector, and its place there
         vec = nvec == 1 ? 0u : fa / n4;                 // no division on the single-vector path
         uint32_t f = fa - vec * n4;
@@ -490,7 +489,7 @@ __device__ __forceinline__ bool quantize_x_to_smem(const float *__restrict__ x, 
                 if (fa < n4_all) r.v[b] = ldcg4_here(reinterpret_cast<const float4 *>(x + (size_t)vec * x_stride) + fl);
             }
             if constexpr (NORM) {
-                r.nw[b] = make_uint2(NORM_ONE_BF16X2, NORM_ONE_BF16X2);
+                r.nw[b] = make_uint2(0x3F803F80u, 0x3F803F80u);
                 if (norm_w && fa < n4_all) r.nw[b] = ldnc2_here(reinterpret_cast<const uint2 *>(norm_w) + fl);
             }
         }
@@ -511,13 +510,12 @@ __device__ __forceinline__ bool quantize_x_to_smem(const float *__restrict__ x, 
             uint32_t vec;
             const uint32_t f = place(fb + lane, vec);
             if constexpr (NORM) {
-                const uint32_t w0 = mul_bf16x2(r.nw[b].x, raise), w1 = mul_bf16x2(r.nw[b].y, raise);
-                r.v[b].x *= __uint_as_float(w0 << 16);
-                r.v[b].y *= __uint_as_float(w0 & 0xffff0000u);
-                r.v[b].z *= __uint_as_float(w1 << 16);
-                r.v[b].w *= __uint_as_float(w1 & 0xffff0000u);
+                r.v[b].x *= __uint_as_float(r.nw[b].x << 16);
+                r.v[b].y *= __uint_as_float(r.nw[b].x & 0xffff0000u);
+                r.v[b].z *= __uint_as_float(r.nw[b].y << 16);
+                r.v[b].w *= __uint_as_float(r.nw[b].y & 0xffff0000u);
             }
-            quantize_piece<NP, G, SUMS>(r.v[b], f, fb + lane < n4_all, lane, xq0 + (size_t)vec * vec_bytes, in_dim);
+            quantize_piece<NP, G, SUMS, NORM>(r.v[b], f, fb + lane < n4_all, lane, xq0 + (size_t)vec * vec_bytes, in_dim, lift);
         }
     }
     if (issued_bar) {      // a warp without a piece of x arrives all the same
