@@ -188,7 +188,8 @@ int  orome_cuda_matvec_group(orome_cuda_ctx *ctx, const OromeTensorRef *refs, in
  * (engine.m:342-392).  gate and up must have identical shape and format.
  * batch > 1 is two batched products (orome_cuda_matvec: its dispatch, scratch and precision class;
  * from OROME_OPT_TC_MIN_BATCH vectors on that is the fp16 tensor-core form) and an elementwise pass,
- * the reference's unfused branch (engine.m:388-404); up to eight vectors all of it may be one launch. */
+ * the reference's unfused branch (engine.m:388-404); up to eight vectors all of it may be one launch behind
+ * the packing of x. */
 int  orome_cuda_gate_up_swiglu(orome_cuda_ctx *ctx, const OromeTensorRef *gate, const OromeTensorRef *up,
                                const float *x_dev, float *out_dev, int batch, int ldx, int ldo, void *stream);
 
