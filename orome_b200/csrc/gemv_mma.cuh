@@ -522,7 +522,7 @@ __device__ __forceinline__ bool quantize_x_mma(const float *__restrict__ x, uint
                 if (lane == (uint32_t)(XB + b)) mine = smax;
             }
         }
-        const float inv_mine = fixed_group<NORM>(mine, QMAX);
+        const float inv_mine = fixed_factor(mine, QMAX);
 #pragma unroll
         for (int b = 0; b < XB; ++b) {
             const uint32_t u = ub + b * nwarps;
@@ -558,7 +558,7 @@ __device__ __forceinline__ bool quantize_x_mma(const float *__restrict__ x, uint
         }
         {
             const uint32_t b = lane < (uint32_t)XB ? lane : lane - XB, u = ub + b * nwarps;
-            if (lane < (uint32_t)(Q6 ? XB : 2 * XB) && u < units) (lane < (uint32_t)XB ? xs : sxs)[u * NTOK + (NTOK == 1 ? 0u : b_tok)] = fixed_unit<NORM>(inv_mine, lift);
+            if (lane < (uint32_t)(Q6 ? XB : 2 * XB) && u < units) (lane < (uint32_t)XB ? xs : sxs)[u * NTOK + (NTOK == 1 ? 0u : b_tok)] = NORM ? fixed_unit(inv_mine) * lift : fixed_unit(inv_mine);
         }
         r = next;
     }

@@ -346,20 +346,29 @@ __device__ __forceinline__ void dot_s(uint32_t q, const XGroup<NP, N> &g, int k,
 }
 
 // Fixed point of a group whose largest magnitude is `m`: X = rn(v * inv), v ~= X * unit.  Any factor near qmax / m will do as long as
-// unit is its exact reciprocal: an approximate one and one rounded reciprocal instead of two divisions, whose ~340 clocks every
-// launch waited for between its input and its first product.  qmax leaves room for the factor's error (2^-22).  m = 0 or infinite:
-// all X are zero (F2I of NaN), unit 0 or infinite.
+// unit is its reciprocal to the last place: an approximate one, and one Newton step for the unit, seven instructions without a branch.
+// (Two divisions were ~340 clocks that every launch waited for between its input and its first product; an approximate reciprocal over
+// fp32's whole range and __frcp_rn were no better where there is much of x to read: experts of 214 tokens, Q6_K down, 1626 us with
+// divisions, 1646 with those, 1606 like this; 9B token 1536 / 1542 / 1501.)  qmax leaves room for the factor's error (2^-22).  m is taken
+// by a quarter, so that the largest one's reciprocal is a normal number, and the factor kept to 2^126, so that zeros and groups below
+// 1e-31 come out with the digits that are left.  m infinite or NaN: the unit is NaN.
+__device__ __forceinline__ float rcp_approx(float v)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
 __device__ __forceinline__ float fixed_factor(float m, float qmax)
 {
     float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(m));
-    return qmax * r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(qmax * 0.25f * rcp_approx(m * 0.25f)), "f"(0x1p126f));
+    return r;
 }
-// NORM: of a normalised x (see norm_rms): the factor stays finite, the unit is lifted.
-template <bool NORM = false>
-__device__ __forceinline__ float fixed_group(float m, float qmax) { return NORM ? fminf(fixed_factor(m, qmax), 0x1p125f) : fixed_factor(m, qmax); }
-template <bool NORM = false>
-__device__ __forceinline__ float fixed_unit(float inv, float lift = 1.0f) { return NORM ? __frcp_rn(inv) * lift : __frcp_rn(inv); }
+__device__ __forceinline__ float fixed_unit(float inv)
+{
+    const float r = rcp_approx(inv);
+    return fmaf(fmaf(-inv, r, 1.0f), r, r);
+}
 
 // ---- x in shared memory, quantized once per CTA --------------------------------------------
 // Layout at xq: NP byte planes of in_dim bytes (plane p holds byte p of every X_i), then one fp32
@@ -384,7 +393,7 @@ __device__ __forceinline__ void quantize_piece(const float4 v, uint32_t f, bool 
     float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
 #pragma unroll
     for (int o = 1; o < G / 4; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    const float inv = fixed_group<NORM>(amax, QMAX);
+    const float inv = fixed_factor(amax, QMAX);
     int X[4];
     X[0] = __float2int_rn(v.x * inv); X[1] = __float2int_rn(v.y * inv);
     X[2] = __float2int_rn(v.z * inv); X[3] = __float2int_rn(v.w * inv);
@@ -402,7 +411,7 @@ __device__ __forceinline__ void quantize_piece(const float4 v, uint32_t f, bool 
             const uint32_t hi = __byte_perm((uint32_t)X[2], (uint32_t)X[3], sel);
             planes[(size_t)p * n4 + 4 * plane_swz(f >> 2) + (f & 3u)] = __byte_perm(lo, hi, 0x5410);
         }
-        if ((lane & (G / 4 - 1)) == 0) scales[f / (G / 4)] = fixed_unit<NORM>(inv, lift);
+        if ((lane & (G / 4 - 1)) == 0) scales[f / (G / 4)] = NORM ? fixed_unit(inv) * lift : fixed_unit(inv);
         if constexpr (SUMS)
             if ((lane & 7u) == 0) sums[f / 8] = NORM ? sum * lift : sum;
     }
@@ -418,9 +427,8 @@ __device__ __forceinline__ float norm_share(const float *norm_parts, uint32_t ti
 // 1 / rms from the warps' sums of their shares (written before the barrier behind the quantization).  It is a common factor of every
 // output, so it is applied to the sums: ahead of the quantization it cost a barrier and a round trip there (with the mma kernel's
 // late loads of the norm weights 5120-wide 4.5 us from x to the barrier, 1.8 without a norm).
-// Small elements are then not raised by up to eps^-1/2 ahead of the fixed point: a group's factor is kept finite (below about 1e-32 with the
-// digits that are left), and its unit, times a block's scale, out of fp32's small end by a lift of 2^32 that this takes back.  (x is
-// below 2^64, or its sum of squares is infinite.)
+// Small elements are then not raised by up to eps^-1/2 ahead of the fixed point: their units, times a block's scale, are kept out of
+// fp32's small end by a lift of 2^32 that this takes back.  (x is below 2^64, or its sum of squares is infinite.)
 constexpr float NORM_LIFT = 0x1p32f;
 __device__ __forceinline__ float norm_rms(const float *s_share, uint32_t nwarps, uint32_t in_dim, float eps)
 {

@@ -21,16 +21,18 @@ def env():
     ctx.close()
 
 
-def _product(env, fmt, rows, cols, x, shift):
-    """matvec with x `shift` floats behind a 256-byte boundary."""
+def _product(env, fmt, rows, cols, x, shift, nan=False):
+    """matvec with x `shift` floats behind a 256-byte boundary: its relative error (nan: the product itself)."""
     torch, F, ctx = env
     w = synth.host_tensor(fmt, rows, cols, seed=cols + shift)
     wt = torch.from_numpy(w).cuda()
     buf = torch.zeros(cols + 64, device="cuda")
     buf[shift:shift + cols] = torch.from_numpy(x).cuda()
-    y = torch.full((rows,), float("nan"), device="cuda")
+    y = torch.full((rows,), 0.0 if nan else float("nan"), device="cuda")
     ctx.matvec(F.tensor_ref(wt.data_ptr(), 0, fmt, rows, cols), buf.data_ptr() + 4 * shift, y.data_ptr())
     torch.cuda.synchronize()
+    if nan:
+        return y.cpu().numpy()
     want = oracle.matvec_f64(fmt, w, rows, cols, x)
     return float(np.linalg.norm(y.cpu().numpy() - want) / np.linalg.norm(want))
 
@@ -52,6 +54,15 @@ def test_scales_of_x(env, fmt, scale):
     x[512:768] *= 1e-6
     x[1024:1056] = 0.0
     assert _product(env, fmt, 48, 2048, (x * np.float32(scale)).astype(np.float32), 0) <= 2e-6
+
+
+# an infinite element, and a group of nothing but NaN, are not lost among the zeros of the fixed point
+@pytest.mark.parametrize("fmt", [synth.Q8_0, synth.Q4_K, synth.Q5_K, synth.Q6_K])
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+def test_x_that_is_not_finite(env, fmt, bad):
+    x = synth.host_x(1024, seed=4)
+    x[256:512] = bad
+    assert np.isnan(_product(env, fmt, 40, 1024, x, 0, nan=True)).all()
 
 
 # norm and residual around one product; 21000 rows: more of them a CTA than its flush buffers (and the residuals read ahead) hold
